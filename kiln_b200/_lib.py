@@ -1,4 +1,5 @@
-"""ctypes loader for libkiln_w4a16.so (the C ABI declared in include/kiln_w4a16.h).
+"""ctypes loader for libkiln_w4a16.so (the C ABI declared in include/kiln_w4a16.h), and the native host path on top of it
+(csrc/host.cpp).
 
 There is no fallback: if the shared library is missing or does not load, importing
 the product raises.  Build it with `python -m kiln_b200.build`.
@@ -96,3 +97,26 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = cdll
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The extension module that runs the entry points' host path (checks, allocation, launch) in one call, bound to the
+    library that `lib()` loaded."""
+    global _native
+    if _native is None:
+        import importlib
+
+        import torch  # noqa: F401 - the extension's libraries come with it
+
+        try:
+            mod = importlib.import_module("kiln_b200._native")
+        except ModuleNotFoundError as e:
+            raise ImportError("kiln_b200/_native.so is missing: run `python -m kiln_b200.build`") from e
+        names = ("kiln_w4a16_gemm_bf16", "kiln_w4a16_workspace_bytes", "kiln_w4a16_gemm_bf16_ex", "kiln_w4a16_workspace_bytes_ex",
+                 "kiln_w4a16_gemm_bf16_grouped", "kiln_w4a16_quantize_and_pack_device")
+        mod.bind(*(ctypes.cast(getattr(lib(), name), _vp).value for name in names))
+        _native = mod
+    return _native

@@ -1,4 +1,5 @@
-"""Builds libkiln_w4a16.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds libkiln_w4a16.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and _native.so, the extension
+module that runs the Python entry points' host path, with g++ against the installed torch.
 
 Usage: python -m kiln_b200.build [--force] [--verbose]
 """
@@ -12,6 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libkiln_w4a16.so")
 SOURCES = ["api.cu", "decode_w4a16.cu", "epilogue_w4a16.cu", "prefill_w4a16_umma.cu", "repack.cu", "smallm_w4a16_tmem.cu"]
+NATIVE = os.path.join(HERE, "_native.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
@@ -19,10 +21,23 @@ FLAGS = [
 ]
 
 
+def _native_command() -> list:
+    import sysconfig
+
+    import torch
+
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
+    inc = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"), cuda, sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *(f"-I{d}" for d in inc), os.path.join(CSRC, "host.cpp"), "-o", NATIVE, "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda",
+            "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+
+
 def _stale() -> bool:
-    if not os.path.exists(LIB):
+    if not (os.path.exists(LIB) and os.path.exists(NATIVE)):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(NATIVE))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "kiln_w4a16.h")]
     return any(os.path.getmtime(d) > t for d in deps)
 
@@ -40,6 +55,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(2, "-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
+    procs.append(("host.cpp", subprocess.Popen(_native_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
@@ -47,7 +63,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(f"--- {src}\n{out}\n")
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed")
+        raise RuntimeError("compilation failed")
     subprocess.check_call([NVCC, "-shared", "-o", LIB, *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt"])
     return LIB
 

@@ -10,26 +10,22 @@ class KilnMarlinError(RuntimeError):
     """Stands in for `candle_core::Error` raised by the reference's `bail!` sites."""
 
 
-_workspaces: dict = {}
-_retired: list = []
-
-
 def workspace_bytes(m: int, n: int, k: int) -> int:
     return int(_lib.lib().kiln_w4a16_workspace_bytes(m, n, k))
 
 
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Scratch that only grows, one buffer per (device, stream): GEMMs on different streams may overlap on the GPU and
-    must not share split-K partial sums.  Replaces the reference's per-call `Tensor::zeros` workspace (lib.rs:176-178).
-    A buffer that is outgrown is kept alive until the process ends (a kernel of an earlier call may still use it)."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        if ws is not None:
-            _retired.append(ws)
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+def scratch(device: torch.device, nbytes: int) -> torch.Tensor | None:
+    """Workspace of one call, from torch's caching allocator.  Its reuse is ordered by the stream, so GEMMs on different
+    streams never share split-K partial sums.  Replaces the reference's `Tensor::zeros` workspace (lib.rs:176-178)."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
+
+
+def status_error(status: int, m: int, n: int, k: int, groupsize: int) -> KilnMarlinError:
+    return KilnMarlinError(
+        f"kiln_marlin_w4a16_gemm failed with status {status} "
+        f"(1=ERR_PROB_SHAPE, 2=ERR_KERN_SHAPE) for m={m}, n={n}, k={k}, groupsize={groupsize}"
+        f" [{_lib.STATUS_NAMES.get(status, '?')}, cuda={_lib.lib().kiln_w4a16_last_cuda_error()}]"
+    )
 
 
 def marlin_w4a16_gemm(a: torch.Tensor, b_packed: torch.Tensor, scales: torch.Tensor, groupsize: int,
@@ -39,6 +35,13 @@ def marlin_w4a16_gemm(a: torch.Tensor, b_packed: torch.Tensor, scales: torch.Ten
     Same checks, in the same order and with the same messages, as lib.rs:103-166.
     `out` (optional, beyond the reference) receives the result in place.
     """
+    if not nvtx.enabled():
+        done = _lib.native().gemm(a, b_packed, scales, groupsize, out)
+        if isinstance(done, torch.Tensor):
+            return done if out is None else out
+        if done is not None:
+            raise status_error(done, a.shape[0], scales.shape[1], a.shape[1], groupsize)
+    # not the plain case: name what is wrong, or copy what has to be contiguous
     if not a.is_cuda:
         raise KilnMarlinError("kiln-marlin-gemm: a must be on CUDA")
     if a.dim() != 2 or b_packed.dim() != 2 or scales.dim() != 2:
@@ -84,16 +87,12 @@ def marlin_w4a16_gemm(a: torch.Tensor, b_packed: torch.Tensor, scales: torch.Ten
         return out
     with torch.cuda.device(a.device), nvtx.range("kiln/marlin/gemm"):
         nbytes = workspace_bytes(m, n, k)
-        ws = _workspace(a.device, nbytes) if nbytes else None
+        ws = scratch(a.device, nbytes)
         stream = torch.cuda.current_stream(a.device).cuda_stream
         status = _lib.lib().kiln_w4a16_gemm_bf16(
             a.data_ptr(), b_packed.data_ptr(), out.data_ptr(), scales.data_ptr(), m, n, k, groupsize,
             ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, stream,
         )
     if status != 0:
-        raise KilnMarlinError(
-            f"kiln_marlin_w4a16_gemm failed with status {status} "
-            f"(1=ERR_PROB_SHAPE, 2=ERR_KERN_SHAPE) for m={m}, n={n}, k={k}, groupsize={groupsize}"
-            f" [{_lib.STATUS_NAMES.get(status, '?')}, cuda={_lib.lib().kiln_w4a16_last_cuda_error()}]"
-        )
+        raise status_error(status, m, n, k, groupsize)
     return out

@@ -8,7 +8,7 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib, nvtx
-from .marlin_gemm import KilnMarlinError, marlin_w4a16_gemm
+from .marlin_gemm import KilnMarlinError, marlin_w4a16_gemm, scratch, status_error
 
 
 @dataclass
@@ -39,6 +39,12 @@ def pack_from_bf16(weight_t: torch.Tensor, groupsize: int = 128) -> Optional[Mar
     Unlike the reference's download -> CPU pack -> upload (marlin_proj.rs:87-182) the
     quantise+pack runs on the device, straight from the tensor.
     """
+    if not nvtx.enabled():
+        done = _lib.native().pack(weight_t, groupsize)
+        if type(done) is tuple:
+            return MarlinPackedProj(*done, groupsize, *weight_t.shape)
+        if done is not None:
+            raise KilnMarlinError(f"marlin_proj: device pack failed: {_lib.STATUS_NAMES.get(done, done)}")
     if not weight_t.is_cuda:
         return None
     if weight_t.dim() != 2:
@@ -201,9 +207,6 @@ def interleave_columns_32(gate_cols: torch.Tensor, up_cols: torch.Tensor) -> tor
     return torch.stack([gate_cols.reshape(n // 32, 32, *rest), up_cols.reshape(n // 32, 32, *rest)], dim=1).reshape(2 * n, *rest)
 
 
-_ex_workspaces: dict = {}
-
-
 def _gemm_ex(x2: torch.Tensor, proj: MarlinPackedProj, swiglu: bool, lora_a, lora_b, lora_scale: float,
              out: Optional[torch.Tensor] = None) -> torch.Tensor:
     import ctypes
@@ -240,10 +243,7 @@ def _gemm_ex(x2: torch.Tensor, proj: MarlinPackedProj, swiglu: bool, lora_a, lor
     name = "kiln/mlp/gate_up_swiglu" if swiglu else ("kiln/marlin/gemm_lora" if lora_a is not None else "kiln/marlin/gemm")
     with torch.cuda.device(x2.device), nvtx.range(name):
         need = int(lib.kiln_w4a16_workspace_bytes_ex(m, proj.n, k, ctypes.byref(ep)))
-        ws = _ex_workspaces.get(x2.device)
-        if need and (ws is None or ws.numel() < need):
-            ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=x2.device)
-            _ex_workspaces[x2.device] = ws
+        ws = scratch(x2.device, need)
         rc = lib.kiln_w4a16_gemm_bf16_ex(
             x2.contiguous().data_ptr(), proj.b_packed.data_ptr(), out.data_ptr(), proj.scales.data_ptr(), m, proj.n, k,
             proj.groupsize, ctypes.byref(ep), ws.data_ptr() if need else None, ws.numel() if need else 0,
@@ -262,11 +262,24 @@ def _flatten(x: torch.Tensor, k: int):
     raise KilnMarlinError(f"marlin_proj: expects rank-2 or rank-3 input, got rank {x.dim()}")
 
 
+def _native_ex(x, proj, swiglu: bool, lora_a, lora_b, lora_scale, out):
+    """The call through the native host path; None: not its plain case (nothing was launched)."""
+    if nvtx.enabled():
+        return None
+    done = _lib.native().gemm_ex(x, proj, swiglu, lora_a, lora_b, lora_scale, out)
+    if done is None or isinstance(done, torch.Tensor):
+        return done if done is None or out is None else out
+    raise KilnMarlinError(f"kiln_w4a16_gemm_bf16_ex failed: {_lib.STATUS_NAMES.get(done, done)}")
+
+
 def matmul_bf16_lora(x: torch.Tensor, proj: MarlinPackedProj, lora_a: torch.Tensor, lora_b: torch.Tensor,
                      lora_scale: float, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """`mlp_proj_forward` / `linear_with_lora` on the Marlin path (kiln-model/src/forward.rs:2925-2945): base GEMM plus
     the LoRA delta x @ A^T @ B^T * scale (lora_loader.rs:213-233), the delta added inside the GEMM's epilogue.
     lora_a [r, k], lora_b [n, r]."""
+    done = _native_ex(x, proj, False, lora_a, lora_b, lora_scale, out)
+    if done is not None:
+        return done
     x2, lead = _flatten(x, proj.k)
     out = _gemm_ex(x2, proj, False, lora_a, lora_b, lora_scale, out)
     return out if lead is None else out.reshape(lead[0], lead[1], -1)
@@ -279,6 +292,9 @@ def swiglu_gate_up(x: torch.Tensor, fused: MarlinPackedProj, lora_a: Optional[to
     kiln-model/src/forward.rs:2769-2839).  `fused` comes from `interleave_gate_up`; the result is [.., n/2] and feeds
     the down projection directly.  An optional LoRA pair applies to the fused matrix (lora_b rows in the same
     interleaved column order, see `interleave_columns_32`)."""
+    done = _native_ex(x, fused, True, lora_a, lora_b, lora_scale, out)
+    if done is not None:
+        return done
     x2, lead = _flatten(x, fused.k)
     out = _gemm_ex(x2, fused, True, lora_a, lora_b, lora_scale, out)
     return out if lead is None else out.reshape(lead[0], lead[1], -1)
@@ -288,6 +304,12 @@ def grouped_matmul_bf16(xs: Sequence[torch.Tensor], projs: Sequence[MarlinPacked
                         outs: Optional[Sequence[torch.Tensor]] = None) -> list:
     """Several independent projections (the q, k, v of an attention layer, say) in ONE launch when the batch is at a
     decode size; xs[i] [m_i, k_i] bf16 (rank 2) goes with projs[i].  Returns the list of outputs."""
+    if not nvtx.enabled():
+        done = _lib.native().grouped(xs, projs, outs)
+        if isinstance(done, list):
+            return done
+        if done is not None:
+            raise KilnMarlinError(f"kiln_w4a16_gemm_bf16_grouped failed: {_lib.STATUS_NAMES.get(done, done)}")
     import ctypes
 
     if len(xs) != len(projs) or not 1 <= len(xs) <= 8:
@@ -310,10 +332,7 @@ def grouped_matmul_bf16(xs: Sequence[torch.Tensor], projs: Sequence[MarlinPacked
                               pr.groupsize)
         need = max(need, int(lib.kiln_w4a16_workspace_bytes(x.shape[0], pr.n, pr.k)))
     with torch.cuda.device(dev), nvtx.range("kiln/proj/grouped"):
-        ws = _ex_workspaces.get(dev)
-        if need and (ws is None or ws.numel() < need):
-            ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-            _ex_workspaces[dev] = ws
+        ws = scratch(dev, need)
         rc = lib.kiln_w4a16_gemm_bf16_grouped(arr, len(xs), ws.data_ptr() if need else None, ws.numel() if need else 0,
                                               torch.cuda.current_stream(dev).cuda_stream)
     if rc != 0:
@@ -323,6 +342,12 @@ def grouped_matmul_bf16(xs: Sequence[torch.Tensor], projs: Sequence[MarlinPacked
 
 def matmul_bf16(x: torch.Tensor, proj: MarlinPackedProj) -> torch.Tensor:
     """marlin_proj.rs:285-319: x [.., k] bf16 -> [.., n] bf16 (rank 2 or 3)."""
+    if not nvtx.enabled():
+        done = _lib.native().matmul(x, proj)
+        if isinstance(done, torch.Tensor):
+            return done
+        if done is not None:
+            raise status_error(done, x.numel() // proj.k, proj.n, proj.k, proj.groupsize)
     if x.dim() == 2:
         lead = None
         if x.shape[1] != proj.k:

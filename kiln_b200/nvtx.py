@@ -20,6 +20,10 @@ def enable(on: bool = True, push=None, pop=None) -> None:
     _push, _pop = push, pop
 
 
+def enabled() -> bool:
+    return _enabled
+
+
 @contextlib.contextmanager
 def range(name: str):  # noqa: A001 - named after the crate's `range!` macro
     if not _enabled:
