@@ -93,7 +93,7 @@ static bool use_prefill(int m, int n, int k, int groupsize, bool plain = false) 
     const int min_m = g_prefill_min_m.load(std::memory_order_relaxed);
     if (min_m != kDefaultPrefillMinM) return m >= min_m;
     if (n <= 1024) return m > 256;
-    if (plain && m <= 64 && smallm_supported(m, n, k, groupsize)) return m >= 17;
+    if (plain && m <= 64) return m >= 17;
     if (n <= 3072 && static_cast<long long>(m) * k * 2 >= (128LL << 10)) return m >= 17;
     return m >= 33;
 }

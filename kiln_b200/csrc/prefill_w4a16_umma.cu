@@ -934,8 +934,8 @@ int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, PrefillParams 
 // SwiGLU can be fused into the tcgen05 kernel's epilogue when its tiling for the problem writes whole tiles as bf16.
 // whether the small-batch kernel runs a plain problem that the planner tiled as `c`
 static bool smallm_takes(const PrefillConfig &c, int m, int n, int k, int groupsize) {
-    return g_smallm_enabled && g_test_drop_a_load < 0 && c.bn == 128 && c.mt == 1 && !c.stream_k && c.splits <= k / 128 &&
-           smallm_supported(m, n, k, groupsize);
+    return g_smallm_enabled && g_test_drop_a_load < 0 && c.bn == 128 && c.mt == 1 && !c.stream_k &&
+           smallm_supported(m, n, k, groupsize, c.splits);
 }
 
 bool prefill_fuses_swiglu(int m, int n, int k) {
@@ -992,22 +992,7 @@ int launch_prefill(const GemmArgs &a) {
                         (a.lora_r == 0 || (a.lora_t && a.lora_b && prefill_fuses_lora(a.groupsize, a.lora_r)));
     if (!smallm && a.swiglu && (fused || c.splits != 1 || c.stream_k || (c.bn == 128 && c.mt == 1)))
         return KILN_W4A16_ERR_KERN_SHAPE;  // (callers ask prefill_fuses_swiglu first)
-    if (smallm) {
-        const size_t need = workspace_for(c, a.m, a.n);
-        if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
-        int rc = launch_smallm(a, c.splits, static_cast<float *>(a.workspace));
-        if (rc == 0 && c.splits > 1) {
-            const size_t total4 = static_cast<size_t>(a.m) * a.n / 4;
-            int blocks = static_cast<int>((total4 + 255) / 256);
-            const int cap = device_sm_count() * 8;
-            if (blocks > cap) blocks = cap;
-            note_launch();
-            rc = record_cuda_error(launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), a.stream, static_cast<float *>(a.workspace),
-                                              static_cast<__nv_bfloat16 *>(a.C), static_cast<const __half *>(a.S), a.m, a.n, c.splits,
-                                              a.groupsize == -1 ? 1 : 0));
-        }
-        return rc;
-    }
+    if (smallm) return launch_smallm(a, c.splits);  // (the K splits of a tile are a cluster: no workspace)
 
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.k), static_cast<cuuint64_t>(a.m)};
