@@ -116,7 +116,7 @@ def native():
         except ModuleNotFoundError as e:
             raise ImportError("kiln_b200/_native.so is missing: run `python -m kiln_b200.build`") from e
         names = ("kiln_w4a16_gemm_bf16", "kiln_w4a16_workspace_bytes", "kiln_w4a16_gemm_bf16_ex", "kiln_w4a16_workspace_bytes_ex",
-                 "kiln_w4a16_gemm_bf16_grouped", "kiln_w4a16_quantize_and_pack_device")
+                 "kiln_w4a16_gemm_bf16_grouped", "kiln_w4a16_quantize_and_pack_device", "kiln_w4a16_repack_gptq_device")
         mod.bind(*(ctypes.cast(getattr(lib(), name), _vp).value for name in names))
         _native = mod
     return _native

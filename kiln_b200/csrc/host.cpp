@@ -40,6 +40,7 @@ struct Abi {
     decltype(&kiln_w4a16_workspace_bytes_ex) workspace_ex;
     decltype(&kiln_w4a16_gemm_bf16_grouped) grouped;
     decltype(&kiln_w4a16_quantize_and_pack_device) pack;
+    decltype(&kiln_w4a16_repack_gptq_device) gptq;
 } abi;
 
 PyObject *name_b, *name_s, *name_g, *name_k, *name_n;  // attribute names of MarlinPackedProj
@@ -302,14 +303,49 @@ PyObject *py_pack(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     });
 }
 
-// bind(gemm, workspace, gemm_ex, workspace_ex, grouped, pack): addresses of the C ABI's entry points
+// pack_gptq(qweight, qzeros, scales, groupsize) -> (b_packed, scales), or False for an asymmetric checkpoint
+PyObject *py_pack_gptq(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 4 || !PyLong_CheckExact(args[3])) Py_RETURN_NONE;
+        const Tensor *qw = plain(args[0], at::kInt), *qz = plain(args[1], at::kInt), *sc = plain(args[2], at::kHalf);
+        const long g = PyLong_AsLong(args[3]);
+        if (PyErr_Occurred()) PyErr_Clear();
+        if (!qw || !qz || !sc || qw->dim() != 2 || qz->dim() != 2 || sc->dim() != 2 || (g != -1 && g != 128)) Py_RETURN_NONE;
+        const int64_t k = qw->size(0) * 8, n = qw->size(1);
+        if (k <= 0 || n <= 0 || k % 128 || n % 256 || k > INT32_MAX || n > INT32_MAX / 2) Py_RETURN_NONE;
+        const int64_t rows = g == -1 ? 1 : k / g;
+        if (qz->size(0) != rows || qz->size(1) != n / 8 || sc->size(0) != rows || sc->size(1) != n || qz->device() != qw->device() ||
+            sc->device() != qw->device())
+            Py_RETURN_NONE;
+        const c10::cuda::CUDAGuard guard(qw->device());
+        const Tensor b = empty({k / 16, 2 * n}, at::kInt, qw->device()), s = empty({rows, n}, at::kHalf, qw->device());
+        const Tensor bad = empty({1}, at::kInt, qw->device());
+        void *const stream = c10::cuda::getCurrentCUDAStream().stream();
+        int rc, count = 0;
+        Py_BEGIN_ALLOW_THREADS;
+        rc = abi.gptq(qw->const_data_ptr<int32_t>(), qz->const_data_ptr<int32_t>(), static_cast<const uint16_t *>(sc->const_data_ptr()),
+                      static_cast<int>(k), static_cast<int>(n), static_cast<int>(g), b.mutable_data_ptr<int32_t>(),
+                      static_cast<uint16_t *>(s.mutable_data_ptr()), static_cast<uint32_t *>(bad.mutable_data_ptr()), stream);
+        if (!rc) count = bad.item<int>();  // (waits for the device)
+        Py_END_ALLOW_THREADS;
+        if (rc) return PyLong_FromLong(rc);
+        if (count) Py_RETURN_FALSE;
+        PyObject *pb = THPVariable_Wrap(b), *ps = pb ? THPVariable_Wrap(s) : nullptr;
+        PyObject *pair = ps ? PyTuple_Pack(2, pb, ps) : nullptr;
+        Py_XDECREF(pb);
+        Py_XDECREF(ps);
+        return pair;
+    });
+}
+
+// bind(gemm, workspace, gemm_ex, workspace_ex, grouped, pack, gptq): addresses of the C ABI's entry points
 PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    void *p[6];
-    if (nargs != 6) {
-        PyErr_SetString(PyExc_TypeError, "bind takes six addresses");
+    void *p[7];
+    if (nargs != 7) {
+        PyErr_SetString(PyExc_TypeError, "bind takes seven addresses");
         return nullptr;
     }
-    for (int i = 0; i < 6; ++i)
+    for (int i = 0; i < 7; ++i)
         if (!(p[i] = PyLong_AsVoidPtr(args[i]))) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null entry point");
             return nullptr;
@@ -320,6 +356,7 @@ PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     abi.workspace_ex = reinterpret_cast<decltype(abi.workspace_ex)>(p[3]);
     abi.grouped = reinterpret_cast<decltype(abi.grouped)>(p[4]);
     abi.pack = reinterpret_cast<decltype(abi.pack)>(p[5]);
+    abi.gptq = reinterpret_cast<decltype(abi.gptq)>(p[6]);
     Py_RETURN_NONE;
 }
 
@@ -330,6 +367,7 @@ PyMethodDef method(const char *name) {
 
 PyMethodDef methods[] = {method<py_bind>("bind"),       method<py_gemm>("gemm"),       method<py_matmul>("matmul"),
                          method<py_gemm_ex>("gemm_ex"), method<py_grouped>("grouped"), method<py_pack>("pack"),
+                         method<py_pack_gptq>("pack_gptq"),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -302,73 +302,248 @@ __global__ void pack_words_kernel(const void *w, int n, int g, const float *scal
     b_packed[static_cast<size_t>(kb) * 2 * n + ch * 128 + tid] = static_cast<int32_t>(word);
 }
 
-// Grouped mode (128 rows per scale), everything in one pass: one block per (scale group, 64-column chunk) reads its
-// 128 x 64 weights once (16-byte loads, 128 contiguous bytes per row), finds the column maxima, writes the 64 fp16
-// scales at their Marlin positions and the eight 512-byte packed blocks.  Same arithmetic as the two kernels above.
-// grid = (n/64, k/128), block = 256.
+// ---- one pass over the weights, grouped (128 rows per scale) or per column --------------------------------------------
+//
+// One block per 128 rows x 64 columns.  A thread holds rows 2qd, 2qd+1, 2qd+8, 2qd+9 of one 16-row tile and eight neighbouring
+// columns: half of the eight weights of each of eight packed words, whose other half (columns c + 8) is the neighbouring
+// lane's.  So the weights go from 16-byte loads (128 contiguous bytes per row and eight lanes) to packed words in registers,
+// with one shuffle per word; shared memory only carries the column maxima and the scales.
+//
+// Bound: HBM once the arithmetic is small.  With the IEEE division and roundf for every weight (about 30 instructions) the
+// arithmetic took 40 us of a 2560 x 9216 weight's 44.  Here w / s is w * (1 / s): its error is below 4 units in the last place,
+// 4e-6 at the largest quotient of 7.51, so rounding it to nearest gives what rounding the correctly rounded quotient half away
+// from zero gives, unless it lies within 1e-5 of a tie.  One bf16 weight in a thousand does (few bits over few bits); those are
+// divided exactly (quantize_near_tie).  NaN, and columns whose scale is zero, subnormal or infinite, take quantize_one.
+// Measured: 2560 x 9216 bf16 44.8 -> 20.7 us per call (18 instructions per weight are what is left: the integer pipe), f32 45.2
+// -> 24.7; per column, whose first version walked each column with one thread, 261 -> 31.
+
+constexpr float kRoundMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to nearest, the integer sits in the low mantissa bits
+constexpr uint32_t kRoundMagicBits = 0x4B400000u;
+
+// two floats per instruction (sm_100)
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {  // NaN if either is
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+struct ColumnScale {
+    float s, inv;  // inv = 0: no fast path for this column
+};
+__device__ __forceinline__ __half scale_of_max(float mx) {
+    if (mx == 0.f) mx = 1.f;
+    return __float2half_rn(__fdiv_rn(2.0f * mx, 15.0f));
+}
+__device__ __forceinline__ ColumnScale column_scale(__half h) {
+    const float s = __half2float(h);
+    return {s, s >= 6.2e-5f && s <= 65504.f ? __fdiv_rn(1.0f, s) : 0.f};
+}
+
+// The quantised weight where w / s may be a tie, without a division: Markstein's theorem (IBM J. Res. Dev. 34, 1990) makes
+// q + (w - q s) * inv the correctly rounded quotient when inv is the correctly rounded 1 / s and q is within one unit in the
+// last place, which the first of the two corrections sees to (s comes from fp16, so its mantissa is not all ones).
+__device__ __forceinline__ uint32_t quantize_near_tie(float w, ColumnScale cs) {
+    float q = w * cs.inv;
+    q = fmaf(fmaf(-q, cs.s, w), cs.inv, q);
+    q = fmaf(fmaf(-q, cs.s, w), cs.inv, q);
+    float r = (q + kRoundMagic) - kRoundMagic;
+    if (fabsf(q - r) == 0.5f) r = q + copysignf(0.5f, q);  // half away from zero
+    return __float_as_uint(fminf(r, 7.f) + (kRoundMagic + 8.f)) & 0xFu;
+}
+
+// Four rows x eight columns of one thread, kept as they were loaded (bf16: two to a register, so that six blocks fit an SM).
 template <bool BF16>
-__global__ void __launch_bounds__(256) pack_group_kernel(const void *w, int n, uint16_t *scales_perm, int32_t *b_packed, float *dequant) {
-    __shared__ float tile[128][65];
-    __shared__ float part_max[4][64];
-    __shared__ float s_col[64];
-    const int ch = blockIdx.x, grp = blockIdx.y, tid = threadIdx.x;
-    const size_t row0 = static_cast<size_t>(grp) * 128;
-    // 128 rows x 8 pieces of 8 weights
-    for (int e = tid; e < 128 * 8; e += 256) {
-        const int r = e >> 3, p8 = e & 7;
-        const size_t off = (row0 + r) * n + ch * 64 + p8 * 8;
-        float v[8];
-        if (BF16) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(w) + off);
-            const uint32_t x[4] = {raw.x, raw.y, raw.z, raw.w};
+struct Rows {
+    uint32_t x[4][BF16 ? 4 : 8];
+    __device__ __forceinline__ void load(const void *w, size_t off, int n) {
+        constexpr int kRow[4] = {0, 1, 8, 9};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                v[2 * i] = __uint_as_float(x[i] << 16);
-                v[2 * i + 1] = __uint_as_float(x[i] & 0xFFFF0000u);
+        for (int r = 0; r < 4; ++r) {
+            const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint8_t *>(w) + (off + static_cast<size_t>(kRow[r]) * n) * (BF16 ? 2 : 4));
+#pragma unroll
+            for (int i = 0; i < (BF16 ? 1 : 2); ++i) {
+                const uint4 raw = __ldg(p + i);
+                x[r][4 * i] = raw.x;
+                x[r][4 * i + 1] = raw.y;
+                x[r][4 * i + 2] = raw.z;
+                x[r][4 * i + 3] = raw.w;
             }
-        } else {
-            const float4 a = *reinterpret_cast<const float4 *>(static_cast<const float *>(w) + off);
-            const float4 b = *reinterpret_cast<const float4 *>(static_cast<const float *>(w) + off + 4);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         }
+    }
+    __device__ __forceinline__ float at(int r, int c) const {
+        if (!BF16) return __uint_as_float(x[r][c & (BF16 ? 3 : 7)]);
+        return __uint_as_float((c & 1) ? (x[r][c >> 1] & 0xFFFF0000u) : (x[r][c >> 1] << 16));
+    }
+};
+
+// Column maxima of the block's 128 x 64 weights -> part[warp][column]; the caller synchronises.
+template <bool BF16>
+__device__ __forceinline__ void block_column_max(const Rows<BF16> &v, float (*part)[64]) {
+    const int warp = threadIdx.x >> 5, p8 = threadIdx.x & 7, qd = (threadIdx.x >> 3) & 3;
+    if constexpr (BF16) {  // two columns at a time (the maximum of bf16 values is one of them: nothing is rounded)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) tile[r][p8 * 8 + i] = v[i];
+        for (int c2 = 0; c2 < 4; ++c2) {
+            auto bf = [](uint32_t u) { return __habs2(*reinterpret_cast<__nv_bfloat162 *>(&u)); };
+            __nv_bfloat162 m = __hmax2(__hmax2(bf(v.x[0][c2]), bf(v.x[1][c2])), __hmax2(bf(v.x[2][c2]), bf(v.x[3][c2])));
+            m = __hmax2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 8));
+            m = __hmax2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 16));
+            if (qd == 0) *reinterpret_cast<float2 *>(&part[warp][p8 * 8 + 2 * c2]) = make_float2(fmaxf(0.f, __low2float(m)), fmaxf(0.f, __high2float(m)));
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            float m = fmaxf(fmaxf(fabsf(v.at(0, c)), fabsf(v.at(1, c))), fmaxf(fabsf(v.at(2, c)), fabsf(v.at(3, c))));
+            m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 8));
+            m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 16));
+            if (qd == 0) part[warp][p8 * 8 + c] = fmaxf(0.f, m);  // (all four NaN: 0, as the reference's comparison leaves it)
+        }
     }
-    __syncthreads();
-    {
-        const int col = tid & 63, part = tid >> 6;
-        float mx = 0.f;
-        for (int r = 0; r < 32; ++r) mx = fmaxf(mx, fabsf(tile[part * 32 + r][col]));
-        part_max[part][col] = mx;
-    }
+}
+
+// Per-column mode, first pass: maxima of every 128-row block, [k/128][n].  grid = (n/64, k/128), block = 256.
+template <bool BF16>
+__global__ void __launch_bounds__(256, BF16 ? 6 : 4) pack_max_kernel(const void *w, int n, float *block_max) {
+    __shared__ float part[8][64];
+    const int tid = threadIdx.x, p8 = tid & 7, qd = (tid >> 3) & 3, kt = tid >> 5;
+    Rows<BF16> v;
+    v.load(w, (static_cast<size_t>(blockIdx.y) * 128 + kt * 16 + 2 * qd) * n + blockIdx.x * 64 + p8 * 8, n);
+    block_column_max(v, part);
     __syncthreads();
     if (tid < 64) {
-        float mx = fmaxf(fmaxf(part_max[0][tid], part_max[1][tid]), fmaxf(part_max[2][tid], part_max[3][tid]));
-        if (mx == 0.f) mx = 1.f;
-        const __half h = __float2half_rn(__fdiv_rn(2.0f * mx, 15.0f));
-        scales_perm[static_cast<size_t>(grp) * n + scale_group_pos(ch * 64 + tid)] = __half_as_ushort(h);
-        s_col[tid] = __half2float(h);
+        float mx = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, part[i][tid]);
+        block_max[static_cast<size_t>(blockIdx.y) * n + blockIdx.x * 64 + tid] = mx;
+    }
+}
+
+// Second pass: the maxima of a column's blocks -> its scale.  (The maxima wait in the buffer of the packed words, which the
+// third pass overwrites; it only needs the scales.)  grid = n/64, block = 256: four threads per column.
+__global__ void __launch_bounds__(256) pack_column_scales_kernel(const float *block_max, int n, int blocks, uint16_t *scales_perm) {
+    __shared__ float part[4][64];
+    const int c = threadIdx.x & 63, col = blockIdx.x * 64 + c;
+    float mx = 0.f;
+    for (int b = threadIdx.x >> 6; b < blocks; b += 4) mx = fmaxf(mx, block_max[static_cast<size_t>(b) * n + col]);
+    part[threadIdx.x >> 6][c] = mx;
+    __syncthreads();
+    if (threadIdx.x < 64)
+        scales_perm[scale_single_pos(col)] = __half_as_ushort(scale_of_max(fmaxf(fmaxf(part[0][c], part[1][c]), fmaxf(part[2][c], part[3][c]))));
+}
+
+// Grouped: scales from the block's own maxima.  Per column: scales from the second pass.  grid = (n/64, k/128), block = 256.
+template <bool BF16>
+__global__ void __launch_bounds__(256, BF16 ? 5 : 4) pack_group_kernel(const void *w, int n, int per_column, uint16_t *scales_perm,
+                                                         int32_t *b_packed, float *dequant) {
+    __shared__ float part[8][64];
+    __shared__ ColumnScale col_scale[64];
+    const int tid = threadIdx.x, p8 = tid & 7, qd = (tid >> 3) & 3, kt = tid >> 5;
+    const int ch = blockIdx.x, grp = blockIdx.y;
+    Rows<BF16> v;
+    const size_t off = (static_cast<size_t>(grp) * 128 + kt * 16 + 2 * qd) * n + ch * 64 + p8 * 8;
+    v.load(w, off, n);
+    if (!per_column) {
+        block_column_max(v, part);
+        __syncthreads();
+    }
+    if (tid < 64) {
+        const int col = ch * 64 + tid;
+        __half h;
+        if (!per_column) {
+            float mx = part[0][tid];
+#pragma unroll
+            for (int i = 1; i < 8; ++i) mx = fmaxf(mx, part[i][tid]);
+            h = scale_of_max(mx);
+            scales_perm[static_cast<size_t>(grp) * n + scale_group_pos(col)] = __half_as_ushort(h);
+        } else {
+            h = __ushort_as_half(scales_perm[scale_single_pos(col)]);
+        }
+        col_scale[tid] = column_scale(h);
     }
     __syncthreads();
-    for (int idx = tid; idx < 8 * 128; idx += 256) {
-        const int kt = idx >> 7, t128 = idx & 127;
-        const int lane = t128 >> 2, j = t128 & 3;
-        const int r0 = kt * 16 + 2 * (lane & 3), c = lane >> 2;
-        uint32_t word = 0;
+    // Half words: nibbles 0, 1, 4, 5 of the word of column c (rows 2qd, 2qd+8, 2qd+1, 2qd+9).
+    uint32_t half[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int cc = 16 * j + c + nib_dc(i);
-            word |= static_cast<uint32_t>(quantize_one(tile[r0 + nib_dr(i)][cc], s_col[cc])) << (4 * i);
+    for (int c = 0; c < 8; ++c) {
+        const ColumnScale cs = col_scale[p8 * 8 + c];
+        constexpr int kOrder[4] = {3, 1, 2, 0};  // rows of nibbles 5, 4, 1, 0: highest first
+        uint32_t word = 0;
+        float worst = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+            const float2 q = f2_unpack(f2_mul(f2_pack(v.at(kOrder[i], c), v.at(kOrder[i + 1], c)), f2_pack(cs.inv, cs.inv)));
+            const unsigned long long t = f2_pack(min_nan(q.x, 7.f), min_nan(q.y, 7.f));  // (above 7 the clamp decides)
+            const unsigned long long r = f2_add(t, f2_pack(kRoundMagic, kRoundMagic));
+            const float2 d = f2_unpack(f2_add(t, f2_fma(r, f2_pack(-1.f, -1.f), f2_pack(kRoundMagic, kRoundMagic))));  // t - rounded(t)
+            worst = max_nan(worst, max_nan(fabsf(d.x), fabsf(d.y)));
+            const float2 rr = f2_unpack(r);
+            word = (word << (i == 2 ? 12 : 4)) + __float_as_uint(rr.x);
+            word = (word << 4) + __float_as_uint(rr.y);
         }
-        b_packed[(static_cast<size_t>(grp) * 8 + kt) * 2 * n + ch * 128 + t128] = static_cast<int32_t>(word);
+        // each nibble came as magic + q: take the magic bits out and add the offset of 8
+        constexpr uint32_t kAdd = 8u - kRoundMagicBits;
+        word += kAdd * (1u + (1u << 4) + (1u << 16) + (1u << 20));
+        if (!(worst < 0.49999f) || cs.inv == 0.f) {  // (NaN among them)
+            const float sum = (v.at(0, c) + v.at(1, c)) + (v.at(2, c) + v.at(3, c));
+            word = 0;
+            if (cs.inv == 0.f || sum != sum) {
+#pragma unroll 1
+                for (int i = 0; i < 4; ++i) {
+                    const float x = i == 0 ? v.at(3, c) : i == 1 ? v.at(1, c) : i == 2 ? v.at(2, c) : v.at(0, c);
+                    word = (word << (i == 2 ? 12 : 4)) | static_cast<uint32_t>(quantize_one(x, cs.s));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) word = (word << (i == 2 ? 12 : 4)) | quantize_near_tie(v.at(kOrder[i], c), cs);
+            }
+        }
+        half[c] = word;
+        if (dequant) {
+            constexpr int kRow[4] = {0, 1, 8, 9}, kShift[4] = {0, 16, 4, 20};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                dequant[off + static_cast<size_t>(kRow[r]) * n + c] =
+                    __fmul_rn(static_cast<float>(static_cast<int>((word >> kShift[r]) & 0xF) - kQOffset), cs.s);
+        }
     }
-    if (dequant) {
-        for (int e = tid; e < 128 * 64; e += 256) {
-            const int r = e >> 6, c = e & 63;
-            const float sc = s_col[c];
-            dequant[(row0 + r) * n + ch * 64 + c] = __fmul_rn(static_cast<float>(quantize_one(tile[r][c], sc) - kQOffset), sc);
-        }
+    // Lane p8 = 2j + e holds columns 16j + 8e + c.  The even lane finishes the words of c = 0..3, the odd one those of 4..7.
+    const int e = p8 & 1, j = p8 >> 1;
+    uint32_t *dst = reinterpret_cast<uint32_t *>(b_packed) + (static_cast<size_t>(grp) * 8 + kt) * 2 * n + ch * 128 + j;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, e ? half[i] : half[4 + i], 1);
+        const uint32_t lo = e ? got : half[i], hi = e ? half[4 + i] : got;
+        const int c = 4 * e + i;
+        dst[(c * 4 + qd) * 4] = lo | (hi << 8);
     }
 }
 
@@ -391,19 +566,35 @@ __global__ void repack_words_kernel(const uint8_t *q, int n, int32_t *b_packed) 
     b_packed[static_cast<size_t>(kb) * 2 * n + ch * 128 + tid] = static_cast<int32_t>(word);
 }
 
-// GPTQ qweight int32 [k/8, n] -> packed words (same gather as above from the two GPTQ words a 16-row tile spans).
-__global__ void repack_gptq_words_kernel(const int32_t *qweight, int n, int32_t *b_packed) {
-    const int ch = blockIdx.x, kb = blockIdx.y, tid = threadIdx.x;
-    const int lane = tid >> 2, j = tid & 3;
-    const int r0 = 2 * (lane & 3), c = lane >> 2;
-    uint32_t word = 0;
+// GPTQ qweight int32 [k/8, n] -> packed words.  A thread takes one c of one 16-row tile and 64-column chunk: the two GPTQ words
+// (rows 0-7 and 8-15 of the tile) of columns 16j + c and 16j + 8 + c give the words (c, qd) for every qd, byte qd of each being
+// rows 2qd and 2qd + 1; the sixteen words of c are 64 contiguous bytes.  grid = (n/64, ceil(k/16/32)), block = 256.
+__global__ void __launch_bounds__(256) repack_gptq_words_kernel(const int32_t *qweight, int n, int k_tiles, int32_t *b_packed) {
+    const int c = threadIdx.x & 7, kb = blockIdx.y * 32 + (threadIdx.x >> 3), ch = blockIdx.x;
+    if (kb >= k_tiles) return;
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(qweight) + static_cast<size_t>(kb) * 2 * n + ch * 64 + c;
+    uint32_t in[2][8];  // [row half][8-column step]
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = r0 + nib_dr(i), col = ch * 64 + 16 * j + c + nib_dc(i);
-        const uint32_t src = static_cast<uint32_t>(qweight[static_cast<size_t>(kb * 2 + (r >> 3)) * n + col]);
-        word |= ((src >> (4 * (r & 7))) & 0xFu) << (4 * i);
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int t = 0; t < 8; ++t) in[r][t] = __ldg(src + static_cast<size_t>(r) * n + t * 8);
+    uint4 *dst = reinterpret_cast<uint4 *>(b_packed + static_cast<size_t>(kb) * 2 * n + ch * 128) + c * 4;
+#pragma unroll
+    for (int qd = 0; qd < 4; ++qd) {
+        uint32_t out[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            // bytes: low nibble = even row, high nibble = odd row
+            const uint32_t a = (in[0][2 * j] >> (8 * qd)) & 0xFFu, b = (in[1][2 * j] >> (8 * qd)) & 0xFFu;
+            const uint32_t a8 = (in[0][2 * j + 1] >> (8 * qd)) & 0xFFu, b8 = (in[1][2 * j + 1] >> (8 * qd)) & 0xFFu;
+            const uint32_t x = a | (b << 8) | (a8 << 16) | (b8 << 24);  // nibbles: A0 A1 B0 B1 A'0 A'1 B'0 B'1
+            const uint32_t ev = x & 0x0F0F0F0Fu, od = (x >> 4) & 0x0F0F0F0Fu;
+            // even rows to nibbles 0..3, odd rows to nibbles 4..7
+            const uint32_t e2 = (ev | (ev >> 4)) & 0x00FF00FFu, o2 = (od | (od >> 4)) & 0x00FF00FFu;
+            out[j] = ((e2 | (e2 >> 8)) & 0xFFFFu) | ((o2 | (o2 >> 8)) << 16);
+        }
+        dst[qd] = make_uint4(out[0], out[1], out[2], out[3]);
     }
-    b_packed[static_cast<size_t>(kb) * 2 * n + ch * 128 + tid] = static_cast<int32_t>(word);
 }
 
 // counts the zero-points that are not 8 (one word = eight of them)
@@ -443,14 +634,25 @@ kiln_w4a16_status_t kiln_w4a16_quantize_and_pack_device(const void *weight, int 
     if (!weight || !b_packed || !scales_f16) return KILN_W4A16_ERR_ARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int num_groups = k / g;
-    if (groupsize == 128 && (reinterpret_cast<uintptr_t>(weight) & 15) == 0) {  // (n is a multiple of 64: rows stay 16-byte aligned)
+    // The one-pass kernel: 16-byte loads, 128-row groups or the whole column.
+    const bool aligned = (reinterpret_cast<uintptr_t>(weight) & 15) == 0;  // (n is a multiple of 64: rows stay 16-byte aligned)
+    if (aligned && (groupsize == 128 || groupsize == -1)) {
         const dim3 grid(n / 64, k / 128);
+        const int per_column = groupsize == -1;
+        if (per_column) {
+            float *block_max = reinterpret_cast<float *>(b_packed);  // (k/128 x n floats: a sixteenth of it)
+            if (weight_is_bf16)
+                pack_max_kernel<true><<<grid, 256, 0, st>>>(weight, n, block_max);
+            else
+                pack_max_kernel<false><<<grid, 256, 0, st>>>(weight, n, block_max);
+            pack_column_scales_kernel<<<n / 64, 256, 0, st>>>(block_max, n, k / 128, scales_f16);
+        }
         if (weight_is_bf16)
-            pack_group_kernel<true><<<grid, 256, 0, st>>>(weight, n, scales_f16, b_packed, dequant);
+            pack_group_kernel<true><<<grid, 256, 0, st>>>(weight, n, per_column, scales_f16, b_packed, dequant);
         else
-            pack_group_kernel<false><<<grid, 256, 0, st>>>(weight, n, scales_f16, b_packed, dequant);
+            pack_group_kernel<false><<<grid, 256, 0, st>>>(weight, n, per_column, scales_f16, b_packed, dequant);
         pack_fence_kernel<<<1, 32, 0, st>>>();
-        note_launch(2);
+        note_launch(per_column ? 4 : 2);
         return record_cuda_error(cudaGetLastError());
     }
     float *scales_nat = nullptr;  // natural-order f32 scales, scratch for the second kernel
@@ -507,7 +709,7 @@ kiln_w4a16_status_t kiln_w4a16_repack_gptq_device(const int32_t *qweight, const 
             qzeros, words, asymmetric);
         ++launches;
     }
-    repack_gptq_words_kernel<<<dim3(n / 64, k / 16), 128, 0, st>>>(qweight, n, b_packed);
+    repack_gptq_words_kernel<<<dim3(n / 64, (k / 16 + 31) / 32), 256, 0, st>>>(qweight, n, k / 16, b_packed);
     permute_scales_kernel<<<dim3((n + 127) / 128, k / g), 128, 0, st>>>(scales, n, groupsize == -1, scales_perm);
     pack_fence_kernel<<<1, 32, 0, st>>>();
     note_launch(launches);

@@ -77,6 +77,14 @@ def pack_from_gptq(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torch.Te
     projection, on the device and without dequantising (kiln: CPU dequantise to bf16, kiln-model/src/quantized.rs:70-163,
     then re-quantise).  Returns None when the shape is unsupported or the checkpoint is not symmetric (a zero-point other
     than 8): the caller then keeps kiln's route.  Reads one counter back from the device."""
+    if not nvtx.enabled():
+        done = _lib.native().pack_gptq(qweight, qzeros, scales, groupsize)
+        if type(done) is tuple:
+            return MarlinPackedProj(*done, groupsize, qweight.shape[0] * 8, qweight.shape[1])
+        if done is False:
+            return None
+        if done is not None:
+            raise KilnMarlinError(f"marlin_proj: GPTQ repack failed: {_lib.STATUS_NAMES.get(done, done)}")
     if not (qweight.is_cuda and qzeros.is_cuda and scales.is_cuda):
         return None
     k, n = qweight.shape[0] * 8, qweight.shape[1]
