@@ -55,6 +55,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(2, "-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
+    obj = os.path.join(CSRC, "pack_host.o")
+    procs.append(("pack_host.cpp", subprocess.Popen([os.environ.get("CXX", "g++"), "-std=c++17", "-O3", "-fPIC", "-c", os.path.join(CSRC, "pack_host.cpp"),
+                                                     "-o", obj], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    objs.append(obj)
     procs.append(("host.cpp", subprocess.Popen(_native_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, p in procs:

@@ -6,11 +6,13 @@
 // 1024-entry gather; every packed word is assembled from the eight weights the consuming lane
 // owns (see the layout note in w4a16_common.cuh).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <thread>
 #include <vector>
 
+#include "pack_host.h"
 #include "w4a16_common.cuh"
 
 namespace kiln {
@@ -77,6 +79,22 @@ void parallel_chunks(int chunks, int num_threads, F &&fn) {
     for (auto &th : pool) th.join();
 }
 
+// fn(i) for i in [0, count), handed out one at a time (blocks differ in what the memory system has to do for them).
+template <class F>
+void parallel_units(int count, int num_threads, F &&fn) {
+    int nt = num_threads > 0 ? num_threads : static_cast<int>(std::thread::hardware_concurrency());
+    nt = std::max(1, std::min(nt, count));
+    std::atomic<int> next{0};
+    auto work = [&] {
+        for (int i; (i = next.fetch_add(1, std::memory_order_relaxed)) < count;) fn(i);
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(nt - 1);
+    for (int t = 1; t < nt; ++t) pool.emplace_back(work);
+    work();
+    for (auto &th : pool) th.join();
+}
+
 // Packs one 64-column chunk of a 16-row K-tile whose nibbles are in nib[16][64].
 inline void pack_tile_host(const uint8_t (*nib)[64], int32_t *out128) {
     for (int lane = 0; lane < 32; ++lane) {
@@ -134,6 +152,17 @@ kiln_w4a16_status_t kiln_w4a16_quantize_and_pack_host(const float *weight, int k
     if (!weight || !b_packed || !scales_f16) return KILN_W4A16_ERR_ARG;
     const int chunks = n / 64, ktiles_per_group = g / 16, num_groups = k / g;
     const size_t row_words = static_cast<size_t>(2) * n;
+    if (pack_host_vectorised()) {
+        int pos[64];
+        for (int c = 0; c < 64; ++c) pos[c] = groupsize == -1 ? scale_single_pos(c) : scale_group_pos(c);
+        const int col_blocks = n / kHostBlockCols;  // (n is a multiple of 256)
+        parallel_units(col_blocks * num_groups, num_threads, [&](int u) {
+            const int grp = u / col_blocks, cb = u - grp * col_blocks;
+            pack_host_block(weight, n, grp * g, g, cb * kHostBlockCols, kHostBlockCols, b_packed, scales_f16 + static_cast<size_t>(grp) * n, pos,
+                            dequant);
+        });
+        return KILN_W4A16_OK;
+    }
     parallel_chunks(chunks, num_threads, [&](int ch) {
         const int c0 = ch * 64;
         float s[64];
