@@ -72,21 +72,15 @@ static int validate(const GemmArgs &a) {
     return -1;  // proceed
 }
 
-// Kernel choice (measured on B200, CUDA-graph replay over rotating weights).  The decode kernel handles 8 or 16 rows per
-// block of CTAs and repeats the int4 dequant for every block; the tcgen05 kernel dequantises once per 128 rows but pays
-// a fixed cost per launch and per K-step of a tile.  Measured crossovers (decode / tcgen05, us):
-//  * wide projections (4096 columns and more): the decode kernel wins up to 32 rows, two blocks of 16 (gate+up M=32:
-//    19.2 / 16.4 but M=24: 18.8 / 22.7; q M=32: 8.2 / 8.9; GDN-in M=32: 11.8 / 11.6), a third block costs it far more than
-//    a tile (gate+up M=40: 32.3 / 16.4, q: 12.7 / 9.4);
-//  * projections of about 2560 columns have few column blocks for the decode kernel to spread over: the tcgen05 kernel
-//    wins from 17 rows (down M=17: 13.4 / 11.8, M=32: 13.7 / 12.5; o M=17: 9.5 / 8.2, M=32: 9.9 / 8.9, M=64: 14.4 / 11.2),
-//    provided the activation matrix is at least 128 KB (smaller ones were measured 40 % slower through its TMA loads);
-//  * projections of 1024 columns or fewer (k, v: four to eight tiles) stay on the decode kernel up to M = 256
-//    (k at M=128: 6.4 / 15.3).
-//  * a GEMM without epilogue options and at most 128 rows runs on the tcgen05 kernel that keeps the
-//    weights in tensor memory (smallm_w4a16_tmem.cu), which moves the crossover to 17 rows for every projection of more
-//    than 1024 columns (M=17: q 7.8 / 6.8, gate+up 18.3 / 13.6, down 12.8 / 10.1, GDN-in 11.0 / 10.0, o 9.1 / 7.0;
-//    M=16, one block of the decode kernel: q 5.7 / 6.6, gate+up 12.0 / 13.4).
+// Kernel choice (measured on B200, CUDA-graph replay over rotating weights).  A decode block of 8 or 16 rows repeats the int4
+// dequant and its MMAs for every further block; a tcgen05 tile dequantises once per 128 rows but pays a fixed cost per launch:
+//  * a plain GEMM (or SwiGLU where it is fused) of at most 128 rows runs on the kernel that keeps the weights in tensor memory
+//    (smallm_w4a16_tmem.cu), from 17 rows for every projection of more than 1024 columns (M = 17, decode / small-batch, us:
+//    2560 x 4096 7.6 / 5.0, 2560 x 18432 17.9 / 10.1, 9216 x 2560 12.7 / 8.9).  It is faster from 9 rows already, but the decode
+//    kernel multiplies the group scale in fp32 where the tcgen05 kernels round it to bf16, so it keeps the sizes it had;
+//  * with a LoRA delta, which the decode kernel adds from an fp32 projection, the line is at 33 rows, or at 17 for projections of
+//    about 2560 columns (few column blocks for the decode kernel) whose activation matrix is at least 128 KB;
+//  * projections of 1024 columns or fewer (four to eight tiles) stay on the decode kernel up to 256 rows.
 // kiln_w4a16_set_prefill_min_m replaces the rule by a plain threshold.
 static bool use_prefill(int m, int n, int k, int groupsize, bool plain = false) {
     if (!prefill_supported(m, n, k, groupsize)) return false;
@@ -105,7 +99,7 @@ static int gemm(const GemmArgs &a) {
     const int v = validate(a);
     if (v >= 0) return v;
     if (use_prefill(a.m, a.n, a.k, a.groupsize, plain_gemm(a))) {
-        const size_t need = a.no_scratch ? 0 : prefill_workspace_bytes(a.m, a.n, a.k);
+        const size_t need = a.no_scratch || smallm_takes(a.m, a.n, a.k, a.groupsize) ? 0 : prefill_workspace_bytes(a.m, a.n, a.k);
         if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
         return launch_prefill(a);
     }

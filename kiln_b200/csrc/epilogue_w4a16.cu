@@ -5,13 +5,13 @@
 //    fp32 sums before rounding, so the delta never exists as a matrix of its own.
 //  * finish_kernel: for batch sizes beyond the decode kernel's range, where the options are not fused yet:
 //    C = epilogue(base), base being the bf16 GEMM result in the workspace (LoRA delta added, SwiGLU applied).
+#include <algorithm>
+
 #include "w4a16_common.cuh"
 
 namespace kiln {
 namespace {
 
-// grid = (ceil(r / 8), m), block = 256: warp w of a CTA computes t[row][8 * blockIdx.x + w].
-// (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernel reads as an operand tile)
 __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_out) {
     if (bf16_out)
         static_cast<__nv_bfloat16 *>(t)[idx] = __float2bfloat16(v);
@@ -19,8 +19,11 @@ __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_o
         static_cast<float *>(t)[idx] = v;
 }
 
-__global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a,
-                                                        float scale, int k, int r, void *__restrict__ t, int bf16_out) {
+// Up to kLoraDotRows rows: one dot product per warp.  grid = (ceil(r / 8), m), block = 256: warp w of a CTA computes
+// t[row][8 * blockIdx.x + w].
+constexpr int kLoraDotRows = 8;
+__global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
+                                                       int k, int r, void *__restrict__ t, int bf16_out) {
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = blockIdx.y, j = blockIdx.x * 8 + warp;
@@ -42,50 +45,92 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
     if (lane == 0) store_t(t, static_cast<size_t>(row) * r + j, sum * scale, bf16_out);
 }
 
-// The same for larger batches: a CTA takes eight rows of x, so that every adapter row it reads serves eight dot products
-// (the kernel above re-reads the whole adapter once per row of x), and two adapter rows, each split over four warps along
-// K (the sums meet in shared memory): enough CTAs to fill the GPU at continuous-batching sizes and a four times shorter
-// loop per warp.  grid = (ceil(r / 2), ceil(m / 8)), block = 256.
-__global__ void __launch_bounds__(256) lora_down_rows8_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a,
-                                                              float scale, int m, int k, int r, void *__restrict__ t, int bf16_out) {
-    __shared__ float part[8][8];  // [warp][row of x]
-    pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int row0 = blockIdx.y * 8, j = blockIdx.x * 2 + (warp >> 2), kq = warp & 3;
-    pdl_wait();  // x may be the previous kernel's output; t may still be read by it
-    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (j < r) {
-        const uint4 *ar = reinterpret_cast<const uint4 *>(a + static_cast<size_t>(j) * k);
-        const int pieces = k / 8, per = (pieces + 3) / 4;  // 16-byte pieces of a row, and of this warp's quarter of K
-        const int i1 = min(pieces, (kq + 1) * per);
-        for (int i = kq * per + lane; i < i1; i += 32) {
-            const uint4 av = ar[i];
-            const uint32_t as[4] = {av.x, av.y, av.z, av.w};
+// More rows: a small tensor-core GEMM, K split over the CTAs of a cluster and, for few rows, over the warps of a CTA.
+//
+// Bound: latency.  The operands are a few hundred KB (x 37 x 9216 and A 64 x 9216: 1.9 MB), so what counts is how many SMs load
+// them at once and how short the chain from the grid-dependency wait to the last store is.  A lane loads 16 contiguous bytes of
+// a row of x and of a row of A and uses them as the K slots {2qd, 2qd+1, 2qd+8, 2qd+9} of two m16n8k16 MMAs: the same K
+// permutation on both sides, so no shared-memory staging and no ldmatrix.
+// A CTA has WM row tiles of 16 and 8 / WM parts of its K range, one (row tile, part) per warp, and 8 NT adapter rows.  Small tiles
+// for few rows (enough CTAs to fill the GPU), large ones for many (x is read once per 8 NT adapter rows).  The parts meet in shared
+// memory, the cluster's partial tiles in rank order through distributed shared memory: the result does not depend on timing.
+// Measured with the GEMM that follows, dot products -> tensor cores: 37 rows rank 64 9216 -> 2560 24 -> 15 us, 2560 -> 4096 13.3 ->
+// 10.7, 2048 rows 96 -> 49; 4 rows 7.6 -> 8.2, hence the line above.
+template <int NT>
+__device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1, const uint4 *const (&a)[NT], int b0, int b1, float (&acc)[NT][4]) {
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) {
+        const uint4 u = ld_cg_v4(x0 + b * 4), v = ld_cg_v4(x1 + b * 4);
+        const uint32_t lo[4] = {u.x, v.x, u.y, v.y}, hi[4] = {u.z, v.z, u.w, v.w};
 #pragma unroll
-            for (int rr = 0; rr < 8; ++rr) {
-                const int row = row0 + rr < m ? row0 + rr : m - 1;  // (rows past m repeat the last one; their sums are dropped)
-                const uint4 xv = ld_cg_v4(reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row) * k) + i);
-                const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    sum[rr] += __uint_as_float(xs[e] << 16) * __uint_as_float(as[e] << 16) +
-                               __uint_as_float(xs[e] & 0xFFFF0000u) * __uint_as_float(as[e] & 0xFFFF0000u);
-            }
+        for (int t = 0; t < NT; ++t) {
+            const uint4 w = __ldg(a[t] + b * 4);
+            mma_bf16_16816(acc[t], lo, w.x, w.y);
+            mma_bf16_16816(acc[t], hi, w.z, w.w);
         }
     }
+}
+
+// grid = (cluster size, ceil(r / (8 NT)), ceil(m / (16 WM))), cluster = (cluster size, 1, 1), block = 256.
+// (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernels read as an operand tile; fp32 otherwise)
+template <int WM, int NT>
+constexpr int lora_smem() {
+    return 8 * 16 * 8 * NT * static_cast<int>(sizeof(float));
+}
+template <int WM, int NT>
+__global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
+                                                        int m, int k, int r, void *__restrict__ t, int bf16_out) {
+    constexpr int kCols = 8 * NT, kRows = 16 * WM, kParts = 8 / WM, kTile = kRows * kCols;
+    extern __shared__ float parts[];  // [kParts][kRows][kCols]; the last one ends up with the sum
+    float *sum = parts + (kParts - 1) * kTile;
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane >> 2, qd = lane & 3;
+    const int wm = warp % WM, part = warp / WM;
+    const int rank = blockIdx.x, size = gridDim.x;
+    const int row0 = blockIdx.z * kRows + wm * 16, col0 = blockIdx.y * kCols;
+    const int blocks = k / 32, slices = size * kParts, slice = rank * kParts + part;
+    const int b0 = static_cast<int>(static_cast<long long>(blocks) * slice / slices), b1 = static_cast<int>(static_cast<long long>(blocks) * (slice + 1) / slices);
+    float acc[NT][4];
+    const uint4 *ap[NT];  // (rows past r or m repeat the last one: their sums are dropped)
 #pragma unroll
-    for (int rr = 0; rr < 8; ++rr) {
-        float v = sum[rr];
+    for (int i = 0; i < NT; ++i) {
+        acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+        ap[i] = reinterpret_cast<const uint4 *>(a + static_cast<size_t>(min(col0 + 8 * i + c, r - 1)) * k) + qd;
+    }
+    const uint4 *x0 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c, m - 1)) * k) + qd;
+    const uint4 *x1 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c + 8, m - 1)) * k) + qd;
+    pdl_wait();  // x may be the previous kernel's output; t may still be read by it
+    lora_mma_range<NT>(x0, x1, ap, b0, b1, acc);
+    float *mine = parts + part * kTile + wm * 16 * kCols;
 #pragma unroll
-        for (int sh = 16; sh >= 1; sh >>= 1) v += __shfl_xor_sync(0xffffffffu, v, sh);
-        if (lane == 0) part[warp][rr] = v;
+    for (int i = 0; i < NT; ++i) {
+        *reinterpret_cast<float2 *>(mine + c * kCols + 8 * i + 2 * qd) = make_float2(acc[i][0], acc[i][1]);
+        *reinterpret_cast<float2 *>(mine + (c + 8) * kCols + 8 * i + 2 * qd) = make_float2(acc[i][2], acc[i][3]);
     }
     __syncthreads();
-    if (threadIdx.x < 16) {  // the CTA's 2 x 8 results: the four K quarters are added in a fixed order
-        const int jj = threadIdx.x >> 3, rr = threadIdx.x & 7, jo = blockIdx.x * 2 + jj;
-        const float v = (part[4 * jj][rr] + part[4 * jj + 1][rr]) + (part[4 * jj + 2][rr] + part[4 * jj + 3][rr]);
-        if (jo < r && row0 + rr < m) store_t(t, static_cast<size_t>(row0 + rr) * r + jo, v * scale, bf16_out);
+    if (kParts > 1) {
+        for (int e = threadIdx.x; e < kTile; e += 256) {
+            float v = parts[e];
+#pragma unroll
+            for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
+            sum[e] = v;  // (of the last part, this thread alone touches this element)
+        }
+        if (size == 1) __syncthreads();
     }
+    if (size > 1) cluster_sync_all();
+    // the CTAs of the cluster take 256 elements of the tile in turn, one per thread, and sum them over the ranks
+    for (int e = threadIdx.x + rank * 256; e < kTile; e += size * 256) {
+        float v = 0.f;
+        const uint32_t addr = smem_u32(sum + e);
+        for (int q = 0; q < size; ++q) {
+            float u;
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(u) : "r"(map_to_cta(addr, q)));
+            v = q ? v + u : u;
+        }
+        const int row = blockIdx.z * kRows + e / kCols, col = col0 + e % kCols;
+        if (row < m && col < r) store_t(t, static_cast<size_t>(row) * r + col, v * scale, bf16_out);
+    }
+    if (size > 1) cluster_sync_all();  // the peers may still be reading this CTA's tile
 }
 
 __device__ __forceinline__ float lora_dot(const float *t, const __nv_bfloat16 *b, int r) {
@@ -122,23 +167,33 @@ __global__ void __launch_bounds__(256) finish_kernel(const __nv_bfloat16 *__rest
 }  // namespace
 
 int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int k, int r, void *t, int bf16_out, cudaStream_t stream) {
+    const bool dot = m <= kLoraDotRows;
+    // row tiles and adapter rows of a CTA: 16 x 16, 64 x 32 or 128 x 64
+    const int wm = m <= 48 ? 1 : (m <= 512 ? 4 : 8), rows = 16 * wm, cols = wm == 1 ? 16 : (wm == 4 ? 32 : 64), parts = 8 / wm;
+    const int row_tiles = (m + rows - 1) / rows, col_tiles = (r + cols - 1) / cols;
+    if (row_tiles > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
+    // K is split over as many CTAs as the tiles leave SMs for, while a warp keeps at least two 32-deep blocks
+    int size = std::min(8, std::max(1, device_sm_count() / (row_tiles * col_tiles)));
+    size = std::max(1, std::min(size, k / 32 / (2 * parts)));
     cudaLaunchConfig_t cfg = {};
-    const bool rows8 = m > 32;
-    cfg.gridDim = rows8 ? dim3((r + 1) / 2, (m + 7) / 8, 1) : dim3((r + 7) / 8, m, 1);
+    cfg.gridDim = dot ? dim3((r + 7) / 8, m) : dim3(size, col_tiles, row_tiles);
     cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = dot ? 0 : (wm == 1 ? lora_smem<1, 2>() : (wm == 4 ? lora_smem<4, 4>() : lora_smem<8, 8>()));
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cfg.gridDim.y > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = size;
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = !dot && size > 1 ? 2 : 1;
+    const auto *xp = static_cast<const __nv_bfloat16 *>(x), *ap = static_cast<const __nv_bfloat16 *>(lora_a);
     note_launch();
-    if (rows8)
-        return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_down_rows8_kernel, static_cast<const __nv_bfloat16 *>(x),
-                                                    static_cast<const __nv_bfloat16 *>(lora_a), scale, m, k, r, t, bf16_out));
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_down_kernel, static_cast<const __nv_bfloat16 *>(x),
-                                                static_cast<const __nv_bfloat16 *>(lora_a), scale, k, r, t, bf16_out));
+    if (dot) return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_dot_kernel, xp, ap, scale, k, r, t, bf16_out));
+    const auto kernel = wm == 1 ? lora_down_kernel<1, 2> : (wm == 4 ? lora_down_kernel<4, 4> : lora_down_kernel<8, 8>);
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out));
 }
 
 int launch_finish(const void *base, void *c, int m, int n, const float *t, const void *lora_b, int r, int swiglu,

@@ -19,6 +19,7 @@
 // Every wait in the kernel is bounded: a wait that runs out records an error code in the
 // device status word, raises a CTA-wide abort flag that every other wait polls, and the CTA
 // drains its outstanding TMA copies, frees its TMEM and returns.
+#include <algorithm>
 #include <mutex>
 
 #include "w4a16_umma.cuh"
@@ -832,6 +833,26 @@ unsigned long long g_wait_limit_ns = kWaitLimitNs;
 int g_test_drop_a_load = -1;
 int g_smallm_enabled = 1;
 
+// K splits of the small-batch kernel.  Its time in microseconds, fitted to 1300 timed launches (CUDA graph over rotating weights;
+// K = 512..9216 x N = 1536..18432 x 1..128 rows x every split): up to half the SMs, consecutive launches run side by side and
+// only the chain from the grid-dependency wait to the exit counts; above that a launch starts on the SMs the one before leaves.
+// A further wave of CTAs repeats that start.  The exchange of partial sums grows with the rows; it is done by all CTAs at once.
+double smallm_cost(int m, int n, int k, int splits) {
+    const int sms = device_sm_count();
+    const int units = n / 128 * splits, waves = (units + sms - 1) / sms;
+    const double stages = (k / 128 + splits - 1) / splits, over = (units < sms ? units : sms) - sms / 2;
+    const double start = over <= 0 ? 1.4 : 2.5 + 0.0246 * over;
+    const double rows = (m + 15) / 16 * 16, step = 0.27 + (over > 0 ? 0.015 : 0.0) + (m > 64 ? 0.03 + (over > 0 ? 0.0024 * over : 0.0) : 0.0);
+    return start + waves * step * stages + (waves - 1) * 3.0 + (splits > 1 ? 0.1 + 0.02 * rows + 0.00012 * rows * rows : 0.0);
+}
+
+int choose_smallm_splits(int m, int n, int k) {
+    int best = 1;
+    for (int s : {2, 3, 4, 6, 8})
+        if (s <= k / 128 && smallm_cost(m, n, k, s) < smallm_cost(m, n, k, best)) best = s;
+    return best;
+}
+
 PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool allow_scratch = true,
                              size_t max_split_bytes = ~static_cast<size_t>(0)) {
     const int sms = device_sm_count();
@@ -844,9 +865,11 @@ PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool 
         // (a forced split larger than max_split_bytes is returned as it is: the no-allocation entry then refuses the call)
         if (legal) return o;
     }
+    // At most 128 rows: 128-column tiles, which the small-batch kernel shares; it may run fewer splits (exec_splits).
+    const bool small = m <= BM && allow_pairs && allow_scratch;
     PrefillConfig best{256, 1, 1, 0};
     double best_t = 1e30;
-    const int bns[2] = {256, 128};
+    const int bns[2] = {small ? 128 : 256, 128};
     const int ss[6] = {1, 2, 3, 4, 6, 8};
     for (int mt = 1; mt <= (allow_pairs ? 2 : 1); ++mt)
         for (int bi = 0; bi < 2; ++bi)
@@ -868,7 +891,7 @@ PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool 
                 }
                 // hybrid stream-K over the same tiling: whole waves as above, the remaining tiles' K-steps in equal
                 // shares, plus the fix-up pass over those tiles
-                if (s == 1 && allow_pairs && allow_scratch) {  // (the no-alloc entry, which passes allow_pairs = false, has no fix-up pass)
+                if (s == 1 && allow_pairs && allow_scratch && !small) {  // (the no-alloc entry, which passes allow_pairs = false, has no fix-up pass)
                     const long long tiles = static_cast<long long>(m_tiles) * (n / bn);
                     const StreamKPlan pl = streamk_plan(static_cast<int>(tiles), k_iters, sms);
                     const long long rem = tiles - pl.first_tile;
@@ -885,7 +908,16 @@ PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool 
                     }
                 }
             }
+    if (small) best.splits = std::max(best.splits, choose_smallm_splits(m, n, k));
     return best;
+}
+
+// The K splits that a plain problem of at most 128 rows runs with, in the small-batch kernel and, when that is switched off, in the
+// general one (so that both give the same bits); `c` is the planner's tiling, whose splits size the workspace and are no fewer.
+int exec_splits(const PrefillConfig &c, int m, int n, int k) {
+    const PrefillConfig &o = g_prefill_override;
+    if (m > BM || (o.bn == c.bn && o.splits == c.splits && o.mt == c.mt && o.stream_k == c.stream_k)) return c.splits;
+    return std::min(c.splits, choose_smallm_splits(m, n, k));
 }
 
 // Tensor map of the bf16 result [m, n] for the epilogue's TMA stores: boxes of 32 rows x 64 columns, 128-byte swizzle.
@@ -931,16 +963,19 @@ int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, PrefillParams 
 
 }  // namespace
 
-// SwiGLU can be fused into the tcgen05 kernel's epilogue when its tiling for the problem writes whole tiles as bf16.
 // whether the small-batch kernel runs a plain problem that the planner tiled as `c`
 static bool smallm_takes(const PrefillConfig &c, int m, int n, int k, int groupsize) {
     return g_smallm_enabled && g_test_drop_a_load < 0 && c.bn == 128 && c.mt == 1 && !c.stream_k &&
-           smallm_supported(m, n, k, groupsize, c.splits);
+           smallm_supported(m, n, k, groupsize, exec_splits(c, m, n, k));
 }
 
+// The small-batch kernel by itself, for a plain problem: no workspace.
+bool smallm_takes(int m, int n, int k, int groupsize) { return m <= BM && smallm_takes(choose_prefill(m, n, k), m, n, k, groupsize); }
+
+// SwiGLU can be fused into the tcgen05 kernel's epilogue when its tiling for the problem writes whole tiles as bf16.
 bool prefill_fuses_swiglu(int m, int n, int k) {
     const PrefillConfig c = choose_prefill(m, n, k);
-    if (c.splits == 1 && smallm_takes(c, m, n, k, 128)) return true;  // (its epilogue pairs the gate and up warps)
+    if (exec_splits(c, m, n, k) == 1 && smallm_takes(c, m, n, k, 128)) return true;  // (its epilogue pairs the gate and up warps)
     // (not the 128-column tiles of one M-tile: their two K-parity accumulators would have to be added first, and at those
     // batch sizes a second pass over the small output costs less than a longer epilogue)
     return c.splits == 1 && !c.stream_k && !(c.bn == 128 && c.mt == 1);
@@ -985,15 +1020,16 @@ int launch_prefill(const GemmArgs &a) {
     uint32_t *status = device_status_word();
     if (!status) return KILN_W4A16_ERR_CUDA;
     const bool fused = a.n_peers > 0 || a.mc_c;  // the peer-store epilogue needs whole tiles: no split-K, no stream-K
-    const PrefillConfig c = choose_prefill(a.m, a.n, a.k, true, !fused && !a.no_scratch);
-    // At most 128 rows in 128-column tiles: the kernel that keeps the dequantised weights in tensor memory (same tiling,
-    // same K splits and workspace, so everything the planner reports holds for it too)
-    const bool smallm = smallm_takes(c, a.m, a.n, a.k, a.groupsize) && !fused && (!a.swiglu || c.splits == 1) &&
-                        (a.lora_r == 0 || (a.lora_t && a.lora_b && prefill_fuses_lora(a.groupsize, a.lora_r)));
-    if (!smallm && a.swiglu && (fused || c.splits != 1 || c.stream_k || (c.bn == 128 && c.mt == 1)))
+    // At most 128 rows: the kernel that keeps the dequantised weights in tensor memory; its K splits need no workspace
+    if (!fused && a.m <= BM && (a.lora_r == 0 || (a.lora_t && a.lora_b && prefill_fuses_lora(a.groupsize, a.lora_r)))) {
+        const PrefillConfig sc = choose_prefill(a.m, a.n, a.k);
+        const int splits = exec_splits(sc, a.m, a.n, a.k);
+        if ((!a.swiglu || splits == 1) && smallm_takes(sc, a.m, a.n, a.k, a.groupsize)) return launch_smallm(a, splits);
+    }
+    PrefillConfig c = choose_prefill(a.m, a.n, a.k, true, !fused && !a.no_scratch);
+    c.splits = exec_splits(c, a.m, a.n, a.k);
+    if (a.swiglu && (fused || c.splits != 1 || c.stream_k || (c.bn == 128 && c.mt == 1)))
         return KILN_W4A16_ERR_KERN_SHAPE;  // (callers ask prefill_fuses_swiglu first)
-    if (smallm) return launch_smallm(a, c.splits);  // (the K splits of a tile are a cluster: no workspace)
-
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.k), static_cast<cuuint64_t>(a.m)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(a.k) * 2};

@@ -166,6 +166,7 @@ void set_wait_limit_ns(unsigned long long ns);
 unsigned long long current_wait_limit_ns();
 void set_smallm_enabled(int on);
 bool smallm_supported(int m, int n, int k, int groupsize, int splits);
+bool smallm_takes(int m, int n, int k, int groupsize);
 int launch_smallm(const GemmArgs &a, int splits);
 void set_test_drop_a_load(int k_step);
 void prefill_plan(int m, int n, int k, int out[4]);
