@@ -12,7 +12,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libkiln_w4a16.so")
-SOURCES = ["api.cu", "decode_w4a16.cu", "epilogue_w4a16.cu", "prefill_w4a16_umma.cu", "repack.cu", "smallm_w4a16_tmem.cu"]
+SOURCES = ["api.cu", "decode_w4a16.cu", "epilogue_w4a16.cu", "pair_w4a16_umma.cu", "prefill_w4a16_umma.cu", "repack.cu", "smallm_w4a16_tmem.cu"]
 NATIVE = os.path.join(HERE, "_native.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [

@@ -22,95 +22,13 @@
 #include <algorithm>
 #include <mutex>
 
-#include "w4a16_umma.cuh"
+#include "w4a16_prefill.cuh"
 
 namespace kiln {
 namespace {
 
-constexpr int BM = 128;
-constexpr int BK = 64;
 constexpr int kDequantWarp0 = 6;
-constexpr uint32_t kEpiWarpBytes = 4096;  // per epilogue warp: 32 rows x 64 columns of bf16, 128B-swizzled (four 1024-byte atoms)
 constexpr int kNumEpilogueThreads = 4 * 32;
-
-struct PrefillParams {
-    const uint4 *B;
-    const __half *S;
-    __nv_bfloat16 *C;
-    float *partial;  // fp32 [splits][m][n] when splits > 1
-    uint32_t *status;
-    int m, n, k;
-    int m_tiles, n_tiles, splits, k_iters;  // k_iters = k / 64
-    int per_column;
-    // fused all-gather epilogue: n_peers > 0 -> every finished tile row segment is stored to the row-major
-    // [m, ldc] buffer of each peer GPU (peer_c[i], plain peer-mapped pointers) at column offset col0
-    __nv_bfloat16 *peer_c[8];
-    int n_peers, ldc, col0;
-    int self_peer;  // index in peer_c of the buffer that lives on this GPU (written through the TMA store), or -1
-    int swiglu;     // columns hold gate and up interleaved in runs of 32; C is [m, n/2] = silu(gate) * up (whole tiles, KP == 1)
-    // LoRA delta as extra K-steps: the piece of work that starts a tile's K range appends lora_steps (1 or 2) 64-deep steps
-    // whose operands are bf16 tiles of t = scale * x * A^T [m, r] and of lora_b [n, r], both fetched by TMA (KS == 1 only)
-    int lora_steps;
-    // mc_c != nullptr: one multimem.st per piece to the group's multicast address instead (the switch replicates
-    // the store into every GPU's buffer, this GPU's included, so each tile leaves this GPU once)
-    __nv_bfloat16 *mc_c;
-    int stream_k;     // 1: whole waves of tiles round-robin, then the remaining tiles' (tile, K-step) space in equal shares
-    int sk_first_tile;  // stream-K: tiles below this index are dealt whole (a multiple of the grid size)
-    int sk_ctas;        // stream-K: CTAs that share the remaining tiles (<= grid size)
-    int tile_elems;   // rows * columns of one output tile (stream-K slabs are tile-shaped)
-    unsigned long long wait_limit_ns;  // every bounded wait of the launch gives up after this long
-    int test_drop_a_load;  // test hook: the activation tile of this K-step (counted per CTA) is announced but never copied; -1 = off
-};
-
-// Hands a CTA its work.  Default: units (tile, K-split) dealt round-robin.  Stream-K (hybrid): the tiles that fill
-// whole waves of the grid are dealt round-robin as above; the flattened (tile, K-step) space of the remaining
-// tiles is cut into sk_ctas equal contiguous ranges, so no SM idles in a last partial wave; a range covers the
-// tail of one tile, whole tiles, and the head of another.  Whole tiles are written straight to C; the at most
-// two partial pieces of a CTA go to fp32 slabs 2*cta and 2*cta+1 of the workspace and are summed per tile, in
-// CTA order, by `streamk_fixup_kernel`.  No CTA waits for another.
-struct WorkIter {
-    int mode, u, units, stride, splits, m_tiles, k_iters, first_tile;
-    long long cur, begin, end;
-    __device__ WorkIter(const PrefillParams &p)
-        : mode(p.stream_k), u(blockIdx.x), units(p.m_tiles * p.n_tiles * p.splits), stride(gridDim.x), splits(p.splits),
-          m_tiles(p.m_tiles), k_iters(p.k_iters), first_tile(p.sk_first_tile) {
-        if (mode) {
-            units = first_tile;  // whole tiles of the full waves (splits == 1 in this mode)
-            const long long total = static_cast<long long>(p.m_tiles * p.n_tiles - first_tile) * p.k_iters;
-            const long long c = blockIdx.x, n = p.sk_ctas;
-            begin = cur = c < n ? total * c / n : 0;
-            end = c < n ? total * (c + 1) / n : 0;
-        } else {
-            begin = cur = end = 0;
-        }
-    }
-    // slab: -1 = the piece is a whole tile (or an ordinary split) and goes where `sp` says; >= 0 = stream-K slab index
-    __device__ bool next(int &mt, int &nt, int &sp, int &ki0, int &ki1, int &slab) {
-        if (u < units) {
-            sp = u % splits;
-            const int t = u / splits;
-            mt = t % m_tiles;
-            nt = t / m_tiles;
-            ki0 = static_cast<int>(static_cast<long long>(k_iters) * sp / splits);
-            ki1 = static_cast<int>(static_cast<long long>(k_iters) * (sp + 1) / splits);
-            slab = -1;
-            u += stride;
-            return true;
-        }
-        if (cur >= end) return false;
-        const int tr = static_cast<int>(cur / k_iters);  // tile within the remainder
-        ki0 = static_cast<int>(cur - static_cast<long long>(tr) * k_iters);
-        const long long left = end - cur;
-        ki1 = left < k_iters - ki0 ? ki0 + static_cast<int>(left) : k_iters;
-        const int t = first_tile + tr;
-        mt = t % m_tiles;
-        nt = t / m_tiles;
-        sp = 0;
-        slab = (ki0 == 0 && ki1 == k_iters) ? -1 : 2 * static_cast<int>(blockIdx.x) + (cur == begin ? 0 : 1);
-        cur += ki1 - ki0;
-        return true;
-    }
-};
 
 // MT = M-tiles of 128 rows that share one dequantised B stage.  With MT = 2 every weight is dequantised
 // once per 256 rows instead of once per 128, which halves the dequant work per MMA flop; the two
@@ -221,7 +139,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             pdl_wait();  // the activations may be the previous kernel's output
             uint32_t it = 0;
             bool ok = true;
-            WorkIter wi(p);
+            WorkIter wi(p, blockIdx.x, gridDim.x);
             while (ok && wi.next(mt, nt, sp, ki0, ki1, slab)) {
                 const int ki1e = ki1 + ((KS == 1 && ki0 == 0) ? p.lora_steps : 0);  // + the LoRA steps of the tile
                 for (int ki = ki0; ki < ki1e; ++ki, ++it) {
@@ -266,7 +184,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             const int q = (KP == 2 && warp != 1) ? 1 : 0;  // K-parity issuer: MMAs 2q, 2q+1 of every K-step, accumulator q
             uint32_t it = 0, tile = 0;
             bool ok = true;
-            WorkIter wi(p);
+            WorkIter wi(p, blockIdx.x, gridDim.x);
             for (; ok && wi.next(mt, nt, sp, ki0, ki1, slab); ++tile) {
                 // MT == 1: the two TMEM buffers alternate between tiles.  MT == 2: buffer h holds M-tile h of the pair.
                 const uint32_t acc0 = MT == 1 ? (tile & 1) : 0u, acc_ph = MT == 1 ? ((tile >> 1) & 1) : (tile & 1);
@@ -304,7 +222,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         pdl_wait();  // C (or the workspace) may still be read or written by the previous kernel
         uint32_t tile = 0;
         bool ok = true;
-        WorkIter wi(p);
+        WorkIter wi(p, blockIdx.x, gridDim.x);
         for (; ok && wi.next(mt, nt, sp, ki0, ki1, slab); ++tile) {
             const uint32_t acc0 = MT == 1 ? (tile & 1) : 0u, acc_ph = MT == 1 ? ((tile >> 1) & 1) : (tile & 1);
 #pragma unroll 1
@@ -572,7 +490,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         bool ok = true;
         int cur_group = -1;
         uint32_t s2[8];  // bf16x2 {s, s} for columns 8t + c of this warp's chunk
-        WorkIter wi(p);
+        WorkIter wi(p, blockIdx.x, gridDim.x);
         while (ok && wi.next(mt, nt, sp, ki0, ki1, slab)) {
             cur_group = -1;
             auto load_regs = [&](Regs &d, int ki) {
@@ -736,8 +654,8 @@ __global__ void splitk_reduce_kernel(const float *partial, __nv_bfloat16 *C, con
 // Stream-K fix-up: gridDim.y blocks per output tile of the remainder.  Recomputes which CTAs covered only a part of
 // the tile's K-steps (the same arithmetic as WorkIter), sums their slabs in CTA order and writes bf16.  A tile that
 // one CTA covered completely was already written by that CTA.
-__global__ void streamk_fixup_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n, int m_tiles,
-                                     int k_iters, int tile_rows, int bn, int ctas, long long total, int first_tile,
+__global__ void streamk_fixup_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n, int m_tiles, int n_tiles,
+                                     int group_m, int k_iters, int tile_rows, int bn, int ctas, long long total, int first_tile,
                                      int per_column) {
     pdl_launch_dependents();
     pdl_wait();  // the slabs come from the kernel launched just before
@@ -756,7 +674,8 @@ __global__ void streamk_fixup_kernel(const float *partial, __nv_bfloat16 *C, con
         if (ns < 40) slabs[ns++] = 2 * r + (a == g0 ? 0 : 1);
     }
     const int t = first_tile + tr;
-    const int mt = t % m_tiles, nt = t / m_tiles;
+    int mt, nt;
+    tile_of(t, m_tiles, n_tiles, group_m, mt, nt);
     const size_t tile_elems = static_cast<size_t>(tile_rows) * bn;
     const int vec_per_row = bn / 4;
     // gridDim.y blocks share a tile by rows
@@ -826,6 +745,12 @@ StreamKPlan streamk_plan(int tiles, int k_iters, int grid) {
     long long c = total / min_share;
     pl.ctas = static_cast<int>(c > grid ? grid : (c < 1 ? 1 : c));
     return pl;
+}
+
+// Rows of tiles in a band (tile_of): about 2048 rows of the problem, in bands of equal height.
+int band_rows(int m_tiles, int mt) {
+    const int most = 2048 / (BM * mt), bands = (m_tiles + most - 1) / most;
+    return (m_tiles + bands - 1) / bands;
 }
 
 PrefillConfig g_prefill_override{0, 0, 0, 0};
@@ -1075,6 +1000,7 @@ int launch_prefill(const GemmArgs &a) {
     p.m_tiles = (a.m + BM * c.mt - 1) / (BM * c.mt);
     p.n_tiles = a.n / c.bn;
     p.splits = c.splits;
+    p.group_m = band_rows(p.m_tiles, c.mt);
     p.k_iters = a.k / BK;
     p.per_column = a.groupsize == -1;
     p.n_peers = a.n_peers;
@@ -1106,14 +1032,18 @@ int launch_prefill(const GemmArgs &a) {
     p.wait_limit_ns = g_wait_limit_ns;
     p.test_drop_a_load = g_test_drop_a_load;
     p.tile_elems = BM * c.mt * c.bn;
-    const StreamKPlan plan = streamk_plan(p.m_tiles * p.n_tiles, p.k_iters, device_sm_count());
+    // 256 x 256 tiles run on CTA pairs (the fused all-gather and the give-up test hook stay on single CTAs)
+    const bool pair = c.mt == 2 && c.bn == 256 && !fused && g_test_drop_a_load < 0;
+    const StreamKPlan plan = streamk_plan(p.m_tiles * p.n_tiles, p.k_iters, pair ? device_sm_count() / 2 : device_sm_count());
     p.sk_first_tile = plan.first_tile;
     p.sk_ctas = plan.ctas;
     const size_t need = workspace_for(c, a.m, a.n);
     if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
 
     int rc;
-    if (c.mt == 2)
+    if (pair)
+        rc = launch_pair(a, p, tmap_c);
+    else if (c.mt == 2)
         rc = c.bn == 256 ? launch_bn<256, 2>(tmap, tmap_c, p, a.stream, pt, plb) : launch_bn<128, 2>(tmap, tmap_c, p, a.stream, pt, plb);
     else
         // (128-column tiles of one M-tile are bound by the MMA issue rate: two issuers, each with an accumulator of its own)
@@ -1142,7 +1072,7 @@ int launch_prefill(const GemmArgs &a) {
         const long long total = static_cast<long long>(rem) * p.k_iters;
         note_launch();
         rc = record_cuda_error(launch_pdl(streamk_fixup_kernel, dim3(rem, 16), dim3(256), a.stream, p.partial, p.C, p.S, a.m, a.n,
-                                          p.m_tiles, p.k_iters, BM * c.mt, c.bn, plan.ctas, total, plan.first_tile,
+                                          p.m_tiles, p.n_tiles, p.group_m, p.k_iters, BM * c.mt, c.bn, plan.ctas, total, plan.first_tile,
                                           static_cast<int>(p.per_column)));
     }
     return rc;
@@ -1271,6 +1201,7 @@ extern "C" kiln_w4a16_status_t kiln_w4a16_gemm_bf16_noalloc(const void *A, const
     p.m_tiles = (m + BM - 1) / BM;
     p.n_tiles = n / c.bn;
     p.splits = c.splits;
+    p.group_m = band_rows(p.m_tiles, 1);
     p.k_iters = k / BK;
     p.per_column = groupsize == -1;
     p.wait_limit_ns = g_wait_limit_ns;
