@@ -193,7 +193,7 @@ int validate_epilogue(const kiln_w4a16_epilogue_t *ep, int n) {
 
 // SwiGLU alone, fused by the tcgen05 kernel that would run it: the kernel choice is the plain GEMM's (from 17 rows)
 static bool ex_plain(const kiln_w4a16_epilogue_t *ep, int m, int n, int k) {
-    return ep->lora_rank == 0 && ep->swiglu && m <= 128 && prefill_fuses_swiglu(m, n, k);
+    return ep->lora_rank == 0 && ep->swiglu && m <= 128 && !prefill_swiglu_room(m, n, k);
 }
 
 size_t kiln_w4a16_workspace_bytes_ex(int m, int n, int k, const kiln_w4a16_epilogue_t *ep) {
@@ -205,7 +205,7 @@ size_t kiln_w4a16_workspace_bytes_ex(int m, int n, int k, const kiln_w4a16_epilo
         // tcgen05 kernel: SwiGLU is fused when the tiling writes whole tiles, the LoRA delta whenever the scales are grouped
         // (this call does not know the group size, so it reserves the composed path's buffer whenever there is a delta);
         // what is not fused is applied by a second pass over the bf16 GEMM result kept in the workspace
-        const bool composed = (ep->swiglu && !prefill_fuses_swiglu(m, n, k)) || ep->lora_rank;
+        const bool composed = (ep->swiglu && prefill_swiglu_room(m, n, k)) || ep->lora_rank;
         if (composed) need += align256(static_cast<size_t>(m) * n * 2);
         need += align256(prefill_workspace_bytes(m, n, k));
     }

@@ -21,23 +21,30 @@
 namespace kiln {
 namespace {
 
-constexpr int kTileM = 256, kTileN = 256;        // of the pair
-constexpr int kHalf = 128;                       // rows of A and columns of B per CTA
-constexpr int kOperandBytes = kHalf * BK * 2;    // 16 KB: one CTA's part of one operand of a stage
-constexpr int kStageBytes = 2 * kOperandBytes;
-constexpr int kStages = 5;
-constexpr int kTmemCols = 512;                   // two accumulators of 256 fp32 columns
+constexpr int kTileM = 256;                      // rows of a tile
+constexpr int kHalf = 128;                       // ... per CTA
+constexpr int kABytes = kHalf * BK * 2;          // a stage's activations, per CTA
 constexpr int kWordWarp = 6, kDequantWarp0 = 7, kTeams = 3, kTeamWarps = 4;
-constexpr int kWordBytes = kHalf * BK / 2, kScaleBytes = kHalf * 2, kWordSlotBytes = kWordBytes + kScaleBytes;
+constexpr int kThreads = (kDequantWarp0 + kTeams * kTeamWarps) * 32;
 // A dequant team asks for its next stage of words, kTeams further, knowing only its own last one: a parity wait tells neighbouring
 // phases apart and no more, so the previous user of a slot has to be the team itself.
 constexpr int kWordSlots = 6;
 static_assert(kWordSlots % kTeams == 0, "see above");
-constexpr int kThreads = (kDequantWarp0 + kTeams * kTeamWarps) * 32;
-constexpr int kBarrierBytes = 1024;  // (the staging tiles behind them are 1024-byte aligned)
-constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 4 * 2 * kEpiWarpBytes + kWordSlots * kWordSlotBytes + 1024;  // + alignment slack
-// D fp32, A/B bf16, both K-major, N = 256, M = 256
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTileN >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
+constexpr int kBarrierBytes = 1024;              // (the staging tiles behind them are 1024-byte aligned)
+
+// TN columns per tile, half of them dequantised by each CTA.
+template <int TN>
+struct Cfg {
+    static constexpr int kCols = TN / 2;                                  // columns of B per CTA
+    static constexpr int kBBytes = kCols * BK * 2, kStageBytes = kABytes + kBBytes;
+    static constexpr int kStages = TN == 256 ? 5 : 6;
+    static constexpr int kTmemCols = 2 * TN;                              // two accumulators
+    static constexpr int kWordBytes = kCols * BK / 2, kScaleBytes = kCols * 2, kWordSlotBytes = kWordBytes + 256;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 4 * 2 * kEpiWarpBytes + kWordSlots * kWordSlotBytes + 1024;  // + alignment slack
+    static constexpr int kBlocks = kCols / 64 * 4 / kTeamWarps;           // 512-byte packed blocks per dequant warp and stage
+    // D fp32, A/B bf16, both K-major, N = TN, M = 256
+    static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(TN >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
+};
 
 __device__ __forceinline__ void arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
@@ -48,12 +55,12 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
                  "l"(map), "r"(x), "r"(y), "r"(cluster_bar)
                  : "memory");
 }
-__device__ __forceinline__ void umma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(accumulate)
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // arrives at the barrier at this offset in both CTAs when the MMAs issued so far are done
@@ -108,10 +115,13 @@ __device__ __forceinline__ void dequant_block(const uint4 &w, const uint32_t (&s
     }
 }
 
+template <int TN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
-                  const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_t, const __grid_constant__ CUtensorMap tmap_lb,
-                  const __grid_constant__ PrefillParams p) {
+                  const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_t,
+                  const __grid_constant__ CUtensorMap tmap_lb, const __grid_constant__ PrefillParams p) {
+    using C = Cfg<TN>;
+    constexpr int kStages = C::kStages, kStageBytes = C::kStageBytes, kCols = C::kCols;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -149,7 +159,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     if (warp == 1) {  // (both CTAs of the pair take part)
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(tmem_ptr_slot))),
-                     "r"(static_cast<uint32_t>(kTmemCols))
+                     "r"(static_cast<uint32_t>(C::kTmemCols))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -176,10 +186,10 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     if (!(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0x100u | s, p.wait_limit_ns))) break;
                     const uint32_t leader_full = map_to_cta(full(s), 0), dst = smem_base + s * kStageBytes;
                     const bool lora = ki >= ki1;  // both operand tiles come by TMA (rows past m, columns past r read zero)
-                    if (rank == 0) mbar_arrive_expect_tx(full(s), (lora ? 4 : 2) * kOperandBytes);
+                    if (rank == 0) mbar_arrive_expect_tx(full(s), 2 * (lora ? kStageBytes : kABytes));
                     if (lora) {
                         tma_load_2d_pair(dst, &tmap_t, (ki - ki1) * BK, mt * kTileM + rank * kHalf, leader_full);
-                        tma_load_2d_pair(dst + kOperandBytes, &tmap_lb, (ki - ki1) * BK, nt * kTileN + rank * kHalf, leader_full);
+                        tma_load_2d_pair(dst + kABytes, &tmap_lb, (ki - ki1) * BK, nt * TN + rank * kCols, leader_full);
                     } else {
                         tma_load_2d_pair(dst, &tmap_a, ki * BK, mt * kTileM + rank * kHalf, leader_full);
                     }
@@ -204,10 +214,10 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 for (int ki = ki0; ki < ki1e; ++ki) {
                     if (!ready && !(ok = mbar_wait(full(s), ph, abort_flag, p.status, 0x300u | s, p.wait_limit_ns))) break;
                     tc_fence_after();
-                    const uint64_t a_desc = make_smem_desc(smem_base + s * kStageBytes), b_desc = make_smem_desc(smem_base + s * kStageBytes + kOperandBytes);
+                    const uint64_t a_desc = make_smem_desc(smem_base + s * kStageBytes), b_desc = make_smem_desc(smem_base + s * kStageBytes + kABytes);
                     if (issue) {
 #pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) umma_pair(tmem_base + acc * kTileN, a_desc + 2 * j, b_desc + 2 * j, (ki > ki0 || j > 0) ? 1u : 0u);
+                        for (int j = 0; j < BK / 16; ++j) umma_pair(tmem_base + acc * TN, a_desc + 2 * j, b_desc + 2 * j, C::kIdesc, (ki > ki0 || j > 0) ? 1u : 0u);
                         umma_commit_pair(empty(s));
                         if (ki == ki1e - 1) umma_commit_pair(tmem_full(acc));
                     }
@@ -230,8 +240,8 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             const uint32_t acc = tile & 1, acc_ph = (tile >> 1) & 1;
             if (!(ok = mbar_wait(tmem_full(acc), acc_ph, abort_flag, p.status, 0x500u | acc, p.wait_limit_ns))) break;
             tc_fence_after();
-            const int row_in_tile = rank * kHalf + quarter * 32 + lane, row = mt * kTileM + row_in_tile;
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kTileN;
+            const int row = mt * kTileM + rank * kHalf + quarter * 32 + lane;
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * TN;
             const uint32_t leader_empty = map_to_cta(tmem_empty(acc), 0);
             auto release = [&] {  // every column of the accumulator is in registers or shared memory
                 tc_fence_before();
@@ -239,23 +249,32 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (lane == 0) arrive_cluster(leader_empty);
             };
             if (slab >= 0 || p.splits > 1) {
-                // fp32: a stream-K piece goes to a tile-shaped slab with all its rows (rows past m hold zeros), a K split to its slab of C
-                float *dst = slab >= 0 ? p.partial + static_cast<size_t>(slab) * p.tile_elems + static_cast<size_t>(row_in_tile) * kTileN
-                                       : p.partial + (static_cast<size_t>(sp) * p.m + row) * p.n + nt * kTileN;
-                const bool live = slab >= 0 || row < p.m;
+                // fp32 piece of a split tile, 32 x 32 at a time through a swizzled staging tile and TMA: a stream-K piece to its
+                // tile-shaped slab, a K split to its slab of C (rows past m are clipped)
 #pragma unroll 1
-                for (int q = 0; q < kTileN / 32; ++q) {
+                for (int q = 0; q < TN / 32; ++q) {
+                    const uint32_t stage = epi_tma0 + static_cast<uint32_t>(q & 1) * kEpiWarpBytes;
                     uint32_t r[32];
                     tmem_ld_32x32b_x32(t_row + q * 32, r);
                     tmem_ld_wait();
-                    if (live) {
-                        float4 *d4 = reinterpret_cast<float4 *>(dst + q * 32);
 #pragma unroll
-                        for (int v = 0; v < 8; ++v)
-                            d4[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+                    for (int v = 0; v < 8; ++v)
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * 128 + ((v ^ (lane & 7)) << 4)), "r"(r[4 * v]),
+                                     "r"(r[4 * v + 1]), "r"(r[4 * v + 2]), "r"(r[4 * v + 3])
+                                     : "memory");
+                    if (q == TN / 32 - 1) release();
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (slab >= 0)
+                            tma_store_3d(&tmap_p, stage, q * 32, rank * kHalf + quarter * 32, slab);
+                        else
+                            tma_store_3d(&tmap_p, stage, nt * TN + q * 32, mt * kTileM + rank * kHalf + quarter * 32, sp);
+                        bulk_commit_group();
+                        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the other staging tile has been read
                     }
+                    __syncwarp();
                 }
-                release();
                 continue;
             }
             uint32_t ra[32], rb[32];
@@ -263,9 +282,9 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             tmem_ld_32x32b_x32(t_row + 32, rb);
             if (p.swiglu) {
                 // a 64-column run is 32 gate columns and their 32 up columns, i.e. the two register buffers of a round
-                __nv_bfloat16 *crow = p.C + static_cast<size_t>(row) * (p.n >> 1) + ((nt * kTileN) >> 1);
+                __nv_bfloat16 *crow = p.C + static_cast<size_t>(row) * (p.n >> 1) + ((nt * TN) >> 1);
 #pragma unroll 1
-                for (int pp = 0; pp < kTileN / 64; ++pp) {
+                for (int pp = 0; pp < TN / 64; ++pp) {
                     tmem_ld_wait();
                     uint4 *dst = reinterpret_cast<uint4 *>(crow + pp * 32);
 #pragma unroll
@@ -277,7 +296,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                             float ga = __uint_as_float(ra[2 * e]), gb = __uint_as_float(ra[2 * e + 1]);
                             float ua = __uint_as_float(rb[2 * e]), ub = __uint_as_float(rb[2 * e + 1]);
                             if (p.per_column) {
-                                const int pg = scale_single_pos(nt * kTileN + pp * 64 + 2 * e), pu = scale_single_pos(nt * kTileN + pp * 64 + 32 + 2 * e);
+                                const int pg = scale_single_pos(nt * TN + pp * 64 + 2 * e), pu = scale_single_pos(nt * TN + pp * 64 + 32 + 2 * e);
                                 ga *= __half2float(p.S[pg]);
                                 gb *= __half2float(p.S[pg + 1]);
                                 ua *= __half2float(p.S[pu]);
@@ -288,7 +307,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                         }
                         if (row < p.m) dst[v] = make_uint4(o[0], o[1], o[2], o[3]);
                     }
-                    if (pp + 1 < kTileN / 64) {
+                    if (pp + 1 < TN / 64) {
                         tmem_ld_32x32b_x32(t_row + (pp + 1) * 64, ra);
                         tmem_ld_32x32b_x32(t_row + (pp + 1) * 64 + 32, rb);
                     } else {
@@ -298,12 +317,12 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 continue;
             }
 #pragma unroll 1
-            for (int pp = 0; pp < kTileN / 64; ++pp) {
+            for (int pp = 0; pp < TN / 64; ++pp) {
                 const uint32_t epi_tma = epi_tma0 + static_cast<uint32_t>(pp & 1) * kEpiWarpBytes;
                 tmem_ld_wait();
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    const int col = nt * kTileN + pp * 64 + half * 32;
+                    const int col = nt * TN + pp * 64 + half * 32;
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
                         uint32_t o[4];
@@ -325,7 +344,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                                      : "memory");
                     }
                 }
-                if (pp + 1 < kTileN / 64) {
+                if (pp + 1 < TN / 64) {
                     tmem_ld_32x32b_x32(t_row + (pp + 1) * 64, ra);
                     tmem_ld_32x32b_x32(t_row + (pp + 1) * 64 + 32, rb);
                 } else {
@@ -334,7 +353,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {  // (rows past m are clipped by the tensor map)
-                    tma_store_2d(&tmap_c, epi_tma, nt * kTileN + pp * 64, mt * kTileM + rank * kHalf + quarter * 32);
+                    tma_store_2d(&tmap_c, epi_tma, nt * TN + pp * 64, mt * kTileM + rank * kHalf + quarter * 32);
                     bulk_commit_group();
                     // the other tile, written two rounds ago, has been read
                     asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -350,16 +369,16 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             int s = 0;
             uint32_t ph = 1;
             while (ok && wi.next(mt, nt, sp, ki0, ki1, slab)) {
-                const int ki1e = ki1 + (ki0 == 0 ? p.lora_steps : 0), col = nt * kTileN + rank * kHalf;
+                const int ki1e = ki1 + (ki0 == 0 ? p.lora_steps : 0), col = nt * TN + rank * kCols;
                 for (int ki = ki0; ki < ki1e; ++ki) {
                     if (!(ok = mbar_wait(word_empty(s), ph, abort_flag, p.status, 0x800u | s, p.wait_limit_ns))) break;
-                    const uint32_t dst = word_base + s * kWordSlotBytes;
+                    const uint32_t dst = word_base + s * C::kWordSlotBytes;
                     if (ki >= ki1) {  // a LoRA step has no words; its slot passes through the ring empty
                         mbar_arrive(word_full(s));
                     } else {
-                        mbar_arrive_expect_tx(word_full(s), kWordBytes + (p.per_column ? 0 : kScaleBytes));
+                        mbar_arrive_expect_tx(word_full(s), C::kWordBytes + (p.per_column ? 0 : C::kScaleBytes));
                         tma_load_2d(dst, &tmap_w, 2 * col, ki * (BK / 16), word_full(s));
-                        if (!p.per_column) tma_load_2d(dst + kWordBytes, &tmap_s, col, ki >> 1, word_full(s));
+                        if (!p.per_column) tma_load_2d(dst + C::kWordBytes, &tmap_s, col, ki >> 1, word_full(s));
                     }
                     if (++s == kWordSlots) {
                         s = 0;
@@ -372,10 +391,11 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // ---------------- dequant: this CTA's 128 columns, packed int4 -> bf16 B tile ----------------
         const int team = (warp - kDequantWarp0) % kTeams, dw = (warp - kDequantWarp0) / kTeams;  // warp `dw` of team `team`
         const int qd = lane & 3, c = lane >> 2;
-        const int ch = dw & 1, kt0 = dw >> 1;  // 64-column chunk of the CTA's two; 16-row K tiles kt0 and kt0 + 2 of a stage
+        // 64-column chunk and first 16-row K tile of a stage: two chunks, K tiles kt0 and kt0 + 2, or one chunk and one K tile
+        const int ch = TN == 256 ? dw & 1 : 0, kt0 = TN == 256 ? dw >> 1 : dw;
         // row (= column of B) 64 ch + 8t + c, 128 B per row; 16-byte chunk (2 kt + half) ^ c
-        const uint32_t row0 = smem_base + kOperandBytes + static_cast<uint32_t>(ch * 64 + c) * 128u + 4u * qd;
-        const uint32_t words = word_base + kt0 * 1024 + ch * 512 + lane * 16, scales = word_base + kWordBytes + ch * 128 + c * 16;
+        const uint32_t row0 = smem_base + kABytes + static_cast<uint32_t>(ch * 64 + c) * 128u + 4u * qd;
+        const uint32_t words = word_base + kt0 * (kCols * 8) + ch * 512 + lane * 16, scales = word_base + C::kWordBytes + ch * 128 + c * 16;
         const uint32_t leader_full0 = map_to_cta(full(0), 0);
         int skip = team;  // steps until this team's next one
         int s = team, ws = team;
@@ -386,12 +406,12 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             int ki = ki0 + skip;
             for (; ki < ki1e; ki += kTeams) {
                 if (!w_ready && !(ok = mbar_wait(word_full(ws), wph, abort_flag, p.status, 0x900u | ws, p.wait_limit_ns))) break;
-                uint4 w[2], sc = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);  // (per-column scales come in the epilogue)
+                uint4 w[C::kBlocks], sc = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);  // (per-column scales come in the epilogue)
                 uint32_t s2[8];
                 if (ki < ki1) {
-                    w[0] = lds_v4(words + ws * kWordSlotBytes);
-                    w[1] = lds_v4(words + ws * kWordSlotBytes + 2 * 1024);
-                    if (!p.per_column) sc = lds_v4(scales + ws * kWordSlotBytes);
+#pragma unroll
+                    for (int b = 0; b < C::kBlocks; ++b) w[b] = lds_v4(words + ws * C::kWordSlotBytes + b * (2 * kCols * 8));
+                    if (!p.per_column) sc = lds_v4(scales + ws * C::kWordSlotBytes);
                     scale_pairs(sc, s2);
                 }
                 __syncwarp();
@@ -399,7 +419,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (!s_ready && !(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0x600u | s, p.wait_limit_ns))) break;
                 if (ki < ki1) {
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
+                    for (int b = 0; b < C::kBlocks; ++b) {
                         const int kt = kt0 + 2 * b;
                         dequant_block(w[b], s2, row0 + s * kStageBytes, static_cast<uint32_t>((2 * kt) ^ c) << 4, static_cast<uint32_t>((2 * kt + 1) ^ c) << 4);
                     }
@@ -429,13 +449,17 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     cluster_sync_all();  // nothing of the pair is in flight any more: MMAs, arrivals, tensor memory
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(kTmemCols)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(C::kTmemCols)) : "memory");
     }
 }
 
 }  // namespace
 
-int launch_pair(const GemmArgs &a, PrefillParams p, const CUtensorMap &tmap_c) {
+// Where the MMAs need 512 cycles per 64 K of a tile of 256 columns, the kernel takes about 540 (16384 x 9216 x 9216: 1367 TFLOP/s at
+// the 1.17 GHz that the power cap leaves; single CTAs 1056).  Writing the dequantised weight out first and feeding both operands by
+// TMA reaches 515 cycles, at 1.10 GHz: the bytes through L2 cost more power than the arithmetic saves (2380 us against 2036).
+// Tiles of 128 columns are for problems that have too few of the wide ones (per 64 K 0.19 us against 0.28).
+int launch_pair(const GemmArgs &a, PrefillParams p, int tile_n, const CUtensorMap &tmap_c, const CUtensorMap &tmap_p) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return KILN_W4A16_ERR_CUDA;
     auto encode = [&](CUtensorMap *map, CUtensorMapDataType type, int elem, const void *ptr, long long cols, int rows, int box_cols, int box_rows,
@@ -445,36 +469,41 @@ int launch_pair(const GemmArgs &a, PrefillParams p, const CUtensorMap &tmap_c) {
         return enc(map, type, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
-    auto operand = [&](CUtensorMap *map, const void *ptr, int cols, int rows) {
-        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, cols, rows, BK, kHalf, CU_TENSOR_MAP_SWIZZLE_128B);
+    auto operand = [&](CUtensorMap *map, const void *ptr, int cols, int rows, int box_rows) {
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, cols, rows, BK, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
     };
+    const int cols = tile_n / 2;  // columns per CTA
     CUtensorMap tmap_a, tmap_w, tmap_s, tmap_t, tmap_lb;
-    if (!operand(&tmap_a, a.A, a.k, a.m) ||
-        !encode(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.B, 2ll * a.n, a.k / 16, 2 * kHalf, BK / 16, CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (!operand(&tmap_a, a.A, a.k, a.m, kHalf) ||
+        !encode(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.B, 2ll * a.n, a.k / 16, 2 * cols, BK / 16, CU_TENSOR_MAP_SWIZZLE_NONE))
         return KILN_W4A16_ERR_CUDA;
     tmap_s = tmap_w;  // (unused with per-column scales)
-    if (!p.per_column && !encode(&tmap_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, a.S, a.n, a.k / 128, kHalf, 1, CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (!p.per_column && !encode(&tmap_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, a.S, a.n, a.k / 128, cols, 1, CU_TENSOR_MAP_SWIZZLE_NONE))
         return KILN_W4A16_ERR_CUDA;
     tmap_t = tmap_lb = tmap_a;  // (unused without a LoRA delta)
-    if (p.lora_steps > 0 && (!operand(&tmap_t, a.lora_t, a.lora_r, a.m) || !operand(&tmap_lb, a.lora_b, a.lora_r, a.n))) return KILN_W4A16_ERR_CUDA;
-    static bool attr_set[64] = {};
+    if (p.lora_steps > 0 && (!operand(&tmap_t, a.lora_t, a.lora_r, a.m, kHalf) || !operand(&tmap_lb, a.lora_b, a.lora_r, a.n, cols)))
+        return KILN_W4A16_ERR_CUDA;
+    const bool wide = tile_n == 256;
+    const auto kernel = wide ? w4a16_pair_kernel<256> : w4a16_pair_kernel<128>;
+    const int smem = wide ? Cfg<256>::kSmemBytes : Cfg<128>::kSmemBytes;
+    static bool attr_set[2][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 64 && !attr_set[dev]) {
-        if (int rc = record_cuda_error(cudaFuncSetAttribute(w4a16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes))) return rc;
-        attr_set[dev] = true;
+    if (dev < 64 && !attr_set[wide][dev]) {
+        if (int rc = record_cuda_error(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return rc;
+        attr_set[wide][dev] = true;
     }
     const int units = p.m_tiles * p.n_tiles * p.splits, pairs = device_sm_count() / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (p.stream_k || units > pairs ? pairs : units));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = a.stream;
     cudaLaunchAttribute attr = pdl_attribute();
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     note_launch();
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, w4a16_pair_kernel, tmap_a, tmap_w, tmap_s, tmap_c, tmap_t, tmap_lb, p));
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, tmap_a, tmap_w, tmap_s, tmap_c, tmap_p, tmap_t, tmap_lb, p));
 }
 
 }  // namespace kiln

@@ -82,7 +82,8 @@ struct DequantRegs {
 template <int BN, int MT, int DW, int DG, int KP, int KS, int AR>
 __global__ void __launch_bounds__((6 + DW + ((MT == 2 || KP == 2) ? 1 : 0)) * 32, 1)
 w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_c,
-                     const __grid_constant__ CUtensorMap tmap_t, const __grid_constant__ CUtensorMap tmap_lb, const PrefillParams p) {
+                     const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_t,
+                     const __grid_constant__ CUtensorMap tmap_lb, const PrefillParams p) {
     using C = Cfg<BN, MT, DW, DG, KP, KS, AR>;
     using Regs = DequantRegs<C::kBlocksPerWarp>;
     extern __shared__ uint8_t smem_raw[];
@@ -249,48 +250,6 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 const uint32_t epi_tma0 = epi_base + static_cast<uint32_t>(warp - 2) * (2 * kEpiWarpBytes);  // 1024-byte aligned swizzle atoms
                 const int x0_out = (p.n_peers > 0 ? p.col0 : 0) + nt * BN;  // first column of the tile in the output buffer
                 uint32_t ra[32], rb[32];
-                if (KP == 1 && p.swiglu) {
-                    // SwiGLU (kiln-model/src/forward.rs:2769-2839 as one GEMM): a 64-column run of the tile is 32 gate columns and
-                    // their 32 up columns, i.e. the two register buffers of a round; silu(gate) * up is computed in fp32 and
-                    // stored straight from registers (64 contiguous bytes per thread and round) while the next round's TMEM
-                    // loads are in flight
-                    __nv_bfloat16 *crow = p.C + static_cast<size_t>(row) * (p.n >> 1) + ((nt * BN) >> 1);
-                    tmem_ld_32x32b_x32(t_row, ra);
-                    tmem_ld_32x32b_x32(t_row + 32, rb);
-#pragma unroll 1
-                    for (int pp = 0; pp < BN / 64; ++pp) {
-                        tmem_ld_wait();
-                        uint4 *dst = reinterpret_cast<uint4 *>(crow + pp * 32);
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) {  // eight output columns at a time: their registers die with the store
-                            uint32_t o[4];
-#pragma unroll
-                            for (int e2 = 0; e2 < 4; ++e2) {
-                                const int e = 4 * v + e2;
-                                float ga = __uint_as_float(ra[2 * e]), gb = __uint_as_float(ra[2 * e + 1]);
-                                float ua = __uint_as_float(rb[2 * e]), ub = __uint_as_float(rb[2 * e + 1]);
-                                if (p.per_column) {
-                                    const int pg = scale_single_pos(nt * BN + pp * 64 + 2 * e), pu = scale_single_pos(nt * BN + pp * 64 + 32 + 2 * e);
-                                    ga *= __half2float(p.S[pg]);
-                                    gb *= __half2float(p.S[pg + 1]);
-                                    ua *= __half2float(p.S[pu]);
-                                    ub *= __half2float(p.S[pu + 1]);
-                                }
-                                __nv_bfloat162 b = __floats2bfloat162_rn(__fdividef(ga, 1.f + __expf(-ga)) * ua, __fdividef(gb, 1.f + __expf(-gb)) * ub);
-                                o[e2] = *reinterpret_cast<uint32_t *>(&b);
-                            }
-                            if (row < p.m) dst[v] = make_uint4(o[0], o[1], o[2], o[3]);
-                        }
-                        if (pp + 1 < BN / 64) {
-                            tmem_ld_32x32b_x32(t_row + (pp + 1) * 64, ra);
-                            tmem_ld_32x32b_x32(t_row + (pp + 1) * 64 + 32, rb);
-                        } else {
-                            tc_fence_before();
-                            mbar_arrive(tmem_empty(acc));
-                        }
-                    }
-                    continue;
-                }
                 if constexpr (KP == 2) {
                     // two accumulators (one per K-parity issuer) to add: 32 columns of each per half-round; the loads of the
                     // next half-round are in flight while a finished 64-column tile is stored
@@ -456,25 +415,25 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
                 }
                 tmem_ld_wait();
-                if (slab >= 0) {
-                    // stream-K piece: tile-shaped fp32 slab, all rows (rows past m hold zeros)
-                    float4 *dst = reinterpret_cast<float4 *>(p.partial + static_cast<size_t>(slab) * p.tile_elems +
-                                                             static_cast<size_t>(h * BM + quarter * 32 + lane) * BN + cc * 32);
+                // fp32 piece of a split tile, 32 x 32 at a time through a swizzled staging tile and TMA: a stream-K piece to its
+                // tile-shaped slab, a K split to its slab of C (rows past m are clipped)
+                const uint32_t stage = epi_base + static_cast<uint32_t>(warp - 2) * (2 * kEpiWarpBytes) + static_cast<uint32_t>(cc & 1) * kEpiWarpBytes;
 #pragma unroll
-                    for (int v = 0; v < 8; ++v)
-                        dst[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                             __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                } else if (row < p.m) {
-                    const int col = nt * BN + cc * 32;
-                    {
-                        float4 *dst = reinterpret_cast<float4 *>(
-                            p.partial + (static_cast<size_t>(sp) * p.m + row) * p.n + col);
-#pragma unroll
-                        for (int v = 0; v < 8; ++v)
-                            dst[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                                 __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                    }
+                for (int v = 0; v < 8; ++v)
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * 128 + ((v ^ (lane & 7)) << 4)), "r"(r[4 * v]), "r"(r[4 * v + 1]),
+                                 "r"(r[4 * v + 2]), "r"(r[4 * v + 3])
+                                 : "memory");
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (slab >= 0)
+                        tma_store_3d(&tmap_p, stage, cc * 32, h * BM + quarter * 32, slab);
+                    else
+                        tma_store_3d(&tmap_p, stage, nt * BN + cc * 32, (mt * MT + h) * BM + quarter * 32, sp);
+                    bulk_commit_group();
+                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the other staging tile has been read
                 }
+                __syncwarp();
             }
             tc_fence_before();
             mbar_arrive(tmem_empty(acc));
@@ -621,92 +580,94 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     }
 }
 
-// out[m][n] = bf16(sum_s partial[s][m][n]) (* per-column scale)
-__global__ void splitk_reduce_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n,
-                                     int splits, int per_column) {
-    pdl_launch_dependents();
-    pdl_wait();  // the partial sums come from the kernel launched just before
-    const size_t total4 = static_cast<size_t>(m) * n / 4;
-    const size_t slab4 = total4;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        float4 acc = reinterpret_cast<const float4 *>(partial)[i];
-        for (int s = 1; s < splits; ++s) {
-            const float4 v = reinterpret_cast<const float4 *>(partial)[i + s * slab4];
-            acc.x += v.x;
-            acc.y += v.y;
-            acc.z += v.z;
-            acc.w += v.w;
-        }
-        if (per_column) {
-            const int col = static_cast<int>((i * 4) % n);
-            const int p0 = scale_single_pos(col), p1 = scale_single_pos(col + 2);
-            acc.x *= __half2float(S[p0]);
-            acc.y *= __half2float(S[p0 + 1]);
-            acc.z *= __half2float(S[p1]);
-            acc.w *= __half2float(S[p1 + 1]);
-        }
-        __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
-        reinterpret_cast<uint2 *>(C)[i] = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+__device__ __forceinline__ uint2 finish4(float4 v, const __half *S, int col, int per_column) {
+    if (per_column) {
+        const int p0 = scale_single_pos(col), p1 = scale_single_pos(col + 2);
+        v.x *= __half2float(S[p0]);
+        v.y *= __half2float(S[p0 + 1]);
+        v.z *= __half2float(S[p1]);
+        v.w *= __half2float(S[p1 + 1]);
     }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+}
+__device__ __forceinline__ void add4(float4 &a, const float4 &v) {
+    a.x += v.x;
+    a.y += v.y;
+    a.z += v.z;
+    a.w += v.w;
 }
 
-// Stream-K fix-up: gridDim.y blocks per output tile of the remainder.  Recomputes which CTAs covered only a part of
-// the tile's K-steps (the same arithmetic as WorkIter), sums their slabs in CTA order and writes bf16.  A tile that
-// one CTA covered completely was already written by that CTA.
-__global__ void streamk_fixup_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n, int m_tiles, int n_tiles,
-                                     int group_m, int k_iters, int tile_rows, int bn, int ctas, long long total, int first_tile,
-                                     int per_column) {
+// out[m][n] = bf16(sum_s partial[s][m][n]) (* per-column scale).  Four sums per thread, whose loads (at most eight) are all in
+// flight at once: the kernel is a few round trips to L2 long and no more.  grid = ceil(m n / 1024), block = 256.
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n,
+                                                            int splits, int per_column) {
     pdl_launch_dependents();
+    const size_t slab4 = static_cast<size_t>(m) * n / 4, i = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;
+    pdl_wait();  // the partial sums come from the kernel launched just before
+    if (i >= slab4) return;
+    float4 v[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+        if (s < splits) v[s] = reinterpret_cast<const float4 *>(partial)[i + s * slab4];
+#pragma unroll
+    for (int s = 1; s < 8; ++s)
+        if (s < splits) add4(v[0], v[s]);
+    reinterpret_cast<uint2 *>(C)[i] = finish4(v[0], S, per_column ? static_cast<int>((i * 4) % n) : 0, per_column);
+}
+
+// Stream-K fix-up: finds out which workers covered only a part of the tile's K-steps (the same arithmetic as WorkIter), sums their
+// slabs in worker order and writes bf16.  A tile that one worker covered completely was already written by it.  Four sums per
+// thread.  (With sixteen blocks per tile and the slabs loaded one after another this pass took 20 us for six tiles.)
+// grid = (tiles of the remainder, tile elements / 1024), block = 256.
+__global__ void __launch_bounds__(256) streamk_fixup_kernel(const float *partial, __nv_bfloat16 *C, const __half *S, int m, int n, int m_tiles,
+                                                            int n_tiles, int group_m, int k_iters, int tile_rows, int bn, int ctas, long long total,
+                                                            int first_tile, int per_column) {
+    __shared__ int slabs[64];  // (a tile has at most 39 candidates)
+    __shared__ int count;
+    pdl_launch_dependents();
+    const int tr = blockIdx.x, lane = threadIdx.x;
+    if (threadIdx.x < 32) {
+        const long long t0 = static_cast<long long>(tr) * k_iters, t1 = t0 + k_iters;
+        const int r_lo = max(0, static_cast<int>(t0 * ctas / total) - 1), r_hi = min(ctas - 1, static_cast<int>(t1 * ctas / total) + 1);
+        int ns = 0;
+        for (int r0 = r_lo; r0 <= r_hi; r0 += 32) {
+            const int r = r0 + lane;
+            const long long g0 = total * r / ctas, g1 = total * (r + 1) / ctas;
+            const long long a = g0 > t0 ? g0 : t0, b = g1 < t1 ? g1 : t1;
+            const bool part = r <= r_hi && a < b, whole = part && a == t0 && b == t1;
+            const unsigned mask = __ballot_sync(0xFFFFFFFFu, part);
+            if (part) slabs[ns + __popc(mask & ((1u << lane) - 1))] = 2 * r + (a == g0 ? 0 : 1);
+            ns += __popc(mask);
+            if (__any_sync(0xFFFFFFFFu, whole)) {
+                ns = 0;
+                break;
+            }
+        }
+        if (lane == 0) count = ns;
+    }
+    __syncthreads();
+    const int ns = count;
     pdl_wait();  // the slabs come from the kernel launched just before
-    const int tr = blockIdx.x;
-    const long long t0 = static_cast<long long>(tr) * k_iters, t1 = t0 + k_iters;
-    int r_lo = static_cast<int>(t0 * ctas / total) - 1, r_hi = static_cast<int>(t1 * ctas / total) + 1;
-    if (r_lo < 0) r_lo = 0;
-    if (r_hi > ctas - 1) r_hi = ctas - 1;
-    int slabs[40];
-    int ns = 0;
-    for (int r = r_lo; r <= r_hi; ++r) {
-        const long long g0 = total * r / ctas, g1 = total * (r + 1) / ctas;
-        const long long a = g0 > t0 ? g0 : t0, b = g1 < t1 ? g1 : t1;
-        if (a >= b) continue;
-        if (a == t0 && b == t1) return;  // whole tile by one CTA: nothing to fix up
-        if (ns < 40) slabs[ns++] = 2 * r + (a == g0 ? 0 : 1);
-    }
-    const int t = first_tile + tr;
     int mt, nt;
-    tile_of(t, m_tiles, n_tiles, group_m, mt, nt);
+    tile_of(first_tile + tr, m_tiles, n_tiles, group_m, mt, nt);
+    const int vec_per_row = bn / 4, i = blockIdx.y * 256 + threadIdx.x;
+    const int rl = i / vec_per_row, cv = i % vec_per_row, row = mt * tile_rows + rl;
+    if (ns == 0 || row >= m) return;
+    const float *src = partial + static_cast<size_t>(rl) * bn + 4 * cv;
     const size_t tile_elems = static_cast<size_t>(tile_rows) * bn;
-    const int vec_per_row = bn / 4;
-    // gridDim.y blocks share a tile by rows
-    const int rows_per_block = (tile_rows + gridDim.y - 1) / gridDim.y;
-    const int r_begin = blockIdx.y * rows_per_block;
-    for (int i = threadIdx.x; i < rows_per_block * vec_per_row; i += blockDim.x) {
-        const int rl = r_begin + i / vec_per_row, cv = i % vec_per_row;
-        if (rl >= tile_rows) break;
-        const int row = mt * tile_rows + rl;
-        if (row >= m) continue;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 0; j < ns; ++j) {
-            const float4 v = *reinterpret_cast<const float4 *>(partial + slabs[j] * tile_elems +
-                                                               static_cast<size_t>(rl) * bn + 4 * cv);
-            acc.x += v.x;
-            acc.y += v.y;
-            acc.z += v.z;
-            acc.w += v.w;
-        }
-        const int col = nt * bn + 4 * cv;
-        if (per_column) {
-            const int p0 = scale_single_pos(col), p1 = scale_single_pos(col + 2);
-            acc.x *= __half2float(S[p0]);
-            acc.y *= __half2float(S[p0 + 1]);
-            acc.z *= __half2float(S[p1]);
-            acc.w *= __half2float(S[p1 + 1]);
-        }
-        __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
-        *reinterpret_cast<uint2 *>(C + static_cast<size_t>(row) * n + col) =
-            make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = 0; j0 < ns; j0 += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j0 + j < ns) v[j] = *reinterpret_cast<const float4 *>(src + slabs[j0 + j] * tile_elems);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j0 + j < ns) add4(acc, v[j]);
     }
+    const int col = nt * bn + 4 * cv;
+    *reinterpret_cast<uint2 *>(C + static_cast<size_t>(row) * n + col) = finish4(acc, S, col, per_column);
 }
 
 // ---- host -----------------------------------------------------------------------------------
@@ -715,21 +676,33 @@ struct PrefillConfig {
     int bn, splits, mt, stream_k;
 };
 
-// Cost model of one launch, least-squares fitted (mean error 6 %) to 1100 timed launches on B200: 5 projection shapes x
-// M = 64..8192 x every tiling the rule considers, each timed alone after an L2 flush.  Microseconds:
-//   launch + waves * (K-steps per unit * step + tile) [+ split-K: fixed + per MB of fp32 slab traffic]
-//   stream-K: launch + whole waves as above + share * step + 2 * tile + per MB of remainder tiles + per slab piece
-// `step` is the time of one 64-K step of a CTA, `tile` what a tile adds on top (epilogue that does not overlap, pipeline
-// restart); both depend on the columns per tile and the M-tiles per stage.  On the fitted set the model's choice is
-// within 0.3 % of the best measured tiling in total.
+// Cost model of one launch for everything that runs on CTA pairs or single CTAs above 128 rows, least-squares fitted (mean error 5 %)
+// to 2700 timed launches (CUDA graph over rotating weights; 12 shapes K = 512..9216 x N = 512..18432, M = 137..8192, every tiling
+// considered; on them the model's choice takes 0.9 % more time than the best one, geometric mean).  Microseconds:
+//   launch + waves * (K-steps per unit * step + tile) + work * (K-steps of all tiles per worker)
+//   + [K split: fixed + per MB of fp32 slab traffic]  or  [stream-K: 2 * tile + per MB of remainder tiles + per slab piece]
+// `work` is what a step costs beyond its time in a wave that leaves part of the chip idle: the power cap lowers the clock.
 struct TileCost {
-    double step, tile;
+    double step, tile, work;
 };
 TileCost tile_cost(int bn, int mt) {
-    if (mt == 2) return bn == 256 ? TileCost{0.584, 11.26} : TileCost{0.463, 3.83};
-    return bn == 256 ? TileCost{0.489, 4.85} : TileCost{0.301, 2.10};
+    if (mt == 2) return bn == 256 ? TileCost{0.276, 1.11, 0.074} : TileCost{0.186, 0.38, 0.069};
+    return TileCost{0.224, 0.61, 0.071};  // (bn = 128; 256-column tiles of one M-tile were never the fastest)
 }
-constexpr double kCostLaunch = 7.02, kCostSplitFixed = 4.21, kCostSplitPerMB = 0.332, kCostSkPerMB = 0.177, kCostSkPerPiece = 0.147;
+constexpr double kCostLaunch = 4.17, kCostSplitFixed = 1.14, kCostSplitPerMB = 0.212, kCostSkPerMB = 0.75, kCostSkPerPiece = 0.044;
+// Stream-K keeps every SM busy to the end, which the power cap takes back under a sustained load: it has to win by this factor.
+constexpr double kSkMargin = 1.04;
+
+// The model for single CTAs alone (the no-allocation entry, the fused all-gather), and for the K splits that size the workspace
+// up to 128 rows: launch + waves * (K-steps per unit * step + tile) [+ split-K: fixed + per MB of slab traffic].
+struct SingleCost {
+    double step, tile;
+};
+SingleCost single_cost(int bn, int mt) {
+    if (mt == 2) return bn == 256 ? SingleCost{0.584, 11.26} : SingleCost{0.463, 3.83};
+    return bn == 256 ? SingleCost{0.489, 4.85} : SingleCost{0.301, 2.10};
+}
+constexpr double kSingleLaunch = 7.02, kSingleSplitFixed = 4.21, kSingleSplitPerMB = 0.332;
 
 // Stream-K split of `tiles` tiles over `grid` CTAs: the tiles of the whole waves are dealt round-robin, the K-steps of
 // the rest go in equal shares to `ctas` CTAs.  A share is at least 8 K-steps and at least 1/36 of a tile, so that no tile
@@ -778,9 +751,69 @@ int choose_smallm_splits(int m, int n, int k) {
     return best;
 }
 
+// Tilings of single CTAs.
+PrefillConfig choose_single(int m, int n, int k, bool narrow, bool allow_pairs, bool allow_scratch, size_t max_split_bytes) {
+    const int sms = device_sm_count(), k_iters = k / BK;
+    PrefillConfig best{narrow ? 128 : 256, 1, 1, 0};
+    double best_t = 1e30;
+    for (int mt = 1; mt <= (allow_pairs && m > BM ? 2 : 1); ++mt)
+        for (int bn = narrow ? 128 : 256; bn >= 128; bn /= 2)
+            for (int s : {1, 2, 3, 4, 6, 8}) {
+                if (k_iters / s < 8) continue;
+                if (s > 1 && (!allow_scratch || static_cast<size_t>(s) * m * n * sizeof(float) > max_split_bytes)) continue;
+                const long long units = static_cast<long long>((m + BM * mt - 1) / (BM * mt)) * (n / bn) * s;
+                const double waves = static_cast<double>((units + sms - 1) / sms);
+                const SingleCost tc = single_cost(bn, mt);
+                double t = kSingleLaunch + waves * (static_cast<double>(k_iters) / s * tc.step + tc.tile);
+                if (s > 1) t += kSingleSplitFixed + kSingleSplitPerMB * (static_cast<double>(s) + 0.5) * m * static_cast<double>(n) * 4.0 / 1.0e6;
+                if (t < best_t) {
+                    best_t = t;
+                    best = PrefillConfig{bn, s, mt, 0};
+                }
+            }
+    return best;
+}
+
+// Tilings of CTA pairs (two M-tiles of 128 rows) and of single CTAs of one M-tile and 128 columns.
+PrefillConfig choose_any(int m, int n, int k, bool allow_scratch, bool pairs_only = false) {
+    const int k_iters = k / BK;
+    PrefillConfig best{128, 1, 1, 0};
+    double best_t = 1e30;
+    for (int mt = m > BM ? 2 : 1; mt >= (pairs_only ? 2 : 1); --mt)
+        for (int bn = mt == 2 ? 256 : 128; bn >= 128; bn /= 2) {
+            const TileCost tc = tile_cost(bn, mt);
+            const int workers = device_sm_count() / mt;
+            const long long tiles = static_cast<long long>((m + BM * mt - 1) / (BM * mt)) * (n / bn);
+            const double base = kCostLaunch + tc.work * static_cast<double>(tiles) * k_iters / workers;
+            for (int s : {1, 2, 3, 4, 6, 8}) {
+                if (s > 1 && (!allow_scratch || k_iters / s < 4)) continue;
+                const double waves = static_cast<double>((tiles * s + workers - 1) / workers);
+                double t = base + waves * (((k_iters + s - 1) / s) * tc.step + tc.tile);
+                if (s > 1) t += kCostSplitFixed + kCostSplitPerMB * (s + 0.5) * m * static_cast<double>(n) * 4.0 / 1.0e6;
+                if (t < best_t) {
+                    best_t = t;
+                    best = PrefillConfig{bn, s, mt, 0};
+                }
+            }
+            if (!allow_scratch || mt == 1) continue;
+            const StreamKPlan pl = streamk_plan(static_cast<int>(tiles), k_iters, workers);
+            const double rem = static_cast<double>(tiles - pl.first_tile);
+            if (rem == 0) continue;
+            const double share = rem * k_iters / pl.ctas;
+            const double t = kSkMargin * (base + static_cast<double>(pl.first_tile / workers) * (k_iters * tc.step + tc.tile) + share * tc.step + 2.0 * tc.tile +
+                                          kCostSkPerMB * rem * BM * mt * bn * 4.0 / 1.0e6 + kCostSkPerPiece * rem * k_iters / share);
+            if (t < best_t) {
+                best_t = t;
+                best = PrefillConfig{bn, 1, mt, 1};
+            }
+        }
+    return best;
+}
+
+// single: the launch has to run on single CTAs (fused all-gather).  !allow_pairs: one M-tile per CTA as well (the no-allocation entry,
+// which has no fix-up pass either).
 PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool allow_scratch = true,
-                             size_t max_split_bytes = ~static_cast<size_t>(0)) {
-    const int sms = device_sm_count();
+                             size_t max_split_bytes = ~static_cast<size_t>(0), bool single = false) {
     const int k_iters = k / BK;
     {  // tuning hook (kiln_w4a16_set_prefill_override): taken when it is legal for this problem, else the rule below
         const PrefillConfig &o = g_prefill_override;
@@ -790,51 +823,12 @@ PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool 
         // (a forced split larger than max_split_bytes is returned as it is: the no-allocation entry then refuses the call)
         if (legal) return o;
     }
+    if (!allow_pairs || single) return choose_single(m, n, k, false, allow_pairs, allow_scratch, max_split_bytes);
+    if (m > BM || !allow_scratch) return choose_any(m, n, k, allow_scratch);
     // At most 128 rows: 128-column tiles, which the small-batch kernel shares; it may run fewer splits (exec_splits).
-    const bool small = m <= BM && allow_pairs && allow_scratch;
-    PrefillConfig best{256, 1, 1, 0};
-    double best_t = 1e30;
-    const int bns[2] = {small ? 128 : 256, 128};
-    const int ss[6] = {1, 2, 3, 4, 6, 8};
-    for (int mt = 1; mt <= (allow_pairs ? 2 : 1); ++mt)
-        for (int bi = 0; bi < 2; ++bi)
-            for (int si = 0; si < 6; ++si) {
-                const int bn = bns[bi], s = ss[si];
-                if (k_iters / s < 8) continue;
-                if (s > 1 && !allow_scratch) continue;
-                if (s > 1 && static_cast<size_t>(s) * m * n * sizeof(float) > max_split_bytes) continue;
-                if (mt == 2 && m <= BM) continue;
-                const int m_tiles = (m + BM * mt - 1) / (BM * mt);
-                const long long units = static_cast<long long>(m_tiles) * (n / bn) * s;
-                const double waves = static_cast<double>((units + sms - 1) / sms);
-                const TileCost tc = tile_cost(bn, mt);
-                double t = kCostLaunch + waves * (static_cast<double>(k_iters) / s * tc.step + tc.tile);
-                if (s > 1) t += kCostSplitFixed + kCostSplitPerMB * (static_cast<double>(s) + 0.5) * m * static_cast<double>(n) * 4.0 / 1.0e6;
-                if (t < best_t) {
-                    best_t = t;
-                    best = PrefillConfig{bn, s, mt, 0};
-                }
-                // hybrid stream-K over the same tiling: whole waves as above, the remaining tiles' K-steps in equal
-                // shares, plus the fix-up pass over those tiles
-                if (s == 1 && allow_pairs && allow_scratch && !small) {  // (the no-alloc entry, which passes allow_pairs = false, has no fix-up pass)
-                    const long long tiles = static_cast<long long>(m_tiles) * (n / bn);
-                    const StreamKPlan pl = streamk_plan(static_cast<int>(tiles), k_iters, sms);
-                    const long long rem = tiles - pl.first_tile;
-                    if (rem > 0 && rem < sms) {
-                        const double share = static_cast<double>(rem) * k_iters / pl.ctas;
-                        const double tile_mb = BM * mt * bn * 4.0 / 1.0e6;
-                        const double tk = kCostLaunch + static_cast<double>(pl.first_tile / sms) * (k_iters * tc.step + tc.tile) +
-                                          share * tc.step + 2.0 * tc.tile + kCostSkPerMB * static_cast<double>(rem) * tile_mb +
-                                          kCostSkPerPiece * static_cast<double>(rem) * k_iters / share;
-                        if (tk < best_t) {
-                            best_t = tk;
-                            best = PrefillConfig{bn, 1, mt, 1};
-                        }
-                    }
-                }
-            }
-    if (small) best.splits = std::max(best.splits, choose_smallm_splits(m, n, k));
-    return best;
+    PrefillConfig c = choose_single(m, n, k, true, true, true, max_split_bytes);
+    c.splits = std::max(c.splits, choose_smallm_splits(m, n, k));
+    return c;
 }
 
 // The K splits that a plain problem of at most 128 rows runs with, in the small-batch kernel and, when that is switched off, in the
@@ -855,8 +849,17 @@ bool encode_c_map(EncodeTiledFn enc, CUtensorMap *map, void *c, int m, int n) {
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tensor map of the fp32 pieces of split tiles: [slabs][rows][cols], boxes of 32 x 32, 128-byte swizzle.
+bool encode_partial_map(EncodeTiledFn enc, CUtensorMap *map, float *partial, int cols, int rows, int slabs) {
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(slabs)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 4, static_cast<cuuint64_t>(cols) * rows * 4};
+    const cuuint32_t box[3] = {32, 32, 1}, estr[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, partial, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int BN, int MT = 1, int DW = 8, int DG = 2, int KP = 1, int KS = 1, int AR = BM>
-int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, PrefillParams p, cudaStream_t stream,
+int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, const CUtensorMap &tmap_p, PrefillParams p, cudaStream_t stream,
               const CUtensorMap *tmap_t = nullptr, const CUtensorMap *tmap_lb = nullptr) {
     using C = Cfg<BN, MT, DW, DG, KP, KS, AR>;
     p.k_iters /= KS;  // the kernel counts pipeline stages of KS atoms (k is a multiple of 128)
@@ -882,7 +885,7 @@ int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, PrefillParams 
     cfg.numAttrs = 1;
     static const CUtensorMap kNoMap = {};  // (never dereferenced when p.lora_steps == 0)
     if (!tmap_t || !tmap_lb || KS != 1) p.lora_steps = 0;
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, w4a16_prefill_kernel<BN, MT, DW, DG, KP, KS, AR>, tmap, tmap_c,
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, w4a16_prefill_kernel<BN, MT, DW, DG, KP, KS, AR>, tmap, tmap_c, tmap_p,
                                                 tmap_t ? *tmap_t : kNoMap, tmap_lb ? *tmap_lb : kNoMap, p));
 }
 
@@ -897,13 +900,24 @@ static bool smallm_takes(const PrefillConfig &c, int m, int n, int k, int groups
 // The small-batch kernel by itself, for a plain problem: no workspace.
 bool smallm_takes(int m, int n, int k, int groupsize) { return m <= BM && smallm_takes(choose_prefill(m, n, k), m, n, k, groupsize); }
 
-// SwiGLU can be fused into the tcgen05 kernel's epilogue when its tiling for the problem writes whole tiles as bf16.
-bool prefill_fuses_swiglu(int m, int n, int k) {
+// SwiGLU is fused into an epilogue that sees whole tiles: the small-batch kernel's without a K split, or the pair kernel's.  A second
+// pass over the bf16 result takes about 4 us, more than a K split saves a SwiGLU-sized projection, except for a long K and few columns.
+constexpr double kCostSwigluPass = 4.0;
+PrefillConfig swiglu_config(int m, int n, int k) {
     const PrefillConfig c = choose_prefill(m, n, k);
-    if (exec_splits(c, m, n, k) == 1 && smallm_takes(c, m, n, k, 128)) return true;  // (its epilogue pairs the gate and up warps)
-    // (not the 128-column tiles of one M-tile: their two K-parity accumulators would have to be added first, and at those
-    // batch sizes a second pass over the small output costs less than a longer epilogue)
-    return c.splits == 1 && !c.stream_k && !(c.bn == 128 && c.mt == 1);
+    return m <= BM || (c.splits == 1 && !c.stream_k && c.mt == 2) ? c : choose_any(m, n, k, false, true);
+}
+bool prefill_fuses_swiglu(int m, int n, int k) {
+    if (m > BM) return g_test_drop_a_load < 0;
+    const PrefillConfig c = choose_prefill(m, n, k);
+    const int splits = exec_splits(c, m, n, k);
+    if (!smallm_takes(c, m, n, k, 128)) return false;
+    return splits == 1 || (smallm_supported(m, n, k, 128, 1) && smallm_cost(m, n, k, 1) < smallm_cost(m, n, k, splits) + kCostSwigluPass);
+}
+// Whether a SwiGLU call reserves room for the bf16 result that a second pass would read: unless the planned tiling writes whole tiles.
+bool prefill_swiglu_room(int m, int n, int k) {
+    const PrefillConfig c = choose_prefill(m, n, k);
+    return m <= BM ? !(c.splits == 1 && smallm_takes(c, m, n, k, 128)) : !(c.splits == 1 && !c.stream_k && c.mt == 2 && c.bn == 256);
 }
 
 // The LoRA delta can ride in the tcgen05 kernel as extra K-steps unless the scales are per column (those are applied to
@@ -949,12 +963,11 @@ int launch_prefill(const GemmArgs &a) {
     if (!fused && a.m <= BM && (a.lora_r == 0 || (a.lora_t && a.lora_b && prefill_fuses_lora(a.groupsize, a.lora_r)))) {
         const PrefillConfig sc = choose_prefill(a.m, a.n, a.k);
         const int splits = exec_splits(sc, a.m, a.n, a.k);
-        if ((!a.swiglu || splits == 1) && smallm_takes(sc, a.m, a.n, a.k, a.groupsize)) return launch_smallm(a, splits);
+        if (smallm_takes(sc, a.m, a.n, a.k, a.groupsize)) return launch_smallm(a, a.swiglu ? 1 : splits);
     }
-    PrefillConfig c = choose_prefill(a.m, a.n, a.k, true, !fused && !a.no_scratch);
+    PrefillConfig c = a.swiglu ? swiglu_config(a.m, a.n, a.k) : choose_prefill(a.m, a.n, a.k, true, !fused && !a.no_scratch, ~static_cast<size_t>(0), fused);
     c.splits = exec_splits(c, a.m, a.n, a.k);
-    if (a.swiglu && (fused || c.splits != 1 || c.stream_k || (c.bn == 128 && c.mt == 1)))
-        return KILN_W4A16_ERR_KERN_SHAPE;  // (callers ask prefill_fuses_swiglu first)
+    if (a.swiglu && (fused || c.splits != 1 || c.stream_k || c.mt == 1)) return KILN_W4A16_ERR_KERN_SHAPE;  // (callers ask prefill_fuses_swiglu first)
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.k), static_cast<cuuint64_t>(a.m)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(a.k) * 2};
@@ -1032,37 +1045,39 @@ int launch_prefill(const GemmArgs &a) {
     p.wait_limit_ns = g_wait_limit_ns;
     p.test_drop_a_load = g_test_drop_a_load;
     p.tile_elems = BM * c.mt * c.bn;
-    // 256 x 256 tiles run on CTA pairs (the fused all-gather and the give-up test hook stay on single CTAs)
-    const bool pair = c.mt == 2 && c.bn == 256 && !fused && g_test_drop_a_load < 0;
+    // tiles of 256 rows run on CTA pairs (the fused all-gather and the give-up test hook stay on single CTAs)
+    const bool pair = c.mt == 2 && !fused && g_test_drop_a_load < 0;
     const StreamKPlan plan = streamk_plan(p.m_tiles * p.n_tiles, p.k_iters, pair ? device_sm_count() / 2 : device_sm_count());
     p.sk_first_tile = plan.first_tile;
     p.sk_ctas = plan.ctas;
     const size_t need = workspace_for(c, a.m, a.n);
     if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
 
+    CUtensorMap tmap_p = tmap_c;  // (unused when no tile is split)
+    if (c.stream_k ? !encode_partial_map(enc, &tmap_p, p.partial, c.bn, BM * c.mt, 2 * plan.ctas)
+                   : c.splits > 1 && !encode_partial_map(enc, &tmap_p, p.partial, a.n, a.m, c.splits))
+        return KILN_W4A16_ERR_CUDA;
+
     int rc;
     if (pair)
-        rc = launch_pair(a, p, tmap_c);
+        rc = launch_pair(a, p, c.bn, tmap_c, tmap_p);
     else if (c.mt == 2)
-        rc = c.bn == 256 ? launch_bn<256, 2>(tmap, tmap_c, p, a.stream, pt, plb) : launch_bn<128, 2>(tmap, tmap_c, p, a.stream, pt, plb);
+        rc = c.bn == 256 ? launch_bn<256, 2>(tmap, tmap_c, tmap_p, p, a.stream, pt, plb) : launch_bn<128, 2>(tmap, tmap_c, tmap_p, p, a.stream, pt, plb);
     else
         // (128-column tiles of one M-tile are bound by the MMA issue rate: two issuers, each with an accumulator of its own)
         // ... and 128-deep pipeline stages, which halve their barrier round trips per K (not with stream-K, whose fix-up pass
         // counts 64-deep steps, nor when a split would be left without a whole stage)
         if (c.bn == 256)
-            rc = launch_bn<256, 1>(tmap, tmap_c, p, a.stream, pt, plb);
+            rc = launch_bn<256, 1>(tmap, tmap_c, tmap_p, p, a.stream, pt, plb);
         else if (c.stream_k || a.k / 128 < c.splits || lora)  // (the LoRA steps are 64 deep)
-            rc = half_a ? launch_bn<128, 1, 8, 2, 2, 1, 64>(tmap, tmap_c, p, a.stream, pt, plb)
-                        : launch_bn<128, 1, 8, 2, 2, 1>(tmap, tmap_c, p, a.stream, pt, plb);
+            rc = half_a ? launch_bn<128, 1, 8, 2, 2, 1, 64>(tmap, tmap_c, tmap_p, p, a.stream, pt, plb)
+                        : launch_bn<128, 1, 8, 2, 2, 1>(tmap, tmap_c, tmap_p, p, a.stream, pt, plb);
         else
-            rc = half_a ? launch_bn<128, 1, 8, 2, 2, 2, 64>(tmap, tmap_c, p, a.stream)
-                        : launch_bn<128, 1, 8, 2, 2, 2>(tmap, tmap_c, p, a.stream);
+            rc = half_a ? launch_bn<128, 1, 8, 2, 2, 2, 64>(tmap, tmap_c, tmap_p, p, a.stream)
+                        : launch_bn<128, 1, 8, 2, 2, 2>(tmap, tmap_c, tmap_p, p, a.stream);
     if (rc) return rc;
     if (c.splits > 1) {
-        const size_t total4 = static_cast<size_t>(a.m) * a.n / 4;
-        int blocks = static_cast<int>((total4 + 255) / 256);
-        const int cap = device_sm_count() * 8;
-        if (blocks > cap) blocks = cap;
+        const unsigned blocks = static_cast<unsigned>((static_cast<size_t>(a.m) * a.n / 4 + 255) / 256);
         note_launch();
         rc = record_cuda_error(launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), a.stream, p.partial, p.C, p.S, a.m, a.n,
                                           c.splits, static_cast<int>(p.per_column)));
@@ -1071,7 +1086,7 @@ int launch_prefill(const GemmArgs &a) {
         const int rem = p.m_tiles * p.n_tiles - plan.first_tile;
         const long long total = static_cast<long long>(rem) * p.k_iters;
         note_launch();
-        rc = record_cuda_error(launch_pdl(streamk_fixup_kernel, dim3(rem, 16), dim3(256), a.stream, p.partial, p.C, p.S, a.m, a.n,
+        rc = record_cuda_error(launch_pdl(streamk_fixup_kernel, dim3(rem, BM * c.mt * c.bn / 1024), dim3(256), a.stream, p.partial, p.C, p.S, a.m, a.n,
                                           p.m_tiles, p.n_tiles, p.group_m, p.k_iters, BM * c.mt, c.bn, plan.ctas, total, plan.first_tile,
                                           static_cast<int>(p.per_column)));
     }
@@ -1210,13 +1225,12 @@ extern "C" kiln_w4a16_status_t kiln_w4a16_gemm_bf16_noalloc(const void *A, const
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     CUtensorMap tmap_c;
     if (!encode_c_map(enc, &tmap_c, C, m, n)) return KILN_W4A16_ERR_CUDA;
-    int rc = c.bn == 256 ? launch_bn<256>(tmap, tmap_c, p, cs) : launch_bn<128>(tmap, tmap_c, p, cs);
+    CUtensorMap tmap_p = tmap_c;  // (unused when no tile is split)
+    if (c.splits > 1 && !encode_partial_map(enc, &tmap_p, p.partial, n, m, c.splits)) return KILN_W4A16_ERR_CUDA;
+    int rc = c.bn == 256 ? launch_bn<256>(tmap, tmap_c, tmap_p, p, cs) : launch_bn<128>(tmap, tmap_c, tmap_p, p, cs);
     if (rc) return rc;
     if (c.splits > 1) {
-        const size_t total4 = static_cast<size_t>(m) * n / 4;
-        int blocks = static_cast<int>((total4 + 255) / 256);
-        const int cap = device_sm_count() * 8;
-        if (blocks > cap) blocks = cap;
+        const unsigned blocks = static_cast<unsigned>((static_cast<size_t>(m) * n / 4 + 255) / 256);
         note_launch();
         rc = record_cuda_error(launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), cs, p.partial, p.C, p.S, m, n, c.splits,
                                           static_cast<int>(p.per_column)));

@@ -172,6 +172,7 @@ void set_test_drop_a_load(int k_step);
 void prefill_plan(int m, int n, int k, int out[4]);
 bool prefill_supported(int m, int n, int k, int groupsize);
 bool prefill_fuses_swiglu(int m, int n, int k);
+bool prefill_swiglu_room(int m, int n, int k);
 int static_status_read_clear(cudaStream_t st, uint32_t *out);
 int decode_status_read_clear(cudaStream_t st, uint32_t *out);
 

@@ -23,7 +23,7 @@ struct PrefillParams {
     __nv_bfloat16 *peer_c[8];
     int n_peers, ldc, col0;
     int self_peer;  // index in peer_c of the buffer that lives on this GPU (written through the TMA store), or -1
-    int swiglu;     // columns hold gate and up interleaved in runs of 32; C is [m, n/2] = silu(gate) * up (whole tiles, KP == 1)
+    int swiglu;     // columns hold gate and up interleaved in runs of 32; C is [m, n/2] = silu(gate) * up (pair kernel, whole tiles)
     // LoRA delta as extra K-steps: the piece of work that starts a tile's K range appends lora_steps (1 or 2) 64-deep steps
     // whose operands are bf16 tiles of t = scale * x * A^T [m, r] and of lora_b [n, r], both fetched by TMA (KS == 1 only)
     int lora_steps;
@@ -49,10 +49,10 @@ __host__ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles
     mt = band * group_m + (r - nt * rows);
 }
 
-// Hands a CTA (or a CTA pair) its work.  Default: units (tile, K-split) dealt round-robin.  Stream-K (hybrid): the tiles that fill
-// whole waves of the grid are dealt round-robin as above; the flattened (tile, K-step) space of the remaining
-// tiles is cut into sk_ctas equal contiguous ranges, so no SM idles in a last partial wave; a range covers the
-// tail of one tile, whole tiles, and the head of another.  Whole tiles are written straight to C; the at most
+// Hands a CTA (or a CTA pair) its work.  Default: units (tile, K-split) dealt round-robin.  Stream-K (hybrid): the flattened (tile,
+// K-step) space of the tiles that do not fill a whole wave of the grid is cut into sk_ctas equal contiguous ranges, so no SM idles in
+// a last partial wave; a range covers the tail of one tile, whole tiles, and the head of another.  They come first, so that the
+// fp32 pieces drain under the main loops of the other tiles, which are dealt round-robin.  Whole tiles are written straight to C; the at most
 // two partial pieces of a CTA go to fp32 slabs 2*cta and 2*cta+1 of the workspace and are summed per tile, in
 // CTA order, by `streamk_fixup_kernel`.  No CTA waits for another.
 struct WorkIter {
@@ -74,31 +74,32 @@ struct WorkIter {
     }
     // slab: -1 = the piece is a whole tile (or an ordinary split) and goes where `sp` says; >= 0 = stream-K slab index
     __device__ bool next(int &mt, int &nt, int &sp, int &ki0, int &ki1, int &slab) {
-        if (u < units) {
-            sp = u % splits;
-            const int t = u / splits;
+        if (cur < end) {
+            const int tr = static_cast<int>(cur / k_iters);  // tile within the remainder
+            ki0 = static_cast<int>(cur - static_cast<long long>(tr) * k_iters);
+            const long long left = end - cur;
+            ki1 = left < k_iters - ki0 ? ki0 + static_cast<int>(left) : k_iters;
+            const int t = first_tile + tr;
             tile_of(t, m_tiles, n_tiles, group_m, mt, nt);
-            ki0 = static_cast<int>(static_cast<long long>(k_iters) * sp / splits);
-            ki1 = static_cast<int>(static_cast<long long>(k_iters) * (sp + 1) / splits);
-            slab = -1;
-            u += stride;
+            sp = 0;
+            slab = (ki0 == 0 && ki1 == k_iters) ? -1 : 2 * me + (cur == begin ? 0 : 1);
+            cur += ki1 - ki0;
             return true;
         }
-        if (cur >= end) return false;
-        const int tr = static_cast<int>(cur / k_iters);  // tile within the remainder
-        ki0 = static_cast<int>(cur - static_cast<long long>(tr) * k_iters);
-        const long long left = end - cur;
-        ki1 = left < k_iters - ki0 ? ki0 + static_cast<int>(left) : k_iters;
-        const int t = first_tile + tr;
+        if (u >= units) return false;
+        sp = u % splits;
+        const int t = u / splits;
         tile_of(t, m_tiles, n_tiles, group_m, mt, nt);
-        sp = 0;
-        slab = (ki0 == 0 && ki1 == k_iters) ? -1 : 2 * me + (cur == begin ? 0 : 1);
-        cur += ki1 - ki0;
+        ki0 = static_cast<int>(static_cast<long long>(k_iters) * sp / splits);
+        ki1 = static_cast<int>(static_cast<long long>(k_iters) * (sp + 1) / splits);
+        slab = -1;
+        u += stride;
         return true;
     }
 };
 
-// The kernel of CTA pairs: 256 x 256 tiles (m_tiles, n_tiles count those), no fused all-gather.
-int launch_pair(const GemmArgs &a, PrefillParams p, const CUtensorMap &tmap_c);
+// The kernel of CTA pairs: tiles of 256 x tile_n (128 or 256; m_tiles, n_tiles count those), no fused all-gather.  tmap_p: the fp32
+// pieces of split tiles (encode_partial_map).
+int launch_pair(const GemmArgs &a, PrefillParams p, int tile_n, const CUtensorMap &tmap_c, const CUtensorMap &tmap_p);
 
 }  // namespace kiln
