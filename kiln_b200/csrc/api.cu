@@ -76,11 +76,11 @@ static int validate(const GemmArgs &a) {
 // dequant and its MMAs for every further block; a tcgen05 tile dequantises once per 128 rows but pays a fixed cost per launch:
 //  * a plain GEMM (or SwiGLU where it is fused) of at most 128 rows runs on the kernel that keeps the weights in tensor memory
 //    (smallm_w4a16_tmem.cu), from 17 rows for every projection of more than 1024 columns (M = 17, decode / small-batch, us:
-//    2560 x 4096 7.6 / 5.0, 2560 x 18432 17.9 / 10.1, 9216 x 2560 12.7 / 8.9).  It is faster from 9 rows already, but the decode
-//    kernel multiplies the group scale in fp32 where the tcgen05 kernels round it to bf16, so it keeps the sizes it had;
+//    2560 x 4096 7.6 / 5.0, 2560 x 18432 17.9 / 10.1, 9216 x 2560 12.7 / 8.9).  Fewer rows have their group scales multiplied in
+//    fp32, where the tcgen05 kernels round them to bf16, and stay with the kernels that do (use_exact);
 //  * with a LoRA delta, which the decode kernel adds from an fp32 projection, the line is at 33 rows, or at 17 for projections of
 //    about 2560 columns (few column blocks for the decode kernel) whose activation matrix is at least 128 KB;
-//  * projections of 1024 columns or fewer (four to eight tiles) stay on the decode kernel up to 256 rows.
+//  * projections of 1024 columns or fewer (four to eight tiles) stay with those kernels up to 256 rows.
 // kiln_w4a16_set_prefill_min_m replaces the rule by a plain threshold.
 static bool use_prefill(int m, int n, int k, int groupsize, bool plain = false) {
     if (!prefill_supported(m, n, k, groupsize)) return false;
@@ -91,6 +91,21 @@ static bool use_prefill(int m, int n, int k, int groupsize, bool plain = false) 
     if (n <= 3072 && static_cast<long long>(m) * k * 2 >= (128LL << 10)) return m >= 17;
     return m >= 33;
 }
+
+// What use_prefill leaves to the kernels that apply the group scales, and add a LoRA delta, in fp32: 16 rows a CTA on the tensor-memory
+// kernel's variant of that arithmetic, or the decode kernel, whose 8-row blocks cost less while there is one of them.  (us, decode kernel /
+// this one: 9 x 2560 x 18432 11.4 / 9.7, 16 x 2560 x 4096 5.7 / 4.6, 64 x 2560 x 512 5.8 / 3.4, but 8 x 2560 x 18432 8.7 / 9.7.)
+//  * from 9 rows, two blocks of the decode kernel, always;
+//  * from 4 rows for a K of at most eight groups and at most 64 tiles: the decode kernel's splits have little to share there
+//    (8 x 512 x 4096 3.8 / 2.9; 8 x 1536 x 8192 5.0 / 4.6 but 4 x 1536 x 8192 4.1 / 4.6);
+//  * with a LoRA delta, which the decode kernel adds slowly, from 5 rows, or 3 for a narrow projection (5 x 2560 x 18432 with SwiGLU
+//    and rank 16 11.8 / 11.1, 3 x 9216 x 1024 rank 16 10.6 / 9.8, 4 x 2560 x 4096 rank 16 6.6 / 7.2).
+static bool use_exact(const GemmArgs &a) {
+    if (g_prefill_min_m.load(std::memory_order_relaxed) != kDefaultPrefillMinM || g_decode_override.cluster_k > 0) return false;
+    const bool wanted = a.lora_r > 0 ? a.m >= 5 || (a.m >= 3 && a.n <= 1024) : a.m >= 9 || (a.m >= 4 && a.k <= 1024 && a.n <= 8192);
+    return wanted && exact_supported(a.m, a.n, a.k, a.groupsize, a.swiglu != 0, a.lora_r);
+}
+static int launch_small(const GemmArgs &a) { return use_exact(a) ? launch_exact(a) : launch_decode(a, g_decode_override); }
 
 // no epilogue option and no fused all-gather: what the small-batch tcgen05 kernel takes
 static bool plain_gemm(const GemmArgs &a) { return !a.swiglu && a.lora_r == 0 && a.n_peers == 0 && !a.mc_c && !a.no_scratch; }
@@ -103,7 +118,7 @@ static int gemm(const GemmArgs &a) {
         if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
         return launch_prefill(a);
     }
-    return launch_decode(a, g_decode_override);
+    return launch_small(a);
 }
 
 }  // namespace kiln
@@ -238,7 +253,7 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
         a.lora_b = ep->lora_b;
         a.lora_r = ep->lora_rank;
         a.swiglu = ep->swiglu ? 1 : 0;
-        return launch_decode(a, g_decode_override);
+        return launch_small(a);
     }
     const bool composed = (ep->swiglu && !fuse_swiglu) || (ep->lora_rank && !fuse_lora);
     void *tmp = nullptr;

@@ -734,10 +734,11 @@ int g_smallm_enabled = 1;
 // K splits of the small-batch kernel.  Its time in microseconds, fitted to 1300 timed launches (CUDA graph over rotating weights;
 // K = 512..9216 x N = 1536..18432 x 1..128 rows x every split): up to half the SMs, consecutive launches run side by side and
 // only the chain from the grid-dependency wait to the exit counts; above that a launch starts on the SMs the one before leaves.
-// A further wave of CTAs repeats that start.  The exchange of partial sums grows with the rows; it is done by all CTAs at once.
+// A further wave of CTAs repeats that start; how many clusters fit decides when there is one (4096 x 6144 has 48 tiles, and 3 splits
+// need 48 clusters of 3 where 45 fit: 12.2 us, 2 splits 7.9).  The exchange of partial sums grows with the rows; it is done by all CTAs at once.
 double smallm_cost(int m, int n, int k, int splits) {
     const int sms = device_sm_count();
-    const int units = n / 128 * splits, waves = (units + sms - 1) / sms;
+    const int units = n / 128 * splits, clusters = smallm_clusters(splits), waves = (n / 128 + clusters - 1) / clusters;
     const double stages = (k / 128 + splits - 1) / splits, over = (units < sms ? units : sms) - sms / 2;
     const double start = over <= 0 ? 1.4 : 2.5 + 0.0246 * over;
     const double rows = (m + 15) / 16 * 16, step = 0.27 + (over > 0 ? 0.015 : 0.0) + (m > 64 ? 0.03 + (over > 0 ? 0.0024 * over : 0.0) : 0.0);
@@ -899,6 +900,14 @@ static bool smallm_takes(const PrefillConfig &c, int m, int n, int k, int groups
 
 // The small-batch kernel by itself, for a plain problem: no workspace.
 bool smallm_takes(int m, int n, int k, int groupsize) { return m <= BM && smallm_takes(choose_prefill(m, n, k), m, n, k, groupsize); }
+
+// The small-batch kernel's variant that applies the group scales in fp32 (the decode kernel's arithmetic): 16 rows a CTA.
+static int exact_splits(int m, int n, int k, bool swiglu) { return swiglu ? 1 : choose_smallm_splits(16, n * ((m + 15) / 16), k); }
+bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r) {
+    return g_smallm_enabled && g_test_drop_a_load < 0 && m <= 256 && (lora_r == 0 || (groupsize != -1 && lora_r <= 128)) &&
+           smallm_supported(std::min(m, 16), n, k, groupsize, exact_splits(m, n, k, swiglu));
+}
+int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
 
 // SwiGLU is fused into an epilogue that sees whole tiles: the small-batch kernel's without a K split, or the pair kernel's.  A second
 // pass over the bf16 result takes about 4 us, more than a K split saves a SwiGLU-sized projection, except for a long K and few columns.

@@ -65,6 +65,8 @@ constexpr int kTeamThreads = kTeams * kTeamWarps * 32;
 constexpr int kThreads = kTeamWarp0 * 32 + kTeamThreads;
 static_assert(kMaxWSlots % kTeams == 0, "see above");
 
+constexpr int kExactRows = 16;  // rows of a CTA of the EXACT variant (see the kernel)
+
 // barriers: [wfull][wempty] x kMaxWSlots, [full][empty] x kMaxSlots, done, exchange, scales
 constexpr int kBarWFull = 0, kBarWEmpty = kMaxWSlots, kBarFull = 2 * kMaxWSlots, kBarEmpty = kBarFull + kMaxSlots,
               kBarDone = kBarEmpty + kMaxSlots, kBarExchange = kBarDone + 1, kBarScales = kBarExchange + 1, kBars = kBarScales + 1;
@@ -77,9 +79,10 @@ struct SmallMParams {
     int m, n, splits, k_stages, npad;
     int scale_rows;                  // most stages of a CTA
     int w_slots;                     // depth of the ring of packed words, in stages
-    int off_x, off_scale, off_recv;  // shared memory: packed words at 0, then these (bytes from the 1024-byte aligned base)
+    int off_x, off_scale, off_recv, off_lora;  // shared memory: packed words at 0, then these (bytes from the 1024-byte aligned base)
     int quads_per_rank, rank_magic;  // K splits: groups of four rows owned by one rank; x / quads_per_rank = (x * rank_magic) >> 16
     // LoRA delta C += t * lora_b^T: t = scale * x * A^T is bf16 [m, lora_r], lora_b bf16 [n, lora_r], lora_r a multiple of 8 up to 128
+    const float *lora_t;  // EXACT: the fp32 projection [m, lora_r]
     const __nv_bfloat16 *lora_b;
     int lora_r;
     int per_column;  // one fp16 scale per column (group size -1): dequantised unscaled, the scale applied to the sums
@@ -113,6 +116,20 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld_32x32b_x4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ float lds_half(uint32_t addr) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+    return __half2float(__ushort_as_half(v));
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void st_shared_bf16(uint32_t addr, __nv_bfloat16 v) {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(__bfloat16_as_ushort(v)) : "memory");
 }
@@ -135,6 +152,7 @@ __device__ __forceinline__ void st_async_v4(uint32_t cluster_addr, float a, floa
 
 // One packed word -> the four bf16x2 registers {column c: K pair qd, column c + 8: K pair qd, c: K pair 4 + qd, c + 8: K pair
 // 4 + qd}, scaled: (128 + nibble) - 136, times the group scale, the same two roundings as the general kernel.
+template <bool SCALE>
 __device__ __forceinline__ void dequant_word(uint32_t x, __nv_bfloat162 s_lo, __nv_bfloat162 s_hi, uint32_t *r) {
     r[0] = lop3_and_or(x, kNibMask, kMagic128);
     r[2] = lop3_and_or(x >> 4, kNibMask, kMagic128);
@@ -145,7 +163,7 @@ __device__ __forceinline__ void dequant_word(uint32_t x, __nv_bfloat162 s_lo, __
     for (int e = 0; e < 4; ++e) {
         __nv_bfloat162 w = *reinterpret_cast<__nv_bfloat162 *>(&r[e]);
         w = __hsub2(w, *reinterpret_cast<const __nv_bfloat162 *>(&k136));
-        w = __hmul2(w, (e & 1) ? s_hi : s_lo);
+        if (SCALE) w = __hmul2(w, (e & 1) ? s_hi : s_lo);
         r[e] = *reinterpret_cast<uint32_t *>(&w);
     }
 }
@@ -156,14 +174,21 @@ constexpr int slots() {
     return (kTmemCols - 2 * R) / kSlotCols;  // 6 for R = 64, 4 for R = 128
 }
 
+// EXACT: the weights go to tensor memory unscaled, as the integers -8..7.  A stage, which is one scale group, has an
+// accumulator of its own, one of four like the teams; before a team hands its next stage to the issuers, and once more at the end, it
+// adds the finished one, times the fp32 group scale of the lane's column, to sums in registers.  That is the decode kernel's
+// arithmetic (exact products, the scale applied once per group, in fp32), so the batches that were the decode kernel's lose no
+// precision here.  The teams' sums meet in tensor memory, and a LoRA delta is added to them in fp32 from the fp32 projection.  More than
+// sixteen rows are so many more CTAs (blockIdx.z): for projections of few columns, which leave the GPU empty otherwise.
 // R: most rows.  SWIGLU is a template parameter so that the plain epilogue is compiled on its own.
-template <int R, bool SWIGLU>
+template <int R, bool SWIGLU, bool EXACT>
 __global__ void __launch_bounds__(kThreads, 1)
 w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_x,
                     const __grid_constant__ CUtensorMap tmap_t, const __grid_constant__ CUtensorMap tmap_c,
                     const __grid_constant__ SmallMParams p) {
     constexpr int kSlots = slots<R>();
     static_assert(kSlots >= kTeams && kSlots <= kMaxSlots, "see kMaxWSlots");
+    static_assert(!EXACT || (kTeams <= kSlots && kTeams * kExactRows <= R && kExactRows == 4 * kTeams), "see above");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(128) uint8_t bar_mem[kBarrierBytes];
@@ -175,9 +200,9 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(bar_mem + 8 * kBars + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = blockIdx.x, nt = blockIdx.y;  // K split (= rank in the cluster), tile
+    const int rank = blockIdx.x, nt = blockIdx.y, m0 = EXACT ? blockIdx.z * kExactRows : 0;  // K split (= rank in the cluster), tile, first row
     const int ks0 = rank * p.k_stages / p.splits, ks1 = (rank + 1) * p.k_stages / p.splits, n_st = ks1 - ks0;
-    const int lora_it = (rank == 0 && p.lora_r > 0) ? 1 : 0;  // the CTA that starts the tile's K range begins with the LoRA iteration
+    const int lora_it = (!EXACT && rank == 0 && p.lora_r > 0) ? 1 : 0;  // the CTA that starts the tile's K range begins with the LoRA iteration
     const int n_it = n_st + lora_it;
 
     pdl_launch_dependents();
@@ -252,7 +277,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     tma_load_2d(dst, &tmap_t, 0, 0, full(s));
                     tma_load_2d(dst + x_bytes, &tmap_t, kAtomK, 0, full(s));
                 } else {
-                    tma_load_3d(dst, &tmap_x, 0, 0, (ks0 + it - lora_it) * 2, full(s));
+                    tma_load_3d(dst, &tmap_x, 0, m0, (ks0 + it - lora_it) * 2, full(s));
                 }
                 if (++s == kSlots) {
                     s = 0;
@@ -280,7 +305,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t a_tmem = tmem_base + 2 * R + s * kSlotCols + t * (kAtomK / 2);
             if (issue) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_bf16_tmem_a(d_tmem, a_tmem + j * 8, b_desc + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
+                for (int j = 0; j < 4; ++j) umma_bf16_tmem_a(d_tmem + (EXACT ? it % kTeams * kExactRows : 0), a_tmem + j * 8, b_desc + 2 * j, idesc,
+                                     ((!EXACT && it > 0) || j > 0) ? 1u : 0u);
                 umma_commit(empty(s));
             }
             if (++s == kSlots) {
@@ -289,7 +315,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
             ready = mbar_test(full(s), ph);
         }
-        if (ok && issue) umma_commit(bar(kBarDone));
+        if (!EXACT && ok && issue) umma_commit(bar(kBarDone));
     } else {
         // ---------------- dequant: packed int4 -> bf16 pairs in tensor memory ----------------
         // team u takes every fourth iteration, from iteration u
@@ -326,6 +352,41 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         int ws = (it - lora_it) % p.w_slots, wph = ((it - lora_it) / p.w_slots) & 1;  // slot of its packed words
         bool w_ready = false, t_ready = false;  // the next waits, asked ahead
         if (it < n_it && !p.per_column) ok = mbar_wait(bar(kBarScales), 0, abort_flag, p.status, 0xEC0u, p.wait_limit_ns);
+        // EXACT: the CTA's part of the LoRA rank (the K splits share it), and its values of lora_b for the tile's columns, a weight that
+        // is there before it is needed; 16 bytes more per row keep the reads off each other's banks
+        const int lora_0 = 8 * (rank * (p.lora_r / 8) / p.splits), lora_n = 8 * ((rank + 1) * (p.lora_r / 8) / p.splits) - lora_0;
+        const int lora_pitch = lora_n * 2 + 16;
+        const uint32_t lora_b_addr = smem_base + p.off_lora, lora_t_addr = lora_b_addr + kTileCols * lora_pitch;
+        if (EXACT && p.lora_r > 0) {
+            const int pieces = lora_n / 8, x = (warp - kTeamWarp0) * 32 + lane;
+            for (int i = x; i < kTileCols * pieces; i += kTeamThreads) {
+                const int col = i / pieces, piece = i - col * pieces;
+                cp_async_16(lora_b_addr + col * lora_pitch + piece * 16,
+                            p.lora_b + (static_cast<size_t>(nt) * kTileCols + col) * p.lora_r + lora_0 + 8 * piece);
+            }
+        }
+        // EXACT: sums of the lane's column, and the step that adds the stage j of this team
+        float y[EXACT ? kExactRows : 1] = {};
+        const int col_in_chunk = col_in_tile & 63;
+        const uint32_t exact_sc = smem_base + p.off_scale + (ch * 64 + 8 * (col_in_chunk & 7) + (col_in_chunk >> 3)) * 2;
+        auto add_stage = [&](int j, bool ready) {
+            if (!ready && !(ok = mbar_wait(empty(j % kSlots), j / kSlots & 1, abort_flag, p.status, 0xF00u | (j % kSlots), p.wait_limit_ns))) return;
+            __syncwarp();
+            tc_fence_after();
+            const float scale = p.per_column ? 1.f : lds_half(exact_sc + j * kScaleBytes);
+#pragma unroll
+            for (int r8 = 0; r8 < kExactRows; r8 += 8) {
+                uint32_t a[8], b[8];
+                tmem_ld_32x32b_x8(t_lane + u * kExactRows + r8, a);
+                tmem_ld_32x32b_x8(t_lane + R + u * kExactRows + r8, b);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float &sum = y[EXACT ? r8 + i : 0];
+                    sum = fmaf(scale, __uint_as_float(a[i]) + __uint_as_float(b[i]), sum);
+                }
+            }
+        };
         for (; it < n_it && ok; it += kTeams) {
             if (it >= kSlots && it < kSlots + kTeams) pdl_wait();  // (park until the MMAs may run)
             if (!w_ready && !(ok = mbar_wait(bar(kBarWFull + ws), wph, abort_flag, p.status, 0xE00u | ws, p.wait_limit_ns))) break;
@@ -339,7 +400,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             __nv_bfloat162 sc[4];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const uint32_t pair = p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + 8 * i);
+                const uint32_t pair = EXACT || p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + 8 * i);
                 const float f0 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair & 0xFFFFu)));
                 const float f1 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair >> 16)));
                 sc[2 * i] = __floats2bfloat162_rn(f0, f0);
@@ -353,12 +414,17 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
             for (int k2 = 0; k2 < 4; ++k2) {  // two K tiles of 16 at a time
                 uint32_t r[8];
-                dequant_word(wa[2 * k2], sc[0], sc[1], r);
-                dequant_word(wa[2 * k2 + 1], sc[0], sc[1], r + 4);
+                dequant_word<!EXACT>(wa[2 * k2], sc[0], sc[1], r);
+                dequant_word<!EXACT>(wa[2 * k2 + 1], sc[0], sc[1], r + 4);
                 tmem_st_16x128b_x4(dst + k2 * 16, r);
-                dequant_word(wb[2 * k2], sc[2], sc[3], r);
-                dequant_word(wb[2 * k2 + 1], sc[2], sc[3], r + 4);
+                dequant_word<!EXACT>(wb[2 * k2], sc[2], sc[3], r);
+                dequant_word<!EXACT>(wb[2 * k2 + 1], sc[2], sc[3], r + 4);
                 tmem_st_16x128b_x4(dst + (16u << 16) + k2 * 16, r);
+            }
+            if (EXACT && it >= kTeams) {
+                if (it < 2 * kTeams) pdl_wait();  // (as above)
+                add_stage(it - kTeams, mbar_test(empty((it - kTeams) % kSlots), (it - kTeams) / kSlots & 1));
+                if (!ok) break;
             }
             const uint32_t done = full(s);
             if ((s += kTeams) >= kSlots) {
@@ -377,10 +443,64 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive(done);
         }
-        // ---------------- epilogue: a thread owns one output column; team u takes every fourth block of 16 rows ----------------
-        if (ok) ok = mbar_wait(bar(kBarDone), 0, abort_flag, p.status, 0xD00u, p.wait_limit_ns);
+        if constexpr (EXACT) {
+            pdl_wait();
+            if (p.lora_r > 0) {  // this CTA's part of the fp32 projection (rows past m are not stored: any row will do for them)
+                const int pieces = lora_n / 4, x = (warp - kTeamWarp0) * 32 + lane;
+                for (int i = x; i < kExactRows * pieces; i += kTeamThreads) {
+                    const int row = i / pieces, piece = i - row * pieces;
+                    cp_async_16(lora_t_addr + i * 16, p.lora_t + static_cast<size_t>(min(m0 + row, p.m - 1)) * p.lora_r + lora_0 + 4 * piece);
+                }
+            }
+            if (ok && it > u) add_stage(it - kTeams, false);
+#pragma unroll
+            for (int r8 = 0; r8 < kExactRows; r8 += 8) {
+                uint32_t r[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(y[r8 + i]);
+                tmem_st_32x32b_x8(t_lane + u * kExactRows + r8, r);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            // the four warps with this quarter of the lanes; all stages are through when they meet
+            asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "n"(kTeams * 32) : "memory");
+            if (p.lora_r > 0) {
+                cp_async_wait_all();
+                asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");
+            }
+            ok = ok && *abort_flag == 0;
+        }
+        // ---------------- epilogue: a thread owns one output column; team u takes every fourth block of 16 rows (EXACT: of 4) ----------------
+        if (!EXACT && ok) ok = mbar_wait(bar(kBarDone), 0, abort_flag, p.status, 0xD00u, p.wait_limit_ns);
         tc_fence_after();
         const int col = nt * kTileCols + col_in_tile;
+        float v4[4] = {};  // EXACT: rows 4u..4u + 3
+        if (EXACT) {
+#pragma unroll
+            for (int w = 0; w < kTeams; ++w) {
+                uint32_t r[4];
+                tmem_ld_32x32b_x4(t_lane + w * kExactRows + 4 * u, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v4[i] += __uint_as_float(r[i]);
+            }
+            if (p.lora_r > 0) {
+                const uint32_t lb = lora_b_addr + col_in_tile * lora_pitch, t = lora_t_addr + 4 * u * lora_n * 4;
+                for (int r = 0; r < lora_n; r += 8) {
+                    const uint4 w4 = lds_v4(lb + r * 2);
+                    const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint4 t0 = lds_v4(t + (i * lora_n + r) * 4), t1 = lds_v4(t + (i * lora_n + r) * 4 + 16);
+                        const uint32_t tv[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            v4[i] = fmaf(__uint_as_float(tv[e]), __uint_as_float(e & 1 ? w[e / 2] & 0xFFFF0000u : w[e / 2] << 16), v4[i]);
+                    }
+                }
+            }
+        }
         if (p.splits == 1) {
             // The bf16 tile is put together in shared memory (over the rings, which are spent) and leaves through TMA: two-byte
             // stores from registers cost 8 cycles of the SM's load / store unit each.
@@ -388,7 +508,21 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const int ocol = SWIGLU ? ch * 32 + 16 * h + (lane & 15) : col_in_tile;  // output column within the tile
             const uint32_t stage = smem_base + (ocol >> 6) * x_bytes + (ocol & 7) * 2;
             const uint32_t chunk16 = (ocol & 63) >> 3;  // 16-byte chunk of a 128-byte row, XORed with row % 8
-            if (ok)
+            if constexpr (EXACT) {
+                const bool up = lane >= 16;
+#pragma unroll
+                for (int i = 0; i < (SWIGLU ? 2 : 4); ++i) {
+                    int row = 4 * u + i;
+                    float out = v4[i] * cs;
+                    if constexpr (SWIGLU) {  // (as below)
+                        const float other = __shfl_xor_sync(0xFFFFFFFFu, up ? v4[2 * i] : v4[2 * i + 1], 16);
+                        const float g = (up ? other : v4[2 * i]) * cs, w = (up ? v4[2 * i + 1] : other) * cs;
+                        row = 4 * u + 2 * i + (up ? 1 : 0);
+                        out = __fdividef(g, 1.f + __expf(-g)) * w;
+                    }
+                    st_shared_bf16(stage + row * 128 + ((chunk16 ^ (row & 7)) << 4), __float2bfloat16_rn(out));
+                }
+            } else if (ok)
 #pragma unroll 1
                 for (int r0 = 16 * u; r0 < p.npad; r0 += 16 * kTeams) {
 #pragma unroll
@@ -423,8 +557,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");  // (every warp of the teams comes here, whatever happened)
             if (ok && warp == kTeamWarp0 && lane == 0) {
                 pdl_wait();  // C may still be read or written by the previous kernel
-                tma_store_2d(&tmap_c, smem_base, nt * (SWIGLU ? kTileCols / 2 : kTileCols), 0);  // (rows past m are clipped)
-                if (!SWIGLU) tma_store_2d(&tmap_c, smem_base + x_bytes, nt * kTileCols + 64, 0);
+                tma_store_2d(&tmap_c, smem_base, nt * (SWIGLU ? kTileCols / 2 : kTileCols), m0);  // (rows past m are clipped)
+                if (!SWIGLU) tma_store_2d(&tmap_c, smem_base + x_bytes, nt * kTileCols + 64, m0);
                 bulk_commit_group();
                 bulk_wait_group0();
             }
@@ -435,8 +569,13 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster runs
             if (R > 64) cluster_sync_all();  // ... and its rings, which the receive buffer lies over, are spent
             if (ok) {
+                if constexpr (EXACT) {
+                    const int owner = (u * p.rank_magic) >> 16, slot = u - owner * p.quads_per_rank;
+                    const uint32_t addr = recv + static_cast<uint32_t>((rank * p.quads_per_rank + slot) * kTileCols + col_in_tile) * 16u;
+                    st_async_v4(map_to_cta(addr, owner), v4[0], v4[1], v4[2], v4[3], map_to_cta(bar(kBarExchange), owner));
+                }
 #pragma unroll 1
-                for (int r0 = 8 * u; r0 < p.npad; r0 += 8 * kTeams) {
+                for (int r0 = 8 * u; r0 < p.npad && !EXACT; r0 += 8 * kTeams) {
                     uint32_t a[8], b[8];
                     tmem_ld_32x32b_x8(t_lane + r0, a);
                     tmem_ld_32x32b_x8(t_lane + R + r0, b);
@@ -470,7 +609,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         v[2] += __uint_as_float(u.z);
                         v[3] += __uint_as_float(u.w);
                     }
-                    const int row0 = (rank * p.quads_per_rank + slot) * 4;
+                    const int row0 = m0 + (rank * p.quads_per_rank + slot) * 4;
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (row0 + i < p.m) p.C[static_cast<size_t>(row0 + i) * p.n + gcol] = __float2bfloat16_rn(v[i] * cs);
@@ -505,15 +644,43 @@ bool smallm_supported(int m, int n, int k, int groupsize, int splits) {
            splits >= 1 && splits <= 8 && splits <= k / kStageK && (k / kStageK + splits - 1) / splits <= kMaxStages;
 }
 
-// C = A * dequant(B) with `splits` K splits (one cluster per tile).
-int launch_smallm(const GemmArgs &a, int splits) {
+// Clusters of `splits` (1..8) CTAs that the device holds at once: what a GPC has left over does not make a cluster (without a device,
+// those of a B200 with 148 SMs).
+int smallm_clusters(int splits) {
+    static const int b200[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    static int cached[64][9] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return b200[splits];
+    if (!cached[dev][splits]) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(splits, 64);
+        cfg.blockDim = dim3(kThreads);
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = splits;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;  // (one CTA per SM, whatever its shared memory: registers)
+        if (cudaOccupancyMaxActiveClusters(&n, w4a16_smallm_kernel<64, false, false>, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = b200[splits];
+        }
+        cached[dev][splits] = n;
+    }
+    return cached[dev][splits];
+}
+
+// C = A * dequant(B) with `splits` K splits (one cluster per tile).  exact: group scales applied in fp32.
+int launch_smallm(const GemmArgs &a, int splits, bool exact) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return KILN_W4A16_ERR_CUDA;
     uint32_t *status = device_status_word();
     if (!status) return KILN_W4A16_ERR_CUDA;
-    if (!smallm_supported(a.m, a.n, a.k, a.groupsize, splits) || (a.swiglu && splits != 1)) return KILN_W4A16_ERR_KERN_SHAPE;
+    const int rows = exact ? std::min(a.m, kExactRows) : a.m;  // of a CTA
+    if (!smallm_supported(rows, a.n, a.k, a.groupsize, splits) || (a.swiglu && splits != 1)) return KILN_W4A16_ERR_KERN_SHAPE;
 
-    const int npad = (a.m + 15) & ~15;
+    const int npad = (rows + 15) & ~15;
     CUtensorMap tmap_w, tmap_s, tmap_x, tmap_t;
     {  // packed words: [k/16][2n] int32, boxes of one tile x eight rows (128 K)
         const cuuint64_t dims[2] = {2ull * a.n, static_cast<cuuint64_t>(a.k / 16)}, strides[1] = {8ull * a.n};
@@ -549,7 +716,7 @@ int launch_smallm(const GemmArgs &a, int splits) {
     const bool lora = a.lora_r > 0 && a.lora_t && a.lora_b;
     if (lora) {
         if (a.groupsize == -1 || a.lora_r % 8 != 0 || a.lora_r > 128) return KILN_W4A16_ERR_KERN_SHAPE;
-        if (!encode(&tmap_t, a.lora_t, a.lora_r)) return KILN_W4A16_ERR_CUDA;
+        if (!exact && !encode(&tmap_t, a.lora_t, a.lora_r)) return KILN_W4A16_ERR_CUDA;
     }
     CUtensorMap tmap_c = tmap_x;  // (unused when K is split)
     if (splits == 1 && !encode(&tmap_c, a.C, a.swiglu ? a.n / 2 : a.n)) return KILN_W4A16_ERR_CUDA;
@@ -567,6 +734,7 @@ int launch_smallm(const GemmArgs &a, int splits) {
     p.rank_magic = (65536 + p.quads_per_rank - 1) / p.quads_per_rank;  // (exact for the at most 32 quads)
     p.per_column = a.groupsize == -1;
     p.lora_b = lora ? static_cast<const __nv_bfloat16 *>(a.lora_b) : nullptr;
+    p.lora_t = lora ? static_cast<const float *>(a.lora_t) : nullptr;
     p.lora_r = lora ? a.lora_r : 0;
     p.wait_limit_ns = current_wait_limit_ns();
 
@@ -575,18 +743,21 @@ int launch_smallm(const GemmArgs &a, int splits) {
     // split lies behind them for up to 64 rows and over them (spent by then) above.
     constexpr int kMostSmem = 226 * 1024 - kBarrierBytes;
     const int recv = splits > 1 ? splits * p.quads_per_rank * kTileCols * 16 : 0;
-    const int x_stages = std::min(stages + (lora ? 1 : 0), a.m <= 64 ? slots<64>() : slots<128>());
-    const int fixed = 2 * x_stages * npad * 128 + (p.per_column ? 0 : stages * kScaleBytes) + 1024;
+    const int x_stages = std::min(stages + (lora && !exact ? 1 : 0), rows <= 64 ? slots<64>() : slots<128>());
+    const int lora_part = lora && exact ? (a.lora_r / 8 + splits - 1) / splits * 8 : 0;  // most of the rank that a CTA has
+    const int lora_bytes = lora_part ? kTileCols * (2 * lora_part + 16) + kExactRows * lora_part * 4 : 0;
+    const int fixed = 2 * x_stages * npad * 128 + (p.per_column ? 0 : stages * kScaleBytes) + lora_bytes + 1024;
     p.scale_rows = stages;
-    for (p.w_slots = kMaxWSlots; p.w_slots > kTeams && fixed + p.w_slots * kWSlotBytes + (a.m <= 64 ? recv : 0) > kMostSmem;) p.w_slots -= kTeams;
+    for (p.w_slots = kMaxWSlots; p.w_slots > kTeams && fixed + p.w_slots * kWSlotBytes + (rows <= 64 ? recv : 0) > kMostSmem;) p.w_slots -= kTeams;
     p.w_slots = std::min(stages, p.w_slots);
     p.off_x = p.w_slots * kWSlotBytes;
     p.off_scale = p.off_x + 2 * x_stages * npad * 128;
-    p.off_recv = a.m <= 64 ? p.off_scale + (p.per_column ? 0 : stages * kScaleBytes) : 0;
-    const int smem = std::max(p.w_slots * kWSlotBytes + fixed, p.off_recv + recv + 1024);
+    p.off_recv = rows <= 64 ? p.off_scale + (p.per_column ? 0 : stages * kScaleBytes) : 0;
+    p.off_lora = p.off_recv + recv;
+    const int smem = std::max(p.w_slots * kWSlotBytes + fixed, p.off_lora + lora_bytes + 1024);
     if (smem > kMostSmem) return KILN_W4A16_ERR_KERN_SHAPE;
 
-    static bool attr_set[4][64] = {};  // per kernel variant and device: the shared-memory attribute is set once
+    static bool attr_set[6][64] = {};  // per kernel variant and device: the shared-memory attribute is set once
     int dev = 0;
     cudaGetDevice(&dev);
     auto launch = [&](auto kernel, int variant) -> int {
@@ -595,7 +766,7 @@ int launch_smallm(const GemmArgs &a, int splits) {
             attr_set[variant][dev] = true;
         }
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(splits, a.n / kTileCols);
+        cfg.gridDim = dim3(splits, a.n / kTileCols, exact ? (a.m + kExactRows - 1) / kExactRows : 1);
         cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = a.stream;
@@ -610,8 +781,9 @@ int launch_smallm(const GemmArgs &a, int splits) {
         note_launch();
         return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, tmap_w, tmap_s, tmap_x, tmap_t, tmap_c, p));
     };
-    if (a.swiglu) return a.m <= 64 ? launch(w4a16_smallm_kernel<64, true>, 2) : launch(w4a16_smallm_kernel<128, true>, 3);
-    return a.m <= 64 ? launch(w4a16_smallm_kernel<64, false>, 0) : launch(w4a16_smallm_kernel<128, false>, 1);
+    if (exact) return a.swiglu ? launch(w4a16_smallm_kernel<64, true, true>, 5) : launch(w4a16_smallm_kernel<64, false, true>, 4);
+    if (a.swiglu) return a.m <= 64 ? launch(w4a16_smallm_kernel<64, true, false>, 2) : launch(w4a16_smallm_kernel<128, true, false>, 3);
+    return a.m <= 64 ? launch(w4a16_smallm_kernel<64, false, false>, 0) : launch(w4a16_smallm_kernel<128, false, false>, 1);
 }
 
 }  // namespace kiln

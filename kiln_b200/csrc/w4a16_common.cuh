@@ -166,8 +166,11 @@ void set_wait_limit_ns(unsigned long long ns);
 unsigned long long current_wait_limit_ns();
 void set_smallm_enabled(int on);
 bool smallm_supported(int m, int n, int k, int groupsize, int splits);
+int smallm_clusters(int splits);
 bool smallm_takes(int m, int n, int k, int groupsize);
-int launch_smallm(const GemmArgs &a, int splits);
+int launch_smallm(const GemmArgs &a, int splits, bool exact = false);
+bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r);
+int launch_exact(const GemmArgs &a);
 void set_test_drop_a_load(int k_step);
 void prefill_plan(int m, int n, int k, int out[4]);
 bool prefill_supported(int m, int n, int k, int groupsize);
