@@ -105,9 +105,10 @@ __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t
                  : "memory");
 }
 // 16 TMEM lanes x 16 cells: two K tiles of 16 of sixteen columns
-__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
-                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+                 "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -116,10 +117,22 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld_32x32b_x4(uint32_t taddr, uint32_t (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
+}
+__device__ __forceinline__ uint2 lds_v2(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
 }
 __device__ __forceinline__ float lds_half(uint32_t addr) {
     unsigned short v;
@@ -305,7 +318,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t a_tmem = tmem_base + 2 * R + s * kSlotCols + t * (kAtomK / 2);
             if (issue) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_bf16_tmem_a(d_tmem + (EXACT ? it % kTeams * kExactRows : 0), a_tmem + j * 8, b_desc + 2 * j, idesc,
+                for (int j = 0; j < 4; ++j)
+                    umma_bf16_tmem_a(d_tmem + (EXACT ? it % kTeams * kExactRows : 0), a_tmem + j * 8, b_desc + 2 * j, idesc,
                                      ((!EXACT && it > 0) || j > 0) ? 1u : 0u);
                 umma_commit(empty(s));
             }
@@ -323,7 +337,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int quarter = warp & 3, ch = quarter >> 1, h = quarter & 1;
         const int c = lane >> 2;
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-        const int col_in_tile = 64 * ch + 16 * h + (lane & 15) + 32 * (lane >> 4);  // of TMEM lane `lane` of this warp
+        const int col_in_tile = 64 * ch + (SWIGLU ? 16 * h + (lane & 15) + 32 * (lane >> 4) : 32 * h + lane);  // of TMEM lane `lane` of this warp
         bool ok = true;
         int it = u;
         if (lora_it && it == 0) {
@@ -346,7 +360,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         // scales of the lane's four columns c, c + 8 (word h) and c + 32, c + 40 (word h + 2): positions 8c + 2h + {0, 1} and
         // 8c + 2h + 4 + {0, 1} of the chunk's scale order (position 8i + j holds column 8j + i)
-        const uint32_t sc_addr = smem_base + p.off_scale + (ch * 64 + 8 * c + 2 * h) * 2;
+        const uint32_t sc_addr = smem_base + p.off_scale + (ch * 64 + 8 * c + (SWIGLU ? 2 : 4) * h) * 2;
         const uint32_t w_addr = smem_base + ch * 512 + lane * 16;
         int s = it % kSlots, ph = (it / kSlots & 1) ^ 1;                               // slot of the iteration
         int ws = (it - lora_it) % p.w_slots, wph = ((it - lora_it) / p.w_slots) & 1;  // slot of its packed words
@@ -369,38 +383,39 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         float y[EXACT ? kExactRows : 1] = {};
         const int col_in_chunk = col_in_tile & 63;
         const uint32_t exact_sc = smem_base + p.off_scale + (ch * 64 + 8 * (col_in_chunk & 7) + (col_in_chunk >> 3)) * 2;
-        auto add_stage = [&](int j, bool ready) {
-            if (!ready && !(ok = mbar_wait(empty(j % kSlots), j / kSlots & 1, abort_flag, p.status, 0xF00u | (j % kSlots), p.wait_limit_ns))) return;
+        auto add_stage = [&](int j, int s, int ph) {
+            if (!mbar_test(empty(s), ph) && !(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xF00u | s, p.wait_limit_ns))) return;
             __syncwarp();
             tc_fence_after();
             const float scale = p.per_column ? 1.f : lds_half(exact_sc + j * kScaleBytes);
+            uint32_t a[kExactRows], b[kExactRows];
+            tmem_ld_32x32b_x16(t_lane + u * kExactRows, a);
+            tmem_ld_32x32b_x16(t_lane + R + u * kExactRows, b);
+            tmem_ld_wait();
 #pragma unroll
-            for (int r8 = 0; r8 < kExactRows; r8 += 8) {
-                uint32_t a[8], b[8];
-                tmem_ld_32x32b_x8(t_lane + u * kExactRows + r8, a);
-                tmem_ld_32x32b_x8(t_lane + R + u * kExactRows + r8, b);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    float &sum = y[EXACT ? r8 + i : 0];
-                    sum = fmaf(scale, __uint_as_float(a[i]) + __uint_as_float(b[i]), sum);
-                }
-            }
+            for (int i = 0; i < (EXACT ? kExactRows : 1); ++i) y[i] = fmaf(scale, __uint_as_float(a[i]) + __uint_as_float(b[i]), y[i]);
         };
+        int s0 = 0, ph0 = 0;  // slot of the team's previous stage, and the phase that ends with it
         for (; it < n_it && ok; it += kTeams) {
             if (it >= kSlots && it < kSlots + kTeams) pdl_wait();  // (park until the MMAs may run)
             if (!w_ready && !(ok = mbar_wait(bar(kBarWFull + ws), wph, abort_flag, p.status, 0xE00u | ws, p.wait_limit_ns))) break;
             uint32_t wa[8], wb[8];  // words h and h + 2 of the eight K tiles
 #pragma unroll
             for (int kt = 0; kt < 8; ++kt) {
-                const uint4 v = lds_v4(w_addr + ws * kWSlotBytes + kt * 1024);
-                wa[kt] = h ? v.y : v.x;
-                wb[kt] = h ? v.w : v.z;
+                if (SWIGLU) {
+                    const uint4 v = lds_v4(w_addr + ws * kWSlotBytes + kt * 1024);
+                    wa[kt] = h ? v.y : v.x;
+                    wb[kt] = h ? v.w : v.z;
+                } else {
+                    const uint2 v = lds_v2(w_addr + 8 * h + ws * kWSlotBytes + kt * 1024);
+                    wa[kt] = v.x;
+                    wb[kt] = v.y;
+                }
             }
             __nv_bfloat162 sc[4];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const uint32_t pair = EXACT || p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + 8 * i);
+                const uint32_t pair = EXACT || p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + (SWIGLU ? 8 : 4) * i);
                 const float f0 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair & 0xFFFFu)));
                 const float f1 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair >> 16)));
                 sc[2 * i] = __floats2bfloat162_rn(f0, f0);
@@ -412,21 +427,23 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             tc_fence_after();
             const uint32_t dst = t_lane + 2 * R + s * kSlotCols;
 #pragma unroll
-            for (int k2 = 0; k2 < 4; ++k2) {  // two K tiles of 16 at a time
-                uint32_t r[8];
-                dequant_word<!EXACT>(wa[2 * k2], sc[0], sc[1], r);
-                dequant_word<!EXACT>(wa[2 * k2 + 1], sc[0], sc[1], r + 4);
-                tmem_st_16x128b_x4(dst + k2 * 16, r);
-                dequant_word<!EXACT>(wb[2 * k2], sc[2], sc[3], r);
-                dequant_word<!EXACT>(wb[2 * k2 + 1], sc[2], sc[3], r + 4);
-                tmem_st_16x128b_x4(dst + (16u << 16) + k2 * 16, r);
+            for (int k4 = 0; k4 < 2; ++k4) {  // four K tiles of 16 at a time
+                uint32_t r[16];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dequant_word<!EXACT>(wa[4 * k4 + i], sc[0], sc[1], r + 4 * i);
+                tmem_st_16x128b_x8(dst + k4 * 32, r);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dequant_word<!EXACT>(wb[4 * k4 + i], sc[2], sc[3], r + 4 * i);
+                tmem_st_16x128b_x8(dst + (16u << 16) + k4 * 32, r);
             }
             if (EXACT && it >= kTeams) {
                 if (it < 2 * kTeams) pdl_wait();  // (as above)
-                add_stage(it - kTeams, mbar_test(empty((it - kTeams) % kSlots), (it - kTeams) / kSlots & 1));
+                add_stage(it - kTeams, s0, ph0);
                 if (!ok) break;
             }
             const uint32_t done = full(s);
+            s0 = s;
+            ph0 = ph ^ 1;  // (the producer side of a slot waits for the phase before)
             if ((s += kTeams) >= kSlots) {
                 s -= kSlots;
                 ph ^= 1;
@@ -452,7 +469,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     cp_async_16(lora_t_addr + i * 16, p.lora_t + static_cast<size_t>(min(m0 + row, p.m - 1)) * p.lora_r + lora_0 + 4 * piece);
                 }
             }
-            if (ok && it > u) add_stage(it - kTeams, false);
+            if (ok && it > u) add_stage(it - kTeams, s0, ph0);
 #pragma unroll
             for (int r8 = 0; r8 < kExactRows; r8 += 8) {
                 uint32_t r[8];
@@ -560,7 +577,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 tma_store_2d(&tmap_c, smem_base, nt * (SWIGLU ? kTileCols / 2 : kTileCols), m0);  // (rows past m are clipped)
                 if (!SWIGLU) tma_store_2d(&tmap_c, smem_base + x_bytes, nt * kTileCols + 64, m0);
                 bulk_commit_group();
-                bulk_wait_group0();
+                bulk_wait_group_read0();  // (the end of the grid completes them)
             }
         }
         if (p.splits > 1) {
