@@ -79,6 +79,7 @@ struct SmallMParams {
     int m, n, splits, k_stages, npad;
     int scale_rows;                  // most stages of a CTA
     int w_slots;                     // depth of the ring of packed words, in stages
+    int recv_over_rings;             // the receive buffer of a K split lies over the rings (more than 64 rows)
     int off_x, off_scale, off_recv, off_lora;  // shared memory: packed words at 0, then these (bytes from the 1024-byte aligned base)
     int quads_per_rank, rank_magic;  // K splits: groups of four rows owned by one rank; x / quads_per_rank = (x * rank_magic) >> 16
     // LoRA delta C += t * lora_b^T: t = scale * x * A^T is bf16 [m, lora_r], lora_b bf16 [n, lora_r], lora_r a multiple of 8 up to 128
@@ -163,6 +164,10 @@ __device__ __forceinline__ void st_async_v4(uint32_t cluster_addr, float a, floa
                  : "memory");
 }
 
+__device__ __forceinline__ void sts_v4(uint32_t addr, float a, float b, float c, float d) {
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 // One packed word -> the four bf16x2 registers {column c: K pair qd, column c + 8: K pair qd, c: K pair 4 + qd, c + 8: K pair
 // 4 + qd}, scaled: (128 + nibble) - 136, times the group scale, the same two roundings as the general kernel.
 template <bool SCALE>
@@ -229,7 +234,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         __syncwarp();
         if (lane == 0 && p.splits > 1) {
             const int quads = p.npad / 4, own = max(0, min(p.quads_per_rank, quads - rank * p.quads_per_rank));
-            mbar_arrive_expect_tx(bar(kBarExchange), static_cast<uint32_t>(p.splits * own) * kTileCols * 16u);
+            mbar_arrive_expect_tx(bar(kBarExchange), static_cast<uint32_t>((p.splits - 1) * own) * kTileCols * 16u);
         }
     } else if (warp == 3 && lane == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
@@ -584,29 +589,33 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t recv = smem_base + p.off_recv;
             __syncwarp();
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster runs
-            if (R > 64) cluster_sync_all();  // ... and its rings, which the receive buffer lies over, are spent
+            if (R > 64 && p.recv_over_rings) cluster_sync_all();  // ... and its rings, which the receive buffer lies over, are spent
+            // (a quad of rows of this CTA's own goes straight to the buffer: the network between SMs bounds the exchange of many rows)
+            auto push = [&](int quad, float a, float b, float c, float d) {
+                const int owner = (quad * p.rank_magic) >> 16, slot = quad - owner * p.quads_per_rank;
+                const uint32_t addr = recv + static_cast<uint32_t>((rank * p.quads_per_rank + slot) * kTileCols + col_in_tile) * 16u;
+                if (owner == rank)
+                    sts_v4(addr, a, b, c, d);
+                else
+                    st_async_v4(map_to_cta(addr, owner), a, b, c, d, map_to_cta(bar(kBarExchange), owner));
+            };
             if (ok) {
-                if constexpr (EXACT) {
-                    const int owner = (u * p.rank_magic) >> 16, slot = u - owner * p.quads_per_rank;
-                    const uint32_t addr = recv + static_cast<uint32_t>((rank * p.quads_per_rank + slot) * kTileCols + col_in_tile) * 16u;
-                    st_async_v4(map_to_cta(addr, owner), v4[0], v4[1], v4[2], v4[3], map_to_cta(bar(kBarExchange), owner));
-                }
+                if constexpr (EXACT) push(u, v4[0], v4[1], v4[2], v4[3]);
 #pragma unroll 1
                 for (int r0 = 8 * u; r0 < p.npad && !EXACT; r0 += 8 * kTeams) {
                     uint32_t a[8], b[8];
                     tmem_ld_32x32b_x8(t_lane + r0, a);
                     tmem_ld_32x32b_x8(t_lane + R + r0, b);
                     tmem_ld_wait();
+                    float v[8];
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const int quad = r0 / 4 + q, owner = (quad * p.rank_magic) >> 16, slot = quad - owner * p.quads_per_rank;
-                        const uint32_t addr = recv + static_cast<uint32_t>((rank * p.quads_per_rank + slot) * kTileCols + col_in_tile) * 16u;
-                        st_async_v4(map_to_cta(addr, owner), __uint_as_float(a[4 * q]) + __uint_as_float(b[4 * q]),
-                                    __uint_as_float(a[4 * q + 1]) + __uint_as_float(b[4 * q + 1]),
-                                    __uint_as_float(a[4 * q + 2]) + __uint_as_float(b[4 * q + 2]),
-                                    __uint_as_float(a[4 * q + 3]) + __uint_as_float(b[4 * q + 3]), map_to_cta(bar(kBarExchange), owner));
-                    }
+                    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) push(r0 / 4 + q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");  // (the rows of its own; every warp of the teams comes here)
+            if (ok) {
                 ok = mbar_wait(bar(kBarExchange), 0, abort_flag, p.status, 0xD80u, p.wait_limit_ns);
             }
             if (ok) {
@@ -638,7 +647,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         tc_fence_before();
     }
 
-    if (R > 64 && p.splits > 1 && warp < kTeamWarp0) {  // (the other warps' part in the barrier above)
+    if (R > 64 && p.recv_over_rings && warp < kTeamWarp0) {  // (the other warps' part in the barrier above)
         __syncwarp();
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -757,7 +766,8 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
 
     // Shared memory: the activation ring mirrors the TMEM slots; packed words take the rest, up to twelve stages (eight, 64 KB
     // in flight, cover the latency of HBM at an SM's share of its bandwidth) or as many as the CTA has.  The receive buffer of a K
-    // split lies behind them for up to 64 rows and over them (spent by then) above.
+    // split lies behind them, or, above 64 rows and where it would leave fewer than those eight, over them: that costs a barrier of the
+    // cluster between the last MMA and the exchange.
     constexpr int kMostSmem = 226 * 1024 - kBarrierBytes;
     const int recv = splits > 1 ? splits * p.quads_per_rank * kTileCols * 16 : 0;
     const int x_stages = std::min(stages + (lora && !exact ? 1 : 0), rows <= 64 ? slots<64>() : slots<128>());
@@ -765,11 +775,17 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
     const int lora_bytes = lora_part ? kTileCols * (2 * lora_part + 16) + kExactRows * lora_part * 4 : 0;
     const int fixed = 2 * x_stages * npad * 128 + (p.per_column ? 0 : stages * kScaleBytes) + lora_bytes + 1024;
     p.scale_rows = stages;
-    for (p.w_slots = kMaxWSlots; p.w_slots > kTeams && fixed + p.w_slots * kWSlotBytes + (rows <= 64 ? recv : 0) > kMostSmem;) p.w_slots -= kTeams;
-    p.w_slots = std::min(stages, p.w_slots);
+    auto w_slots = [&](int bytes) {  // beside the rest and that many bytes
+        int slots = kMaxWSlots;
+        while (slots > kTeams && fixed + slots * kWSlotBytes + bytes > kMostSmem) slots -= kTeams;
+        return std::min(stages, slots);
+    };
+    p.w_slots = w_slots(recv);
+    p.recv_over_rings = rows > 64 && recv > 0 && (p.w_slots < std::min(stages, 8) || fixed + p.w_slots * kWSlotBytes + recv > kMostSmem);
+    if (p.recv_over_rings) p.w_slots = w_slots(0);
     p.off_x = p.w_slots * kWSlotBytes;
     p.off_scale = p.off_x + 2 * x_stages * npad * 128;
-    p.off_recv = rows <= 64 ? p.off_scale + (p.per_column ? 0 : stages * kScaleBytes) : 0;
+    p.off_recv = p.recv_over_rings ? 0 : p.off_scale + (p.per_column ? 0 : stages * kScaleBytes);
     p.off_lora = p.off_recv + recv;
     const int smem = std::max(p.w_slots * kWSlotBytes + fixed, p.off_lora + lora_bytes + 1024);
     if (smem > kMostSmem) return KILN_W4A16_ERR_KERN_SHAPE;
