@@ -74,11 +74,11 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16(const void *A, const void *B, void *C, 
  *             32 (columns 64c .. 64c+31 are gate columns 32c .. 32c+31, columns 64c+32 .. 64c+63 the up columns of the
  *             same indices; n = 2 * intermediate size).  C is then [m, n/2] = silu(gate) * up, computed in fp32 from the
  *             unrounded sums (the reference rounds gate and up to bf16 first).  lora_b follows the same column order.
- * For batch sizes the decode kernel serves the options are fused into that kernel's final reduction.  For larger ones
- * the LoRA delta rides in the tcgen05 kernels as extra K-steps (grouped scales; t is then written as bf16), and SwiGLU is
- * fused into the epilogue of the small-batch kernel (up to 128 rows, K not split) and of the general kernel's tilings
- * that write whole tiles from one accumulator per M-tile; what is not fused is applied by a second kernel to the bf16
- * GEMM result kept in the workspace. */
+ * At decode batch sizes the options are fused into the final reduction, in fp32, of the decode kernel or of the small-batch
+ * kernel's fp32-scale variant.  For larger ones the LoRA delta rides in the tcgen05 kernels as extra K-steps (grouped
+ * scales; t is then written as bf16), and SwiGLU is fused into the epilogue of the small-batch kernel (up to 128 rows, K not
+ * split) and of the CTA-pair kernel; what is not fused is applied by a second kernel to the bf16 GEMM result kept in the
+ * workspace. */
 typedef struct kiln_w4a16_epilogue {
     int swiglu;
     const void *lora_a;
@@ -159,7 +159,8 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_allgather_multicast(const void *A, cons
                                                              int ldc, int col0, void *stream);
 
 /* Scratch bytes the GEMM needs for (m, n, k); replaces the reference wrapper's
- * fixed `(n/128) * 16` int32 lock array (crates/kiln-marlin-gemm/src/lib.rs:176-178). */
+ * fixed `(n/128) * 16` int32 lock array (crates/kiln-marlin-gemm/src/lib.rs:176-178).  It is the planned tiling's scratch;
+ * a launch that needs less (the small-batch kernel keeps its split sums in shared memory) leaves it alone. */
 size_t kiln_w4a16_workspace_bytes(int m, int n, int k);
 
 /* Shape rule of the path (crates/kiln-model/src/marlin_proj.rs:53-55): 1 if supported. */
@@ -240,11 +241,12 @@ void kiln_w4a16_decode_plan(int m, int n, int k, int out[4]);
  * built-in rule (M > 256 for projections of at most 1024 columns; otherwise M >= 17 for a plain GEMM,
  * which the small-batch kernel takes up to 128 rows; with fused epilogue options M >= 33, or M >= 17
  * for projections of 1025..3072 columns whose activation matrix is at least 128 KB); a huge value disables those kernels,
- * 1 forces them. */
+ * 1 forces them.  With the built-in rule, what is below it runs on the small-batch kernel's fp32-scale variant from 9 rows (fewer for a
+ * short K or with a LoRA delta), else on the decode kernel; any other value leaves all of it to the decode kernel. */
 void kiln_w4a16_set_prefill_min_m(int min_m);
 
 /* Tuning hook for sweeps: force the tcgen05 kernel's tiling: bn = 128 or 256 columns per tile, K splits (1..8, fp32
- * slabs in the workspace), m_tiles = 1 or 2 (128-row tiles sharing a dequantised stage), stream_k = 1 for equal shares of the
+ * slabs in the workspace), m_tiles = 1 or 2 (2: CTA pairs, 256 rows per tile), stream_k = 1 for equal shares of the
  * (tile, K-step) space per CTA.  A combination that is not legal for a problem falls back to the built-in rule; 0,0,0,0
  * restores the rule.  kiln_w4a16_workspace_bytes follows the override.  Process-wide, not thread-safe; no counterpart in
  * the reference. */
@@ -252,7 +254,7 @@ void kiln_w4a16_set_prefill_override(int bn, int splits, int m_tiles, int stream
 
 /* Tuning hook: 0 keeps problems of at most 128 rows on the general tcgen05 kernel instead of the one that holds the
  * dequantised weights in tensor memory (default 1).  Results of the two kernels are the same up to fp32 summation
- * order.  Process-wide, not thread-safe; no counterpart in the reference. */
+ * order; what runs on its fp32-scale variant goes to the decode kernel.  Process-wide, not thread-safe; no counterpart in the reference. */
 void kiln_w4a16_set_small_batch_kernel(int enabled);
 
 /* How long a bounded device-side wait of the tcgen05 kernel polls before it gives up (nanoseconds; 0 restores the

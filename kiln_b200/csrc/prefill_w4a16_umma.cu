@@ -16,6 +16,10 @@
 // stores: lane (qd, c) owns K-pairs (2qd, 2qd+1), (2qd+8, 2qd+9) of column 8t + c, and the
 // 128B swizzle XORs the 16-byte chunk index with (column % 8) = c.
 //
+// Most prefill runs on CTA pairs (pair_w4a16_umma.cu), which shares the tile walk, the reduction and the fix-up with this kernel.
+// It keeps what pairs do not pay for or do not take: few row tiles of few columns, the fused all-gather, and problems of at most
+// 128 rows that the small-batch kernel does not take.  This file also holds the planner that picks between the three.
+//
 // Every wait in the kernel is bounded: a wait that runs out records an error code in the
 // device status word, raises a CTA-wide abort flag that every other wait polls, and the CTA
 // drains its outstanding TMA copies, frees its TMEM and returns.

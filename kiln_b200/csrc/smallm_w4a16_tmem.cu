@@ -24,21 +24,22 @@
 // 128-column tiles; the epilogue adds the two), so the two kernels' results are bit-identical.
 // Roles (640 threads): warp 0 packed words, warps 1 and 2 MMA issuers, warp 3 scales and activations, warps 4-19 dequant, then
 // the epilogue.
-// Warp x of a team owns TMEM lanes 32(x%4)..+31 = words h and h + 2 (h = x % 2) of chunk (x%4)/2: lanes 0..15 hold columns
-// 16h + r, lanes 16..31 columns 32 + 16h + r of the chunk.  With gate and up interleaved in runs of 32 columns (SwiGLU) a
-// gate column and its up column are thus 16 lanes apart and meet through one shuffle.
+// Warp x of a team owns TMEM lanes 32(x%4)..+31 = words 2h and 2h + 1 (h = x % 2) of chunk (x%4)/2, columns 32h..+31, which one
+// 8-byte read per lane brings.  With SwiGLU, words h and h + 2 (of a 16-byte read): lanes 0..15 hold columns 16h + r, lanes 16..31
+// columns 32 + 16h + r, so that with gate and up interleaved in runs of 32 columns a gate column and its up column are 16 lanes
+// apart and meet through one shuffle.
 // LoRA delta (grouped scales): an extra iteration at the start of a tile's K range, its tensor-memory operand the tile's rows of
 // lora_b and its activation tile t = scale * x * A^T (bf16, written by the kernel launched just before).
 // Every wait is bounded (w4a16_async.cuh).  Per-column scales (group size -1): the weights are dequantised unscaled and the
 // scale multiplies the finished sums.
 //
-// What bounds it: about 0.32 us per 128 K and CTA up to 64 rows.  The dequant arithmetic needs 334 cycles of every
-// sub-partition (16 instructions per packed word, each two cycles on its pipe), shared memory about 450 (words in and out,
-// activations in and out), and a launch has 3.4 us that no stage hides (the first words' latency after a CTA of the
-// previous kernel has left the SM, the exchange, the exit).  CUDA graph over rotating weights, before (register-streamed
-// words, quad transposes, split-K through global slabs and a second kernel) -> now: 64 rows 2560 -> 18432 14.0 -> 10.4 us,
-// 2560 -> 4096 8.5 -> 6.7, 4096 -> 2560 8.9 -> 6.9, 2560 -> 8192 10.9 -> 8.4, 9216 -> 2560 12.0 -> 9.2; 128 rows 2560 -> 18432
-// 16.0 -> 12.2, 9216 -> 2560 13.6 -> 12.7.
+// What bounds it: about 0.3 us per 128 K and CTA up to 64 rows.  The dequant needs 250 to 330 issue slots of every
+// sub-partition (eleven instructions per packed word, fifteen with scales), the eight MMAs 430 cycles of one issuer, and a launch has
+// 2.5 to 3.4 us that no stage hides (the first words' latency after a CTA of the previous kernel has left the SM, the exchange, the
+// exit).  CUDA graph over rotating weights, before (register-streamed words, quad transposes, split-K through global slabs and
+// a second kernel) -> now: 64 rows 2560 -> 18432 14.0 -> 10.3 us, 2560 -> 4096 8.5 -> 5.3, 4096 -> 2560 8.9 -> 5.7, 2560 -> 8192
+// 10.9 -> 7.1, 9216 -> 2560 12.0 -> 9.0; 128 rows 2560 -> 18432 16.0 -> 12.1.  EXACT, against the decode kernel: 16 rows
+// 2560 -> 18432 12.2 -> 9.6, 2560 -> 4096 5.7 -> 4.5; 64 rows 2560 -> 512 5.8 -> 3.4.
 #include <algorithm>
 
 #include "w4a16_common.cuh"
@@ -363,8 +364,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (lane == 0) mbar_arrive(full(0));
             it = kTeams;
         }
-        // scales of the lane's four columns c, c + 8 (word h) and c + 32, c + 40 (word h + 2): positions 8c + 2h + {0, 1} and
-        // 8c + 2h + 4 + {0, 1} of the chunk's scale order (position 8i + j holds column 8j + i)
+        // scales of the lane's four columns c and c + 8 of its two words: word w has them at positions 8c + 2w + {0, 1} of the
+        // chunk's scale order (position 8i + j holds column 8j + i)
         const uint32_t sc_addr = smem_base + p.off_scale + (ch * 64 + 8 * c + (SWIGLU ? 2 : 4) * h) * 2;
         const uint32_t w_addr = smem_base + ch * 512 + lane * 16;
         int s = it % kSlots, ph = (it / kSlots & 1) ^ 1;                               // slot of the iteration
@@ -404,7 +405,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         for (; it < n_it && ok; it += kTeams) {
             if (it >= kSlots && it < kSlots + kTeams) pdl_wait();  // (park until the MMAs may run)
             if (!w_ready && !(ok = mbar_wait(bar(kBarWFull + ws), wph, abort_flag, p.status, 0xE00u | ws, p.wait_limit_ns))) break;
-            uint32_t wa[8], wb[8];  // words h and h + 2 of the eight K tiles
+            uint32_t wa[8], wb[8];  // the two words of the eight K tiles
 #pragma unroll
             for (int kt = 0; kt < 8; ++kt) {
                 if (SWIGLU) {
