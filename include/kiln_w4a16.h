@@ -163,6 +163,10 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_allgather_multicast(const void *A, cons
  * a launch that needs less (the small-batch kernel keeps its split sums in shared memory) leaves it alone. */
 size_t kiln_w4a16_workspace_bytes(int m, int n, int k);
 
+/* The part of it that this call will use, at most kiln_w4a16_workspace_bytes_ex: for callers that allocate per call.  ep may
+ * be NULL.  No counterpart in the reference. */
+size_t kiln_w4a16_scratch_bytes(int m, int n, int k, int groupsize, const kiln_w4a16_epilogue_t *ep);
+
 /* Shape rule of the path (crates/kiln-model/src/marlin_proj.rs:53-55): 1 if supported. */
 int kiln_w4a16_shape_is_supported(int k, int n);
 

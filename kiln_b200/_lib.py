@@ -48,6 +48,7 @@ SIGNATURES = {
     "kiln_marlin_w4a16_gemm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i]),
     "kiln_w4a16_gemm_bf16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
     "kiln_w4a16_workspace_bytes_ex": (_sz, [_i, _i, _i, ctypes.POINTER(Epilogue)]),
+    "kiln_w4a16_scratch_bytes": (ctypes.c_size_t, [_i, _i, _i, _i, _vp]),
     "kiln_w4a16_gemm_bf16_ex": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, ctypes.POINTER(Epilogue), _vp, _sz, _vp]),
     "kiln_w4a16_gemm_bf16_grouped": (_i, [ctypes.POINTER(Problem), _i, _vp, _sz, _vp]),
     "kiln_w4a16_gemm_bf16_noalloc": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
@@ -115,8 +116,8 @@ def native():
             mod = importlib.import_module("kiln_b200._native")
         except ModuleNotFoundError as e:
             raise ImportError("kiln_b200/_native.so is missing: run `python -m kiln_b200.build`") from e
-        names = ("kiln_w4a16_gemm_bf16", "kiln_w4a16_workspace_bytes", "kiln_w4a16_gemm_bf16_ex", "kiln_w4a16_workspace_bytes_ex",
-                 "kiln_w4a16_gemm_bf16_grouped", "kiln_w4a16_quantize_and_pack_device", "kiln_w4a16_repack_gptq_device")
+        names = ("kiln_w4a16_gemm_bf16", "kiln_w4a16_scratch_bytes", "kiln_w4a16_gemm_bf16_ex", "kiln_w4a16_gemm_bf16_grouped",
+                 "kiln_w4a16_quantize_and_pack_device", "kiln_w4a16_repack_gptq_device")
         mod.bind(*(ctypes.cast(getattr(lib(), name), _vp).value for name in names))
         _native = mod
     return _native

@@ -110,11 +110,16 @@ static int launch_small(const GemmArgs &a) { return use_exact(a) ? launch_exact(
 // no epilogue option and no fused all-gather: what the small-batch tcgen05 kernel takes
 static bool plain_gemm(const GemmArgs &a) { return !a.swiglu && a.lora_r == 0 && a.n_peers == 0 && !a.mc_c && !a.no_scratch; }
 
+// What a plain GEMM on the tcgen05 kernels uses of its workspace: the small-batch kernel keeps its split sums in shared memory.
+static size_t gemm_scratch(int m, int n, int k, int groupsize) {
+    return smallm_takes(m, n, k, groupsize) ? 0 : prefill_workspace_bytes(m, n, k);
+}
+
 static int gemm(const GemmArgs &a) {
     const int v = validate(a);
     if (v >= 0) return v;
     if (use_prefill(a.m, a.n, a.k, a.groupsize, plain_gemm(a))) {
-        const size_t need = a.no_scratch || smallm_takes(a.m, a.n, a.k, a.groupsize) ? 0 : prefill_workspace_bytes(a.m, a.n, a.k);
+        const size_t need = a.no_scratch ? 0 : gemm_scratch(a.m, a.n, a.k, a.groupsize);
         if (need > 0 && (!a.workspace || a.workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
         return launch_prefill(a);
     }
@@ -227,6 +232,33 @@ size_t kiln_w4a16_workspace_bytes_ex(int m, int n, int k, const kiln_w4a16_epilo
     return need;
 }
 
+// How a call with epilogue options runs, and the bytes of its workspace that this takes: at most what kiln_w4a16_workspace_bytes_ex,
+// which knows neither the group size nor what the small-batch kernel saves, asks for.
+struct ExPlan {
+    bool tc, fuse_lora, fuse_swiglu, composed;
+    size_t gemm, scratch;
+};
+static ExPlan plan_ex(int m, int n, int k, int groupsize, const kiln_w4a16_epilogue_t *ep) {
+    ExPlan x = {};
+    x.tc = use_prefill(m, n, k, groupsize, ex_plain(ep, m, n, k));
+    x.scratch = align256(static_cast<size_t>(m) * ep->lora_rank * sizeof(float));
+    if (!x.tc) return x;
+    x.fuse_lora = ep->lora_rank && prefill_fuses_lora(groupsize, ep->lora_rank);
+    x.fuse_swiglu = ep->swiglu && prefill_fuses_swiglu(m, n, k);
+    x.composed = (ep->swiglu && !x.fuse_swiglu) || (ep->lora_rank && !x.fuse_lora);
+    // (SwiGLU is fused into whole tiles, which need none)
+    x.gemm = !x.composed && x.fuse_swiglu ? 0 : gemm_scratch(m, n, k, groupsize);
+    if (x.composed) x.scratch += align256(static_cast<size_t>(m) * n * 2);
+    x.scratch += align256(x.gemm);
+    return x;
+}
+
+size_t kiln_w4a16_scratch_bytes(int m, int n, int k, int groupsize, const kiln_w4a16_epilogue_t *ep) {
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    if (ep && (ep->swiglu || ep->lora_rank)) return plan_ex(m, n, k, groupsize, ep).scratch;
+    return use_prefill(m, n, k, groupsize, true) ? gemm_scratch(m, n, k, groupsize) : 0;
+}
+
 kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *C, const void *s, int m, int n, int k,
                                             int groupsize, const kiln_w4a16_epilogue_t *ep, void *workspace,
                                             size_t workspace_bytes, void *stream) {
@@ -236,12 +268,10 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
     GemmArgs a{A, B, s, C, m, n, k, groupsize, workspace, workspace_bytes, static_cast<cudaStream_t>(stream)};
     const int v = validate(a);
     if (v >= 0) return v;
-    const size_t need = kiln_w4a16_workspace_bytes_ex(m, n, k, ep);
-    if (need > 0 && (!workspace || workspace_bytes < need)) return KILN_W4A16_ERR_WORKSPACE;
+    const ExPlan x = plan_ex(m, n, k, groupsize, ep);
+    if (x.scratch > 0 && (!workspace || workspace_bytes < x.scratch)) return KILN_W4A16_ERR_WORKSPACE;
     uint8_t *ws = static_cast<uint8_t *>(workspace);
-    const bool tc = use_prefill(m, n, k, groupsize, ex_plain(ep, m, n, k));
-    const bool fuse_lora = tc && ep->lora_rank && prefill_fuses_lora(groupsize, ep->lora_rank);
-    const bool fuse_swiglu = tc && ep->swiglu && prefill_fuses_swiglu(m, n, k);
+    const bool tc = x.tc, fuse_lora = x.fuse_lora, fuse_swiglu = x.fuse_swiglu;
     void *t = nullptr;
     if (ep->lora_rank) {
         t = ws;  // fp32 [m, r] for the decode kernel and the composed pass, bf16 [m, r] as an operand of the tcgen05 kernel
@@ -255,13 +285,13 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
         a.swiglu = ep->swiglu ? 1 : 0;
         return launch_small(a);
     }
-    const bool composed = (ep->swiglu && !fuse_swiglu) || (ep->lora_rank && !fuse_lora);
+    const bool composed = x.composed;
     void *tmp = nullptr;
     if (composed) {
         tmp = ws;
         ws += align256(static_cast<size_t>(m) * n * 2);
     }
-    GemmArgs b{A, B, s, composed ? tmp : C, m, n, k, groupsize, ws, prefill_workspace_bytes(m, n, k), a.stream};
+    GemmArgs b{A, B, s, composed ? tmp : C, m, n, k, groupsize, ws, x.gemm, a.stream};
     if (fuse_lora) {
         b.lora_t = t;
         b.lora_b = ep->lora_b;

@@ -35,9 +35,8 @@ using at::Tensor;
 
 struct Abi {
     decltype(&kiln_w4a16_gemm_bf16) gemm;
-    decltype(&kiln_w4a16_workspace_bytes) workspace;
+    decltype(&kiln_w4a16_scratch_bytes) scratch;
     decltype(&kiln_w4a16_gemm_bf16_ex) gemm_ex;
-    decltype(&kiln_w4a16_workspace_bytes_ex) workspace_ex;
     decltype(&kiln_w4a16_gemm_bf16_grouped) grouped;
     decltype(&kiln_w4a16_quantize_and_pack_device) pack;
     decltype(&kiln_w4a16_repack_gptq_device) gptq;
@@ -127,7 +126,7 @@ PyObject *guarded(F &&f) {  // C++ exceptions (out of memory, say) -> Python
 PyObject *run_gemm(const Tensor &x, long m, const Proj &p, Tensor out) {
     const c10::cuda::CUDAGuard guard(x.device());
     if (!out.defined()) out = new_output(x, p.n);
-    const size_t need = abi.workspace(static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k));
+    const size_t need = abi.scratch(static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k), static_cast<int>(p.groupsize), nullptr);
     Tensor ws;
     if (need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x.device());
     void *const wp = need ? ws.mutable_data_ptr() : nullptr, *const stream = c10::cuda::getCurrentCUDAStream().stream();
@@ -197,7 +196,7 @@ PyObject *py_gemm_ex(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const c10::cuda::CUDAGuard guard(x->device());
         if (!out.defined()) out = new_output(*x, n_out);
         const int mi = static_cast<int>(m), ni = static_cast<int>(p.n), ki = static_cast<int>(p.k);
-        const size_t need = abi.workspace_ex(mi, ni, ki, &ep);
+        const size_t need = abi.scratch(mi, ni, ki, static_cast<int>(p.groupsize), &ep);
         Tensor ws;
         if (need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x->device());
         void *const wp = need ? ws.mutable_data_ptr() : nullptr, *const stream = c10::cuda::getCurrentCUDAStream().stream();
@@ -243,7 +242,7 @@ PyObject *py_grouped(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         for (Py_ssize_t i = 0; i < count; ++i) {
             if (!given) outs[i] = new_output(*xs[i], prob[i].n);
             prob[i].C = outs[i].mutable_data_ptr();
-            const size_t w = abi.workspace(prob[i].m, prob[i].n, prob[i].k);
+            const size_t w = abi.scratch(prob[i].m, prob[i].n, prob[i].k, prob[i].groupsize, nullptr);
             if (w > need) need = w;
         }
         Tensor ws;
@@ -338,25 +337,24 @@ PyObject *py_pack_gptq(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     });
 }
 
-// bind(gemm, workspace, gemm_ex, workspace_ex, grouped, pack, gptq): addresses of the C ABI's entry points
+// bind(gemm, scratch, gemm_ex, grouped, pack, gptq): addresses of the C ABI's entry points
 PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    void *p[7];
-    if (nargs != 7) {
-        PyErr_SetString(PyExc_TypeError, "bind takes seven addresses");
+    void *p[6];
+    if (nargs != 6) {
+        PyErr_SetString(PyExc_TypeError, "bind takes six addresses");
         return nullptr;
     }
-    for (int i = 0; i < 7; ++i)
+    for (int i = 0; i < 6; ++i)
         if (!(p[i] = PyLong_AsVoidPtr(args[i]))) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null entry point");
             return nullptr;
         }
     abi.gemm = reinterpret_cast<decltype(abi.gemm)>(p[0]);
-    abi.workspace = reinterpret_cast<decltype(abi.workspace)>(p[1]);
+    abi.scratch = reinterpret_cast<decltype(abi.scratch)>(p[1]);
     abi.gemm_ex = reinterpret_cast<decltype(abi.gemm_ex)>(p[2]);
-    abi.workspace_ex = reinterpret_cast<decltype(abi.workspace_ex)>(p[3]);
-    abi.grouped = reinterpret_cast<decltype(abi.grouped)>(p[4]);
-    abi.pack = reinterpret_cast<decltype(abi.pack)>(p[5]);
-    abi.gptq = reinterpret_cast<decltype(abi.gptq)>(p[6]);
+    abi.grouped = reinterpret_cast<decltype(abi.grouped)>(p[3]);
+    abi.pack = reinterpret_cast<decltype(abi.pack)>(p[4]);
+    abi.gptq = reinterpret_cast<decltype(abi.gptq)>(p[5]);
     Py_RETURN_NONE;
 }
 

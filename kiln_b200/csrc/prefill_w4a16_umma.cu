@@ -754,11 +754,47 @@ double smallm_cost(int m, int n, int k, int splits) {
     return start + waves * step * stages + (waves - 1) * 3.0 + exchange;
 }
 
+// The models are asked several times per call with the same sizes and take 0.3 to 0.6 us each, as long as a quarter of a launch:
+// a thread keeps what they said for the sizes it met last.  (They depend on sizes and device alone.)
+template <class T>
+struct PlanMemo {
+    static constexpr int kEntries = 64;
+    struct Entry {
+        int dev = -1, m = 0, n = 0, k = 0;
+        T plan{};
+    } entry[kEntries];
+    template <class F>
+    T get(int m, int n, int k, F &&model) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return model();
+        const unsigned hash = (static_cast<unsigned>(m) * 31u + static_cast<unsigned>(n >> 7)) * 31u + static_cast<unsigned>(k >> 7);
+        Entry &e = entry[(hash * 2654435761u) >> 26];
+        if (e.dev != dev || e.m != m || e.n != n || e.k != k) {
+            e.plan = model();
+            e.dev = dev;
+            e.m = m;
+            e.n = n;
+            e.k = k;
+        }
+        return e.plan;
+    }
+};
+
 int choose_smallm_splits(int m, int n, int k) {
-    int best = 1;
-    for (int s : {2, 3, 4, 6, 8})
-        if (s <= k / 128 && smallm_cost(m, n, k, s) < smallm_cost(m, n, k, best)) best = s;
-    return best;
+    static thread_local PlanMemo<int> memo;
+    return memo.get(m, n, k, [=] {
+        int best = 1;
+        double best_t = smallm_cost(m, n, k, 1);
+        for (int s : {2, 3, 4, 6, 8}) {
+            if (s > k / 128) break;
+            const double t = smallm_cost(m, n, k, s);
+            if (t < best_t) {
+                best_t = t;
+                best = s;
+            }
+        }
+        return best;
+    });
 }
 
 // Tilings of single CTAs.
@@ -834,11 +870,15 @@ PrefillConfig choose_prefill(int m, int n, int k, bool allow_pairs = true, bool 
         if (legal) return o;
     }
     if (!allow_pairs || single) return choose_single(m, n, k, false, allow_pairs, allow_scratch, max_split_bytes);
-    if (m > BM || !allow_scratch) return choose_any(m, n, k, allow_scratch);
-    // At most 128 rows: 128-column tiles, which the small-batch kernel shares; it may run fewer splits (exec_splits).
-    PrefillConfig c = choose_single(m, n, k, true, true, true, max_split_bytes);
-    c.splits = std::max(c.splits, choose_smallm_splits(m, n, k));
-    return c;
+    if (!allow_scratch) return choose_any(m, n, k, false);
+    static thread_local PlanMemo<PrefillConfig> memo;
+    return memo.get(m, n, k, [=] {
+        if (m > BM) return choose_any(m, n, k, true);
+        // At most 128 rows: 128-column tiles, which the small-batch kernel shares; it may run fewer splits (exec_splits).
+        PrefillConfig c = choose_single(m, n, k, true, true, true, ~static_cast<size_t>(0));
+        c.splits = std::max(c.splits, choose_smallm_splits(m, n, k));
+        return c;
+    });
 }
 
 // The K splits that a plain problem of at most 128 rows runs with, in the small-batch kernel and, when that is switched off, in the
