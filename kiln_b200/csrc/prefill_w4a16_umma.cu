@@ -735,8 +735,8 @@ unsigned long long g_wait_limit_ns = kWaitLimitNs;
 int g_test_drop_a_load = -1;
 int g_smallm_enabled = 1;
 
-// K splits of the small-batch kernel.  Its time in microseconds, fitted to 360 timed launches (CUDA graph over rotating weights;
-// K = 1024..9216 x N = 1536..18432 x 17..128 rows x every split; the splits it picks are within 2% of the best).  While its clusters
+// K splits of the small-batch kernel.  Its time in microseconds, fitted to 570 timed launches (CUDA graph over rotating weights;
+// K = 1024..9216 x N = 512..18432 x 9..128 rows x every split; the splits it picks are within 2% of the best).  While its clusters
 // take at most half the GPU, consecutive launches run side by side and only the chain from the grid-dependency wait to the exit
 // counts; above that a launch starts on the SMs the one before leaves.  A further wave of CTAs repeats that start; how many clusters
 // fit decides when there is one (4096 x 6144 has 48 tiles, and 3 splits need 48 clusters of 3 where 45 fit: 12.2 us, 2 splits 7.9).
@@ -745,13 +745,13 @@ double smallm_cost(int m, int n, int k, int splits) {
     const int tiles = n / 128, clusters = smallm_clusters(splits), waves = (tiles + clusters - 1) / clusters;
     const double stages = (k / 128 + splits - 1) / splits, rows = (m + 15) / 16 * 16;
     const double over = ((tiles < clusters ? tiles : clusters) / static_cast<double>(clusters) - 0.5) * device_sm_count();
-    double start = 2.08, step = 0.183 + 0.00137 * rows, exchange = 0.0;
+    double start = 1.86, step = 0.221 + 0.00092 * rows + (m > 64 ? 0.0091 : 0.0), exchange = 0.0;
     if (over > 0) {
-        start = 2.60 + 0.0224 * over;
-        step += 0.055 + (m > 64 ? 0.00038 * over - 0.0085 : 0.0);
+        start = 2.55 + 0.0228 * over;
+        step += 0.0433 + (m > 64 ? 0.00044 * over : 0.0);
     }
-    if (splits > 1) exchange = 0.0204 * rows * (splits - 1) / splits + (m > 64 ? 0.58 : 0.0);
-    return start + waves * step * stages + (waves - 1) * 3.0 + exchange;
+    if (splits > 1) exchange = 0.22 + 0.0174 * rows * (splits - 1) / splits + (m > 64 ? 0.65 : 0.0);
+    return start + waves * step * stages + (waves - 1) * 2.73 + exchange;
 }
 
 // The models are asked several times per call with the same sizes and take 0.3 to 0.6 us each, as long as a quarter of a launch:
