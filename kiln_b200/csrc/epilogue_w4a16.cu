@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__re
 // a row of x and of a row of A and uses them as the K slots {2qd, 2qd+1, 2qd+8, 2qd+9} of two m16n8k16 MMAs: the same K
 // permutation on both sides, so no shared-memory staging and no ldmatrix.
 // A CTA has WM row tiles of 16 and 8 / WM parts of its K range, one (row tile, part) per warp, and 8 NT adapter rows.  Small tiles
-// for few rows (enough CTAs to fill the GPU), large ones for many (x is read once per 8 NT adapter rows).  The parts meet in shared
+// nearly always (many CTAs, short chains: 64 rows, 9216 -> 2560 with its GEMM 21 -> 13 us against tiles of 64 x 32), large ones for
+// very many rows (x is read once per 8 NT adapter rows).  The parts meet in shared
 // memory, the cluster's partial tiles in rank order through distributed shared memory: the result does not depend on timing.
 // Measured with the GEMM that follows, dot products -> tensor cores: 37 rows rank 64 9216 -> 2560 24 -> 15 us, 2560 -> 4096 13.3 ->
 // 10.7, 2048 rows 96 -> 49; 4 rows 7.6 -> 8.2, hence the line above.
@@ -168,17 +169,19 @@ __global__ void __launch_bounds__(256) finish_kernel(const __nv_bfloat16 *__rest
 
 int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int k, int r, void *t, int bf16_out, cudaStream_t stream) {
     const bool dot = m <= kLoraDotRows;
-    // row tiles and adapter rows of a CTA: 16 x 16, 64 x 32 or 128 x 64
-    const int wm = m <= 48 ? 1 : (m <= 512 ? 4 : 8), rows = 16 * wm, cols = wm == 1 ? 16 : (wm == 4 ? 32 : 64), parts = 8 / wm;
+    // Rows and adapter rows of a CTA: 16 x 16, or 128 x 64 for more than 1024 rows of a large rank, where reading x once per 16
+    // adapter rows costs more than the longer chains of large tiles (2048 x 9216, rank 64, with its GEMM: 118 / 114 us; 1024 rows: 65 / 83).
+    const int wm = m > 1024 && r > 32 ? 8 : 1, rows = 16 * wm, cols = wm == 1 ? 16 : 64, parts = 8 / wm;
     const int row_tiles = (m + rows - 1) / rows, col_tiles = (r + cols - 1) / cols;
     if (row_tiles > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
-    // K is split over as many CTAs as the tiles leave SMs for, while a warp keeps at least two 32-deep blocks
-    int size = std::min(8, std::max(1, device_sm_count() / (row_tiles * col_tiles)));
+    // K is split over as many CTAs as the tiles leave room for (four small ones to an SM: 768 x 9216, rank 64 57.6 -> 51.3 us against
+    // one), while a warp keeps at least two 32-deep blocks
+    int size = std::min(8, std::max(1, (wm == 1 ? 4 : 1) * device_sm_count() / (row_tiles * col_tiles)));
     size = std::max(1, std::min(size, k / 32 / (2 * parts)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dot ? dim3((r + 7) / 8, m) : dim3(size, col_tiles, row_tiles);
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = dot ? 0 : (wm == 1 ? lora_smem<1, 2>() : (wm == 4 ? lora_smem<4, 4>() : lora_smem<8, 8>()));
+    cfg.dynamicSmemBytes = dot ? 0 : (wm == 1 ? lora_smem<1, 2>() : lora_smem<8, 8>());
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -192,7 +195,7 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     const auto *xp = static_cast<const __nv_bfloat16 *>(x), *ap = static_cast<const __nv_bfloat16 *>(lora_a);
     note_launch();
     if (dot) return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_dot_kernel, xp, ap, scale, k, r, t, bf16_out));
-    const auto kernel = wm == 1 ? lora_down_kernel<1, 2> : (wm == 4 ? lora_down_kernel<4, 4> : lora_down_kernel<8, 8>);
+    const auto kernel = wm == 1 ? lora_down_kernel<1, 2> : lora_down_kernel<8, 8>;
     return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out));
 }
 
