@@ -534,12 +534,14 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if constexpr (EXACT) {
                 const bool up = lane >= 16;
 #pragma unroll
+                for (int i = 0; i < 4; ++i) v4[i] *= cs;  // (before the exchange: the partner's column has a scale of its own)
+#pragma unroll
                 for (int i = 0; i < (SWIGLU ? 2 : 4); ++i) {
                     int row = 4 * u + i;
-                    float out = v4[i] * cs;
+                    float out = v4[i];
                     if constexpr (SWIGLU) {  // (as below)
                         const float other = __shfl_xor_sync(0xFFFFFFFFu, up ? v4[2 * i] : v4[2 * i + 1], 16);
-                        const float g = (up ? other : v4[2 * i]) * cs, w = (up ? v4[2 * i + 1] : other) * cs;
+                        const float g = up ? other : v4[2 * i], w = up ? v4[2 * i + 1] : other;
                         row = 4 * u + 2 * i + (up ? 1 : 0);
                         out = __fdividef(g, 1.f + __expf(-g)) * w;
                     }

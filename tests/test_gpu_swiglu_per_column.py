@@ -1,0 +1,29 @@
+"""SwiGLU with per-column scales (group size -1): gate and up columns that meet in an epilogue have scales of their own.  Against the fp64
+oracle, max|out - ref| / max|ref| <= 1e-2."""
+import numpy as np
+import pytest
+import torch
+
+import kiln_b200
+import oracle
+from kiln_b200 import _lib
+from oracle import C
+from tests.test_gpu_epilogue import _proj, _silu
+from tests.util import REL_TOL, from_torch_bf16, rel_err, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+# decode kernel; the small-batch kernel's fp32-scale variant from its smallest problem to its most rows, K of one stage and of more
+# than the teams; the small-batch kernel itself, 64 and 128 rows; CTA pairs
+@pytest.mark.parametrize("m,k,n_half", [(1, 2560, 512), (5, 640, 512), (9, 128, 128), (13, 2560, 256), (16, 9216, 1280), (17, 640, 384),
+                                        (129, 1536, 384), (256, 640, 512), (24, 2560, 9216), (64, 2560, 9216), (100, 640, 9216), (300, 1152, 512)])
+def test_each_column_keeps_its_own_scale(cuda_device, m, k, n_half):
+    a, qg, sg = oracle.synth_inputs(m, k, n_half, seed=m + k, groupsize=-1)
+    _, qu, su = oracle.synth_inputs(1, k, n_half, seed=m + k + 1, groupsize=-1)
+    fused = kiln_b200.interleave_gate_up(_proj(qg, sg, -1, cuda_device), _proj(qu, su, -1, cuda_device))
+    out = kiln_b200.swiglu_gate_up(to_torch_bf16(a, cuda_device), fused)
+    torch.cuda.synchronize()
+    assert _lib.lib().kiln_w4a16_check_device_status(None, None) == 0
+    ref = _silu(C.gemm_fp64(a, qg, sg, -1).astype(np.float64)) * C.gemm_fp64(a, qu, su, -1).astype(np.float64)
+    assert rel_err(from_torch_bf16(out), ref.astype(np.float32)) <= REL_TOL
