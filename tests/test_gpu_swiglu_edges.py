@@ -1,5 +1,5 @@
-"""SwiGLU with per-column scales (group size -1): gate and up columns that meet in an epilogue have scales of their own.  Against the fp64
-oracle, max|out - ref| / max|ref| <= 1e-2."""
+"""SwiGLU where its parts are easy to lose: per-column scales (group size -1), whose gate and up columns meet in an epilogue with scales of
+their own (against the fp64 oracle, max|out - ref| / max|ref| <= 1e-2), and gates near the end of the exponential's range."""
 import numpy as np
 import pytest
 import torch
@@ -27,3 +27,23 @@ def test_each_column_keeps_its_own_scale(cuda_device, m, k, n_half):
     assert _lib.lib().kiln_w4a16_check_device_status(None, None) == 0
     ref = _silu(C.gemm_fp64(a, qg, sg, -1).astype(np.float64)) * C.gemm_fp64(a, qu, su, -1).astype(np.float64)
     assert rel_err(from_torch_bf16(out), ref.astype(np.float32)) <= REL_TOL
+
+
+@pytest.mark.parametrize("m", [8, 9, 16])
+def test_silu_of_a_gate_near_its_underflow(cuda_device, m):
+    """gate = -87.5 .. -88.5: 1 + exp(-gate) lies above 2^126, where an approximate quotient is 0 and silu(gate) * up is still a normal
+    number of about 1e-35.  Relative error: half a unit of bf16, whose
+    eight-bit significand makes that at most 2^-8, plus the exponential's 2 + 1.173 * 88 units of fp32 (1e-5)."""
+    k, n_half = 128, 128
+    qg, qu = np.zeros((k, n_half), np.uint8), np.zeros((k, n_half), np.uint8)
+    qg[:], qu[:] = 8, 8          # zero, but for the first row: gate 7 x, up x
+    qg[0], qu[0] = 15, 9
+    s = np.ones((1, n_half), np.float16)
+    x = np.zeros((m, k), np.float32)
+    x[:, 0] = np.linspace(-12.64, -12.5, m)
+    x_t = torch.from_numpy(x).to(torch.bfloat16)
+    fused = kiln_b200.interleave_gate_up(_proj(qg, s, 128, cuda_device), _proj(qu, s, 128, cuda_device))
+    out = from_torch_bf16(kiln_b200.swiglu_gate_up(x_t.to(cuda_device), fused)).astype(np.float64)
+    v = x_t[:, 0].double().numpy()
+    ref = (7 * v / (1 + np.exp(-7 * v)) * v)[:, None]
+    assert np.abs(out / ref - 1).max() <= 2.0 ** -8 + 2e-5
