@@ -94,7 +94,7 @@ bool read_proj(PyObject *obj, const at::Device &dev, Proj &p) {
 
 // x [m, k], or [b, s, k] where that is allowed: rows of k bf16 values.
 bool activations_ok(const Tensor *x, long k, bool allow_rank3, long &m) {
-    if (!x || !(x->dim() == 2 || (allow_rank3 && x->dim() == 3)) || x->size(-1) != k) return false;
+    if (!x || !(x->dim() == 2 || (allow_rank3 && x->dim() == 3)) || k <= 0 || x->size(-1) != k) return false;
     m = x->numel() / k;
     return m > 0 && m <= INT32_MAX;
 }
