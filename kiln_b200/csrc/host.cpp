@@ -55,9 +55,11 @@ Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device &dev) {
     return Tensor(at::detail::empty_cuda(size, type, dev, std::nullopt));
 }
 
-// A packed projection whose tensors fit together and live on `dev`.
+// A packed projection whose tensors fit together and live on `dev`.  It owns them until the launch is enqueued: an attribute may be a
+// property that makes them on each read (weights kept in host memory, say), or be assigned by another thread while the GIL is free, and
+// memory that is given back before the launch is the next tensor's.
 struct Proj {
-    const void *b, *s;
+    Tensor b, s;
     long k, n, groupsize;
 };
 
@@ -67,10 +69,15 @@ bool weight_ok(Proj &p, const Tensor *b, const Tensor *s, const at::Device &dev)
     if (p.k <= 0 || p.n <= 0 || p.k % 128 || p.n % 256 || p.k > INT32_MAX || p.n > INT32_MAX / 2) return false;
     if (b->size(0) != p.k / 16 || b->size(1) != 2 * p.n) return false;
     if (s->size(0) != (p.groupsize == -1 ? 1 : p.k / 128) || s->size(1) != p.n) return false;
-    p.b = b->const_data_ptr();
-    p.s = s->const_data_ptr();
+    p.b = *b;
+    p.s = *s;
     return true;
 }
+
+struct Ref {  // an owned reference, or nullptr
+    PyObject *o;
+    ~Ref() { Py_XDECREF(o); }
+};
 
 bool read_long(PyObject *obj, PyObject *name, long &out) {
     PyObject *v = PyObject_GetAttr(obj, name);
@@ -86,7 +93,7 @@ bool read_proj(PyObject *obj, const at::Device &dev, Proj &p) {
     PyObject *b = PyObject_GetAttr(obj, name_b), *s = b ? PyObject_GetAttr(obj, name_s) : nullptr;
     bool ok = s && read_long(obj, name_g, p.groupsize) && read_long(obj, name_k, p.k) && read_long(obj, name_n, p.n) &&
               weight_ok(p, plain(b, at::kInt), plain(s, at::kHalf), dev);
-    Py_XDECREF(b);  // (the projection keeps its tensors for the length of the call)
+    Py_XDECREF(b);
     Py_XDECREF(s);
     if (PyErr_Occurred()) PyErr_Clear();
     return ok;
@@ -130,11 +137,11 @@ PyObject *run_gemm(const Tensor &x, long m, const Proj &p, Tensor out) {
     Tensor ws;
     if (need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x.device());
     void *const wp = need ? ws.mutable_data_ptr() : nullptr, *const stream = c10::cuda::getCurrentCUDAStream().stream();
-    const void *xp = x.const_data_ptr();
+    const void *xp = x.const_data_ptr(), *bp = p.b.const_data_ptr(), *sp = p.s.const_data_ptr();
     void *op = out.mutable_data_ptr();
     int rc;
     Py_BEGIN_ALLOW_THREADS;  // a launch blocks while the stream's queue is full
-    rc = abi.gemm(xp, p.b, op, p.s, static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k),
+    rc = abi.gemm(xp, bp, op, sp, static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k),
                   static_cast<int>(p.groupsize), wp, need, stream);
     Py_END_ALLOW_THREADS;
     return finish(rc, out);
@@ -146,7 +153,7 @@ PyObject *py_gemm(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         if (nargs != 5) Py_RETURN_NONE;
         const Tensor *x = plain(args[0], at::kBFloat16), *b = plain(args[1], at::kInt), *s = plain(args[2], at::kHalf);
         if (!x || !b || !s || !PyLong_CheckExact(args[3]) || x->dim() != 2 || s->dim() != 2) Py_RETURN_NONE;
-        Proj p{nullptr, nullptr, x->size(1), s->size(1), PyLong_AsLong(args[3])};
+        Proj p{Tensor(), Tensor(), x->size(1), s->size(1), PyLong_AsLong(args[3])};
         if (PyErr_Occurred()) PyErr_Clear();
         long m;
         Tensor out;
@@ -200,11 +207,11 @@ PyObject *py_gemm_ex(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         Tensor ws;
         if (need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x->device());
         void *const wp = need ? ws.mutable_data_ptr() : nullptr, *const stream = c10::cuda::getCurrentCUDAStream().stream();
-        const void *xp = x->const_data_ptr();
+        const void *xp = x->const_data_ptr(), *bp = p.b.const_data_ptr(), *sp = p.s.const_data_ptr();
         void *op = out.mutable_data_ptr();
         int rc;
         Py_BEGIN_ALLOW_THREADS;
-        rc = abi.gemm_ex(xp, p.b, op, p.s, mi, ni, ki, static_cast<int>(p.groupsize), &ep, wp, need, stream);
+        rc = abi.gemm_ex(xp, bp, op, sp, mi, ni, ki, static_cast<int>(p.groupsize), &ep, wp, need, stream);
         Py_END_ALLOW_THREADS;
         return finish(rc, out);
     });
@@ -218,24 +225,27 @@ PyObject *py_grouped(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
             Py_RETURN_NONE;
         const bool given = args[2] != Py_None;
         if (given && !(PyList_CheckExact(args[2]) || PyTuple_CheckExact(args[2]))) Py_RETURN_NONE;
-        const Py_ssize_t count = PySequence_Fast_GET_SIZE(args[0]);
-        if (count < 1 || count > KILN_W4A16_MAX_GROUP || PySequence_Fast_GET_SIZE(args[1]) != count ||
-            (given && PySequence_Fast_GET_SIZE(args[2]) != count))
+        // (tuples of our own: a list may change while a property of a projection runs, or while the GIL is free)
+        const Ref xt{PySequence_Tuple(args[0])}, pt{PySequence_Tuple(args[1])}, ot{given ? PySequence_Tuple(args[2]) : nullptr};
+        if (!xt.o || !pt.o || (given && !ot.o)) return nullptr;
+        const Py_ssize_t count = PyTuple_GET_SIZE(xt.o);
+        if (count < 1 || count > KILN_W4A16_MAX_GROUP || PyTuple_GET_SIZE(pt.o) != count || (given && PyTuple_GET_SIZE(ot.o) != count))
             Py_RETURN_NONE;
         kiln_w4a16_problem_t prob[KILN_W4A16_MAX_GROUP] = {};
         const Tensor *xs[KILN_W4A16_MAX_GROUP];
         Tensor outs[KILN_W4A16_MAX_GROUP];
+        Proj projs[KILN_W4A16_MAX_GROUP];
         size_t need = 0;
         for (Py_ssize_t i = 0; i < count; ++i) {
-            xs[i] = plain(PySequence_Fast_GET_ITEM(args[0], i), at::kBFloat16);
-            Proj p;
+            xs[i] = plain(PyTuple_GET_ITEM(xt.o, i), at::kBFloat16);
+            Proj &p = projs[i];
             long m;
-            if (!xs[i] || xs[i]->device() != xs[0]->device() || !read_proj(PySequence_Fast_GET_ITEM(args[1], i), xs[0]->device(), p) ||
+            if (!xs[i] || xs[i]->device() != xs[0]->device() || !read_proj(PyTuple_GET_ITEM(pt.o, i), xs[0]->device(), p) ||
                 !activations_ok(xs[i], p.k, false, m))
                 Py_RETURN_NONE;
-            if (given && !out_ok(PySequence_Fast_GET_ITEM(args[2], i), outs[i], m, p.n, xs[0]->device())) Py_RETURN_NONE;
-            prob[i] = {xs[i]->const_data_ptr(), p.b, nullptr, p.s, static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k),
-                       static_cast<int>(p.groupsize)};
+            if (given && !out_ok(PyTuple_GET_ITEM(ot.o, i), outs[i], m, p.n, xs[0]->device())) Py_RETURN_NONE;
+            prob[i] = {xs[i]->const_data_ptr(), p.b.const_data_ptr(), nullptr, p.s.const_data_ptr(), static_cast<int>(m), static_cast<int>(p.n),
+                       static_cast<int>(p.k), static_cast<int>(p.groupsize)};
         }
         const at::Device dev = xs[0]->device();
         const c10::cuda::CUDAGuard guard(dev);
@@ -258,7 +268,7 @@ PyObject *py_grouped(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         for (Py_ssize_t i = 0; i < count; ++i) {
             PyObject *o;
             if (given) {
-                o = PySequence_Fast_GET_ITEM(args[2], i);
+                o = PyTuple_GET_ITEM(ot.o, i);
                 Py_INCREF(o);
             } else if (!(o = THPVariable_Wrap(outs[i]))) {
                 Py_DECREF(list);

@@ -26,3 +26,42 @@ except kiln_b200.KilnMarlinError as e:
     print(e)
 """)
     assert "k=0 must be divisible by groupsize=128" in out
+
+
+class _Offloaded:
+    """A projection whose tensors are brought to the GPU whenever they are read."""
+
+    def __init__(self, proj):
+        self.b_cpu, self.s_cpu, self.groupsize, self.k, self.n = proj.b_packed.cpu(), proj.scales.cpu(), proj.groupsize, proj.k, proj.n
+
+    @property
+    def b_packed(self):
+        return self.b_cpu.to("cuda")
+
+    @property
+    def scales(self):
+        return self.s_cpu.to("cuda")
+
+
+def test_weights_made_on_each_read_live_until_the_launch(cuda_device):
+    """Memory of a weight that nobody holds goes to the next tensor of its size: the second projection of a group, the output, the
+    workspace.  Sizes on both sides of the allocator's 1 MB, so that each of those can happen."""
+    gen = torch.Generator().manual_seed(5)
+    for k, n, m in [(512, 256, 64), (512, 256, 5), (2560, 2560, 64), (1024, 2048, 1024)]:
+        def proj():
+            b = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 16, 2 * n), dtype=torch.int32, generator=gen)
+            s = (0.01 * torch.rand((k // 128, n), generator=gen) + 1e-3).to(torch.float16)
+            return kiln_b200.MarlinPackedProj(b.to(cuda_device), s.to(cuda_device), 128, k, n)
+
+        p, q = proj(), proj()
+        x = torch.randn((m, k), generator=gen).to(torch.bfloat16).to(cuda_device)
+        la, lb = torch.randn((16, k), generator=gen).to(torch.bfloat16).to(cuda_device), torch.randn((n, 16), generator=gen).to(torch.bfloat16).to(cuda_device)
+
+        def calls(p, q):
+            return [kiln_b200.matmul_bf16(x, p), kiln_b200.swiglu_gate_up(x, p), kiln_b200.matmul_bf16_lora(x, p, la, lb, 0.5),
+                    *kiln_b200.grouped_matmul_bf16([x, x], [p, q])]
+
+        want = calls(p, q)
+        for _ in range(5):
+            for got, ref in zip(calls(_Offloaded(p), _Offloaded(q)), want):
+                assert torch.equal(got, ref)
