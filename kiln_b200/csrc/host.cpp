@@ -120,6 +120,13 @@ Tensor new_output(const Tensor &x, long n) {
 
 PyObject *finish(int status, const Tensor &out) { return status ? PyLong_FromLong(status) : THPVariable_Wrap(out); }
 
+// Frees the GIL for as long as it lives (a launch blocks while the stream's queue is full).  An exception that leaves its scope takes the
+// GIL back before anything touches the interpreter.
+struct NoGil {
+    PyThreadState *state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 template <class F>
 PyObject *guarded(F &&f) {  // C++ exceptions (out of memory, say) -> Python
     try {
@@ -140,10 +147,11 @@ PyObject *run_gemm(const Tensor &x, long m, const Proj &p, Tensor out) {
     const void *xp = x.const_data_ptr(), *bp = p.b.const_data_ptr(), *sp = p.s.const_data_ptr();
     void *op = out.mutable_data_ptr();
     int rc;
-    Py_BEGIN_ALLOW_THREADS;  // a launch blocks while the stream's queue is full
-    rc = abi.gemm(xp, bp, op, sp, static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k),
-                  static_cast<int>(p.groupsize), wp, need, stream);
-    Py_END_ALLOW_THREADS;
+    {
+        const NoGil free;
+        rc = abi.gemm(xp, bp, op, sp, static_cast<int>(m), static_cast<int>(p.n), static_cast<int>(p.k),
+                      static_cast<int>(p.groupsize), wp, need, stream);
+    }
     return finish(rc, out);
 }
 
@@ -210,9 +218,10 @@ PyObject *py_gemm_ex(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const void *xp = x->const_data_ptr(), *bp = p.b.const_data_ptr(), *sp = p.s.const_data_ptr();
         void *op = out.mutable_data_ptr();
         int rc;
-        Py_BEGIN_ALLOW_THREADS;
-        rc = abi.gemm_ex(xp, bp, op, sp, mi, ni, ki, static_cast<int>(p.groupsize), &ep, wp, need, stream);
-        Py_END_ALLOW_THREADS;
+        {
+            const NoGil free;
+            rc = abi.gemm_ex(xp, bp, op, sp, mi, ni, ki, static_cast<int>(p.groupsize), &ep, wp, need, stream);
+        }
         return finish(rc, out);
     });
 }
@@ -259,9 +268,10 @@ PyObject *py_grouped(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         if (need) ws = empty({static_cast<int64_t>(need)}, at::kByte, dev);
         void *const wp = need ? ws.mutable_data_ptr() : nullptr, *const stream = c10::cuda::getCurrentCUDAStream().stream();
         int rc;
-        Py_BEGIN_ALLOW_THREADS;
-        rc = abi.grouped(prob, static_cast<int>(count), wp, need, stream);
-        Py_END_ALLOW_THREADS;
+        {
+            const NoGil free;
+            rc = abi.grouped(prob, static_cast<int>(count), wp, need, stream);
+        }
         if (rc) return PyLong_FromLong(rc);
         PyObject *list = PyList_New(count);
         if (!list) return nullptr;
@@ -300,9 +310,10 @@ PyObject *py_pack(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         int32_t *bp = static_cast<int32_t *>(b.mutable_data_ptr());
         uint16_t *sp = static_cast<uint16_t *>(s.mutable_data_ptr());
         int rc;
-        Py_BEGIN_ALLOW_THREADS;
-        rc = abi.pack(wp, bf16 ? 1 : 0, static_cast<int>(k), static_cast<int>(n), static_cast<int>(g), bp, sp, nullptr, stream);
-        Py_END_ALLOW_THREADS;
+        {
+            const NoGil free;
+            rc = abi.pack(wp, bf16 ? 1 : 0, static_cast<int>(k), static_cast<int>(n), static_cast<int>(g), bp, sp, nullptr, stream);
+        }
         if (rc) return PyLong_FromLong(rc);
         PyObject *pb = THPVariable_Wrap(b), *ps = pb ? THPVariable_Wrap(s) : nullptr;
         PyObject *pair = ps ? PyTuple_Pack(2, pb, ps) : nullptr;
@@ -331,12 +342,13 @@ PyObject *py_pack_gptq(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const Tensor bad = empty({1}, at::kInt, qw->device());
         void *const stream = c10::cuda::getCurrentCUDAStream().stream();
         int rc, count = 0;
-        Py_BEGIN_ALLOW_THREADS;
-        rc = abi.gptq(qw->const_data_ptr<int32_t>(), qz->const_data_ptr<int32_t>(), static_cast<const uint16_t *>(sc->const_data_ptr()),
-                      static_cast<int>(k), static_cast<int>(n), static_cast<int>(g), b.mutable_data_ptr<int32_t>(),
-                      static_cast<uint16_t *>(s.mutable_data_ptr()), static_cast<uint32_t *>(bad.mutable_data_ptr()), stream);
-        if (!rc) count = bad.item<int>();  // (waits for the device)
-        Py_END_ALLOW_THREADS;
+        {
+            const NoGil free;
+            rc = abi.gptq(qw->const_data_ptr<int32_t>(), qz->const_data_ptr<int32_t>(), static_cast<const uint16_t *>(sc->const_data_ptr()),
+                          static_cast<int>(k), static_cast<int>(n), static_cast<int>(g), b.mutable_data_ptr<int32_t>(),
+                          static_cast<uint16_t *>(s.mutable_data_ptr()), static_cast<uint32_t *>(bad.mutable_data_ptr()), stream);
+            if (!rc) count = bad.item<int>();  // (waits for the device)
+        }
         if (rc) return PyLong_FromLong(rc);
         if (count) Py_RETURN_FALSE;
         PyObject *pb = THPVariable_Wrap(b), *ps = pb ? THPVariable_Wrap(s) : nullptr;

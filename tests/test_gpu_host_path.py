@@ -65,3 +65,23 @@ def test_weights_made_on_each_read_live_until_the_launch(cuda_device):
         for _ in range(5):
             for got, ref in zip(calls(_Offloaded(p), _Offloaded(q)), want):
                 assert torch.equal(got, ref)
+
+
+def test_an_error_while_the_gil_is_free_arrives_as_a_python_exception(cuda_device):
+    """pack_from_gptq reads a counter back, which is refused while the stream is being captured."""
+    out = _child("""
+q = torch.zeros((16, 256), dtype=torch.int32, device=dev)
+z = torch.full((1, 32), -0x77777778, dtype=torch.int32, device=dev)
+s = torch.ones((1, 256), dtype=torch.float16, device=dev)
+assert kiln_b200.pack_from_gptq(q, z, s) is not None
+try:
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        try:
+            kiln_b200.pack_from_gptq(q, z, s)
+        except RuntimeError:
+            print("raised", flush=True)
+            raise
+except RuntimeError:
+    print("alive", flush=True)
+""")
+    assert out.split() == ["raised", "alive"]
