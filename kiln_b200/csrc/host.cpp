@@ -23,6 +23,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -128,11 +129,11 @@ struct NoGil {
 };
 
 template <class F>
-PyObject *guarded(F &&f) {  // C++ exceptions (out of memory, say) -> Python
+PyObject *guarded(F &&f) {  // C++ exceptions become the Python ones that torch's own functions raise (torch.OutOfMemoryError, say)
     try {
         return f();
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
 }

@@ -85,3 +85,23 @@ except RuntimeError:
     print("alive", flush=True)
 """)
     assert out.split() == ["raised", "alive"]
+
+
+def test_out_of_memory_keeps_its_type(cuda_device):
+    """What a server catches to evict and try again: for an output, a workspace and a packed weight alike."""
+    out = _child("""
+torch.cuda.set_per_process_memory_fraction((64 << 20) / torch.cuda.mem_get_info()[1])
+proj = kiln_b200.pack_from_bf16(torch.zeros((128, 1024), dtype=torch.bfloat16, device=dev))
+x = torch.zeros((8192, 128), dtype=torch.bfloat16, device=dev)
+w = torch.zeros((4096, 4096), dtype=torch.bfloat16, device=dev)
+big = kiln_b200.MarlinPackedProj(proj.b_packed.repeat(1, 8), proj.scales.repeat(1, 8), 128, 128, 8192)
+for call in (lambda: kiln_b200.matmul_bf16(x, big), lambda: kiln_b200.swiglu_gate_up(x, big), lambda: kiln_b200.grouped_matmul_bf16([x], [big]),
+             lambda: [kiln_b200.pack_from_bf16(w) for _ in range(8)]):
+    try:
+        held = call()
+        print("allocated")
+    except torch.OutOfMemoryError as e:
+        print("C++" if "Exception raised from" in str(e) else "out of memory")
+    held = None
+""")
+    assert out.split("\n")[:4] == ["out of memory"] * 4
