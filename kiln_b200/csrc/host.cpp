@@ -80,14 +80,15 @@ struct Ref {  // an owned reference, or nullptr
     ~Ref() { Py_XDECREF(o); }
 };
 
+bool as_long(PyObject *v, long &out) {  // false: not an int, or beyond a long (PyLong_AsLong says -1 then, which is a group size)
+    int overflow = 1;
+    if (PyLong_CheckExact(v)) out = PyLong_AsLongAndOverflow(v, &overflow);
+    return overflow == 0;
+}
+
 bool read_long(PyObject *obj, PyObject *name, long &out) {
-    PyObject *v = PyObject_GetAttr(obj, name);
-    if (!v) return false;
-    const bool ok = PyLong_CheckExact(v);
-    if (ok) out = PyLong_AsLong(v);
-    Py_DECREF(v);
-    if (PyErr_Occurred()) PyErr_Clear();
-    return ok;
+    const Ref v{PyObject_GetAttr(obj, name)};
+    return v.o && as_long(v.o, out);
 }
 
 bool read_proj(PyObject *obj, const at::Device &dev, Proj &p) {
@@ -161,9 +162,9 @@ PyObject *py_gemm(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
         if (nargs != 5) Py_RETURN_NONE;
         const Tensor *x = plain(args[0], at::kBFloat16), *b = plain(args[1], at::kInt), *s = plain(args[2], at::kHalf);
-        if (!x || !b || !s || !PyLong_CheckExact(args[3]) || x->dim() != 2 || s->dim() != 2) Py_RETURN_NONE;
-        Proj p{Tensor(), Tensor(), x->size(1), s->size(1), PyLong_AsLong(args[3])};
-        if (PyErr_Occurred()) PyErr_Clear();
+        if (!x || !b || !s || x->dim() != 2 || s->dim() != 2) Py_RETURN_NONE;
+        Proj p{Tensor(), Tensor(), x->size(1), s->size(1), 0};
+        if (!as_long(args[3], p.groupsize)) Py_RETURN_NONE;
         long m;
         Tensor out;
         if (!activations_ok(x, p.k, false, m) || !weight_ok(p, b, s, x->device())) Py_RETURN_NONE;
@@ -294,12 +295,11 @@ PyObject *py_grouped(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // pack(weight, groupsize) -> (b_packed, scales)
 PyObject *py_pack(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
-        if (nargs != 2 || !PyLong_CheckExact(args[1])) Py_RETURN_NONE;
+        long g;
+        if (nargs != 2 || !as_long(args[1], g)) Py_RETURN_NONE;
         const Tensor *w = plain(args[0], at::kBFloat16);
         const bool bf16 = w != nullptr;
         if (!w) w = plain(args[0], at::kFloat);
-        const long g = PyLong_AsLong(args[1]);
-        if (PyErr_Occurred()) PyErr_Clear();
         if (!w || w->dim() != 2 || (g != -1 && g != 128)) Py_RETURN_NONE;
         const int64_t k = w->size(0), n = w->size(1);
         if (k <= 0 || n <= 0 || k % 128 || n % 256 || k > INT32_MAX || n > INT32_MAX / 2) Py_RETURN_NONE;
@@ -327,10 +327,9 @@ PyObject *py_pack(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // pack_gptq(qweight, qzeros, scales, groupsize) -> (b_packed, scales), or False for an asymmetric checkpoint
 PyObject *py_pack_gptq(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
-        if (nargs != 4 || !PyLong_CheckExact(args[3])) Py_RETURN_NONE;
+        long g;
+        if (nargs != 4 || !as_long(args[3], g)) Py_RETURN_NONE;
         const Tensor *qw = plain(args[0], at::kInt), *qz = plain(args[1], at::kInt), *sc = plain(args[2], at::kHalf);
-        const long g = PyLong_AsLong(args[3]);
-        if (PyErr_Occurred()) PyErr_Clear();
         if (!qw || !qz || !sc || qw->dim() != 2 || qz->dim() != 2 || sc->dim() != 2 || (g != -1 && g != 128)) Py_RETURN_NONE;
         const int64_t k = qw->size(0) * 8, n = qw->size(1);
         if (k <= 0 || n <= 0 || k % 128 || n % 256 || k > INT32_MAX || n > INT32_MAX / 2) Py_RETURN_NONE;

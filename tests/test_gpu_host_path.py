@@ -105,3 +105,16 @@ for call in (lambda: kiln_b200.matmul_bf16(x, big), lambda: kiln_b200.swiglu_gat
     held = None
 """)
     assert out.split("\n")[:4] == ["out of memory"] * 4
+
+
+def test_a_group_size_beyond_a_long_is_refused(cuda_device):
+    w = torch.randn((128, 256), device=cuda_device).to(torch.bfloat16)
+    proj = kiln_b200.pack_from_bf16(w, -1)
+    x = torch.zeros((3, 128), dtype=torch.bfloat16, device=cuda_device)
+    for g in (2 ** 70, -2 ** 63 - 1, 2 ** 32 + 128):
+        for call in (lambda: kiln_b200.marlin_w4a16_gemm(x, proj.b_packed, proj.scales, g), lambda: kiln_b200.pack_from_bf16(w, g),
+                     lambda: kiln_b200.matmul_bf16(x, kiln_b200.MarlinPackedProj(proj.b_packed, proj.scales, g, 128, 256))):
+            with pytest.raises(kiln_b200.KilnMarlinError, match="groupsize must be -1 or 128"):
+                call()
+        qzeros = torch.full((1, 32), -0x77777778, dtype=torch.int32, device=cuda_device)
+        assert kiln_b200.pack_from_gptq(torch.zeros((16, 256), dtype=torch.int32, device=cuda_device), qzeros, proj.scales, g) is None
