@@ -48,8 +48,8 @@ typedef int kiln_w4a16_status_t;
  *     or the reference's own legal values are accepted, and they do not select a tile.
  * B is int32 [prob_k/16, 2*prob_n] in the Marlin layout, s is fp16
  * [prob_k/groupsize, prob_n] (one row for groupsize -1) in the Marlin scale order.
- * Stream-ordered, asynchronous, capturable in a CUDA graph after one warm-up call
- * per device (function attributes and tensor maps are created on first use). */
+ * Stream-ordered, asynchronous, capturable in a CUDA graph; a warm-up call is not needed (first use sets
+ * function attributes and finds addresses, and allocates nothing). */
 kiln_w4a16_status_t kiln_marlin_w4a16_gemm(const void *A, const void *B, void *C, void *s, int prob_m,
                                            int prob_n, int prob_k, void *workspace, int groupsize,
                                            int dev, void *stream, int thread_k, int thread_n, int sms,

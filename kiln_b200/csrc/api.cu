@@ -5,7 +5,6 @@
 // status mapping) and in its host dispatcher (kiln-marlin-gemm/csrc/marlin_kernel.cu:731-819:
 // shape -> kernel/tile choice), so that both are testable without a Rust toolchain.
 #include <atomic>
-#include <mutex>
 
 #include "w4a16_common.cuh"
 
@@ -41,21 +40,22 @@ int device_sm_count() {
     return cached[dev];
 }
 
-// One status word per device, in its own small allocation made on first use (outside any
-// stream capture: call the GEMM once before capturing).
+// One status word per device, in the library's image as the decode kernel's is: no launch allocates for it, so that a call of any size may be
+// the first of its kind inside a stream capture.
+static __device__ __align__(256) uint32_t g_status_word;
+
 uint32_t *device_status_word() {
-    static uint32_t *words[64] = {};
-    static std::mutex mu;
+    static std::atomic<uint32_t *> words[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!words[dev]) {
-        uint32_t *p = nullptr;
-        if (record_cuda_error(cudaMalloc(&p, 256))) return nullptr;
-        if (record_cuda_error(cudaMemset(p, 0, 256))) return nullptr;
-        words[dev] = p;
+    uint32_t *word = words[dev].load(std::memory_order_acquire);
+    if (!word) {
+        void *p = nullptr;
+        if (record_cuda_error(cudaGetSymbolAddress(&p, g_status_word))) return nullptr;
+        word = static_cast<uint32_t *>(p);
+        words[dev].store(word, std::memory_order_release);
     }
-    return words[dev];
+    return word;
 }
 
 static int validate(const GemmArgs &a) {
