@@ -597,7 +597,9 @@ __global__ void repack_words_kernel(const uint8_t *q, int n, int32_t *b_packed) 
 
 // GPTQ qweight int32 [k/8, n] -> packed words.  A thread takes one c of one 16-row tile and 64-column chunk: the two GPTQ words
 // (rows 0-7 and 8-15 of the tile) of columns 16j + c and 16j + 8 + c give the words (c, qd) for every qd, byte qd of each being
-// rows 2qd and 2qd + 1; the sixteen words of c are 64 contiguous bytes.  grid = (n/64, ceil(k/16/32)), block = 256.
+// rows 2qd and 2qd + 1; the sixteen words of c are 64 contiguous bytes.  WIDE: b_packed is 16-byte aligned (an int32 buffer of a C caller
+// need not be).  grid = (n/64, ceil(k/16/32)), block = 256.
+template <bool WIDE>
 __global__ void __launch_bounds__(256) repack_gptq_words_kernel(const int32_t *qweight, int n, int k_tiles, int32_t *b_packed) {
     const int c = threadIdx.x & 7, kb = blockIdx.y * 32 + (threadIdx.x >> 3), ch = blockIdx.x;
     if (kb >= k_tiles) return;
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(256) repack_gptq_words_kernel(const int32_t *q
     for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int t = 0; t < 8; ++t) in[r][t] = __ldg(src + static_cast<size_t>(r) * n + t * 8);
-    uint4 *dst = reinterpret_cast<uint4 *>(b_packed + static_cast<size_t>(kb) * 2 * n + ch * 128) + c * 4;
+    int32_t *dst = b_packed + static_cast<size_t>(kb) * 2 * n + ch * 128 + c * 16;
 #pragma unroll
     for (int qd = 0; qd < 4; ++qd) {
         uint32_t out[4];
@@ -622,7 +624,12 @@ __global__ void __launch_bounds__(256) repack_gptq_words_kernel(const int32_t *q
             const uint32_t e2 = (ev | (ev >> 4)) & 0x00FF00FFu, o2 = (od | (od >> 4)) & 0x00FF00FFu;
             out[j] = ((e2 | (e2 >> 8)) & 0xFFFFu) | ((o2 | (o2 >> 8)) << 16);
         }
-        dst[qd] = make_uint4(out[0], out[1], out[2], out[3]);
+        if constexpr (WIDE) {
+            reinterpret_cast<uint4 *>(dst)[qd] = make_uint4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[qd * 4 + j] = static_cast<int32_t>(out[j]);
+        }
     }
 }
 
@@ -738,7 +745,8 @@ kiln_w4a16_status_t kiln_w4a16_repack_gptq_device(const int32_t *qweight, const 
             qzeros, words, asymmetric);
         ++launches;
     }
-    repack_gptq_words_kernel<<<dim3(n / 64, (k / 16 + 31) / 32), 256, 0, st>>>(qweight, n, k / 16, b_packed);
+    const auto repack = (reinterpret_cast<uintptr_t>(b_packed) & 15) == 0 ? repack_gptq_words_kernel<true> : repack_gptq_words_kernel<false>;
+    repack<<<dim3(n / 64, (k / 16 + 31) / 32), 256, 0, st>>>(qweight, n, k / 16, b_packed);
     permute_scales_kernel<<<dim3((n + 127) / 128, k / g), 128, 0, st>>>(scales, n, groupsize == -1, scales_perm);
     pack_fence_kernel<<<1, 32, 0, st>>>();
     note_launch(launches);
