@@ -541,8 +541,9 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     float out = v4[i];
                     if constexpr (SWIGLU) {  // (as below)
                         const float other = __shfl_xor_sync(0xFFFFFFFFu, up ? v4[2 * i] : v4[2 * i + 1], 16);
-                        const float g = up ? other : v4[2 * i], w = up ? v4[2 * i + 1] : other;
                         row = 4 * u + 2 * i + (up ? 1 : 0);
+                        // (the division is slow for a dividend of zero, which rows past m would have)
+                        const float g = m0 + row < p.m ? (up ? other : v4[2 * i]) : 1.f, w = up ? v4[2 * i + 1] : other;
                         out = g / (1.f + __expf(-g)) * w;  // (as the decode kernel divides: __fdividef gives 0 for a divisor above 2^126)
                     }
                     st_shared_bf16(stage + row * 128 + ((chunk16 ^ (row & 7)) << 4), __float2bfloat16_rn(out));
