@@ -238,7 +238,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         bool ok = true;
         for (; ok && wi.next(mt, nt, sp, ki0, ki1, slab); ++tile) {
             const uint32_t acc = tile & 1, acc_ph = (tile >> 1) & 1;
-            if (!(ok = mbar_wait(tmem_full(acc), acc_ph, abort_flag, p.status, 0x500u | acc, p.wait_limit_ns))) break;
+            if (!(ok = warp_all(mbar_wait(tmem_full(acc), acc_ph, abort_flag, p.status, 0x500u | acc, p.wait_limit_ns)))) break;
             tc_fence_after();
             const int row = mt * kTileM + rank * kHalf + quarter * 32 + lane;
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * TN;
@@ -401,11 +401,11 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         int s = team, ws = team;
         uint32_t ph = 1, wph = 0;
         bool ok = true, w_ready = false, s_ready = false;  // the next waits, asked ahead
-        while (ok && wi.next(mt, nt, sp, ki0, ki1, slab)) {
+        while (wi.next(mt, nt, sp, ki0, ki1, slab)) {
             const int ki1e = ki1 + (ki0 == 0 ? p.lora_steps : 0);
             int ki = ki0 + skip;
-            for (; ki < ki1e; ki += kTeams) {
-                if (!w_ready && !(ok = mbar_wait(word_full(ws), wph, abort_flag, p.status, 0x900u | ws, p.wait_limit_ns))) break;
+            for (; ki < ki1e; ki += kTeams) {  // (to the end, whatever a wait says: see warp_all)
+                if (ok && !w_ready) ok = mbar_wait(word_full(ws), wph, abort_flag, p.status, 0x900u | ws, p.wait_limit_ns);
                 uint4 w[C::kBlocks], sc = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);  // (per-column scales come in the epilogue)
                 uint32_t s2[8];
                 if (ki < ki1) {
@@ -415,8 +415,8 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     scale_pairs(sc, s2);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(word_empty(ws));  // in registers: the slot can load again
-                if (!s_ready && !(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0x600u | s, p.wait_limit_ns))) break;
+                if (ok && lane == 0) mbar_arrive(word_empty(ws));  // in registers: the slot can load again
+                if (ok && !s_ready) ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0x600u | s, p.wait_limit_ns);
                 if (ki < ki1) {
 #pragma unroll
                     for (int b = 0; b < C::kBlocks; ++b) {
@@ -426,7 +426,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 }
                 fence_proxy_async_smem();  // every thread publishes its own stores to the async proxy
                 __syncwarp();
-                if (lane == 0) arrive_cluster(leader_full0 + 8u * s);
+                if (ok && lane == 0) arrive_cluster(leader_full0 + 8u * s);
                 if ((s += kTeams) >= kStages) {
                     s -= kStages;
                     ph ^= 1;

@@ -233,7 +233,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll 1
             for (int h = 0; h < MT && ok; ++h) {
             const uint32_t acc = acc0 + h;
-            if (!(ok = mbar_wait(tmem_full(acc), acc_ph, abort_flag, p.status, 0x500u | acc, p.wait_limit_ns))) break;
+            if (!(ok = warp_all(mbar_wait(tmem_full(acc), acc_ph, abort_flag, p.status, 0x500u | acc, p.wait_limit_ns)))) break;
             tc_fence_after();
             const int row = (mt * MT + h) * BM + quarter * 32 + lane;
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * KP * BN;

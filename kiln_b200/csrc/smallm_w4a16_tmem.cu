@@ -371,7 +371,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         int s = it % kSlots, ph = (it / kSlots & 1) ^ 1;                               // slot of the iteration
         int ws = (it - lora_it) % p.w_slots, wph = ((it - lora_it) / p.w_slots) & 1;  // slot of its packed words
         bool w_ready = false, t_ready = false;  // the next waits, asked ahead
-        if (it < n_it && !p.per_column) ok = mbar_wait(bar(kBarScales), 0, abort_flag, p.status, 0xEC0u, p.wait_limit_ns);
+        if (it < n_it && !p.per_column) ok = warp_all(mbar_wait(bar(kBarScales), 0, abort_flag, p.status, 0xEC0u, p.wait_limit_ns));
         // EXACT: the CTA's part of the LoRA rank (the K splits share it), and its values of lora_b for the tile's columns, a weight that
         // is there before it is needed; 16 bytes more per row keep the reads off each other's banks
         const int lora_0 = 8 * (rank * (p.lora_r / 8) / p.splits), lora_n = 8 * ((rank + 1) * (p.lora_r / 8) / p.splits) - lora_0;
@@ -390,7 +390,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int col_in_chunk = col_in_tile & 63;
         const uint32_t exact_sc = smem_base + p.off_scale + (ch * 64 + 8 * (col_in_chunk & 7) + (col_in_chunk >> 3)) * 2;
         auto add_stage = [&](int j, int s, int ph) {
-            if (!mbar_test(empty(s), ph) && !(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xF00u | s, p.wait_limit_ns))) return;
+            if (ok && !mbar_test(empty(s), ph)) ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xF00u | s, p.wait_limit_ns);
             __syncwarp();
             tc_fence_after();
             const float scale = p.per_column ? 1.f : lds_half(exact_sc + j * kScaleBytes);
@@ -402,9 +402,9 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             for (int i = 0; i < (EXACT ? kExactRows : 1); ++i) y[i] = fmaf(scale, __uint_as_float(a[i]) + __uint_as_float(b[i]), y[i]);
         };
         int s0 = 0, ph0 = 0;  // slot of the team's previous stage, and the phase that ends with it
-        for (; it < n_it && ok; it += kTeams) {
+        for (; it < n_it; it += kTeams) {  // (to the end, whatever a wait says: see warp_all)
             if (it >= kSlots && it < kSlots + kTeams) pdl_wait();  // (park until the MMAs may run)
-            if (!w_ready && !(ok = mbar_wait(bar(kBarWFull + ws), wph, abort_flag, p.status, 0xE00u | ws, p.wait_limit_ns))) break;
+            if (ok && !w_ready) ok = mbar_wait(bar(kBarWFull + ws), wph, abort_flag, p.status, 0xE00u | ws, p.wait_limit_ns);
             uint32_t wa[8], wb[8];  // the two words of the eight K tiles
 #pragma unroll
             for (int kt = 0; kt < 8; ++kt) {
@@ -428,8 +428,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 sc[2 * i + 1] = __floats2bfloat162_rn(f1, f1);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(kBarWEmpty + ws));  // the stage's words are in registers: its slot can load again
-            if (it >= kSlots && !t_ready && !(ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xE80u | s, p.wait_limit_ns))) break;
+            if (ok && lane == 0) mbar_arrive(bar(kBarWEmpty + ws));  // the stage's words are in registers: its slot can load again
+            if (it >= kSlots && ok && !t_ready) ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xE80u | s, p.wait_limit_ns);
             tc_fence_after();
             const uint32_t dst = t_lane + 2 * R + s * kSlotCols;
 #pragma unroll
@@ -445,7 +445,6 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (EXACT && it >= kTeams) {
                 if (it < 2 * kTeams) pdl_wait();  // (as above)
                 add_stage(it - kTeams, s0, ph0);
-                if (!ok) break;
             }
             const uint32_t done = full(s);
             s0 = s;
@@ -464,7 +463,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(done);
+            if (ok && lane == 0) mbar_arrive(done);
         }
         if constexpr (EXACT) {
             pdl_wait();
@@ -475,7 +474,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     cp_async_16(lora_t_addr + i * 16, p.lora_t + static_cast<size_t>(min(m0 + row, p.m - 1)) * p.lora_r + lora_0 + 4 * piece);
                 }
             }
-            if (ok && it > u) add_stage(it - kTeams, s0, ph0);
+            if (it > u) add_stage(it - kTeams, s0, ph0);
 #pragma unroll
             for (int r8 = 0; r8 < kExactRows; r8 += 8) {
                 uint32_t r[8];
@@ -492,10 +491,10 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 cp_async_wait_all();
                 asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");
             }
-            ok = ok && *abort_flag == 0;
+            ok = warp_all(ok && *abort_flag == 0);
         }
         // ---------------- epilogue: a thread owns one output column; team u takes every fourth block of 16 rows (EXACT: of 4) ----------------
-        if (!EXACT && ok) ok = mbar_wait(bar(kBarDone), 0, abort_flag, p.status, 0xD00u, p.wait_limit_ns);
+        if (!EXACT) ok = warp_all(ok && mbar_wait(bar(kBarDone), 0, abort_flag, p.status, 0xD00u, p.wait_limit_ns));
         tc_fence_after();
         const int col = nt * kTileCols + col_in_tile;
         float v4[4] = {};  // EXACT: rows 4u..4u + 3

@@ -71,6 +71,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return false;
 }
 
+// What a whole warp goes on from.  Each lane polls for itself, so when a wait runs out at the moment its barrier completes, lanes can
+// disagree, and the ones that went on would wait at the next warp-wide instruction for the ones that left.  A lane whose wait failed
+// therefore goes on with its warp, on whatever the barrier was to guard and without arriving anywhere, until the warp votes.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xFFFFFFFFu, ok); }
+
 // Drain helper for abort paths: bounded (about 20 ms), ignores the abort flag.
 __device__ __forceinline__ void mbar_wait_quiet(uint32_t bar, uint32_t parity) {
     const unsigned long long t0 = global_ns();
