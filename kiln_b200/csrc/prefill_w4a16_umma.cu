@@ -943,7 +943,7 @@ int launch_bn(const CUtensorMap &tmap, const CUtensorMap &tmap_c, const CUtensor
 
 // whether the small-batch kernel runs a plain problem that the planner tiled as `c`
 static bool smallm_takes(const PrefillConfig &c, int m, int n, int k, int groupsize) {
-    return g_smallm_enabled && g_test_drop_a_load < 0 && c.bn == 128 && c.mt == 1 && !c.stream_k &&
+    return g_smallm_enabled && c.bn == 128 && c.mt == 1 && !c.stream_k &&
            smallm_supported(m, n, k, groupsize, exec_splits(c, m, n, k));
 }
 
@@ -953,7 +953,7 @@ bool smallm_takes(int m, int n, int k, int groupsize) { return m <= BM && smallm
 // The small-batch kernel's variant that applies the group scales in fp32 (the decode kernel's arithmetic): 16 rows a CTA.
 static int exact_splits(int m, int n, int k, bool swiglu) { return swiglu ? 1 : choose_smallm_splits(16, n * ((m + 15) / 16), k); }
 bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r) {
-    return g_smallm_enabled && g_test_drop_a_load < 0 && m <= 256 && (lora_r == 0 || (groupsize != -1 && lora_r <= 128)) &&
+    return g_smallm_enabled && m <= 256 && (lora_r == 0 || (groupsize != -1 && lora_r <= 128)) &&
            smallm_supported(std::min(m, 16), n, k, groupsize, exact_splits(m, n, k, swiglu));
 }
 int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
@@ -986,6 +986,7 @@ void set_wait_limit_ns(unsigned long long ns) { g_wait_limit_ns = ns ? ns : kWai
 unsigned long long current_wait_limit_ns() { return g_wait_limit_ns; }
 void set_smallm_enabled(int on) { g_smallm_enabled = on; }
 void set_test_drop_a_load(int k_step) { g_test_drop_a_load = k_step; }
+int test_drop_a_load() { return g_test_drop_a_load; }
 
 void set_prefill_override(int bn, int splits, int mt, int stream_k) {
     g_prefill_override = PrefillConfig{bn, splits, mt, stream_k};

@@ -317,7 +317,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const uint64_t desc0 = make_smem_desc(smem_base + p.off_x + t * x_bytes);
         int s = 0, ph = 0;
         bool ok = true, ready = false;
-        for (int it = 0; it < n_it; ++it) {
+        int it = 0;
+        for (; it < n_it; ++it) {
             if (!ready && !(ok = mbar_wait(full(s), ph, abort_flag, p.status, 0xB00u | s, p.wait_limit_ns))) break;
             tc_fence_after();
             const uint64_t b_desc = desc0 + static_cast<uint64_t>((s * 2 * x_bytes) >> 4);
@@ -336,6 +337,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             ready = mbar_test(full(s), ph);
         }
         if (!EXACT && ok && issue) umma_commit(bar(kBarDone));
+        if (!ok && it > 0) mbar_wait_quiet(empty((it - 1) % kSlots), ((it - 1) / kSlots) & 1);  // the MMAs it has issued
     } else {
         // ---------------- dequant: packed int4 -> bf16 pairs in tensor memory ----------------
         // team u takes every fourth iteration, from iteration u
@@ -494,6 +496,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             ok = warp_all(ok && *abort_flag == 0);
         }
         // ---------------- epilogue: a thread owns one output column; team u takes every fourth block of 16 rows (EXACT: of 4) ----------------
+        if (!EXACT) pdl_wait();  // (park until the MMAs may run)
         if (!EXACT) ok = warp_all(ok && mbar_wait(bar(kBarDone), 0, abort_flag, p.status, 0xD00u, p.wait_limit_ns));
         tc_fence_after();
         const int col = nt * kTileCols + col_in_tile;
@@ -523,6 +526,11 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
             }
         }
+        auto drain = [&] {  // a wait of the teams has run out: copies that may be in flight though no wait of the loading warps has
+            if (!p.per_column) mbar_wait_quiet(bar(kBarScales), 0);
+            for (int j = max(0, n_st - p.w_slots); j < n_st; ++j) mbar_wait_quiet(bar(kBarWFull + j % p.w_slots), (j / p.w_slots) & 1);
+            for (int j = max(0, n_it - kSlots); j < n_it; ++j) mbar_wait_quiet(full(j % kSlots), (j / kSlots) & 1);
+        };
         if (p.splits == 1) {
             // The bf16 tile is put together in shared memory (over the rings, which are spent) and leaves through TMA: two-byte
             // stores from registers cost 8 cycles of the SM's load / store unit each.
@@ -586,6 +594,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 if (!SWIGLU) tma_store_2d(&tmap_c, smem_base + x_bytes, nt * kTileCols + 64, m0);
                 bulk_commit_group();
                 bulk_wait_group_read0();  // (the end of the grid completes them)
+            } else if (!ok && warp == kTeamWarp0 && lane == 0) {
+                drain();
             }
         }
         if (p.splits > 1) {
@@ -602,20 +612,20 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 else
                     st_async_v4(map_to_cta(addr, owner), a, b, c, d, map_to_cta(bar(kBarExchange), owner));
             };
-            if (ok) {
-                if constexpr (EXACT) push(u, v4[0], v4[1], v4[2], v4[3]);
+            // A CTA that has given up pushes all the same, whatever its sums are (the status word tells what the results are worth): every CTA stays
+            // until it has everything, so a push always finds its owner there.
+            if constexpr (EXACT) push(u, v4[0], v4[1], v4[2], v4[3]);
 #pragma unroll 1
-                for (int r0 = 8 * u; r0 < p.npad && !EXACT; r0 += 8 * kTeams) {
-                    uint32_t a[8], b[8];
-                    tmem_ld_32x32b_x8(t_lane + r0, a);
-                    tmem_ld_32x32b_x8(t_lane + R + r0, b);
-                    tmem_ld_wait();
-                    float v[8];
+            for (int r0 = 8 * u; r0 < p.npad && !EXACT; r0 += 8 * kTeams) {
+                uint32_t a[8], b[8];
+                tmem_ld_32x32b_x8(t_lane + r0, a);
+                tmem_ld_32x32b_x8(t_lane + R + r0, b);
+                tmem_ld_wait();
+                float v[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
+                for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) push(r0 / 4 + q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                }
+                for (int q = 0; q < 2; ++q) push(r0 / 4 + q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");  // (the rows of its own; every warp of the teams comes here)
             if (ok) {
@@ -644,7 +654,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         if (row0 + i < p.m) p.C[static_cast<size_t>(row0 + i) * p.n + gcol] = __float2bfloat16_rn(v[i] * cs);
                 }
             } else {
-                mbar_wait_quiet(bar(kBarExchange), 0);  // peers may still be pushing into this CTA
+                if (warp == kTeamWarp0 && lane == 0) drain();
+                mbar_wait_quiet(bar(kBarExchange), 0, 32 * p.wait_limit_ns);  // peers push into this CTA until they are through or have given up
             }
         }
         tc_fence_before();
@@ -736,7 +747,8 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
     {  // activations [m, k] seen as [k/64][m][64], so that one copy brings both 64-deep tiles of a stage
         const cuuint64_t dims[3] = {kAtomK, static_cast<cuuint64_t>(a.m), static_cast<cuuint64_t>(a.k / kAtomK)};
         const cuuint64_t strides[2] = {static_cast<cuuint64_t>(a.k) * 2, kAtomK * 2};
-        const cuuint32_t box[3] = {kAtomK, static_cast<cuuint32_t>(npad), 2}, estr[3] = {1, 1, 1};
+        // (test hook: boxes of eight rows less than the kernel announces, so that its waits for them run out)
+        const cuuint32_t box[3] = {kAtomK, static_cast<cuuint32_t>(test_drop_a_load() >= 0 ? npad - 8 : npad), 2}, estr[3] = {1, 1, 1};
         if (enc(&tmap_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(a.A), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return KILN_W4A16_ERR_CUDA;

@@ -76,10 +76,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // therefore goes on with its warp, on whatever the barrier was to guard and without arriving anywhere, until the warp votes.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xFFFFFFFFu, ok); }
 
-// Drain helper for abort paths: bounded (about 20 ms), ignores the abort flag.
-__device__ __forceinline__ void mbar_wait_quiet(uint32_t bar, uint32_t parity) {
+// Drain helper for abort paths: bounded (about 20 ms unless told otherwise), ignores the abort flag.
+__device__ __forceinline__ void mbar_wait_quiet(uint32_t bar, uint32_t parity, unsigned long long limit_ns = 20ull * 1000 * 1000) {
     const unsigned long long t0 = global_ns();
-    while (!mbar_try_wait(bar, parity) && global_ns() - t0 < 20ull * 1000 * 1000) {
+    while (!mbar_try_wait(bar, parity) && global_ns() - t0 < limit_ns) {
     }
 }
 

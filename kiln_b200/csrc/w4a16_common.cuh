@@ -172,6 +172,7 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact = false);
 bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r);
 int launch_exact(const GemmArgs &a);
 void set_test_drop_a_load(int k_step);
+int test_drop_a_load();
 void prefill_plan(int m, int n, int k, int out[4]);
 bool prefill_supported(int m, int n, int k, int groupsize);
 bool prefill_fuses_swiglu(int m, int n, int k);
