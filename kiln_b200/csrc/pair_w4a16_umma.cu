@@ -14,7 +14,8 @@
 // Roles (448 threads): warp 0 TMA, warp 1 MMA issuer (leader) and the TMEM allocation, warps 2-5 epilogue, warps 6-13 dequant in
 // two teams that take the stages in turn.  Work distribution, K splits and the hybrid stream-K are those of the other kernel, a
 // worker being a pair.  Dequantisation, LoRA steps, SwiGLU and per-column scales as there: same roundings.
-// Every wait is bounded (w4a16_async.cuh); a wait gives up after milliseconds, when copies in flight have long landed.
+// Every wait is bounded (w4a16_async.cuh).  When one runs out, its CTA tells the other one, lets what is in flight land, and the two leave
+// together (see the teardown).
 // No load is multicast.
 #include "w4a16_prefill.cuh"
 
@@ -48,6 +49,9 @@ struct Cfg {
 
 __device__ __forceinline__ void arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 // a load into this CTA's shared memory that counts on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t cluster_bar) {
@@ -446,6 +450,13 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag && threadIdx.x == 0) {
+        // A wait has run out, and every warp of this CTA has given up.  The other one would learn of it by its own limit.  Copies and MMAs that have
+        // been issued take microseconds, in whatever state the rings are, and land during this pause; neither CTA leaves before it.
+        st_cluster_u32(map_to_cta(smem_u32(const_cast<uint32_t *>(abort_flag)), cluster_ctarank() ^ 1), 1u);
+        pause_ns(20ull * 1000 * 1000);
+    }
+    __syncwarp();
     cluster_sync_all();  // nothing of the pair is in flight any more: MMAs, arrivals, tensor memory
     if (warp == 1) {
         tc_fence_after();
@@ -474,7 +485,8 @@ int launch_pair(const GemmArgs &a, PrefillParams p, int tile_n, const CUtensorMa
     };
     const int cols = tile_n / 2;  // columns per CTA
     CUtensorMap tmap_a, tmap_w, tmap_s, tmap_t, tmap_lb;
-    if (!operand(&tmap_a, a.A, a.k, a.m, kHalf) ||
+    // (test hook: boxes of eight rows less than the kernel announces, so that its waits for them run out)
+    if (!operand(&tmap_a, a.A, a.k, a.m, p.test_drop_a_load >= 0 ? kHalf - 8 : kHalf) ||
         !encode(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.B, 2ll * a.n, a.k / 16, 2 * cols, BK / 16, CU_TENSOR_MAP_SWIZZLE_NONE))
         return KILN_W4A16_ERR_CUDA;
     tmap_s = tmap_w;  // (unused with per-column scales)

@@ -966,7 +966,7 @@ PrefillConfig swiglu_config(int m, int n, int k) {
     return m <= BM || (c.splits == 1 && !c.stream_k && c.mt == 2) ? c : choose_any(m, n, k, false, true);
 }
 bool prefill_fuses_swiglu(int m, int n, int k) {
-    if (m > BM) return g_test_drop_a_load < 0;
+    if (m > BM) return true;
     const PrefillConfig c = choose_prefill(m, n, k);
     const int splits = exec_splits(c, m, n, k);
     if (!smallm_takes(c, m, n, k, 128)) return false;
@@ -1104,8 +1104,8 @@ int launch_prefill(const GemmArgs &a) {
     p.wait_limit_ns = g_wait_limit_ns;
     p.test_drop_a_load = g_test_drop_a_load;
     p.tile_elems = BM * c.mt * c.bn;
-    // tiles of 256 rows run on CTA pairs (the fused all-gather and the give-up test hook stay on single CTAs)
-    const bool pair = c.mt == 2 && !fused && g_test_drop_a_load < 0;
+    // tiles of 256 rows run on CTA pairs (the fused all-gather stays on single CTAs)
+    const bool pair = c.mt == 2 && !fused;
     const StreamKPlan plan = streamk_plan(p.m_tiles * p.n_tiles, p.k_iters, pair ? device_sm_count() / 2 : device_sm_count());
     p.sk_first_tile = plan.first_tile;
     p.sk_ctas = plan.ctas;

@@ -54,6 +54,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+__device__ __forceinline__ void pause_ns(unsigned long long ns) {
+    const unsigned long long t0 = global_ns();
+    while (global_ns() - t0 < ns) __nanosleep(10000);
+}
+
 // Bounded wait.  Returns false if the CTA is aborting (this wait or another one ran out).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
                                           uint32_t *status, uint32_t code, unsigned long long limit_ns = kWaitLimitNs) {

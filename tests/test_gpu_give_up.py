@@ -84,3 +84,23 @@ def test_kernel_of_single_ctas(cuda_device, bn, m, splits):
     finally:
         lib.kiln_w4a16_set_prefill_override(0, 0, 0, 0)
         lib.kiln_w4a16_set_prefill_min_m(0)
+
+
+# both widths of tiles; K splits and stream-K, whose later passes run on what there is; several tiles per pair; an adapter, SwiGLU, per-column
+# scales; a K shorter than the ring of stages
+@pytest.mark.parametrize("bn,m,k,n,groupsize,rank,swiglu,splits,stream_k", [
+    (128, 300, 1024, 512, 128, 0, False, 1, 0), (256, 300, 1024, 512, 128, 0, False, 1, 0), (256, 512, 2560, 2560, 128, 0, False, 3, 0),
+    (256, 1000, 2560, 2560, 128, 0, False, 1, 1), (128, 4300, 256, 4096, 128, 0, False, 1, 0), (256, 300, 640, 1024, 128, 64, False, 1, 0),
+    (256, 300, 640, 1024, 128, 0, True, 1, 0), (128, 300, 640, 512, -1, 0, False, 1, 0)])
+def test_kernel_of_cta_pairs(cuda_device, bn, m, k, n, groupsize, rank, swiglu, splits, stream_k):
+    x, proj, adapter = _inputs(cuda_device, m, k, n, groupsize, rank)
+    call = (lambda: kiln_b200.swiglu_gate_up(x, proj)) if swiglu else \
+        (lambda: kiln_b200.matmul_bf16_lora(x, proj, *adapter, 0.5) if rank else kiln_b200.matmul_bf16(x, proj))
+    lib = _lib.lib()
+    lib.kiln_w4a16_set_prefill_min_m(1)
+    lib.kiln_w4a16_set_prefill_override(bn, splits, 2, stream_k)
+    try:
+        _give_up(call, 0, (0x100, 0x200, 0x300, 0x500, 0x600, 0x800, 0x900))
+    finally:
+        lib.kiln_w4a16_set_prefill_override(0, 0, 0, 0)
+        lib.kiln_w4a16_set_prefill_min_m(0)
