@@ -30,6 +30,7 @@ def _native_command() -> list:
     cuda = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
     inc = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"), cuda, sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f'-DKILN_NATIVE_KEY="{_native_key()}"',
             *(f"-I{d}" for d in inc), os.path.join(CSRC, "host.cpp"), "-o", NATIVE, "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda",
             "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
 
@@ -38,8 +39,22 @@ def _stale() -> bool:
     if not (os.path.exists(LIB) and os.path.exists(NATIVE)):
         return True
     t = min(os.path.getmtime(LIB), os.path.getmtime(NATIVE))
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "kiln_w4a16.h")]
-    return any(os.path.getmtime(d) > t for d in deps)
+    # (sources only: the objects lie beside them, and the last of them is younger than _native.so, which is compiled meanwhile)
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".cpp", ".h"))]
+    deps.append(os.path.join(HERE, "..", "include", "kiln_w4a16.h"))
+    return any(os.path.getmtime(d) > t for d in deps) or not _built_for_this_torch()
+
+
+def _native_key() -> str:
+    """What _native.so depends on besides its source; compiled into it (csrc/host.cpp)."""
+    import torch
+
+    return f"kiln_b200 native: python {sys.version_info[0]}.{sys.version_info[1]}, torch {torch.__version__}, abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)};"
+
+
+def _built_for_this_torch() -> bool:
+    with open(NATIVE, "rb") as f:
+        return _native_key().encode() in f.read()
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -389,7 +389,8 @@ PyMethodDef methods[] = {method<py_bind>("bind"),       method<py_gemm>("gemm"),
                          method<py_gemm_ex>("gemm_ex"), method<py_grouped>("grouped"), method<py_pack>("pack"),
                          method<py_pack_gptq>("pack_gptq"),
                          {nullptr, nullptr, 0, nullptr}};
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+// (its doc string says what it was compiled for: the build compares it with what is installed)
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", KILN_NATIVE_KEY, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
