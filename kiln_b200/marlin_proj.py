@@ -96,13 +96,13 @@ def pack_from_gptq(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torch.Te
     if qweight.dtype != torch.int32 or qzeros.dtype != torch.int32:
         raise KilnMarlinError("marlin_proj: GPTQ qweight and qzeros must be i32")
     dev = qweight.device
-    sc = scales.to(torch.float16).contiguous()
+    qw, qz, sc = qweight.contiguous(), qzeros.contiguous(), scales.to(torch.float16).contiguous()  # (held: a copy given back would be the next one's)
     b_packed = torch.empty((k // 16, 2 * n), dtype=torch.int32, device=dev)
     s_perm = torch.empty((k // g, n), dtype=torch.float16, device=dev)
     bad = torch.zeros(1, dtype=torch.int32, device=dev)
     with torch.cuda.device(dev):
         rc = _lib.lib().kiln_w4a16_repack_gptq_device(
-            qweight.contiguous().data_ptr(), qzeros.contiguous().data_ptr(), sc.data_ptr(), k, n, groupsize,
+            qw.data_ptr(), qz.data_ptr(), sc.data_ptr(), k, n, groupsize,
             b_packed.data_ptr(), s_perm.data_ptr(), bad.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
     if rc != 0:
         raise KilnMarlinError(f"marlin_proj: GPTQ repack failed: {_lib.STATUS_NAMES.get(rc, rc)}")
@@ -226,7 +226,6 @@ def _gemm_ex(x2: torch.Tensor, proj: MarlinPackedProj, swiglu: bool, lora_a, lor
         raise KilnMarlinError("marlin_proj: x must be a CUDA bf16 tensor")
     ep = _lib.Epilogue()
     ep.swiglu = 1 if swiglu else 0
-    keep = []
     if lora_a is not None:
         r = lora_a.shape[0]
         if tuple(lora_a.shape) != (r, k) or tuple(lora_b.shape) != (proj.n, r):
@@ -238,8 +237,8 @@ def _gemm_ex(x2: torch.Tensor, proj: MarlinPackedProj, swiglu: bool, lora_a, lor
             a_ = torch.cat([a_, a_.new_zeros((pad, k))], dim=0).contiguous()
             b_ = torch.cat([b_, b_.new_zeros((proj.n, pad))], dim=1).contiguous()
             r += pad
-        keep += [a_, b_]
         ep.lora_a, ep.lora_b, ep.lora_rank, ep.lora_scale = a_.data_ptr(), b_.data_ptr(), r, float(lora_scale)
+    xc, b, s = x2.contiguous(), proj.b_packed, proj.scales  # (held until the launch is enqueued: copies, or what a property makes)
     n_out = proj.n // 2 if swiglu else proj.n
     if out is None:
         out = torch.empty((m, n_out), dtype=torch.bfloat16, device=x2.device)
@@ -253,7 +252,7 @@ def _gemm_ex(x2: torch.Tensor, proj: MarlinPackedProj, swiglu: bool, lora_a, lor
         need = int(lib.kiln_w4a16_workspace_bytes_ex(m, proj.n, k, ctypes.byref(ep)))
         ws = scratch(x2.device, need)
         rc = lib.kiln_w4a16_gemm_bf16_ex(
-            x2.contiguous().data_ptr(), proj.b_packed.data_ptr(), out.data_ptr(), proj.scales.data_ptr(), m, proj.n, k,
+            xc.data_ptr(), b.data_ptr(), out.data_ptr(), s.data_ptr(), m, proj.n, k,
             proj.groupsize, ctypes.byref(ep), ws.data_ptr() if need else None, ws.numel() if need else 0,
             torch.cuda.current_stream(x2.device).cuda_stream)
     if rc != 0:
@@ -330,13 +329,13 @@ def grouped_matmul_bf16(xs: Sequence[torch.Tensor], projs: Sequence[MarlinPacked
     for i, (x, pr) in enumerate(zip(xs, projs)):
         if x.dim() != 2 or x.shape[1] != pr.k or x.dtype != torch.bfloat16 or x.device != dev:
             raise KilnMarlinError("marlin_proj: every x must be a rank-2 bf16 tensor [m, k] on one device")
-        xc = x.contiguous()
-        keep.append(xc)
+        xc, b, s = x.contiguous(), pr.b_packed, pr.scales
+        keep += [xc, b, s]
         o = given[i] if given is not None else torch.empty((x.shape[0], pr.n), dtype=torch.bfloat16, device=dev)
         if tuple(o.shape) != (x.shape[0], pr.n) or o.dtype != torch.bfloat16 or not o.is_contiguous():
             raise KilnMarlinError("marlin_proj: every out must be a contiguous bf16 [m, n] tensor")
         outs.append(o)
-        arr[i] = _lib.Problem(xc.data_ptr(), pr.b_packed.data_ptr(), o.data_ptr(), pr.scales.data_ptr(), x.shape[0], pr.n, pr.k,
+        arr[i] = _lib.Problem(xc.data_ptr(), b.data_ptr(), o.data_ptr(), s.data_ptr(), x.shape[0], pr.n, pr.k,
                               pr.groupsize)
         need = max(need, int(lib.kiln_w4a16_workspace_bytes(x.shape[0], pr.n, pr.k)))
     with torch.cuda.device(dev), nvtx.range("kiln/proj/grouped"):

@@ -57,13 +57,15 @@ def test_weights_made_on_each_read_live_until_the_launch(cuda_device):
         x = torch.randn((m, k), generator=gen).to(torch.bfloat16).to(cuda_device)
         la, lb = torch.randn((16, k), generator=gen).to(torch.bfloat16).to(cuda_device), torch.randn((n, 16), generator=gen).to(torch.bfloat16).to(cuda_device)
 
-        def calls(p, q):
+        def calls(p, q, x=x):
             return [kiln_b200.matmul_bf16(x, p), kiln_b200.swiglu_gate_up(x, p), kiln_b200.matmul_bf16_lora(x, p, la, lb, 0.5),
                     *kiln_b200.grouped_matmul_bf16([x, x], [p, q])]
 
         want = calls(p, q)
         for _ in range(5):
             for got, ref in zip(calls(_Offloaded(p), _Offloaded(q)), want):
+                assert torch.equal(got, ref)
+            for got, ref in zip(calls(_Offloaded(p), _Offloaded(q), x.t().contiguous().t()), want):  # the Python path, which copies x
                 assert torch.equal(got, ref)
 
 
@@ -118,3 +120,16 @@ def test_a_group_size_beyond_a_long_is_refused(cuda_device):
                 call()
         qzeros = torch.full((1, 32), -0x77777778, dtype=torch.int32, device=cuda_device)
         assert kiln_b200.pack_from_gptq(torch.zeros((16, 256), dtype=torch.int32, device=cuda_device), qzeros, proj.scales, g) is None
+
+
+def test_gptq_tensors_that_have_to_be_copied_do_not_overlap(cuda_device):
+    """Neither tensor is contiguous: both copies have to live until the repack is enqueued."""
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(1)
+    for k, n in [(1024, 1024), (256, 256), (4096, 2048)]:
+        qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), dtype=torch.int32, device=cuda_device, generator=gen)
+        qz = torch.full((k // 128, n // 8), -0x77777778, dtype=torch.int32, device=cuda_device)
+        s = torch.rand((k // 128, n), device=cuda_device, generator=gen).to(torch.float16)
+        want = kiln_b200.pack_from_gptq(qw, qz, s)
+        got = kiln_b200.pack_from_gptq(qw.t().contiguous().t(), qz.t().contiguous().t(), s.t().contiguous().t())
+        assert torch.equal(got.b_packed, want.b_packed) and torch.equal(got.scales, want.scales)
