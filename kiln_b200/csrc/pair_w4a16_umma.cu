@@ -1,18 +1,18 @@
-// Prefill-shape W4A16 GEMM on CTA pairs (tcgen05.mma.cta_group::2): 256 x 256 tiles, 64 K per pipeline stage.
+// Prefill-shape W4A16 GEMM on CTA pairs (tcgen05.mma.cta_group::2): tiles of 256 rows x 256 or 128 columns, 64 K per pipeline stage.
 //
 // The kernel of single CTAs (prefill_w4a16_umma.cu) dequantises a weight once per 256 rows by giving a CTA two 128-row tiles.
 // That costs it shared memory (per 256 x 256 x 64 it reads 96 KB of operands and writes 64 KB: 1250 cycles at 128 bytes a cycle
 // against 1024 cycles of MMAs) and tensor memory (both accumulators belong to one tile, so its epilogue, 14,000 of 59,000 cycles
 // at K = 2560, hides under nothing).  Here two SMs share the tile: each holds 128 rows of the activations and dequantises 128
-// of the 256 weight columns, every MMA multiplies both halves, and an SM's tensor memory holds two accumulators of 128 x 256.
+// of the 256 weight columns (64 of 128), every MMA multiplies both halves, and an SM's tensor memory holds two accumulators of 128 x 256.
 // Per SM and 64 K that is 32 KB read and 32 KB written in 512 cycles of MMAs, and the epilogue of a tile runs under the next one.
 //
 // Cluster of two CTAs; CTA 0 (the leader) issues the MMAs.  Per stage:
 //  * full (leader's): the activation bytes of both CTAs (TMA loads of either count on it) + one arrival per dequant warp of both;
 //  * empty (each CTA's own): the commit of the stage's MMAs, multicast to both.
 // Per accumulator: full (each CTA's own, multicast commit), empty (leader's): one arrival per epilogue warp of both.
-// Roles (448 threads): warp 0 TMA, warp 1 MMA issuer (leader) and the TMEM allocation, warps 2-5 epilogue, warps 6-13 dequant in
-// two teams that take the stages in turn.  Work distribution, K splits and the hybrid stream-K are those of the other kernel, a
+// Roles (608 threads): warp 0 TMA of the activations, warp 1 MMA issuer (leader) and the TMEM allocation, warps 2-5 epilogue, warp 6 TMA of the
+// packed words and scales, warps 7-18 dequant in three teams that take the stages in turn.  Work distribution, K splits and the hybrid stream-K are those of the other kernel, a
 // worker being a pair.  Dequantisation, LoRA steps, SwiGLU and per-column scales as there: same roundings.
 // Every wait is bounded (w4a16_async.cuh).  When one runs out, its CTA tells the other one, lets what is in flight land, and the two leave
 // together (see the teardown).

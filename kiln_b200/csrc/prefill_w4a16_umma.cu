@@ -1103,7 +1103,6 @@ int launch_prefill(const GemmArgs &a) {
     p.stream_k = c.stream_k;
     p.wait_limit_ns = g_wait_limit_ns;
     p.test_drop_a_load = g_test_drop_a_load;
-    p.tile_elems = BM * c.mt * c.bn;
     // tiles of 256 rows run on CTA pairs (the fused all-gather stays on single CTAs)
     const bool pair = c.mt == 2 && !fused;
     const StreamKPlan plan = streamk_plan(p.m_tiles * p.n_tiles, p.k_iters, pair ? device_sm_count() / 2 : device_sm_count());

@@ -88,12 +88,4 @@ __device__ __forceinline__ void mbar_wait_quiet(uint32_t bar, uint32_t parity, u
     }
 }
 
-// 1-D bulk copy global -> shared; dst, src and bytes are multiples of 16.
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-
 }  // namespace kiln

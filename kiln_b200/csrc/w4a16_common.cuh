@@ -30,8 +30,7 @@ __device__ __forceinline__ uint32_t lop3_and_or(uint32_t x, uint32_t mask, uint3
 // gives exactly 128 + v.
 constexpr uint32_t kNibMask = 0x000F000Fu;
 constexpr uint32_t kMagic128 = 0x43004300u;  // bf16x2 {128, 128}
-constexpr uint32_t kNeg136x2 = 0xC308C308u;  // bf16x2 {-136, -136} = -(128 + 8)
-constexpr uint32_t kPos136x2 = 0x43084308u;  // bf16x2 {136, 136}
+constexpr uint32_t kPos136x2 = 0x43084308u;  // bf16x2 {136, 136}: 128 + 8
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                                uint32_t b1) {
@@ -93,16 +92,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta));
     return r;
 }
-__device__ __forceinline__ float2 ld_dsmem_f2(uint32_t cluster_addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr));
-    return v;
-}
-
-__device__ __forceinline__ void st_dsmem_f2(uint32_t cluster_addr, float2 v) {
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" ::"r"(cluster_addr), "f"(v.x), "f"(v.y) : "memory");
-}
-
 // Position of natural column `col` inside the per-column (groupsize -1) scale order
 // (kiln-marlin-gemm/src/lib.rs:348-357): within each 32, out[8i + j] = in[2i + {0,1,8,9,16,17,24,25}[j]].
 __device__ __host__ __forceinline__ int scale_single_pos(int col) {
@@ -126,8 +115,9 @@ struct GemmArgs {
     int n_peers = 0, ldc = 0, col0 = 0;
     // the same with one NVSwitch multicast address for the whole group instead of per-GPU pointers (multimem.st)
     void *mc_c = nullptr;
-    // epilogue options (LoRA: decode kernel; SwiGLU: decode kernel, and the tcgen05 kernel's whole-tile tilings): LoRA delta C += lora_t * lora_b^T with lora_t [m, lora_r] = scale * x * A^T (fp32 for the decode kernel, bf16 for the tcgen05 kernel)
-    // and lora_b bf16 [n, lora_r]; swiglu: columns are gate/up interleaved in runs of 32, C is [m, n/2]
+    // epilogue options.  LoRA delta C += lora_t * lora_b^T: lora_t [m, lora_r] = scale * x * A^T, fp32 for the decode kernel and the small-batch
+    // kernel's fp32-scale variant, bf16 where it is an operand tile of a tcgen05 kernel; lora_b bf16 [n, lora_r].  swiglu: columns are gate / up
+    // interleaved in runs of 32, C is [m, n/2] (decode kernel, small-batch kernel without a K split, pair kernel)
     bool no_scratch = false;  // the tcgen05 kernel may not use the workspace (legacy entry point: its caller's buffer is tiny)
     const void *lora_t = nullptr;
     const void *lora_b = nullptr;

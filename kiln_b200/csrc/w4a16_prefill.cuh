@@ -34,7 +34,6 @@ struct PrefillParams {
     int sk_first_tile;  // stream-K: tiles below this index are dealt whole (a multiple of the grid size)
     int sk_ctas;        // stream-K: CTAs that share the remaining tiles (<= grid size)
     int group_m;        // tiles are dealt in bands of this many rows of tiles (tile_of)
-    int tile_elems;   // rows * columns of one output tile (stream-K slabs are tile-shaped)
     unsigned long long wait_limit_ns;  // every bounded wait of the launch gives up after this long
     int test_drop_a_load;  // test hook: the activation tile of this K-step (counted per CTA) is announced but never copied; -1 = off
 };
