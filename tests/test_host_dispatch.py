@@ -1,7 +1,9 @@
 """Host-side kernel selection and workspace rules, through the C ABI, without a GPU (148 SMs are assumed when no device is
 present).  The workspace a caller must lend follows from which kernel a problem goes to and how that kernel splits K:
-  * up to 16 rows, and projections of at most 1024 columns up to 256 rows: decode kernel, no workspace;
-  * from 17 rows on wider projections: a tcgen05 kernel, `splits * m * n * 4` bytes when the planner splits K;
+  * up to 16 rows, and projections of at most 1024 columns up to 256 rows: decode kernel, or the small-batch kernel's fp32-scale variant
+    (from 9 rows, or fewer for a short K or with a LoRA delta): no workspace either way;
+  * from 17 rows on wider projections: a tcgen05 kernel, `splits * m * n * 4` bytes when the planner splits K (reserved for any of them: the
+    small-batch kernel keeps its sums in shared memory);
   * epilogue options add the fp32 [m, rank] projection of a LoRA delta and, when an option is not fused, a bf16 copy of
     the GEMM result for the second pass."""
 import ctypes
@@ -21,8 +23,8 @@ def _plan(lib, m, n, k):
 
 def test_plain_gemm_workspace_follows_the_kernel_choice():
     lib = _lib.lib()
-    assert lib.kiln_w4a16_workspace_bytes(16, 4096, 2560) == 0          # decode kernel
-    assert lib.kiln_w4a16_workspace_bytes(256, 512, 2560) == 0          # narrow projection: decode kernel up to 256 rows
+    assert lib.kiln_w4a16_workspace_bytes(16, 4096, 2560) == 0          # fp32-scale variant
+    assert lib.kiln_w4a16_workspace_bytes(256, 512, 2560) == 0          # narrow projection: the same up to 256 rows
     for m in (17, 64, 128):                                             # small-batch tcgen05 kernel, the planner's K splits
         bn, splits, mt, sk = _plan(lib, m, 4096, 2560)
         assert (bn, mt, sk) == (128, 1, 0) and splits > 1
