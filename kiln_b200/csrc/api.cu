@@ -316,7 +316,8 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_grouped(const kiln_w4a16_problem_t *pro
         const int v = validate(a);
         if (v > 0) return v;
         if (v == 0) continue;  // an empty problem
-        if (use_prefill(q.m, q.n, q.k, q.groupsize)) one_launch = false;  // (one decode launch for the group beats per-problem small-batch launches)
+        if (use_prefill(q.m, q.n, q.k, q.groupsize)) one_launch = false;  // (one decode launch for the group beat per-problem launches of
+                                                                                       // the first small-batch kernel; not measured against the present one)
         items[live++] = DecodeItem{q.A, q.B, q.s, q.C, q.m, q.n, q.k, q.groupsize, nullptr, nullptr, 0, 0};
     }
     if (live == 0) return KILN_W4A16_OK;
