@@ -276,7 +276,9 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
     if (ep->lora_rank) {
         t = ws;  // fp32 [m, r] for the decode kernel and the composed pass, bf16 [m, r] as an operand of the tcgen05 kernel
         ws += align256(static_cast<size_t>(m) * ep->lora_rank * sizeof(float));
-        if (int rc = launch_lora_down(A, ep->lora_a, ep->lora_scale, m, k, ep->lora_rank, t, fuse_lora ? 1 : 0, a.stream)) return rc;
+        // (an operand tile of the tcgen05 kernels, which form their weights at that factor of their value)
+        const float factor = fuse_lora ? kWeightFactor : 1.f;
+        if (int rc = launch_lora_down(A, ep->lora_a, ep->lora_scale * factor, m, k, ep->lora_rank, t, fuse_lora ? 1 : 0, a.stream)) return rc;
     }
     if (!tc) {
         a.lora_t = t;

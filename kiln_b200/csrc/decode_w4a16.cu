@@ -77,6 +77,12 @@ constexpr uint32_t kMagicHi = 0x54005400u;   // fp16x2 {64, 64}: ulp 1/16, a nib
 constexpr uint32_t kNegOffLo = 0xE408E408u;  // fp16x2 {-1032, -1032}
 constexpr uint32_t kNegOffHi = 0xD480D480u;  // fp16x2 {-72, -72}
 
+__device__ __forceinline__ uint32_t lop3_and_or(uint32_t x, uint32_t mask, uint32_t orv) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "r"(mask), "r"(orv));
+    return r;
+}
+
 __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                               uint32_t b0, uint32_t b1) {
     asm volatile(

@@ -80,37 +80,14 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
     return v;
 }
 
-// bf16x2 {s, s} for the lane's columns 8t + c of a 64-column chunk, from 16 bytes of its scale order
-__device__ __forceinline__ void scale_pairs(const uint4 &sc, uint32_t (&s2)[8]) {
-    const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        const float f = __half2float(__ushort_as_half(static_cast<unsigned short>((t & 1) ? (sw[t >> 1] >> 16) : (sw[t >> 1] & 0xFFFFu))));
-        __nv_bfloat162 b = __floats2bfloat162_rn(f, f);
-        s2[t] = *reinterpret_cast<uint32_t *>(&b);
-    }
-}
-
 // One 512-byte packed block (16 K x 64 columns) -> the K-major 128B-swizzled tile: row (column of B) 8t + c at row_base + 1024 t, its
 // two 16-byte chunks of the block at sw_lo and sw_hi.
-__device__ __forceinline__ void dequant_block(const uint4 &w, const uint32_t (&s2)[8], uint32_t row_base, uint32_t sw_lo, uint32_t sw_hi) {
+__device__ __forceinline__ void dequant_block(const uint4 &w, const WeightScale (&sc)[4], uint32_t row_base, uint32_t sw_lo, uint32_t sw_hi) {
     const uint32_t xs[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const uint32_t x = xs[j];
         uint32_t v[4];
-        v[0] = lop3_and_or(x, kNibMask, kMagic128);        // K 2qd, 2qd+1     col 16j + c
-        v[1] = lop3_and_or(x >> 4, kNibMask, kMagic128);   // K 2qd+8, 2qd+9   col 16j + c
-        v[2] = lop3_and_or(x >> 8, kNibMask, kMagic128);   // K 2qd, 2qd+1     col 16j + 8 + c
-        v[3] = lop3_and_or(x >> 12, kNibMask, kMagic128);  // K 2qd+8, 2qd+9   col 16j + 8 + c
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            __nv_bfloat162 d = *reinterpret_cast<__nv_bfloat162 *>(&v[e]);
-            const uint32_t k136 = kPos136x2;
-            d = __hsub2(d, *reinterpret_cast<const __nv_bfloat162 *>(&k136));
-            d = __hmul2(d, *reinterpret_cast<const __nv_bfloat162 *>(&s2[2 * j + (e >> 1)]));
-            v[e] = *reinterpret_cast<uint32_t *>(&d);
-        }
+        dequant_word(xs[j], sc[j], v[0], v[1], v[2], v[3]);
         const uint32_t r_lo = row_base + static_cast<uint32_t>(16 * j) * 128u, r_hi = r_lo + 8u * 128u;
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(r_lo + sw_lo), "r"(v[0]) : "memory");
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(r_lo + sw_hi), "r"(v[1]) : "memory");
@@ -306,7 +283,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                                 ua *= __half2float(p.S[pu]);
                                 ub *= __half2float(p.S[pu + 1]);
                             }
-                            __nv_bfloat162 b = __floats2bfloat162_rn(__fdividef(ga, 1.f + __expf(-ga)) * ua, __fdividef(gb, 1.f + __expf(-gb)) * ub);
+                            __nv_bfloat162 b = __floats2bfloat162_rn(swiglu_scaled(ga, ua), swiglu_scaled(gb, ub));
                             o[e2] = *reinterpret_cast<uint32_t *>(&b);
                         }
                         if (row < p.m) dst[v] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -339,8 +316,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                                 x0 *= __half2float(p.S[pos]);
                                 x1 *= __half2float(p.S[pos + 1]);
                             }
-                            __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-                            o[e] = *reinterpret_cast<uint32_t *>(&b);
+                            o[e] = unscale_bf16x2(x0, x1);
                         }
                         // 128-byte rows, 16-byte chunk index XOR (row % 8): the layout of the 128B-swizzled tensor map
                         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(epi_tma + lane * 128 + (((half * 4 + v) ^ (lane & 7)) << 4)), "r"(o[0]),
@@ -411,12 +387,12 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (; ki < ki1e; ki += kTeams) {  // (to the end, whatever a wait says: see warp_all)
                 if (ok && !w_ready) ok = mbar_wait(word_full(ws), wph, abort_flag, p.status, 0x900u | ws, p.wait_limit_ns);
                 uint4 w[C::kBlocks], sc = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);  // (per-column scales come in the epilogue)
-                uint32_t s2[8];
+                WeightScale s2[4];  // of columns 16j + c, 16j + 8 + c
                 if (ki < ki1) {
 #pragma unroll
                     for (int b = 0; b < C::kBlocks; ++b) w[b] = lds_v4(words + ws * C::kWordSlotBytes + b * (2 * kCols * 8));
                     if (!p.per_column) sc = lds_v4(scales + ws * C::kWordSlotBytes);
-                    scale_pairs(sc, s2);
+                    s2[0] = weight_scale(sc.x), s2[1] = weight_scale(sc.y), s2[2] = weight_scale(sc.z), s2[3] = weight_scale(sc.w);
                 }
                 __syncwarp();
                 if (ok && lane == 0) mbar_arrive(word_empty(ws));  // in registers: the slot can load again

@@ -277,8 +277,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                     x0 *= __half2float(p.S[pos]);
                                     x1 *= __half2float(p.S[pos + 1]);
                                 }
-                                __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-                                o[e] = *reinterpret_cast<uint32_t *>(&b);
+                                o[e] = unscale_bf16x2(x0, x1);
                             }
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
                                              epi_tma + lane * 128 + (((half * 4 + v) ^ (lane & 7)) << 4)),
@@ -350,8 +349,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                     x0 *= __half2float(p.S[pos]);
                                     x1 *= __half2float(p.S[pos + 1]);
                                 }
-                                __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-                                o[e] = *reinterpret_cast<uint32_t *>(&b);
+                                o[e] = unscale_bf16x2(x0, x1);
                             }
                             // 128-byte rows, 16-byte chunk index XOR (row % 8): the layout of the 128B-swizzled tensor map
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
@@ -452,7 +450,7 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         uint32_t it_base = 0;  // stages issued before this piece of work (all teams count alike)
         bool ok = true;
         int cur_group = -1;
-        uint32_t s2[8];  // bf16x2 {s, s} for columns 8t + c of this warp's chunk
+        WeightScale s2[4];  // of columns 16j + c, 16j + 8 + c of this warp's chunk
         WorkIter wi(p, blockIdx.x, gridDim.x);
         while (ok && wi.next(mt, nt, sp, ki0, ki1, slab)) {
             cur_group = -1;
@@ -499,19 +497,9 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 const int g = p.per_column ? 0 : group_of(ki);
                 if (g != cur_group) {
                     cur_group = g;
-                    if (p.per_column) {
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) s2[t] = 0x3F803F80u;  // bf16x2 {1, 1}; scale applied in the epilogue
-                    } else {
-                        const uint32_t sw[4] = {rs[u].x, rs[u].y, rs[u].z, rs[u].w};
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            const float f = __half2float(__ushort_as_half(
-                                static_cast<unsigned short>((t & 1) ? (sw[t >> 1] >> 16) : (sw[t >> 1] & 0xFFFFu))));
-                            __nv_bfloat162 b = __floats2bfloat162_rn(f, f);
-                            s2[t] = *reinterpret_cast<uint32_t *>(&b);
-                        }
-                    }
+                    // (per-column scales are applied in the epilogue)
+                    const uint4 sw = p.per_column ? make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u) : rs[u];
+                    s2[0] = weight_scale(sw.x), s2[1] = weight_scale(sw.y), s2[2] = weight_scale(sw.z), s2[3] = weight_scale(sw.w);
                 }
                 if (!(ok = mbar_wait(empty(s), ph ^ 1, abort_flag, p.status, 0x600u | s, p.wait_limit_ns))) break;
                 const uint32_t b_tile = smem_base + s * C::kStageBytes + C::kABytes;
@@ -527,20 +515,8 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     const uint32_t sw_hi = static_cast<uint32_t>((2 * kt + 1) ^ c) << 4;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const uint32_t x = xs[j];
                         uint32_t v[4];
-                        v[0] = lop3_and_or(x, kNibMask, kMagic128);        // K 2qd, 2qd+1     col 16j + c
-                        v[1] = lop3_and_or(x >> 4, kNibMask, kMagic128);   // K 2qd+8, 2qd+9   col 16j + c
-                        v[2] = lop3_and_or(x >> 8, kNibMask, kMagic128);   // K 2qd, 2qd+1     col 16j + 8 + c
-                        v[3] = lop3_and_or(x >> 12, kNibMask, kMagic128);  // K 2qd+8, 2qd+9   col 16j + 8 + c
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            __nv_bfloat162 w = *reinterpret_cast<__nv_bfloat162 *>(&v[e]);
-                            const uint32_t k136 = kPos136x2;
-                            w = __hsub2(w, *reinterpret_cast<const __nv_bfloat162 *>(&k136));
-                            w = __hmul2(w, *reinterpret_cast<const __nv_bfloat162 *>(&s2[2 * j + (e >> 1)]));
-                            v[e] = *reinterpret_cast<uint32_t *>(&w);
-                        }
+                        dequant_word(xs[j], s2[j], v[0], v[1], v[2], v[3]);
                         const uint32_t r_lo = row_base + static_cast<uint32_t>(16 * j) * 128u;
                         const uint32_t r_hi = r_lo + 8u * 128u;
                         asm volatile("st.shared.b32 [%0], %1;" ::"r"(r_lo + sw_lo), "r"(v[0]) : "memory");
@@ -584,7 +560,9 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     }
 }
 
+// complete sums of four columns, times the factor that the weights were formed at -> bf16
 __device__ __forceinline__ uint2 finish4(float4 v, const __half *S, int col, int per_column) {
+    v.x *= kWeightUnscale, v.y *= kWeightUnscale, v.z *= kWeightUnscale, v.w *= kWeightUnscale;
     if (per_column) {
         const int p0 = scale_single_pos(col), p1 = scale_single_pos(col + 2);
         v.x *= __half2float(S[p0]);

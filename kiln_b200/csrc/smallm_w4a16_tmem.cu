@@ -33,9 +33,9 @@
 // Every wait is bounded (w4a16_async.cuh).  Per-column scales (group size -1): the weights are dequantised unscaled and the
 // scale multiplies the finished sums.
 //
-// What bounds it: about 0.3 us per 128 K and CTA up to 64 rows.  The dequant needs 250 to 330 issue slots of every
-// sub-partition (eleven instructions per packed word, fifteen with scales), the eight MMAs 430 cycles of one issuer, and a launch has
-// 2.5 to 3.4 us that no stage hides (the first words' latency after a CTA of the previous kernel has left the SM, the exchange, the
+// What bounds it: about 0.3 us per 128 K and CTA up to 64 rows.  The dequant needs some 200 issue slots of every
+// sub-partition (nine instructions per packed word), an MMA 32 cycles at 64 rows and 9 at 16, a barrier 160 cycles to answer beside
+// them, and a launch has 2.5 to 3.4 us that no stage hides (the first words' latency after a CTA of the previous kernel has left the SM, the exchange, the
 // exit).  CUDA graph over rotating weights, before (register-streamed words, quad transposes, split-K through global slabs and
 // a second kernel) -> now: 64 rows 2560 -> 18432 14.0 -> 10.3 us, 2560 -> 4096 8.5 -> 5.3, 4096 -> 2560 8.9 -> 5.7, 2560 -> 8192
 // 10.9 -> 7.1, 9216 -> 2560 12.0 -> 9.0; 128 rows 2560 -> 18432 16.0 -> 12.1.  EXACT, against the decode kernel: 16 rows
@@ -170,22 +170,8 @@ __device__ __forceinline__ void sts_v4(uint32_t addr, float a, float b, float c,
 }
 
 // One packed word -> the four bf16x2 registers {column c: K pair qd, column c + 8: K pair qd, c: K pair 4 + qd, c + 8: K pair
-// 4 + qd}, scaled: (128 + nibble) - 136, times the group scale, the same two roundings as the general kernel.
-template <bool SCALE>
-__device__ __forceinline__ void dequant_word(uint32_t x, __nv_bfloat162 s_lo, __nv_bfloat162 s_hi, uint32_t *r) {
-    r[0] = lop3_and_or(x, kNibMask, kMagic128);
-    r[2] = lop3_and_or(x >> 4, kNibMask, kMagic128);
-    r[1] = lop3_and_or(x >> 8, kNibMask, kMagic128);
-    r[3] = lop3_and_or(x >> 12, kNibMask, kMagic128);
-    const uint32_t k136 = kPos136x2;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        __nv_bfloat162 w = *reinterpret_cast<__nv_bfloat162 *>(&r[e]);
-        w = __hsub2(w, *reinterpret_cast<const __nv_bfloat162 *>(&k136));
-        if (SCALE) w = __hmul2(w, (e & 1) ? s_hi : s_lo);
-        r[e] = *reinterpret_cast<uint32_t *>(&w);
-    }
-}
+// 4 + qd}.
+__device__ __forceinline__ void dequant_word(uint32_t x, const WeightScale &s, uint32_t *r) { dequant_word(x, s, r[0], r[2], r[1], r[3]); }
 
 // Stages in flight: TMEM slots of weights, and activation slots in shared memory
 template <int R>
@@ -395,7 +381,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (ok && !mbar_test(empty(s), ph)) ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xF00u | s, p.wait_limit_ns);
             __syncwarp();
             tc_fence_after();
-            const float scale = p.per_column ? 1.f : lds_half(exact_sc + j * kScaleBytes);
+            const float scale = p.per_column ? kWeightUnscale : lds_half(exact_sc + j * kScaleBytes) * kWeightUnscale;
             uint32_t a[kExactRows], b[kExactRows];
             tmem_ld_32x32b_x16(t_lane + u * kExactRows, a);
             tmem_ld_32x32b_x16(t_lane + R + u * kExactRows, b);
@@ -420,15 +406,10 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     wb[kt] = v.y;
                 }
             }
-            __nv_bfloat162 sc[4];
+            WeightScale sc[2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const uint32_t pair = EXACT || p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + (SWIGLU ? 8 : 4) * i);
-                const float f0 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair & 0xFFFFu)));
-                const float f1 = __half2float(__ushort_as_half(static_cast<unsigned short>(pair >> 16)));
-                sc[2 * i] = __floats2bfloat162_rn(f0, f0);
-                sc[2 * i + 1] = __floats2bfloat162_rn(f1, f1);
-            }
+            for (int i = 0; i < 2; ++i)
+                sc[i] = weight_scale(EXACT || p.per_column ? 0x3C003C00u : lds_u32(sc_addr + (it - lora_it) * kScaleBytes + (SWIGLU ? 8 : 4) * i));
             __syncwarp();
             if (ok && lane == 0) mbar_arrive(bar(kBarWEmpty + ws));  // the stage's words are in registers: its slot can load again
             if (it >= kSlots && ok && !t_ready) ok = mbar_wait(empty(s), ph, abort_flag, p.status, 0xE80u | s, p.wait_limit_ns);
@@ -438,10 +419,10 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             for (int k4 = 0; k4 < 2; ++k4) {  // four K tiles of 16 at a time
                 uint32_t r[16];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dequant_word<!EXACT>(wa[4 * k4 + i], sc[0], sc[1], r + 4 * i);
+                for (int i = 0; i < 4; ++i) dequant_word(wa[4 * k4 + i], sc[0], r + 4 * i);
                 tmem_st_16x128b_x8(dst + k4 * 32, r);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dequant_word<!EXACT>(wb[4 * k4 + i], sc[2], sc[3], r + 4 * i);
+                for (int i = 0; i < 4; ++i) dequant_word(wb[4 * k4 + i], sc[1], r + 4 * i);
                 tmem_st_16x128b_x8(dst + (16u << 16) + k4 * 32, r);
             }
             if (EXACT && it >= kTeams) {
@@ -534,7 +515,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (p.splits == 1) {
             // The bf16 tile is put together in shared memory (over the rings, which are spent) and leaves through TMA: two-byte
             // stores from registers cost 8 cycles of the SM's load / store unit each.
-            const float cs = p.per_column ? __half2float(p.S[scale_single_pos(col)]) : 1.f;
+            const float cs = (p.per_column ? __half2float(p.S[scale_single_pos(col)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
             const int ocol = SWIGLU ? ch * 32 + 16 * h + (lane & 15) : col_in_tile;  // output column within the tile
             const uint32_t stage = smem_base + (ocol >> 6) * x_bytes + (ocol & 7) * 2;
             const uint32_t chunk16 = (ocol & 63) >> 3;  // 16-byte chunk of a 128-byte row, XORed with row % 8
@@ -636,7 +617,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 const int own = min(p.quads_per_rank, p.npad / 4 - rank * p.quads_per_rank);
                 const int x = (warp - kTeamWarp0) * 32 + lane, cc = x & (kTileCols - 1);
                 const int gcol = nt * kTileCols + cc;
-                const float cs = p.per_column ? __half2float(p.S[scale_single_pos(gcol)]) : 1.f;
+                const float cs = (p.per_column ? __half2float(p.S[scale_single_pos(gcol)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
                 for (int slot = x >> 7; slot < own; slot += kTeamThreads / kTileCols) {
                     const uint32_t src = recv + static_cast<uint32_t>(slot * kTileCols + cc) * 16u;
                     const uint4 v0 = lds_v4(src);

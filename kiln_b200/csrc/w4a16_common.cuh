@@ -20,17 +20,56 @@ namespace kiln {
 constexpr int kGroup = 128;     // K elements per scale group
 constexpr int kChunkCols = 64;  // N columns per 512-byte block
 
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t x, uint32_t mask, uint32_t orv) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "r"(mask), "r"(orv));
-    return r;
-}
 
-// bf16 has 7 mantissa bits: OR-ing a nibble into the low mantissa bits of 128.0 (0x4300)
-// gives exactly 128 + v.
-constexpr uint32_t kNibMask = 0x000F000Fu;
-constexpr uint32_t kMagic128 = 0x43004300u;  // bf16x2 {128, 128}
-constexpr uint32_t kPos136x2 = 0x43084308u;  // bf16x2 {136, 136}: 128 + 8
+// Two packed nibbles -> (nibble - 8) * s * 2^-22 as bf16x2, in one AND and one fused multiply-add.
+// Read as bf16, a nibble at bits 0..3 of a half word is the subnormal nibble * 2^-133, and one at bits 4..7, whose top bit is the
+// exponent's lowest, is nibble * 2^-129: subnormals and the first normal binade are one linear scale.  So the fused multiply-add
+// brings nibble * s - 8 s, rounded once, which is what subtracting 8 and multiplying by s in two steps gives.  s * 2^133 would be
+// too large for bf16; with the factor of 2^-22 it is not, whatever the fp16 scale is (the largest rounds to 2^16).  The
+// factor is a power of two, so it changes no rounding; what reads the sums takes it out (kWeightUnscale).
+// An infinite scale gives NaN.  Sums below 2^-104 lose precision, as they did below 2^-126 without the factor.
+// Nine instructions for a packed word's eight weights; OR-ing the nibbles into 128.0, subtracting 136 and multiplying took fifteen, and
+// the dequantising warps bound every kernel that uses this up to a few hundred rows (37 rows 2560 -> 18432 10.4 -> 9.4 us, 9216 -> 2560
+// 8.3 -> 7.6); above, it saves power (16384 x 9216 x 9216 2026 -> 1969 us).
+constexpr uint32_t kNibMask = 0x000F000Fu, kHiNibMask = 0x00F000F0u;
+constexpr float kWeightFactor = 1.f / 4194304.f, kWeightUnscale = 4194304.f;  // 2^-22
+struct WeightScale {  // of two columns
+    __nv_bfloat162 lo, hi, off;  // s * 2^111, s * 2^107, -8 s * 2^-22
+};
+__device__ __forceinline__ WeightScale weight_scale(uint32_t half2_bits) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&half2_bits));
+    const __nv_bfloat162 s = __floats2bfloat162_rn(f.x, f.y);
+    const uint32_t lo = 0x77007700u, hi = 0x75007500u, off = 0xB600B600u;  // bf16x2 2^111, 2^107, -2^-19
+    return {__hmul2(s, *reinterpret_cast<const __nv_bfloat162 *>(&lo)), __hmul2(s, *reinterpret_cast<const __nv_bfloat162 *>(&hi)),
+            __hmul2(s, *reinterpret_cast<const __nv_bfloat162 *>(&off))};
+}
+__device__ __forceinline__ uint32_t dequant_pair(uint32_t nibbles, __nv_bfloat162 mul, __nv_bfloat162 off) {
+    const __nv_bfloat162 w = __hfma2(*reinterpret_cast<const __nv_bfloat162 *>(&nibbles), mul, off);
+    return *reinterpret_cast<const uint32_t *>(&w);
+}
+// bf16 results, the weights' factor taken out after the rounding, which it does not change: one instruction for two
+__device__ __forceinline__ uint32_t unscale_bf16x2(float lo, float hi) {
+    const uint32_t f = 0x4A804A80u;  // bf16x2 2^22
+    const __nv_bfloat162 v = __hmul2(__floats2bfloat162_rn(lo, hi), *reinterpret_cast<const __nv_bfloat162 *>(&f));
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+// silu(g) * u of sums that still have the factor, g' = g 2^-22 and u' = u 2^-22, which costs no instruction: e^-g = 2^(-g log2 e) takes
+// g's out in the product with log2 e, and g / (1 + e^-g) both of them in the sum, g' / (2^-44 + 2^-44 e^-g) = 2^22 g / (1 + e^-g).
+__device__ __forceinline__ float swiglu_scaled(float g, float u) {
+    constexpr float kLog2e = 1.4426950408889634f, kBoth = kWeightFactor * kWeightFactor;
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * (-kLog2e * kWeightUnscale)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(e, kBoth, kBoth)));  // (__fdividef is slow for a divisor this small)
+    return g * r * u;
+}
+// the eight weights of a packed word: K 2qd, 2qd + 1 and 2qd + 8, 2qd + 9 of the first column (c), then of the second (c + 8)
+__device__ __forceinline__ void dequant_word(uint32_t x, const WeightScale &s, uint32_t &k0, uint32_t &k8, uint32_t &second_k0, uint32_t &second_k8) {
+    const uint32_t y = x >> 8;
+    k0 = dequant_pair(x & kNibMask, __low2bfloat162(s.lo), __low2bfloat162(s.off));
+    k8 = dequant_pair(x & kHiNibMask, __low2bfloat162(s.hi), __low2bfloat162(s.off));
+    second_k0 = dequant_pair(y & kNibMask, __high2bfloat162(s.lo), __high2bfloat162(s.off));
+    second_k8 = dequant_pair(y & kHiNibMask, __high2bfloat162(s.hi), __high2bfloat162(s.off));
+}
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                                uint32_t b1) {
