@@ -309,28 +309,50 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
 kiln_w4a16_status_t kiln_w4a16_gemm_bf16_grouped(const kiln_w4a16_problem_t *problems, int count, void *workspace,
                                                  size_t workspace_bytes, void *stream) {
     if (!problems || count < 1 || count > KILN_W4A16_MAX_GROUP) return KILN_W4A16_ERR_ARG;
-    DecodeItem items[KILN_W4A16_MAX_GROUP] = {};
-    bool one_launch = true;
-    int live = 0;
+    GemmArgs live[KILN_W4A16_MAX_GROUP];
+    int count_live = 0;
+    bool decode = true, same = true;  // all for the kernels that apply the scales in fp32; rows, K and group size alike
     for (int i = 0; i < count; ++i) {
         const kiln_w4a16_problem_t &q = problems[i];
-        GemmArgs a{q.A, q.B, q.s, q.C, q.m, q.n, q.k, q.groupsize, workspace, workspace_bytes, static_cast<cudaStream_t>(stream)};
+        const GemmArgs a{q.A, q.B, q.s, q.C, q.m, q.n, q.k, q.groupsize, workspace, workspace_bytes, static_cast<cudaStream_t>(stream)};
         const int v = validate(a);
         if (v > 0) return v;
         if (v == 0) continue;  // an empty problem
-        if (use_prefill(q.m, q.n, q.k, q.groupsize)) one_launch = false;  // (one decode launch for the group beat per-problem launches of
-                                                                                       // the first small-batch kernel; not measured against the present one)
-        items[live++] = DecodeItem{q.A, q.B, q.s, q.C, q.m, q.n, q.k, q.groupsize, nullptr, nullptr, 0, 0};
+        if (use_prefill(q.m, q.n, q.k, q.groupsize)) decode = false;
+        const GemmArgs &first = count_live ? live[0] : a;
+        if (a.m != first.m || a.k != first.k || a.groupsize != first.groupsize) same = false;
+        live[count_live++] = a;
     }
-    if (live == 0) return KILN_W4A16_OK;
-    // one batch class per launch: up to 8 rows, or 9 and more
-    for (int i = 1; i < live; ++i)
-        if ((items[i].m <= 8) != (items[0].m <= 8)) one_launch = false;
-    if (one_launch) return launch_decode_list(items, live, static_cast<cudaStream_t>(stream), g_decode_override);
-    for (int i = 0; i < live; ++i) {  // batch sizes of the tcgen05 kernel, or mixed classes: one launch each
-        const DecodeItem &q = items[i];
-        if (int rc = kiln_w4a16_gemm_bf16(q.A, q.B, q.C, q.S, q.m, q.n, q.k, q.groupsize, workspace, workspace_bytes, stream))
-            return rc;
+    if (count_live == 0) return KILN_W4A16_OK;
+    // One launch where the problems are alike and each would run on the small-batch kernel's variant by itself (2560 -> 4096, 512 and 512,
+    // us, decode kernel / this: 9 rows 5.5 / 5.5, 16 6.2 / 5.6, 17 11.3 / 7.5, 32 11.6 / 7.5).
+    bool exact = same && count_live > 1;
+    for (int i = 0; i < count_live; ++i) exact = exact && decode && use_exact(live[i]);
+    if (exact) return launch_exact_group(live, count_live);
+    // one batch class per launch of the decode kernel: up to 8 rows, or 9 and more
+    for (int i = 1; i < count_live; ++i)
+        if ((live[i].m <= 8) != (live[0].m <= 8)) decode = false;
+    if (decode) {
+        DecodeItem items[KILN_W4A16_MAX_GROUP] = {};
+        for (int i = 0; i < count_live; ++i) {
+            const GemmArgs &q = live[i];
+            items[i] = DecodeItem{q.A, q.B, q.S, q.C, q.m, q.n, q.k, q.groupsize, nullptr, nullptr, 0, 0};
+        }
+        return launch_decode_list(items, count_live, static_cast<cudaStream_t>(stream), g_decode_override);
+    }
+    // Batch sizes of the tcgen05 kernels, or mixed classes: one launch each, except that neighbours which are alike and which the small-batch
+    // kernel, or its variant with fp32 scales, runs by themselves share theirs (2560 -> 512 twice beside 2560 -> 4096, 64 rows 12.0 -> 9.6 us).
+    auto variant = [&](const GemmArgs &q) {  // 1: small-batch kernel, 2: its variant, 0: another
+        if (!use_prefill(q.m, q.n, q.k, q.groupsize, true)) return use_exact(q) ? 2 : 0;
+        return smallm_takes(q.m, q.n, q.k, q.groupsize) ? 1 : 0;
+    };
+    for (int i = 0; i < count_live;) {
+        const GemmArgs &q = live[i];
+        const int kind = variant(q);
+        int next = i + 1;
+        while (kind && next < count_live && live[next].m == q.m && live[next].k == q.k && live[next].groupsize == q.groupsize && variant(live[next]) == kind) ++next;
+        if (int rc = next == i + 1 ? gemm(q) : kind == 2 ? launch_exact_group(&q, next - i) : launch_plain_group(&q, next - i)) return rc;
+        i = next;
     }
     return KILN_W4A16_OK;
 }

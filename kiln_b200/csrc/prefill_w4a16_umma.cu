@@ -935,6 +935,19 @@ bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r
            smallm_supported(std::min(m, 16), n, k, groupsize, exact_splits(m, n, k, swiglu));
 }
 int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
+// GEMMs of the same rows, K and group size, in launches of as many as one takes; the K splits are those of one with all columns.
+static int launch_groups(const GemmArgs *items, int count, bool exact) {
+    for (int i = 0; i < count; i += smallm_most_grouped()) {
+        const int c = std::min(count - i, smallm_most_grouped());
+        int n = 0;
+        for (int j = i; j < i + c; ++j) n += items[j].n;
+        const int splits = exact ? exact_splits(items[i].m, n, items[i].k, false) : choose_smallm_splits(items[i].m, n, items[i].k);
+        if (int rc = launch_smallm_group(items + i, c, splits, exact)) return rc;
+    }
+    return 0;
+}
+int launch_exact_group(const GemmArgs *items, int count) { return launch_groups(items, count, true); }
+int launch_plain_group(const GemmArgs *items, int count) { return launch_groups(items, count, false); }
 
 // SwiGLU is fused into an epilogue that sees whole tiles: the small-batch kernel's without a K split, or the pair kernel's.  A second
 // pass over the bf16 result takes about 4 us, more than a K split saves a SwiGLU-sized projection, except for a long K and few columns.

@@ -174,6 +174,20 @@ __device__ __forceinline__ void sts_v4(uint32_t addr, float a, float b, float c,
 // 4 + qd}.
 __device__ __forceinline__ void dequant_word(uint32_t x, const WeightScale &s, uint32_t *r) { dequant_word(x, s, r[0], r[2], r[1], r[3]); }
 
+// Further GEMMs of one launch, which have the rows, the K, the group size and the K splits of the first in common: blockIdx.y runs over the
+// tiles of all of them.  (A template parameter, because what a launch passes and looks up for them costs a single GEMM a few per cent.)
+constexpr int kMaxGroup = 4;
+template <bool GROUP>
+struct SmallMGroup {};
+template <>
+struct SmallMGroup<true> {
+    CUtensorMap w[kMaxGroup], s[kMaxGroup], x[kMaxGroup], c[kMaxGroup];
+    const __half *S[kMaxGroup];
+    __nv_bfloat16 *C[kMaxGroup];
+    int n[kMaxGroup], tile0[kMaxGroup];
+    int count;
+};
+
 // Stages in flight: TMEM slots of weights, and activation slots in shared memory
 template <int R>
 constexpr int slots() {
@@ -187,11 +201,11 @@ constexpr int slots() {
 // precision here.  The teams' sums meet in tensor memory, and a LoRA delta is added to them in fp32 from the fp32 projection.  More than
 // sixteen rows are so many more CTAs (blockIdx.z): for projections of few columns, which leave the GPU empty otherwise.
 // R: most rows.  SWIGLU is a template parameter so that the plain epilogue is compiled on its own.
-template <int R, bool SWIGLU, bool EXACT>
+template <int R, bool SWIGLU, bool EXACT, bool GROUP = false>
 __global__ void __launch_bounds__(kThreads, 1)
 w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_x,
                     const __grid_constant__ CUtensorMap tmap_t, const __grid_constant__ CUtensorMap tmap_c,
-                    const __grid_constant__ SmallMParams p) {
+                    const __grid_constant__ SmallMParams p, const __grid_constant__ SmallMGroup<GROUP> g) {
     constexpr int kSlots = slots<R>();
     static_assert(kSlots >= kTeams && kSlots <= kMaxSlots, "see kMaxWSlots");
     static_assert(!EXACT || (kTeams <= kSlots && kTeams * kExactRows <= R && kExactRows == 4 * kTeams), "see above");
@@ -206,7 +220,22 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(bar_mem + 8 * kBars + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = blockIdx.x, nt = blockIdx.y, m0 = EXACT ? blockIdx.z * kExactRows : 0;  // K split (= rank in the cluster), tile, first row
+    int tile = blockIdx.y, width = p.n;
+    const CUtensorMap *map_w = &tmap_w, *map_s = &tmap_s, *map_x = &tmap_x, *map_c = &tmap_c;
+    const __half *scales = p.S;
+    __nv_bfloat16 *result = p.C;
+    if constexpr (GROUP) {
+        int i = 0;
+#pragma unroll
+        for (int j = 1; j < kMaxGroup; ++j)
+            if (j < g.count && tile >= g.tile0[j]) i = j;
+        tile -= g.tile0[i];
+        width = g.n[i];
+        map_w = &g.w[i], map_s = &g.s[i], map_x = &g.x[i], map_c = &g.c[i];
+        scales = g.S[i];
+        result = g.C[i];
+    }
+    const int rank = blockIdx.x, nt = tile, m0 = EXACT ? blockIdx.z * kExactRows : 0;  // K split (= rank in the cluster), tile, first row
     const int ks0 = rank * p.k_stages / p.splits, ks1 = (rank + 1) * p.k_stages / p.splits, n_st = ks1 - ks0;
     const int lora_it = (!EXACT && rank == 0 && p.lora_r > 0) ? 1 : 0;  // the CTA that starts the tile's K range begins with the LoRA iteration
     const int n_it = n_st + lora_it;
@@ -225,10 +254,10 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             mbar_arrive_expect_tx(bar(kBarExchange), static_cast<uint32_t>((p.splits - 1) * own) * kTileCols * 16u);
         }
     } else if (warp == 3 && lane == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_s) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_c) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map_w) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map_s) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map_x) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map_c) : "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -256,7 +285,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 if (i == p.w_slots) pdl_wait();  // (park until the consumers run)
                 if (i >= p.w_slots && !(ok = mbar_wait(bar(kBarWEmpty + s), ph, abort_flag, p.status, 0xA00u | s, p.wait_limit_ns))) break;
                 mbar_arrive_expect_tx(bar(kBarWFull + s), kWSlotBytes);
-                tma_load_2d(smem_base + s * kWSlotBytes, &tmap_w, nt * (2 * kTileCols), (ks0 + i) * (kStageK / 16), bar(kBarWFull + s));
+                tma_load_2d(smem_base + s * kWSlotBytes, map_w, nt * (2 * kTileCols), (ks0 + i) * (kStageK / 16), bar(kBarWFull + s));
                 if (++s == p.w_slots) {
                     s = 0;
                     ph ^= 1;
@@ -270,7 +299,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) {
             if (!p.per_column) {  // the scales of all stages (rows past the CTA's last one are not used)
                 mbar_arrive_expect_tx(bar(kBarScales), p.scale_rows * kScaleBytes);
-                tma_load_2d(smem_base + p.off_scale, &tmap_s, nt * kTileCols, ks0, bar(kBarScales));
+                tma_load_2d(smem_base + p.off_scale, map_s, nt * kTileCols, ks0, bar(kBarScales));
             }
             pdl_wait();  // the activations may be the previous kernel's output
             bool ok = true;
@@ -283,7 +312,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     tma_load_2d(dst, &tmap_t, 0, 0, full(s));
                     tma_load_2d(dst + x_bytes, &tmap_t, kAtomK, 0, full(s));
                 } else {
-                    tma_load_3d(dst, &tmap_x, 0, m0, (ks0 + it - lora_it) * 2, full(s));
+                    tma_load_3d(dst, map_x, 0, m0, (ks0 + it - lora_it) * 2, full(s));
                 }
                 if (++s == kSlots) {
                     s = 0;
@@ -516,7 +545,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (p.splits == 1) {
             // The bf16 tile is put together in shared memory (over the rings, which are spent) and leaves through TMA: two-byte
             // stores from registers cost 8 cycles of the SM's load / store unit each.
-            const float cs = (p.per_column ? __half2float(p.S[scale_single_pos(col)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
+            const float cs = (p.per_column ? __half2float(scales[scale_single_pos(col)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
             const int ocol = SWIGLU ? ch * 32 + 16 * h + (lane & 15) : col_in_tile;  // output column within the tile
             const uint32_t stage = smem_base + (ocol >> 6) * x_bytes + (ocol & 7) * 2;
             const uint32_t chunk16 = (ocol & 63) >> 3;  // 16-byte chunk of a 128-byte row, XORed with row % 8
@@ -571,8 +600,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             fence_proxy_async_smem();
             asm volatile("bar.sync 1, %0;" ::"n"(kTeamThreads) : "memory");  // (every warp of the teams comes here, whatever happened)
             if (ok && warp == kTeamWarp0 && lane == 0) {
-                tma_store_2d(&tmap_c, smem_base, nt * (SWIGLU ? kTileCols / 2 : kTileCols), m0);  // (rows past m are clipped)
-                if (!SWIGLU) tma_store_2d(&tmap_c, smem_base + x_bytes, nt * kTileCols + 64, m0);
+                tma_store_2d(map_c, smem_base, nt * (SWIGLU ? kTileCols / 2 : kTileCols), m0);  // (rows past m are clipped)
+                if (!SWIGLU) tma_store_2d(map_c, smem_base + x_bytes, nt * kTileCols + 64, m0);
                 bulk_commit_group();
                 bulk_wait_group_read0();  // (the end of the grid completes them)
             } else if (!ok && warp == kTeamWarp0 && lane == 0) {
@@ -620,7 +649,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     const int own = min(p.quads_per_rank, p.quads - rank * p.quads_per_rank);
                     const int x = (warp - kTeamWarp0) * 32 + lane, cc = x & (kTileCols - 1);
                     const int gcol = nt * kTileCols + cc;
-                    const float cs = (p.per_column ? __half2float(p.S[scale_single_pos(gcol)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
+                    const float cs = (p.per_column ? __half2float(scales[scale_single_pos(gcol)]) : 1.f) * (EXACT ? 1.f : kWeightUnscale);
                     for (int slot = x >> 7; slot < own; slot += kTeamThreads / kTileCols) {
                         const uint32_t src = recv + static_cast<uint32_t>(slot * kTileCols + cc) * 16u;
                         const uint4 v0 = lds_v4(src);
@@ -635,7 +664,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         const int row0 = m0 + (rank * p.quads_per_rank + slot) * 4;
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
-                            if (row0 + i < p.m) p.C[static_cast<size_t>(row0 + i) * p.n + gcol] = __float2bfloat16_rn(v[i] * cs);
+                            if (row0 + i < p.m) result[static_cast<size_t>(row0 + i) * width + gcol] = __float2bfloat16_rn(v[i] * cs);
                     }
                 } else {
                     // A warp finishes a quad of rows, four adjacent columns a lane, and stores 256 contiguous bytes of each row: two-byte
@@ -662,8 +691,8 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         const int row0 = m0 + (rank * p.quads_per_rank + slot) * 4;
                         float cs[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) cs[j] = (p.per_column ? __half2float(p.S[scale_single_pos(gcol + j)]) : 1.f) * kWeightUnscale;
-                        __nv_bfloat16 *dst = p.C + static_cast<size_t>(row0) * p.n + gcol;
+                        for (int j = 0; j < 4; ++j) cs[j] = (p.per_column ? __half2float(scales[scale_single_pos(gcol + j)]) : 1.f) * kWeightUnscale;
+                        __nv_bfloat16 *dst = result + static_cast<size_t>(row0) * width + gcol;
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float a0 = turn & 1 ? v[3][i] : v[0][i], a1 = turn & 1 ? v[0][i] : v[1][i], a2 = turn & 1 ? v[1][i] : v[2][i],
@@ -671,7 +700,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                             const float c0 = turn & 2 ? a2 : a0, c1 = turn & 2 ? a3 : a1, c2 = turn & 2 ? a0 : a2, c3 = turn & 2 ? a1 : a3;
                             __nv_bfloat162 lo = __floats2bfloat162_rn(c0 * cs[0], c1 * cs[1]), hi = __floats2bfloat162_rn(c2 * cs[2], c3 * cs[3]);
                             if (row0 + i < p.m)
-                                *reinterpret_cast<uint2 *>(dst + static_cast<size_t>(i) * p.n) =
+                                *reinterpret_cast<uint2 *>(dst + static_cast<size_t>(i) * width) =
                                     make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
                         }
                     }
@@ -734,8 +763,10 @@ int smallm_clusters(int splits) {
     return cached[dev][splits];
 }
 
-// C = A * dequant(B) with `splits` K splits (one cluster per tile).  exact: group scales applied in fp32.
-int launch_smallm(const GemmArgs &a, int splits, bool exact) {
+// C = A * dequant(B) with `splits` K splits (one cluster per tile), for up to kMaxGroup GEMMs that share rows, K and group size (several:
+// no epilogue options).  exact: group scales applied in fp32.
+int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact) {
+    const GemmArgs &a = items[0];
     EncodeTiledFn enc = encode_fn();
     if (!enc) return KILN_W4A16_ERR_CUDA;
     uint32_t *status = device_status_word();
@@ -743,47 +774,60 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
     const int rows = exact ? std::min(a.m, kExactRows) : a.m;  // of a CTA
     if (!smallm_supported(rows, a.n, a.k, a.groupsize, splits) || (a.swiglu && splits != 1)) return KILN_W4A16_ERR_KERN_SHAPE;
 
-    const int npad = (rows + 15) & ~15;
-    CUtensorMap tmap_w, tmap_s, tmap_x, tmap_t;
-    {  // packed words: [k/16][2n] int32, boxes of one tile x eight rows (128 K)
-        const cuuint64_t dims[2] = {2ull * a.n, static_cast<cuuint64_t>(a.k / 16)}, strides[1] = {8ull * a.n};
-        const cuuint32_t box[2] = {2 * kTileCols, kStageK / 16}, estr[2] = {1, 1};
-        if (enc(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void *>(a.B), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return KILN_W4A16_ERR_CUDA;
+    if (count < 1 || count > kMaxGroup) return KILN_W4A16_ERR_ARG;
+    int tiles = a.n / kTileCols;
+    for (int i = 1; i < count; ++i) {
+        const GemmArgs &b = items[i];
+        if (b.m != a.m || b.k != a.k || b.groupsize != a.groupsize || b.n % kTileCols != 0) return KILN_W4A16_ERR_KERN_SHAPE;
+        tiles += b.n / kTileCols;
     }
-    tmap_s = tmap_w;  // (unused with per-column scales)
-    const int stages = (a.k / kStageK + splits - 1) / splits;
-    if (a.groupsize != -1) {  // scales [k/128][n] fp16, boxes of one tile x the most stages a CTA has (rows past the matrix read zero)
-        const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.n), static_cast<cuuint64_t>(a.k / kStageK)}, strides[1] = {2ull * a.n};
-        const cuuint32_t box[2] = {kTileCols, static_cast<cuuint32_t>(stages)}, estr[2] = {1, 1};
-        if (enc(&tmap_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(a.S), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return KILN_W4A16_ERR_CUDA;
-    }
+    if (tiles > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
+
+    const int npad = (rows + 15) & ~15, stages = (a.k / kStageK + splits - 1) / splits;
     auto encode = [&](CUtensorMap *map, const void *ptr, int cols) {  // boxes of 64 columns x all rows, 128-byte swizzle
         const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(a.m)}, strides[1] = {static_cast<cuuint64_t>(cols) * 2};
         const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(npad)}, estr[2] = {1, 1};
         return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
-    {  // activations [m, k] seen as [k/64][m][64], so that one copy brings both 64-deep tiles of a stage
-        const cuuint64_t dims[3] = {kAtomK, static_cast<cuuint64_t>(a.m), static_cast<cuuint64_t>(a.k / kAtomK)};
-        const cuuint64_t strides[2] = {static_cast<cuuint64_t>(a.k) * 2, kAtomK * 2};
-        // (test hook: boxes of eight rows less than the kernel announces, so that its waits for them run out)
-        const cuuint32_t box[3] = {kAtomK, static_cast<cuuint32_t>(test_drop_a_load() >= 0 ? npad - 8 : npad), 2}, estr[3] = {1, 1, 1};
-        if (enc(&tmap_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(a.A), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return KILN_W4A16_ERR_CUDA;
-    }
+    // tensor maps of one GEMM: packed words, scales (unused with per-column scales), activations, result (unused when K is split)
+    auto encode_maps = [&](const GemmArgs &q, CUtensorMap *w, CUtensorMap *s, CUtensorMap *x, CUtensorMap *c) {
+        {  // packed words: [k/16][2n] int32, boxes of one tile x eight rows (128 K)
+            const cuuint64_t dims[2] = {2ull * q.n, static_cast<cuuint64_t>(q.k / 16)}, strides[1] = {8ull * q.n};
+            const cuuint32_t box[2] = {2 * kTileCols, kStageK / 16}, estr[2] = {1, 1};
+            if (enc(w, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void *>(q.B), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return false;
+        }
+        *s = *w;
+        if (q.groupsize != -1) {  // scales [k/128][n] fp16, boxes of one tile x the most stages a CTA has (rows past the matrix read zero)
+            const cuuint64_t dims[2] = {static_cast<cuuint64_t>(q.n), static_cast<cuuint64_t>(q.k / kStageK)}, strides[1] = {2ull * q.n};
+            const cuuint32_t box[2] = {kTileCols, static_cast<cuuint32_t>(stages)}, estr[2] = {1, 1};
+            if (enc(s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(q.S), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return false;
+        }
+        {  // activations [m, k] seen as [k/64][m][64], so that one copy brings both 64-deep tiles of a stage
+            const cuuint64_t dims[3] = {kAtomK, static_cast<cuuint64_t>(q.m), static_cast<cuuint64_t>(q.k / kAtomK)};
+            const cuuint64_t strides[2] = {static_cast<cuuint64_t>(q.k) * 2, kAtomK * 2};
+            // (test hook: boxes of eight rows less than the kernel announces, so that its waits for them run out)
+            const cuuint32_t box[3] = {kAtomK, static_cast<cuuint32_t>(test_drop_a_load() >= 0 ? npad - 8 : npad), 2}, estr[3] = {1, 1, 1};
+            if (enc(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(q.A), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return false;
+        }
+        *c = *x;
+        return splits != 1 || encode(c, q.C, q.swiglu ? q.n / 2 : q.n);
+    };
+    CUtensorMap tmap_w, tmap_s, tmap_x, tmap_t, tmap_c;
+    if (!encode_maps(a, &tmap_w, &tmap_s, &tmap_x, &tmap_c)) return KILN_W4A16_ERR_CUDA;
     tmap_t = tmap_x;  // (unused without a LoRA delta)
     const bool lora = a.lora_r > 0 && a.lora_t && a.lora_b;
     if (lora) {
         if (a.groupsize == -1 || a.lora_r % 8 != 0 || a.lora_r > 128) return KILN_W4A16_ERR_KERN_SHAPE;
         if (!exact && !encode(&tmap_t, a.lora_t, a.lora_r)) return KILN_W4A16_ERR_CUDA;
     }
-    CUtensorMap tmap_c = tmap_x;  // (unused when K is split)
-    if (splits == 1 && !encode(&tmap_c, a.C, a.swiglu ? a.n / 2 : a.n)) return KILN_W4A16_ERR_CUDA;
+    if (count > 1 && (lora || a.swiglu)) return KILN_W4A16_ERR_KERN_SHAPE;
 
     SmallMParams p{};
     p.S = static_cast<const __half *>(a.S);
@@ -829,16 +873,16 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
     const int smem = std::max(p.w_slots * kWSlotBytes + fixed, p.off_lora + lora_bytes + 1024);
     if (smem > kMostSmem) return KILN_W4A16_ERR_KERN_SHAPE;
 
-    static bool attr_set[6][64] = {};  // per kernel variant and device: the shared-memory attribute is set once
+    static bool attr_set[9][64] = {};  // per kernel variant and device: the shared-memory attribute is set once
     int dev = 0;
     cudaGetDevice(&dev);
-    auto launch = [&](auto kernel, int variant) -> int {
+    auto launch = [&](auto kernel, int variant, const auto &group) -> int {
         if (dev < 64 && !attr_set[variant][dev]) {
             if (int rc = record_cuda_error(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem))) return rc;
             attr_set[variant][dev] = true;
         }
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(splits, a.n / kTileCols, exact ? (a.m + kExactRows - 1) / kExactRows : 1);
+        cfg.gridDim = dim3(splits, tiles, exact ? (a.m + kExactRows - 1) / kExactRows : 1);
         cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = a.stream;
@@ -851,11 +895,30 @@ int launch_smallm(const GemmArgs &a, int splits, bool exact) {
         cfg.attrs = attrs;
         cfg.numAttrs = splits > 1 ? 2 : 1;
         note_launch();
-        return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, tmap_w, tmap_s, tmap_x, tmap_t, tmap_c, p));
+        return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, tmap_w, tmap_s, tmap_x, tmap_t, tmap_c, p, group));
     };
-    if (exact) return a.swiglu ? launch(w4a16_smallm_kernel<64, true, true>, 5) : launch(w4a16_smallm_kernel<64, false, true>, 4);
-    if (a.swiglu) return a.m <= 64 ? launch(w4a16_smallm_kernel<64, true, false>, 2) : launch(w4a16_smallm_kernel<128, true, false>, 3);
-    return a.m <= 64 ? launch(w4a16_smallm_kernel<64, false, false>, 0) : launch(w4a16_smallm_kernel<128, false, false>, 1);
+    if (count > 1) {
+        SmallMGroup<true> g;
+        int tile0 = 0;
+        g.count = count;
+        for (int i = 0; i < count; ++i) {
+            const GemmArgs &q = items[i];
+            if (!encode_maps(q, &g.w[i], &g.s[i], &g.x[i], &g.c[i])) return KILN_W4A16_ERR_CUDA;
+            g.S[i] = static_cast<const __half *>(q.S);
+            g.C[i] = static_cast<__nv_bfloat16 *>(q.C);
+            g.n[i] = q.n;
+            g.tile0[i] = tile0;
+            tile0 += q.n / kTileCols;
+        }
+        if (exact) return launch(w4a16_smallm_kernel<64, false, true, true>, 8, g);
+        return rows <= 64 ? launch(w4a16_smallm_kernel<64, false, false, true>, 6, g) : launch(w4a16_smallm_kernel<128, false, false, true>, 7, g);
+    }
+    const SmallMGroup<false> none;
+    if (exact) return a.swiglu ? launch(w4a16_smallm_kernel<64, true, true>, 5, none) : launch(w4a16_smallm_kernel<64, false, true>, 4, none);
+    if (a.swiglu) return a.m <= 64 ? launch(w4a16_smallm_kernel<64, true, false>, 2, none) : launch(w4a16_smallm_kernel<128, true, false>, 3, none);
+    return a.m <= 64 ? launch(w4a16_smallm_kernel<64, false, false>, 0, none) : launch(w4a16_smallm_kernel<128, false, false>, 1, none);
 }
+int launch_smallm(const GemmArgs &a, int splits, bool exact) { return launch_smallm_group(&a, 1, splits, exact); }
+int smallm_most_grouped() { return kMaxGroup; }
 
 }  // namespace kiln

@@ -198,8 +198,12 @@ bool smallm_supported(int m, int n, int k, int groupsize, int splits);
 int smallm_clusters(int splits);
 bool smallm_takes(int m, int n, int k, int groupsize);
 int launch_smallm(const GemmArgs &a, int splits, bool exact = false);
+int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact);
+int smallm_most_grouped();
 bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r);
 int launch_exact(const GemmArgs &a);
+int launch_exact_group(const GemmArgs *items, int count);
+int launch_plain_group(const GemmArgs *items, int count);
 void set_test_drop_a_load(int k_step);
 int test_drop_a_load();
 void prefill_plan(int m, int n, int k, int out[4]);

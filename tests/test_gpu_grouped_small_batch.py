@@ -1,0 +1,38 @@
+"""Grouped launches of the small-batch kernel and of its variant with fp32 scales, against the fp64 oracle, and their number of launches.
+Tolerance: max|out - ref| / max|ref| <= 1e-2, as for single launches."""
+import numpy as np
+import pytest
+import torch
+
+import kiln_b200
+from kiln_b200 import _lib
+import oracle
+from oracle import C
+from tests.util import REL_TOL, from_torch_bf16, rel_err, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+# (rows, K, columns of each, group size, launches): nine to 32 rows in one launch; above, neighbours of one kind; five problems, two launches;
+# rows that are no multiple of four, and several CTAs of 16 rows; group sizes -1; the 128-row variant; one K stage; decode up to 8 rows
+@pytest.mark.parametrize("m,k,ns,groupsize,launches", [
+    (9, 640, (512, 256, 256), 128, 1), (16, 2560, (4096, 512, 512), 128, 1), (29, 640, (4096, 512, 512), 128, 1), (13, 384, (256,) * 5, 128, 2),
+    (13, 640, (512, 256), -1, 1), (37, 640, (4096, 512, 512), 128, 2), (50, 640, (512, 4096, 2048, 512), 128, 3), (101, 1280, (2048, 4096), 128, 1),
+    (64, 2560, (2048, 2048, 2048), 128, 1), (128, 128, (1280, 1280), 128, 1), (77, 640, (2048, 2048), -1, 1), (8, 640, (512, 256), 128, 1)])
+def test_alike_problems_share_a_launch(cuda_device, m, k, ns, groupsize, launches):
+    xs, projs, refs = [], [], []
+    for i, n in enumerate(ns):
+        a, q, s = oracle.synth_inputs(m, k, n, seed=m + n + i, groupsize=groupsize)
+        packed, sp = kiln_b200.pack.repack(q, s, groupsize)
+        projs.append(kiln_b200.MarlinPackedProj(torch.from_numpy(packed).to(cuda_device),
+                                                torch.from_numpy(sp.view(np.int16).copy()).view(torch.float16).to(cuda_device), groupsize, k, n))
+        xs.append(to_torch_bf16(a, cuda_device))
+        refs.append(C.gemm_fp64(a, q, s, groupsize))
+    lib = _lib.lib()
+    before = lib.kiln_w4a16_launch_count()
+    outs = kiln_b200.grouped_matmul_bf16(xs, projs)
+    torch.cuda.synchronize()
+    assert lib.kiln_w4a16_check_device_status(None, None) == 0
+    assert lib.kiln_w4a16_launch_count() - before == launches
+    for out, ref in zip(outs, refs):
+        assert rel_err(from_torch_bf16(out), ref) <= REL_TOL
