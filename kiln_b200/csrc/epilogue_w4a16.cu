@@ -6,7 +6,9 @@
 //  * finish_kernel: for batch sizes beyond the decode kernel's range, where the options are not fused yet:
 //    C = epilogue(base), base being the bf16 GEMM result in the workspace (LoRA delta added, SwiGLU applied).
 #include <algorithm>
+#include <atomic>
 
+#include "w4a16_async.cuh"
 #include "w4a16_common.cuh"
 
 namespace kiln {
@@ -19,33 +21,7 @@ __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_o
         static_cast<float *>(t)[idx] = v;
 }
 
-// Up to kLoraDotRows rows: one dot product per warp.  grid = (ceil(r / 8), m), block = 256: warp w of a CTA computes
-// t[row][8 * blockIdx.x + w].
-constexpr int kLoraDotRows = 8;
-__global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
-                                                       int k, int r, void *__restrict__ t, int bf16_out) {
-    pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int row = blockIdx.y, j = blockIdx.x * 8 + warp;
-    pdl_wait();  // x may be the previous kernel's output; t may still be read by it
-    if (j >= r) return;
-    const uint4 *xr = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row) * k);
-    const uint4 *ar = reinterpret_cast<const uint4 *>(a + static_cast<size_t>(j) * k);
-    float sum = 0.f;
-    for (int i = lane; i < k / 8; i += 32) {
-        const uint4 xv = ld_cg_v4(xr + i), av = ar[i];
-        const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, as[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            sum += __uint_as_float(xs[e] << 16) * __uint_as_float(as[e] << 16) +
-                   __uint_as_float(xs[e] & 0xFFFF0000u) * __uint_as_float(as[e] & 0xFFFF0000u);
-    }
-#pragma unroll
-    for (int sh = 16; sh >= 1; sh >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, sh);
-    if (lane == 0) store_t(t, static_cast<size_t>(row) * r + j, sum * scale, bf16_out);
-}
-
-// More rows: a small tensor-core GEMM, K split over the CTAs of a cluster and, for few rows, over the warps of a CTA.
+// A small tensor-core GEMM, K split over the CTAs of a cluster and, for few rows, over the warps of a CTA.
 //
 // Bound: latency.  The operands are a few hundred KB (x 37 x 9216 and A 64 x 9216: 1.9 MB), so what counts is how many SMs load
 // them at once and how short the chain from the grid-dependency wait to the last store is.  A lane loads 16 contiguous bytes of
@@ -53,10 +29,22 @@ __global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__re
 // permutation on both sides, so no shared-memory staging and no ldmatrix.
 // A CTA has WM row tiles of 16 and 8 / WM parts of its K range, one (row tile, part) per warp, and 8 NT adapter rows.  Small tiles
 // nearly always (many CTAs, short chains: 64 rows, 9216 -> 2560 with its GEMM 21 -> 13 us against tiles of 64 x 32), large ones for
-// very many rows (x is read once per 8 NT adapter rows).  The parts meet in shared
-// memory, the cluster's partial tiles in rank order through distributed shared memory: the result does not depend on timing.
-// Measured with the GEMM that follows, dot products -> tensor cores: 37 rows rank 64 9216 -> 2560 24 -> 15 us, 2560 -> 4096 13.3 ->
-// 10.7, 2048 rows 96 -> 49; 4 rows 7.6 -> 8.2, hence the line above.
+// very many rows (x is read once per 8 NT adapter rows).  The parts meet in shared memory; the cluster's partial tiles are pushed to
+// the rank that owns the elements (st.async, counted on its barrier; two cluster barriers around reads took 0.7 us more) and added there
+// in rank order: the result does not depend on timing.
+// AHEAD: the first blocks of a warp whose loads are all in flight at once, and the adapter, cold in HBM in a model of many layers, is asked
+// into L2 before the grid-dependency wait.  (Reading it before the wait would be another 2 % faster, but a caller may have written it.)
+// By itself, us: 37 rows rank 64 K = 2560 3.0 -> 2.3, K = 9216 4.0 -> 3.0.  Few rows were dot products, a warp each: 4 rows rank 64 K = 2560
+// 2.35 -> 1.96, K = 9216 5.35 -> 2.5.  Four layers with it: 8 rows 254 -> 188, 37 rows 218 -> 188, 128 rows 301 -> 275.
+template <int NT>
+__device__ __forceinline__ void lora_mma_block(const uint4 &u, const uint4 &v, const uint4 (&w)[NT], float (&acc)[NT][4]) {
+    const uint32_t lo[4] = {u.x, v.x, u.y, v.y}, hi[4] = {u.z, v.z, u.w, v.w};
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        mma_bf16_16816(acc[t], lo, w[t].x, w[t].y);
+        mma_bf16_16816(acc[t], hi, w[t].z, w[t].w);
+    }
+}
 template <int NT>
 __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1, const uint4 *const (&a)[NT], int b0, int b1, float (&acc)[NT][4]) {
 #pragma unroll 4
@@ -76,18 +64,34 @@ __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1,
 // (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernels read as an operand tile; fp32 otherwise)
 template <int WM, int NT>
 constexpr int lora_smem() {
-    return 8 * 16 * 8 * NT * static_cast<int>(sizeof(float));
+    return (8 * 16 * 8 * NT + 16 * WM * 8 * NT + 8) * static_cast<int>(sizeof(float));
 }
-template <int WM, int NT>
+template <int WM, int NT, int AHEAD>
 __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
-                                                        int m, int k, int r, void *__restrict__ t, int bf16_out) {
+                                                        int m, int k, int r, void *__restrict__ t, int bf16_out, uint32_t *status,
+                                                        unsigned long long wait_limit_ns) {
     constexpr int kCols = 8 * NT, kRows = 16 * WM, kParts = 8 / WM, kTile = kRows * kCols;
-    extern __shared__ float parts[];  // [kParts][kRows][kCols]; the last one ends up with the sum
-    float *sum = parts + (kParts - 1) * kTile;
+    extern __shared__ float parts[];  // [kParts][kRows][kCols], then what the ranks push
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane >> 2, qd = lane & 3;
     const int wm = warp % WM, part = warp / WM;
     const int rank = blockIdx.x, size = gridDim.x;
+    // A rank of the cluster owns `each` elements of the tile, the last ones fewer or none.  (armed before the wait; that every CTA runs is
+    // checked before the first push)
+    const int each = (kTile + size - 1) / size, own = max(0, min(each, kTile - rank * each));
+    __shared__ __align__(8) unsigned long long exchange;
+    __shared__ uint32_t gave_up;
+    const uint32_t bar = smem_u32(&exchange);
+    if (size > 1) {
+        if (threadIdx.x == 0) {
+            gave_up = 0;
+            mbar_init(bar, 1);
+            mbar_init_fence();
+            mbar_arrive_expect_tx(bar, static_cast<uint32_t>((size - 1) * own) * 4u);
+        }
+        __syncthreads();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
     const int row0 = blockIdx.z * kRows + wm * 16, col0 = blockIdx.y * kCols;
     const int blocks = k / 32, slices = size * kParts, slice = rank * kParts + part;
     const int b0 = static_cast<int>(static_cast<long long>(blocks) * slice / slices), b1 = static_cast<int>(static_cast<long long>(blocks) * (slice + 1) / slices);
@@ -100,8 +104,23 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
     }
     const uint4 *x0 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c, m - 1)) * k) + qd;
     const uint4 *x1 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c + 8, m - 1)) * k) + qd;
+    // The adapter's rows come to L2 before the wait, and are read after it: a kernel before this one may have written them.
+    for (int b = b0; AHEAD > 0 && b < b1; ++b)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) asm volatile("prefetch.global.L2 [%0];" ::"l"(ap[t] + b * 4));
     pdl_wait();  // x may be the previous kernel's output; t may still be read by it
-    lora_mma_range<NT>(x0, x1, ap, b0, b1, acc);
+    uint4 w[AHEAD + 1][NT], u[AHEAD + 1], v[AHEAD + 1];  // (the first blocks' loads are all in flight at once)
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+        if (b0 + i < b1) {
+            u[i] = ld_cg_v4(x0 + (b0 + i) * 4), v[i] = ld_cg_v4(x1 + (b0 + i) * 4);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) w[i][t] = ld_cg_v4(ap[t] + (b0 + i) * 4);
+        }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+        if (b0 + i < b1) lora_mma_block<NT>(u[i], v[i], w[i], acc);
+    lora_mma_range<NT>(x0, x1, ap, b0 + AHEAD, b1, acc);
     float *mine = parts + part * kTile + wm * 16 * kCols;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
@@ -109,29 +128,33 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
         *reinterpret_cast<float2 *>(mine + (c + 8) * kCols + 8 * i + 2 * qd) = make_float2(acc[i][2], acc[i][3]);
     }
     __syncthreads();
-    if (kParts > 1) {
-        for (int e = threadIdx.x; e < kTile; e += 256) {
-            float v = parts[e];
+    // Every CTA sums its parts and pushes each rank its share (counted on that rank's barrier), the owner adds the shares in rank order.
+    float *recv = parts + kParts * kTile;  // [rank][each]
+    if (size > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int e = threadIdx.x; e < kTile; e += 256) {
+        float v = parts[e];
 #pragma unroll
-            for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
-            sum[e] = v;  // (of the last part, this thread alone touches this element)
-        }
-        if (size == 1) __syncthreads();
+        for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
+        const int owner = e / each;
+        const uint32_t slot = smem_u32(recv + rank * each + e - owner * each);
+        if (owner == rank)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(v) : "memory");
+        else
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(map_to_cta(slot, owner)), "f"(v),
+                         "r"(map_to_cta(bar, owner))
+                         : "memory");
     }
-    if (size > 1) cluster_sync_all();
-    // the CTAs of the cluster take 256 elements of the tile in turn, one per thread, and sum them over the ranks
-    for (int e = threadIdx.x + rank * 256; e < kTile; e += size * 256) {
-        float v = 0.f;
-        const uint32_t addr = smem_u32(sum + e);
-        for (int q = 0; q < size; ++q) {
-            float u;
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(u) : "r"(map_to_cta(addr, q)));
-            v = q ? v + u : u;
-        }
-        const int row = blockIdx.z * kRows + e / kCols, col = col0 + e % kCols;
+    __syncthreads();
+    if (size > 1 && !mbar_wait(bar, 0, &gave_up, status, 0xC00u, wait_limit_ns)) {
+        mbar_wait_quiet(bar, 0, 32 * wait_limit_ns);  // (a peer pushes into this CTA until it is through)
+        return;
+    }
+    for (int i = threadIdx.x; i < own; i += 256) {
+        float v = recv[i];
+        for (int q = 1; q < size; ++q) v += recv[q * each + i];
+        const int e = rank * each + i, row = blockIdx.z * kRows + e / kCols, col = col0 + e % kCols;
         if (row < m && col < r) store_t(t, static_cast<size_t>(row) * r + col, v * scale, bf16_out);
     }
-    if (size > 1) cluster_sync_all();  // the peers may still be reading this CTA's tile
 }
 
 __device__ __forceinline__ float lora_dot(const float *t, const __nv_bfloat16 *b, int r) {
@@ -168,7 +191,6 @@ __global__ void __launch_bounds__(256) finish_kernel(const __nv_bfloat16 *__rest
 }  // namespace
 
 int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int k, int r, void *t, int bf16_out, cudaStream_t stream) {
-    const bool dot = m <= kLoraDotRows;
     // Rows and adapter rows of a CTA: 16 x 16, or 128 x 64 for more than 1024 rows of a large rank, where reading x once per 16
     // adapter rows costs more than the longer chains of large tiles (2048 x 9216, rank 64, with its GEMM: 118 / 114 us; 1024 rows: 65 / 83).
     const int wm = m > 1024 && r > 32 ? 8 : 1, rows = 16 * wm, cols = wm == 1 ? 16 : 64, parts = 8 / wm;
@@ -179,9 +201,9 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     int size = std::min(8, std::max(1, (wm == 1 ? 4 : 1) * device_sm_count() / (row_tiles * col_tiles)));
     size = std::max(1, std::min(size, k / 32 / (2 * parts)));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dot ? dim3((r + 7) / 8, m) : dim3(size, col_tiles, row_tiles);
+    cfg.gridDim = dim3(size, col_tiles, row_tiles);
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = dot ? 0 : (wm == 1 ? lora_smem<1, 2>() : lora_smem<8, 8>());
+    cfg.dynamicSmemBytes = wm == 1 ? lora_smem<1, 2>() : lora_smem<8, 8>();
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -191,12 +213,23 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     attrs[1].val.clusterDim.y = 1;
     attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
-    cfg.numAttrs = !dot && size > 1 ? 2 : 1;
+    cfg.numAttrs = size > 1 ? 2 : 1;
+    uint32_t *status = device_status_word();
+    if (!status) return KILN_W4A16_ERR_CUDA;
     const auto *xp = static_cast<const __nv_bfloat16 *>(x), *ap = static_cast<const __nv_bfloat16 *>(lora_a);
     note_launch();
-    if (dot) return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_dot_kernel, xp, ap, scale, k, r, t, bf16_out));
-    const auto kernel = wm == 1 ? lora_down_kernel<1, 2> : lora_down_kernel<8, 8>;
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out));
+    if (wm != 1) {  // (its shared memory is beyond what a launch may have unasked)
+        static std::atomic<bool> asked[64] = {};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 64 || !asked[dev].load(std::memory_order_acquire)) {
+            if (int rc = record_cuda_error(cudaFuncSetAttribute(lora_down_kernel<8, 8, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lora_smem<8, 8>()))) return rc;
+            if (dev < 64) asked[dev].store(true, std::memory_order_release);
+        }
+    }
+    // (76 registers against 62: only where all CTAs are resident either way, three to an SM)
+    const auto kernel = wm != 1 ? lora_down_kernel<8, 8, 0> : size * row_tiles * col_tiles <= 3 * device_sm_count() ? lora_down_kernel<1, 2, 2> : lora_down_kernel<1, 2, 0>;
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out, status, current_wait_limit_ns()));
 }
 
 int launch_finish(const void *base, void *c, int m, int n, const float *t, const void *lora_b, int r, int swiglu,

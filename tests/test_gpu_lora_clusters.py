@@ -1,0 +1,26 @@
+"""The LoRA projection for every cluster size (K = 512 d gives d CTAs), also those that do not divide a tile, rows of one tile and of two, and
+ranks that fill a column tile or not.  The base weight is tiny, so the result is the delta: tolerance 1e-2 of the largest, as elsewhere."""
+import pytest
+import torch
+
+import kiln_b200
+from kiln_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("r", [8, 24, 64])
+@pytest.mark.parametrize("k", [128, 512, 1024, 1536, 2048, 2560, 3072, 3584, 4096])
+def test_projection(cuda_device, k, r):
+    n, gen = 256, torch.Generator(device=cuda_device).manual_seed(k + r)
+    w = torch.full((k // 16, 2 * n), -0x77777778, dtype=torch.int32, device=cuda_device)  # every weight (8 - 8) s = 0
+    proj = kiln_b200.MarlinPackedProj(w, torch.full((k // 128, n), 0.01, dtype=torch.float16, device=cuda_device), 128, k, n)
+    for m in (1, 4, 8, 17, 40, 130):
+        x = torch.randn((m, k), device=cuda_device, generator=gen).bfloat16()
+        a = torch.randn((r, k), device=cuda_device, generator=gen).bfloat16()
+        b = torch.randn((n, r), device=cuda_device, generator=gen).bfloat16()
+        out = kiln_b200.matmul_bf16_lora(x, proj, a, b, 0.5)
+        torch.cuda.synchronize()
+        assert _lib.lib().kiln_w4a16_check_device_status(None, None) == 0
+        ref = 0.5 * (x.double() @ a.double().T) @ b.double().T
+        assert float((out.double() - ref).abs().max() / ref.abs().max()) <= 1e-2, m
