@@ -937,12 +937,11 @@ bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r
 int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
 // GEMMs of the same rows, K and group size, in launches of as many as one takes; the K splits are those of one with all columns.
 static int launch_groups(const GemmArgs *items, int count, bool exact) {
-    for (int i = 0; i < count; i += smallm_most_grouped()) {
-        const int c = std::min(count - i, smallm_most_grouped());
-        int n = 0;
-        for (int j = i; j < i + c; ++j) n += items[j].n;
+    for (int i = 0, end; i < count; i = end) {
+        int n = items[i].n;
+        for (end = i + 1; end < count && end < i + smallm_most_grouped() && static_cast<long long>(n) + items[end].n <= 65535LL * 128; ++end) n += items[end].n;
         const int splits = exact ? exact_splits(items[i].m, n, items[i].k, false) : choose_smallm_splits(items[i].m, n, items[i].k);
-        if (int rc = launch_smallm_group(items + i, c, splits, exact)) return rc;
+        if (int rc = launch_smallm_group(items + i, end - i, splits, exact)) return rc;
     }
     return 0;
 }
