@@ -935,12 +935,16 @@ bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r
            smallm_supported(std::min(m, 16), n, k, groupsize, exact_splits(m, n, k, swiglu));
 }
 int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
-// GEMMs of the same rows, K and group size, in launches of as many as one takes; the K splits are those of one with all columns.
+// GEMMs of the same rows, K and group size, in launches of as many as one takes.  The K splits are those of one GEMM with all columns, but
+// no fewer than a CTA's most stages ask for: more columns want fewer splits, and each member by itself may need the splits that it has.
 static int launch_groups(const GemmArgs *items, int count, bool exact) {
     for (int i = 0, end; i < count; i = end) {
-        int n = items[i].n;
+        const GemmArgs &a = items[i];
+        int n = a.n;
         for (end = i + 1; end < count && end < i + smallm_most_grouped() && static_cast<long long>(n) + items[end].n <= 65535LL * 128; ++end) n += items[end].n;
-        const int splits = exact ? exact_splits(items[i].m, n, items[i].k, false) : choose_smallm_splits(items[i].m, n, items[i].k);
+        int splits = exact ? exact_splits(a.m, n, a.k, false) : choose_smallm_splits(a.m, n, a.k);
+        for (int s : {2, 3, 4, 6, 8})
+            if (s > splits && !smallm_supported(exact ? std::min(a.m, 16) : a.m, a.n, a.k, a.groupsize, splits)) splits = s;
         if (int rc = launch_smallm_group(items + i, end - i, splits, exact)) return rc;
     }
     return 0;

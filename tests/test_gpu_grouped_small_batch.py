@@ -36,3 +36,28 @@ def test_alike_problems_share_a_launch(cuda_device, m, k, ns, groupsize, launche
     assert lib.kiln_w4a16_launch_count() - before == launches
     for out, ref in zip(outs, refs):
         assert rel_err(from_torch_bf16(out), ref) <= REL_TOL
+
+
+# K of 112 and 128 stages, where a CTA takes at most 96 and each problem by itself has two splits or more: the columns of all of them ask for fewer
+@pytest.mark.parametrize("m,k,ns,launches", [(16, 14336, (7168, 7168), 1), (64, 16384, (9216, 9216), 1), (100, 16384, (8192, 1024, 1024), 2),
+                                             (13, 28672, (4096, 1024, 1024), 1)])
+def test_alike_problems_of_a_long_k(cuda_device, m, k, ns, launches):
+    gen = torch.Generator(device=cuda_device).manual_seed(m + k)
+    xs, projs, refs = [], [], []
+    for n in ns:
+        q = torch.randint(0, 16, (k, n), dtype=torch.uint8, device=cuda_device, generator=gen)
+        s = (0.01 * torch.rand((k // 128, n), device=cuda_device, generator=gen) + 1e-3).half()
+        packed, sp = kiln_b200.pack.repack(q.cpu().numpy(), s.cpu().numpy(), 128)
+        projs.append(kiln_b200.MarlinPackedProj(torch.from_numpy(packed).to(cuda_device),
+                                                torch.from_numpy(sp.view(np.int16).copy()).view(torch.float16).to(cuda_device), 128, k, n))
+        xs.append(torch.randn((m, k), device=cuda_device, generator=gen).bfloat16())
+        w = (q.view(k // 128, 128, n).double() - 8.0) * s.double()[:, None]
+        refs.append((xs[-1].double() @ w.view(k, n)).float().cpu().numpy())
+    lib = _lib.lib()
+    before = lib.kiln_w4a16_launch_count()
+    outs = kiln_b200.grouped_matmul_bf16(xs, projs)
+    torch.cuda.synchronize()
+    assert lib.kiln_w4a16_check_device_status(None, None) == 0
+    assert lib.kiln_w4a16_launch_count() - before == launches
+    for out, ref in zip(outs, refs):
+        assert rel_err(from_torch_bf16(out), ref) <= REL_TOL
