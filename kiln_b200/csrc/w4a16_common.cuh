@@ -53,14 +53,15 @@ __device__ __forceinline__ uint32_t unscale_bf16x2(float lo, float hi) {
     const __nv_bfloat162 v = __hmul2(__floats2bfloat162_rn(lo, hi), *reinterpret_cast<const __nv_bfloat162 *>(&f));
     return *reinterpret_cast<const uint32_t *>(&v);
 }
-// silu(g) * u of sums that still have the factor, g' = g 2^-22 and u' = u 2^-22, which costs no instruction: e^-g = 2^(-g log2 e) takes
-// g's out in the product with log2 e, and g / (1 + e^-g) both of them in the sum, g' / (2^-44 + 2^-44 e^-g) = 2^22 g / (1 + e^-g).
+// silu(g) * u of sums that still have the factor, g' = g 2^-22 and u' = u 2^-22: e^-g = 2^(-g log2 e) takes g's out in the product with
+// log2 e, and 1 / (2^-22 + 2^-22 e^-g) once more for the quotient.  u's goes in a product of its own: no partial product is then larger or
+// smaller than its value, so nothing overflows or vanishes that the result does not.
 __device__ __forceinline__ float swiglu_scaled(float g, float u) {
-    constexpr float kLog2e = 1.4426950408889634f, kBoth = kWeightFactor * kWeightFactor;
+    constexpr float kLog2e = 1.4426950408889634f;
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * (-kLog2e * kWeightUnscale)));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(e, kBoth, kBoth)));  // (__fdividef is slow for a divisor this small)
-    return g * r * u;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(e, kWeightFactor, kWeightFactor)));
+    return g * r * (u * kWeightUnscale);
 }
 // the eight weights of a packed word: K 2qd, 2qd + 1 and 2qd + 8, 2qd + 9 of the first column (c), then of the second (c + 8)
 __device__ __forceinline__ void dequant_word(uint32_t x, const WeightScale &s, uint32_t &k0, uint32_t &k8, uint32_t &second_k0, uint32_t &second_k8) {

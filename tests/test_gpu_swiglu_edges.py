@@ -47,3 +47,33 @@ def test_silu_of_a_gate_near_its_underflow(cuda_device, m):
     v = x_t[:, 0].double().numpy()
     ref = (7 * v / (1 + np.exp(-7 * v)) * v)[:, None]
     assert np.abs(out / ref - 1).max() <= 2.0 ** -8 + 2e-5
+
+
+# the kernel of CTA pairs, 256 and 128 columns a tile
+@pytest.mark.parametrize("groupsize", [128, -1])
+@pytest.mark.parametrize("m,n_half", [(129, 1024), (300, 1024), (512, 9216)])
+def test_extreme_gates_and_ups_of_the_pair_kernel(cuda_device, m, n_half, groupsize):
+    """No step from the sums to silu(gate) * up may overflow or vanish where the result does not.  Relative error: half a unit of bf16 (at most
+    2^-8), plus the exponential's error for |gate| up to 88 (2e-5, as above).  Zeros and infinities are exact."""
+    k = 256
+    q = np.full((k, n_half), 8, np.uint8)
+    qg, qu = q.copy(), q.copy()
+    qg[0], qu[1] = 9, 9          # gate = x[0], up = x[1]
+    s = np.ones((1 if groupsize == -1 else 2, n_half), np.float16)
+    pairs = [(1e32, 1.0), (1e32, 0.0), (1e35, -1e-10), (3e38, 1e-30), (3e38, 1.0), (1e30, 1e30), (-87.0, 1.0), (-87.0, 40.0), (-60.0, 1e-6), (-20.0, 1e30),
+             (-1e5, 1e5), (0.0, 7.0), (1e-30, 1.0), (50.0, 1e-30), (2.0, 3e38), (-0.5, 0.25), (5.0, -3.0)]
+    x = torch.zeros((m, k))
+    x[:, :2] = torch.tensor([pairs[i % len(pairs)] for i in range(m)])
+    x = x.bfloat16()
+    fused = kiln_b200.interleave_gate_up(_proj(qg, s, groupsize, cuda_device), _proj(qu, s, groupsize, cuda_device))
+    out = kiln_b200.swiglu_gate_up(x.to(cuda_device), fused).cpu().double().numpy()
+    assert _lib.lib().kiln_w4a16_check_device_status(None, None) == 0
+    g, u = x[:, 0].double().numpy(), x[:, 1].double().numpy()
+    with np.errstate(over="ignore"):
+        ref = (g / (1.0 + np.exp(-g)) * u)[:, None] * np.ones((1, n_half))
+    large = np.abs(ref) > 3.4e38
+    exact = large | (np.abs(ref) < 2.0 ** -149)
+    want = np.where(exact, 0.0, ref)
+    want[large] = np.sign(ref[large]) * np.inf
+    assert (out[exact] == want[exact]).all()
+    assert np.abs(out[~exact] / want[~exact] - 1).max() <= 2.0 ** -8 + 2e-5

@@ -11,7 +11,7 @@ from kiln_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-# rows -> kernel: 16 fp32 scales; 48, 128 small-batch; 129, 256 CTA pairs (split K or whole tiles); 1024 x 256 columns: single-CTA tiles
+# rows -> kernel: 16 fp32 scales; 48, 128 small-batch; 129, 256 CTA pairs (split K or whole tiles); 300 x 256 columns: single-CTA tiles
 @pytest.mark.parametrize("groupsize", [128, -1])
 @pytest.mark.parametrize("m,n", [(16, 2048), (48, 2048), (128, 2048), (129, 2048), (256, 18432), (300, 256)])
 def test_a_weight_comes_out_as_it_was_packed(cuda_device, m, n, groupsize):
