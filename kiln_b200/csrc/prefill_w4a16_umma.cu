@@ -270,14 +270,14 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             uint32_t o[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                float x0 = __uint_as_float(ra[8 * v + 2 * e]) + __uint_as_float(rb[8 * v + 2 * e]);
-                                float x1 = __uint_as_float(ra[8 * v + 2 * e + 1]) + __uint_as_float(rb[8 * v + 2 * e + 1]);
+                                float x0 = (__uint_as_float(ra[8 * v + 2 * e]) + __uint_as_float(rb[8 * v + 2 * e])) * kWeightUnscale;
+                                float x1 = (__uint_as_float(ra[8 * v + 2 * e + 1]) + __uint_as_float(rb[8 * v + 2 * e + 1])) * kWeightUnscale;
                                 if (p.per_column) {
                                     const int pos = scale_single_pos(col + 8 * v + 2 * e);
                                     x0 *= __half2float(p.S[pos]);
                                     x1 *= __half2float(p.S[pos + 1]);
                                 }
-                                o[e] = unscale_bf16x2(x0, x1);
+                                o[e] = pack_bf16x2(x0, x1);
                             }
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
                                              epi_tma + lane * 128 + (((half * 4 + v) ^ (lane & 7)) << 4)),
@@ -342,14 +342,14 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             uint32_t o[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]);
-                                float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]);
+                                float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]) * kWeightUnscale;
+                                float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]) * kWeightUnscale;
                                 if (p.per_column) {
                                     const int pos = scale_single_pos(col + 8 * v + 2 * e);
                                     x0 *= __half2float(p.S[pos]);
                                     x1 *= __half2float(p.S[pos + 1]);
                                 }
-                                o[e] = unscale_bf16x2(x0, x1);
+                                o[e] = pack_bf16x2(x0, x1);
                             }
                             // 128-byte rows, 16-byte chunk index XOR (row % 8): the layout of the 128B-swizzled tensor map
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(

@@ -26,8 +26,11 @@ constexpr int kChunkCols = 64;  // N columns per 512-byte block
 // exponent's lowest, is nibble * 2^-129: subnormals and the first normal binade are one linear scale.  So the fused multiply-add
 // brings nibble * s - 8 s, rounded once, which is what subtracting 8 and multiplying by s in two steps gives.  s * 2^133 would be
 // too large for bf16; with the factor of 2^-22 it is not, whatever the fp16 scale is (the largest rounds to 2^16).  The
-// factor is a power of two, so it changes no rounding; what reads the sums takes it out (kWeightUnscale).
-// An infinite scale gives NaN.  Sums below 2^-104 lose precision, as they did below 2^-126 without the factor.
+// factor is a power of two, so it changes no rounding; what reads the sums takes it out (kWeightUnscale), in fp32: a product after
+// the rounding to bf16, one instruction for two, would round sums below 2^-104 as the subnormals that they are with it (0 to 1 % of a launch).
+// An infinite scale gives NaN (without the factor, infinity except for a nibble of 8; a sum over a group of 128 was NaN either way unless no
+// activation is 0, no nibble 8 and all products have one sign).  Sums in fp32 reach down to 2^-149 at the factor, so a sum has eight good
+// bits from 2^-119 on (from 2^-126, where bf16's subnormals begin, without it).
 // Nine instructions for a packed word's eight weights; OR-ing the nibbles into 128.0, subtracting 136 and multiplying took fifteen, and
 // the dequantising warps bound every kernel that uses this up to a few hundred rows (37 rows 2560 -> 18432 10.4 -> 9.4 us, 9216 -> 2560
 // 8.3 -> 7.6); above, it saves power (16384 x 9216 x 9216 2026 -> 1969 us).
@@ -47,10 +50,8 @@ __device__ __forceinline__ uint32_t dequant_pair(uint32_t nibbles, __nv_bfloat16
     const __nv_bfloat162 w = __hfma2(*reinterpret_cast<const __nv_bfloat162 *>(&nibbles), mul, off);
     return *reinterpret_cast<const uint32_t *>(&w);
 }
-// bf16 results, the weights' factor taken out after the rounding, which it does not change: one instruction for two
-__device__ __forceinline__ uint32_t unscale_bf16x2(float lo, float hi) {
-    const uint32_t f = 0x4A804A80u;  // bf16x2 2^22
-    const __nv_bfloat162 v = __hmul2(__floats2bfloat162_rn(lo, hi), *reinterpret_cast<const __nv_bfloat162 *>(&f));
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 // silu(g) * u of sums that still have the factor, g' = g 2^-22 and u' = u 2^-22: e^-g = 2^(-g log2 e) takes g's out in the product with
