@@ -33,7 +33,8 @@ __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_o
 // the rank that owns the elements (st.async, counted on its barrier; two cluster barriers around reads took 0.7 us more) and added there
 // in rank order: the result does not depend on timing.
 // AHEAD: the first blocks of a warp whose loads are all in flight at once, and the adapter, cold in HBM in a model of many layers, is asked
-// into L2 before the grid-dependency wait.  (Reading it before the wait would be another 2 % faster, but a caller may have written it.)
+// into L2 before the grid-dependency wait.  (Reading it before the wait would be another 2 % faster, but a caller may have written it: so
+// no load of it is one that the compiler may move, as __ldg is.)
 // By itself, us: 37 rows rank 64 K = 2560 3.0 -> 2.3, K = 9216 4.0 -> 3.0.  Few rows were dot products, a warp each: 4 rows rank 64 K = 2560
 // 2.35 -> 1.96, K = 9216 5.35 -> 2.5.  Four layers with it: 8 rows 254 -> 188, 37 rows 218 -> 188, 128 rows 301 -> 275.
 template <int NT>
@@ -53,7 +54,7 @@ __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1,
         const uint32_t lo[4] = {u.x, v.x, u.y, v.y}, hi[4] = {u.z, v.z, u.w, v.w};
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            const uint4 w = __ldg(a[t] + b * 4);
+            const uint4 w = ld_v4(a[t] + b * 4);
             mma_bf16_16816(acc[t], lo, w.x, w.y);
             mma_bf16_16816(acc[t], hi, w.z, w.w);
         }
