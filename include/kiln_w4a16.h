@@ -273,8 +273,8 @@ void kiln_w4a16_set_wait_limit_ns(unsigned long long ns);
 
 /* TEST HOOK for the give-up path above: the activation tile of K-step `k_step` (counted per CTA from 0) is announced
  * to its barrier but never copied, so the wait for it runs out (small-batch and CTA-pair kernel: of every
- * K-step, a tile eight rows short of what was announced).  Nothing faults or spins past the limit.  -1 switches
- * the hook off.  Process-wide, not thread-safe; no counterpart in the reference. */
+ * K-step, a tile eight rows short of what was announced).  -2: the exchange between the CTAs of a LoRA projection is
+ * announced four bytes more than are pushed.  Nothing faults or spins past the limit.  -1 switches the hook off.  Process-wide, not thread-safe; no counterpart in the reference. */
 void kiln_w4a16_test_drop_activation_load(int k_step);
 
 /* Diagnostic: the tiling the tcgen05 kernel would use for (m, n, k) on the current device, as

@@ -62,7 +62,8 @@ __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1,
 }
 
 // grid = (cluster size, ceil(r / (8 NT)), ceil(m / (16 WM))), cluster = (cluster size, 1, 1), block = 256.
-// (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernels read as an operand tile; fp32 otherwise)
+// (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernels read as an operand tile; fp32 otherwise.  test_missing: bytes that are
+// announced to the exchange but never pushed)
 template <int WM, int NT>
 constexpr int lora_smem() {
     return (8 * 16 * 8 * NT + 16 * WM * 8 * NT + 8) * static_cast<int>(sizeof(float));
@@ -70,7 +71,7 @@ constexpr int lora_smem() {
 template <int WM, int NT, int AHEAD>
 __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
                                                         int m, int k, int r, void *__restrict__ t, int bf16_out, uint32_t *status,
-                                                        unsigned long long wait_limit_ns) {
+                                                        unsigned long long wait_limit_ns, uint32_t test_missing) {
     constexpr int kCols = 8 * NT, kRows = 16 * WM, kParts = 8 / WM, kTile = kRows * kCols;
     extern __shared__ float parts[];  // [kParts][kRows][kCols], then what the ranks push
     pdl_launch_dependents();
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
             gave_up = 0;
             mbar_init(bar, 1);
             mbar_init_fence();
-            mbar_arrive_expect_tx(bar, static_cast<uint32_t>((size - 1) * own) * 4u);
+            mbar_arrive_expect_tx(bar, static_cast<uint32_t>((size - 1) * own) * 4u + test_missing);
         }
         __syncthreads();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
     }
     __syncthreads();
     if (size > 1 && !mbar_wait(bar, 0, &gave_up, status, 0xC00u, wait_limit_ns)) {
-        mbar_wait_quiet(bar, 0, 32 * wait_limit_ns);  // (a peer pushes into this CTA until it is through)
+        mbar_wait_quiet(bar, 0, peers_limit_ns(wait_limit_ns));  // (a peer pushes into this CTA until it is through)
         return;
     }
     for (int i = threadIdx.x; i < own; i += 256) {
@@ -230,7 +231,8 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     }
     // (76 registers against 62: only where all CTAs are resident either way, three to an SM)
     const auto kernel = wm != 1 ? lora_down_kernel<8, 8, 0> : size * row_tiles * col_tiles <= 3 * device_sm_count() ? lora_down_kernel<1, 2, 2> : lora_down_kernel<1, 2, 0>;
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out, status, current_wait_limit_ns()));
+    const bool test = test_drop_a_load() == kTestShortExchange;  // (gives up well before a kernel that waits for this one does)
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out, status, current_wait_limit_ns() / (test ? 4 : 1), test ? 4u : 0u));
 }
 
 int launch_finish(const void *base, void *c, int m, int n, const float *t, const void *lora_b, int r, int swiglu,

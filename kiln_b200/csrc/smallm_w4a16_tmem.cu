@@ -707,7 +707,7 @@ w4a16_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
             } else {
                 if (warp == kTeamWarp0 && lane == 0) drain();
-                mbar_wait_quiet(bar(kBarExchange), 0, 32 * p.wait_limit_ns);  // peers push into this CTA until they are through or have given up
+                mbar_wait_quiet(bar(kBarExchange), 0, peers_limit_ns(p.wait_limit_ns));  // peers push into this CTA until they are through or have given up
             }
         }
         tc_fence_before();

@@ -88,4 +88,11 @@ __device__ __forceinline__ void mbar_wait_quiet(uint32_t bar, uint32_t parity, u
     }
 }
 
+// How long a CTA that gave up stays for its peers, which push into its shared memory until they are through or have given up themselves: a
+// peer may come to the end of several waits in turn, and takes its time for loads whatever the limit is.
+__device__ __forceinline__ unsigned long long peers_limit_ns(unsigned long long wait_limit_ns) {
+    constexpr unsigned long long kLeast = 20ull * 1000 * 1000;
+    return wait_limit_ns > kLeast / 32 ? 32 * wait_limit_ns : kLeast;
+}
+
 }  // namespace kiln

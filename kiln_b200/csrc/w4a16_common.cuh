@@ -215,6 +215,7 @@ int launch_exact_group(const GemmArgs *items, int count);
 int launch_plain_group(const GemmArgs *items, int count);
 void set_test_drop_a_load(int k_step);
 int test_drop_a_load();
+constexpr int kTestShortExchange = -2;  // its value for the LoRA projection's exchange
 void prefill_plan(int m, int n, int k, int out[4]);
 bool prefill_supported(int m, int n, int k, int groupsize);
 bool prefill_fuses_swiglu(int m, int n, int k);

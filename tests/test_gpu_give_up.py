@@ -104,3 +104,12 @@ def test_kernel_of_cta_pairs(cuda_device, bn, m, k, n, groupsize, rank, swiglu, 
     finally:
         lib.kiln_w4a16_set_prefill_override(0, 0, 0, 0)
         lib.kiln_w4a16_set_prefill_min_m(0)
+
+
+# clusters of 2, 5 and 8 CTAs (K = 512 each), one row tile and three, with the fp32 projection and with the bf16 one; a limit so short that
+# only the least time that a CTA stays for its peers lets them finish
+@pytest.mark.parametrize("m,k,rank,limit_ns", [(9, 1024, 16, 2_000_000), (16, 2560, 64, 2_000_000), (40, 4096, 64, 2_000_000), (100, 4096, 24, 2_000_000),
+                                               (40, 4096, 64, 100_000)])
+def test_exchange_of_the_lora_projection(cuda_device, m, k, rank, limit_ns):
+    x, proj, adapter = _inputs(cuda_device, m, k, 2048, 128, rank)
+    _give_up(lambda: kiln_b200.matmul_bf16_lora(x, proj, *adapter, 0.5), -2, (0xC00,), limit_ns)
