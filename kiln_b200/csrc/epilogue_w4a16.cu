@@ -63,21 +63,21 @@ __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1,
 
 // grid = (cluster size, ceil(r / (8 NT)), ceil(m / (16 WM))), cluster = (cluster size, 1, 1), block = 256.
 // (bf16_out: t is a bf16 [m, r] matrix, the form the tcgen05 kernels read as an operand tile; fp32 otherwise.  test_missing: bytes that are
-// announced to the exchange but never pushed)
+// announced to the exchange but never pushed.  ALONE: one CTA has a tile's whole K, and its threads store the sums of its parts at once.)
 template <int WM, int NT>
 constexpr int lora_smem() {
     return (8 * 16 * 8 * NT + 16 * WM * 8 * NT + 8) * static_cast<int>(sizeof(float));
 }
-template <int WM, int NT, int AHEAD>
+template <int WM, int NT, int AHEAD, bool ALONE>
 __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
                                                         int m, int k, int r, void *__restrict__ t, int bf16_out, uint32_t *status,
-                                                        unsigned long long wait_limit_ns, uint32_t test_missing) {
+                                                        unsigned long long wait_limit_ns, uint32_t test_missing, bool prefetch) {
     constexpr int kCols = 8 * NT, kRows = 16 * WM, kParts = 8 / WM, kTile = kRows * kCols;
     extern __shared__ float parts[];  // [kParts][kRows][kCols], then what the ranks push
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane >> 2, qd = lane & 3;
     const int wm = warp % WM, part = warp / WM;
-    const int rank = blockIdx.x, size = gridDim.x;
+    const int rank = ALONE ? 0 : blockIdx.x, size = ALONE ? 1 : gridDim.x;
     // A rank of the cluster owns `each` elements of the tile, the last ones fewer or none.  (armed before the wait; that every CTA runs is
     // checked before the first push)
     const int each = (kTile + size - 1) / size, own = max(0, min(each, kTile - rank * each));
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
     const uint4 *x0 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c, m - 1)) * k) + qd;
     const uint4 *x1 = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(min(row0 + c + 8, m - 1)) * k) + qd;
     // The adapter's rows come to L2 before the wait, and are read after it: a kernel before this one may have written them.
-    for (int b = b0; AHEAD > 0 && b < b1; ++b)
+    for (int b = b0; (AHEAD > 0 || (ALONE && prefetch)) && b < b1; ++b)
 #pragma unroll
         for (int t = 0; t < NT; ++t) asm volatile("prefetch.global.L2 [%0];" ::"l"(ap[t] + b * 4));
     pdl_wait();  // x may be the previous kernel's output; t may still be read by it
@@ -130,6 +130,16 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
         *reinterpret_cast<float2 *>(mine + (c + 8) * kCols + 8 * i + 2 * qd) = make_float2(acc[i][2], acc[i][3]);
     }
     __syncthreads();
+    if (ALONE) {
+        for (int e = threadIdx.x; e < kTile; e += 256) {
+            float v = parts[e];
+#pragma unroll
+            for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
+            const int row = blockIdx.z * kRows + e / kCols, col = col0 + e % kCols;
+            if (row < m && col < r) store_t(t, static_cast<size_t>(row) * r + col, v * scale, bf16_out);
+        }
+        return;
+    }
     // Every CTA sums its parts and pushes each rank its share (counted on that rank's barrier), the owner adds the shares in rank order.
     float *recv = parts + kParts * kTile;  // [rank][each]
     if (size > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -193,46 +203,56 @@ __global__ void __launch_bounds__(256) finish_kernel(const __nv_bfloat16 *__rest
 }  // namespace
 
 int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int k, int r, void *t, int bf16_out, cudaStream_t stream) {
+    const auto *xp = static_cast<const __nv_bfloat16 *>(x), *ap = static_cast<const __nv_bfloat16 *>(lora_a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = 1;
     // Rows and adapter rows of a CTA: 16 x 16, or 128 x 64 for more than 1024 rows of a large rank, where reading x once per 16
     // adapter rows costs more than the longer chains of large tiles (2048 x 9216, rank 64, with its GEMM: 118 / 114 us; 1024 rows: 65 / 83).
     const int wm = m > 1024 && r > 32 ? 8 : 1, rows = 16 * wm, cols = wm == 1 ? 16 : 64, parts = 8 / wm;
     const int row_tiles = (m + rows - 1) / rows, col_tiles = (r + cols - 1) / cols;
     if (row_tiles > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
+    const int tiles = row_tiles * col_tiles;
     // K is split over as many CTAs as the tiles leave room for (four small ones to an SM: 768 x 9216, rank 64 57.6 -> 51.3 us against
-    // one), while a warp keeps at least two 32-deep blocks
-    int size = std::min(8, std::max(1, (wm == 1 ? 4 : 1) * device_sm_count() / (row_tiles * col_tiles)));
+    // one), while a warp keeps at least two 32-deep blocks.
+    int size = std::min(8, std::max(1, (wm == 1 ? 4 : 1) * device_sm_count() / tiles));
     size = std::max(1, std::min(size, k / 32 / (2 * parts)));
-    cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(size, col_tiles, row_tiles);
-    cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = wm == 1 ? lora_smem<1, 2>() : lora_smem<8, 8>();
-    cfg.stream = stream;
-    cudaLaunchAttribute attrs[2];
-    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[0].val.programmaticStreamSerializationAllowed = 1;
-    attrs[1].id = cudaLaunchAttributeClusterDimension;
-    attrs[1].val.clusterDim.x = size;
-    attrs[1].val.clusterDim.y = 1;
-    attrs[1].val.clusterDim.z = 1;
-    cfg.attrs = attrs;
-    cfg.numAttrs = size > 1 ? 2 : 1;
-    uint32_t *status = device_status_word();
-    if (!status) return KILN_W4A16_ERR_CUDA;
-    const auto *xp = static_cast<const __nv_bfloat16 *>(x), *ap = static_cast<const __nv_bfloat16 *>(lora_a);
-    note_launch();
+    if (size > 1) {
+        attrs[1].id = cudaLaunchAttributeClusterDimension;
+        attrs[1].val.clusterDim.x = size;
+        attrs[1].val.clusterDim.y = 1;
+        attrs[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
+    uint32_t *status = size > 1 ? device_status_word() : nullptr;  // (of the exchange's wait)
+    if (size > 1 && !status) return KILN_W4A16_ERR_CUDA;
+    // The look-ahead takes 76 registers against 62, three CTAs to an SM: only where all are resident either way.  A projection whose
+    // tiles have one CTA each has a short K and little to look ahead to, and its CTAs may have to start on the few SMs that the GEMM before
+    // leaves free (256 rows rank 64 K = 512: 64 CTAs beside 128 of a GEMM; four to an SM 7.6 us with the next GEMM, three 8.6).  There it is for
+    // a few tiles alone (8 x 512 -> 2560 rank 64 5.4 -> 5.1); the prefetch, which needs no register, stays.
+    const bool few = size * tiles <= 3 * device_sm_count(), alone = size == 1;
+    const auto kernel = wm != 1 ? lora_down_kernel<8, 8, 0, false>
+                        : alone ? (tiles <= 8 ? lora_down_kernel<1, 2, 2, true> : lora_down_kernel<1, 2, 0, true>)
+                                : (few ? lora_down_kernel<1, 2, 2, false> : lora_down_kernel<1, 2, 0, false>);
     if (wm != 1) {  // (its shared memory is beyond what a launch may have unasked)
         static std::atomic<bool> asked[64] = {};
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev >= 64 || !asked[dev].load(std::memory_order_acquire)) {
-            if (int rc = record_cuda_error(cudaFuncSetAttribute(lora_down_kernel<8, 8, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lora_smem<8, 8>()))) return rc;
+            if (int rc = record_cuda_error(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lora_smem<8, 8>()))) return rc;
             if (dev < 64) asked[dev].store(true, std::memory_order_release);
         }
     }
-    // (76 registers against 62: only where all CTAs are resident either way, three to an SM)
-    const auto kernel = wm != 1 ? lora_down_kernel<8, 8, 0> : size * row_tiles * col_tiles <= 3 * device_sm_count() ? lora_down_kernel<1, 2, 2> : lora_down_kernel<1, 2, 0>;
+    note_launch();
     const bool test = test_drop_a_load() == kTestShortExchange;  // (gives up well before a kernel that waits for this one does)
-    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out, status, current_wait_limit_ns() / (test ? 4 : 1), test ? 4u : 0u));
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kernel, xp, ap, scale, m, k, r, t, bf16_out, status, current_wait_limit_ns() / (test ? 4 : 1), test ? 4u : 0u, wm == 1 && few));
 }
 
 int launch_finish(const void *base, void *c, int m, int n, const float *t, const void *lora_b, int r, int swiglu,

@@ -12,10 +12,14 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("r", [8, 24, 64])
 @pytest.mark.parametrize("k", [128, 512, 1024, 1536, 2048, 2560, 3072, 3584, 4096])
 def test_projection(cuda_device, k, r):
+    _check(cuda_device, k, r, (1, 4, 8, 17, 40, 130))
+
+
+def _check(cuda_device, k, r, rows):
     n, gen = 256, torch.Generator(device=cuda_device).manual_seed(k + r)
     w = torch.full((k // 16, 2 * n), -0x77777778, dtype=torch.int32, device=cuda_device)  # every weight (8 - 8) s = 0
     proj = kiln_b200.MarlinPackedProj(w, torch.full((k // 128, n), 0.01, dtype=torch.float16, device=cuda_device), 128, k, n)
-    for m in (1, 4, 8, 17, 40, 130):
+    for m in rows:
         x = torch.randn((m, k), device=cuda_device, generator=gen).bfloat16()
         a = torch.randn((r, k), device=cuda_device, generator=gen).bfloat16()
         b = torch.randn((n, r), device=cuda_device, generator=gen).bfloat16()
