@@ -21,7 +21,32 @@ __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_o
         static_cast<float *>(t)[idx] = v;
 }
 
-// A small tensor-core GEMM, K split over the CTAs of a cluster and, for few rows, over the warps of a CTA.
+// Up to four rows of a short K and a small rank: one dot product per warp, fewer steps from the wait to the store than the tiles below have.
+// grid = (ceil(r / 8), m), block = 256: warp w of a CTA computes t[row][8 * blockIdx.x + w].
+__global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
+                                                       int k, int r, void *__restrict__ t, int bf16_out) {
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.y, j = blockIdx.x * 8 + warp;
+    pdl_wait();  // x may be the previous kernel's output, and so may the adapter; t may still be read by it
+    if (j >= r) return;
+    const uint4 *xr = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row) * k);
+    const uint4 *ar = reinterpret_cast<const uint4 *>(a + static_cast<size_t>(j) * k);
+    float sum = 0.f;
+    for (int i = lane; i < k / 8; i += 32) {
+        const uint4 xv = ld_cg_v4(xr + i), av = ld_cg_v4(ar + i);
+        const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, as[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            sum += __uint_as_float(xs[e] << 16) * __uint_as_float(as[e] << 16) +
+                   __uint_as_float(xs[e] & 0xFFFF0000u) * __uint_as_float(as[e] & 0xFFFF0000u);
+    }
+#pragma unroll
+    for (int sh = 16; sh >= 1; sh >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, sh);
+    if (lane == 0) store_t(t, static_cast<size_t>(row) * r + j, sum * scale, bf16_out);
+}
+
+// Otherwise a small tensor-core GEMM, K split over the CTAs of a cluster and, for few rows, over the warps of a CTA.
 //
 // Bound: latency.  The operands are a few hundred KB (x 37 x 9216 and A 64 x 9216: 1.9 MB), so what counts is how many SMs load
 // them at once and how short the chain from the grid-dependency wait to the last store is.  A lane loads 16 contiguous bytes of
@@ -35,7 +60,7 @@ __device__ __forceinline__ void store_t(void *t, size_t idx, float v, int bf16_o
 // AHEAD: the first blocks of a warp whose loads are all in flight at once, and the adapter, cold in HBM in a model of many layers, is asked
 // into L2 before the grid-dependency wait.  (Reading it before the wait would be another 2 % faster, but a caller may have written it: so
 // no load of it is one that the compiler may move, as __ldg is.)
-// By itself, us: 37 rows rank 64 K = 2560 3.0 -> 2.3, K = 9216 4.0 -> 3.0.  Few rows were dot products, a warp each: 4 rows rank 64 K = 2560
+// By itself, us: 37 rows rank 64 K = 2560 3.0 -> 2.3, K = 9216 4.0 -> 3.0.  Against dot products, a warp each: 4 rows rank 64 K = 2560
 // 2.35 -> 1.96, K = 9216 5.35 -> 2.5.  Four layers with it: 8 rows 254 -> 188, 37 rows 218 -> 188, 128 rows 301 -> 275.
 template <int NT>
 __device__ __forceinline__ void lora_mma_block(const uint4 &u, const uint4 &v, const uint4 (&w)[NT], float (&acc)[NT][4]) {
@@ -212,6 +237,13 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     attrs[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = 1;
+    // Dot products or tiles (us with the GEMM, rank 16, K = 640 / 1024 / 1280 / 1536 -> 512: one row 4.3 / 4.3 / 4.5 / 4.5 against 4.4 / 4.4 / 4.7 /
+    // 4.5, four rows 4.4 / 4.3 / 4.6 / 4.7 against 4.4 / 4.4 / 4.9 / 4.6; four rows rank 64 1280 -> 2560 6.8 against 6.4).
+    if (m <= 4 && m * r <= 128 && k <= 1280) {
+        cfg.gridDim = dim3((r + 7) / 8, m);
+        note_launch();
+        return record_cuda_error(cudaLaunchKernelEx(&cfg, lora_dot_kernel, xp, ap, scale, k, r, t, bf16_out));
+    }
     // Rows and adapter rows of a CTA: 16 x 16, or 128 x 64 for more than 1024 rows of a large rank, where reading x once per 16
     // adapter rows costs more than the longer chains of large tiles (2048 x 9216, rank 64, with its GEMM: 118 / 114 us; 1024 rows: 65 / 83).
     const int wm = m > 1024 && r > 32 ? 8 : 1, rows = 16 * wm, cols = wm == 1 ? 16 : 64, parts = 8 / wm;

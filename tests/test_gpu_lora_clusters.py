@@ -28,3 +28,9 @@ def _check(cuda_device, k, r, rows):
         assert _lib.lib().kiln_w4a16_check_device_status(None, None) == 0
         ref = 0.5 * (x.double() @ a.double().T) @ b.double().T
         assert float((out.double() - ref).abs().max() / ref.abs().max()) <= 1e-2, m
+
+
+# the line between dot products and tiles: four rows, rows x rank of 128, K of 1280; ranks that are no multiple of a block's eight warps x rows
+@pytest.mark.parametrize("k,r,rows", [(128, 8, (1, 4, 5)), (1280, 32, (1, 2, 4, 5)), (1280, 40, (3, 4)), (1408, 32, (4,)), (640, 128, (1, 2)), (1024, 120, (1,))])
+def test_few_rows_of_a_short_k(cuda_device, k, r, rows):
+    _check(cuda_device, k, r, rows)
