@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(256) lora_dot_kernel(const __nv_bfloat16 *__re
 // A CTA has WM row tiles of 16 and 8 / WM parts of its K range, one (row tile, part) per warp, and 8 NT adapter rows.  Small tiles
 // nearly always (many CTAs, short chains: 64 rows, 9216 -> 2560 with its GEMM 21 -> 13 us against tiles of 64 x 32), large ones for
 // very many rows (x is read once per 8 NT adapter rows).  The parts meet in shared memory; the cluster's partial tiles are pushed to
-// the rank that owns the elements (st.async, counted on its barrier; two cluster barriers around reads took 0.7 us more) and added there
-// in rank order: the result does not depend on timing.
+// the rank that owns the elements (st.async, counted on its barrier; two cluster barriers around reads took 0.7 us more; of the large tiles
+// 16 bytes a push, with 4 bytes 2100 rows rank 64 512 -> 1024 16.9 -> 19.8 us) and added there in rank order: the result does not depend on timing.
 // AHEAD: the first blocks of a warp whose loads are all in flight at once, and the adapter, cold in HBM in a model of many layers, is asked
 // into L2 before the grid-dependency wait.  (Reading it before the wait would be another 2 % faster, but a caller may have written it: so
 // no load of it is one that the compiler may move, as __ldg is.)
@@ -91,21 +91,22 @@ __device__ __forceinline__ void lora_mma_range(const uint4 *x0, const uint4 *x1,
 // announced to the exchange but never pushed.  ALONE: one CTA has a tile's whole K, and its threads store the sums of its parts at once.)
 template <int WM, int NT>
 constexpr int lora_smem() {
-    return (8 * 16 * 8 * NT + 16 * WM * 8 * NT + 8) * static_cast<int>(sizeof(float));
+    return (8 * 16 * 8 * NT + 16 * WM * 8 * NT + 32) * static_cast<int>(sizeof(float));
 }
 template <int WM, int NT, int AHEAD, bool ALONE>
 __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a, float scale,
                                                         int m, int k, int r, void *__restrict__ t, int bf16_out, uint32_t *status,
                                                         unsigned long long wait_limit_ns, uint32_t test_missing, bool prefetch) {
     constexpr int kCols = 8 * NT, kRows = 16 * WM, kParts = 8 / WM, kTile = kRows * kCols;
-    extern __shared__ float parts[];  // [kParts][kRows][kCols], then what the ranks push
+    extern __shared__ __align__(16) float parts[];  // [kParts][kRows][kCols], then what the ranks push
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane >> 2, qd = lane & 3;
     const int wm = warp % WM, part = warp / WM;
     const int rank = ALONE ? 0 : blockIdx.x, size = ALONE ? 1 : gridDim.x;
     // A rank of the cluster owns `each` elements of the tile, the last ones fewer or none.  (armed before the wait; that every CTA runs is
     // checked before the first push)
-    const int each = (kTile + size - 1) / size, own = max(0, min(each, kTile - rank * each));
+    constexpr int kVec = kParts == 1 ? 4 : 1;  // floats of a push
+    const int each = (kTile / kVec + size - 1) / size * kVec, own = max(0, min(each, kTile - rank * each));
     __shared__ __align__(8) unsigned long long exchange;
     __shared__ uint32_t gave_up;
     const uint32_t bar = smem_u32(&exchange);
@@ -168,18 +169,28 @@ __global__ void __launch_bounds__(256) lora_down_kernel(const __nv_bfloat16 *__r
     // Every CTA sums its parts and pushes each rank its share (counted on that rank's barrier), the owner adds the shares in rank order.
     float *recv = parts + kParts * kTile;  // [rank][each]
     if (size > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    for (int e = threadIdx.x; e < kTile; e += 256) {
-        float v = parts[e];
-#pragma unroll
-        for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
+    for (int e = kVec * threadIdx.x; e < kTile; e += kVec * 256) {
         const int owner = e / each;
         const uint32_t slot = smem_u32(recv + rank * each + e - owner * each);
-        if (owner == rank)
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(v) : "memory");
-        else
-            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(map_to_cta(slot, owner)), "f"(v),
-                         "r"(map_to_cta(bar, owner))
-                         : "memory");
+        if constexpr (kVec == 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(parts + e);
+            if (owner == rank)
+                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(slot), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+            else
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1,%2,%3,%4}, [%5];" ::"r"(map_to_cta(slot, owner)),
+                             "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(map_to_cta(bar, owner))
+                             : "memory");
+        } else {
+            float v = parts[e];
+#pragma unroll
+            for (int q = 1; q < kParts; ++q) v += parts[q * kTile + e];
+            if (owner == rank)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(v) : "memory");
+            else
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(map_to_cta(slot, owner)), "f"(v),
+                             "r"(map_to_cta(bar, owner))
+                             : "memory");
+        }
     }
     __syncthreads();
     if (size > 1 && !mbar_wait(bar, 0, &gave_up, status, 0xC00u, wait_limit_ns)) {
@@ -251,8 +262,10 @@ int launch_lora_down(const void *x, const void *lora_a, float scale, int m, int 
     if (row_tiles > 65535) return KILN_W4A16_ERR_KERN_SHAPE;
     const int tiles = row_tiles * col_tiles;
     // K is split over as many CTAs as the tiles leave room for (four small ones to an SM: 768 x 9216, rank 64 57.6 -> 51.3 us against
-    // one), while a warp keeps at least two 32-deep blocks.
+    // one), while a warp keeps at least two 32-deep blocks.  Of the large ones, one to an SM for their 142 registers, all clusters have to
+    // fit at once: not all SMs are in clusters of eight (2100 rows rank 64, 17 clusters where 15 of eight fit: 9216 -> 2560 128 us, six to a cluster 110).
     int size = std::min(8, std::max(1, (wm == 1 ? 4 : 1) * device_sm_count() / tiles));
+    while (wm != 1 && size > 1 && smallm_clusters(size) < tiles) --size;
     size = std::max(1, std::min(size, k / 32 / (2 * parts)));
     cfg.gridDim = dim3(size, col_tiles, row_tiles);
     cfg.dynamicSmemBytes = wm == 1 ? lora_smem<1, 2>() : lora_smem<8, 8>();

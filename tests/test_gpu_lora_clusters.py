@@ -34,3 +34,10 @@ def _check(cuda_device, k, r, rows):
 @pytest.mark.parametrize("k,r,rows", [(128, 8, (1, 4, 5)), (1280, 32, (1, 2, 4, 5)), (1280, 40, (3, 4)), (1408, 32, (4,)), (640, 128, (1, 2)), (1024, 120, (1,))])
 def test_few_rows_of_a_short_k(cuda_device, k, r, rows):
     _check(cuda_device, k, r, rows)
+
+
+# large tiles: clusters of 1 to 8 CTAs, shares that are no multiple of the threads, and counts of tiles for which clusters of eight do not fit at once
+@pytest.mark.parametrize("m,k,r", [(1100, 128, 64), (2100, 512, 128), (1100, 256, 72), (3000, 512, 64), (1100, 384, 64), (2100, 512, 40), (1100, 512, 64),
+                                   (16384, 128, 40)])
+def test_large_tiles(cuda_device, m, k, r):
+    _check(cuda_device, k, r, (m,))
