@@ -97,9 +97,9 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_ex(const void *A, const void *B, void *
 /* Several independent GEMMs in one launch: sibling projections of one layer that the reference issues as separate
  * Marlin calls (q, k, v: crates/kiln-model/src/forward.rs; gate and up: forward.rs:2769-2839).  The problems may
  * differ in every argument.  When every problem is at a decode batch size (kiln_w4a16_workspace_bytes == 0) and all
- * have either at most 8 rows or more than 8, ONE launch covers all their column blocks: of the small-batch kernel's fp32-scale
- * variant (up to four problems a launch) where rows, K and group size are the same for all and each would run on it by itself, else of
- * the decode kernel.  Otherwise the problems are launched one after another with the given workspace (sized for the largest), except that
+ * have either at most 8 rows or more than 8, one launch of the decode kernel covers all their column blocks, or, where rows, K and
+ * group size are the same for all, each would run on it by itself and the group is faster there, one launch of the small-batch
+ * kernel's fp32-scale variant per four problems.  Otherwise the problems are launched one after another with the given workspace (sized for the largest), except that
  * neighbours of the same rows, K and group size share a launch of the small-batch kernel, or of that variant, where that is what
  * runs them.  count <= 8. */
 #define KILN_W4A16_MAX_GROUP 8

@@ -324,11 +324,10 @@ kiln_w4a16_status_t kiln_w4a16_gemm_bf16_grouped(const kiln_w4a16_problem_t *pro
         live[count_live++] = a;
     }
     if (count_live == 0) return KILN_W4A16_OK;
-    // One launch where the problems are alike and each would run on the small-batch kernel's variant by itself (2560 -> 4096, 512 and 512,
-    // us, decode kernel / this: 9 rows 5.5 / 5.5, 16 6.2 / 5.6, 17 11.3 / 7.5, 32 11.6 / 7.5).
-    bool exact = same && count_live > 1;
-    for (int i = 0; i < count_live; ++i) exact = exact && decode && use_exact(live[i]);
-    if (exact) return launch_exact_group(live, count_live);
+    // One launch where the problems are alike, each would run on the small-batch kernel's variant by itself, and all of them are faster there.
+    bool exact = same && decode && count_live > 1;
+    for (int i = 0; i < count_live; ++i) exact = exact && use_exact(live[i]);
+    if (exact && exact_group_pays(live, count_live)) return launch_exact_group(live, count_live);
     // one batch class per launch of the decode kernel: up to 8 rows, or 9 and more
     for (int i = 1; i < count_live; ++i)
         if ((live[i].m <= 8) != (live[0].m <= 8)) decode = false;

@@ -937,17 +937,55 @@ bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r
 int launch_exact(const GemmArgs &a) { return launch_smallm(a, exact_splits(a.m, a.n, a.k, a.swiglu), true); }
 // GEMMs of the same rows, K and group size, in launches of as many as one takes.  The K splits are those of one GEMM with all columns, but
 // no fewer than a CTA's most stages ask for: more columns want fewer splits, and each member by itself may need the splits that it has.
+struct GroupLaunch {
+    int end, n, splits;  // the members before `end`, their columns
+};
+static GroupLaunch group_launch(const GemmArgs *items, int i, int count, bool exact) {
+    const GemmArgs &a = items[i];
+    GroupLaunch g{i + 1, a.n, 1};
+    for (; g.end < count && g.end < i + smallm_most_grouped() && static_cast<long long>(g.n) + items[g.end].n <= 65535LL * 128; ++g.end) g.n += items[g.end].n;
+    g.splits = exact ? exact_splits(a.m, g.n, a.k, false) : choose_smallm_splits(a.m, g.n, a.k);
+    for (int s : {2, 3, 4, 6, 8})
+        if (s > g.splits && !smallm_supported(exact ? std::min(a.m, 16) : a.m, a.n, a.k, a.groupsize, g.splits)) g.splits = s;
+    return g;
+}
 static int launch_groups(const GemmArgs *items, int count, bool exact) {
-    for (int i = 0, end; i < count; i = end) {
-        const GemmArgs &a = items[i];
-        int n = a.n;
-        for (end = i + 1; end < count && end < i + smallm_most_grouped() && static_cast<long long>(n) + items[end].n <= 65535LL * 128; ++end) n += items[end].n;
-        int splits = exact ? exact_splits(a.m, n, a.k, false) : choose_smallm_splits(a.m, n, a.k);
-        for (int s : {2, 3, 4, 6, 8})
-            if (s > splits && !smallm_supported(exact ? std::min(a.m, 16) : a.m, a.n, a.k, a.groupsize, splits)) splits = s;
-        if (int rc = launch_smallm_group(items + i, end - i, splits, exact)) return rc;
+    for (int i = 0; i < count;) {
+        const GroupLaunch g = group_launch(items, i, count, exact);
+        if (int rc = launch_smallm_group(items + i, g.end - i, g.splits, exact)) return rc;
+        i = g.end;
     }
     return 0;
+}
+// Whether a group of decode-sized GEMMs that the fp32-scale variant could run is faster there than in one launch of the decode kernel.  Measured
+// from 4 to 32 rows for K = 128 .. 12288 and 512 .. 25600 columns in all (weights cold in HBM); us, decode kernel / this one:
+//  * up to 8 rows, one block of the decode kernel: while the tiles take half the GPU (8 x 512 x 8192 4.7 / 2.7, 5 x 512 x 12288 3.6 / 3.8), four rows
+//    only between the shortest K and eight groups (4 x 512 x 8192 3.6 / 2.6, 4 x 128 x 1024 2.2 / 2.3, 4 x 1024 x 6144 3.1 / 3.5);
+//  * in one wave of CTAs always (16 x 2560 x 5120 6.4 / 5.7, 32 x 4096 x 4864 12.3 / 7.0), but for the widest of a short K (9 x 256 x 18944 3.5 / 4.2);
+//  * a further wave repeats a CTA's start, which only a long K makes up for, where the decode kernel dequantises twice (from 17 rows; from 13 above
+//    5120): whole tiles or many from 2560 (17 x 2560 x 10240 16.9 / 15.1, 17 x 4864 x 13824 41 / 28; 17 x 4608 x 10240, split, 20.6 / 24.9, 17 x 2304 x 10240
+//    12.4 / 14.1, 17 x 256 x 24576 5.4 / 10.8), around 12288 columns from 1408 (17 x 1792 x 13568 14.5 / 12.4, x 18432 14.2 / 14.7), all above 5120
+//    (17 x 6144 x 10240 37.6 / 29.2, 16 x 8192 x 9728 22.6 / 19.7; 9 x 12288 x 11008 24.4 / 25.8);
+//  * a second launch, for more than four members, under the same condition (five of 3840 columns, 17 rows: K = 1408 6.0 / 7.5, 6144 22.1 / 13.1).
+bool exact_group_pays(const GemmArgs *items, int count) {
+    const int m = items[0].m, k = items[0].k;
+    if (count > smallm_most_grouped() && (m < 17 || k <= 5120)) return false;
+    for (int i = 0; i < count;) {
+        const GroupLaunch g = group_launch(items, i, count, true);
+        const int tiles = g.n / 128, units = tiles * ((m + 15) / 16);
+        bool pays;
+        if (m <= 8)
+            pays = 2 * tiles <= device_sm_count() && (m > 4 || (k > 128 && (k < 1024 || g.n <= 4096)));
+        else if (units <= smallm_clusters(g.splits))
+            pays = k > 512 || g.n <= 16384;
+        else if (k > 5120)
+            pays = m >= 13;
+        else
+            pays = m >= 17 && (k >= 2560 ? g.splits == 1 || g.n > 12288 : k >= 1408 && g.n >= 12288 && g.n <= 16384);
+        if (!pays) return false;
+        i = g.end;
+    }
+    return true;
 }
 int launch_exact_group(const GemmArgs *items, int count) { return launch_groups(items, count, true); }
 int launch_plain_group(const GemmArgs *items, int count) { return launch_groups(items, count, false); }

@@ -211,6 +211,7 @@ int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact
 int smallm_most_grouped();
 bool exact_supported(int m, int n, int k, int groupsize, bool swiglu, int lora_r);
 int launch_exact(const GemmArgs &a);
+bool exact_group_pays(const GemmArgs *items, int count);
 int launch_exact_group(const GemmArgs *items, int count);
 int launch_plain_group(const GemmArgs *items, int count);
 void set_test_drop_a_load(int k_step);

@@ -13,12 +13,17 @@ from tests.util import REL_TOL, from_torch_bf16, rel_err, to_torch_bf16
 pytestmark = pytest.mark.gpu
 
 
-# (rows, K, columns of each, group size, launches): nine to 32 rows in one launch; above, neighbours of one kind; five problems, two launches;
-# rows that are no multiple of four, and several CTAs of 16 rows; group sizes -1; the 128-row variant; one K stage; decode up to 8 rows
+# (rows, K, columns of each, group size, launches): nine to 32 rows in one launch; above, neighbours of one kind; five problems, the decode kernel
+# or, for more rows of a long K, two launches; rows that are no multiple of four, and several CTAs of 16 rows; group sizes -1; the 128-row
+# variant; one K stage; decode up to 8 rows; either side of the lines between the decode kernel and the variant that the columns of all draw:
+# half the GPU's tiles up to 8 rows, a second wave of CTAs, split or not
 @pytest.mark.parametrize("m,k,ns,groupsize,launches", [
-    (9, 640, (512, 256, 256), 128, 1), (16, 2560, (4096, 512, 512), 128, 1), (29, 640, (4096, 512, 512), 128, 1), (13, 384, (256,) * 5, 128, 2),
+    (9, 640, (512, 256, 256), 128, 1), (16, 2560, (4096, 512, 512), 128, 1), (29, 640, (4096, 512, 512), 128, 1), (13, 384, (256,) * 5, 128, 1), (17, 5248, (256,) * 5, 128, 2),
     (13, 640, (512, 256), -1, 1), (37, 640, (4096, 512, 512), 128, 2), (50, 640, (512, 4096, 2048, 512), 128, 3), (101, 1280, (2048, 4096), 128, 1),
-    (64, 2560, (2048, 2048, 2048), 128, 1), (128, 128, (1280, 1280), 128, 1), (77, 640, (2048, 2048), -1, 1), (8, 640, (512, 256), 128, 1)])
+    (64, 2560, (2048, 2048, 2048), 128, 1), (128, 128, (1280, 1280), 128, 1), (77, 640, (2048, 2048), -1, 1), (8, 640, (512, 256), 128, 1),
+    (7, 256, (4864, 4608), 128, 1), (7, 256, (4864, 4864), 128, 1), (4, 1024, (3072, 1024), 128, 1), (16, 256, (9472, 9728), 128, 1),
+    (17, 640, (4864, 4608), 128, 1), (17, 640, (4864, 4864), 128, 1), (17, 2560, (4864, 4864), 128, 1), (13, 5248, (3328, 6400), 128, 1),
+    (12, 5248, (3328, 6400), 128, 1)])
 def test_alike_problems_share_a_launch(cuda_device, m, k, ns, groupsize, launches):
     xs, projs, refs = [], [], []
     for i, n in enumerate(ns):
