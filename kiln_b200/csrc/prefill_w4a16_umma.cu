@@ -270,8 +270,9 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             uint32_t o[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                float x0 = (__uint_as_float(ra[8 * v + 2 * e]) + __uint_as_float(rb[8 * v + 2 * e])) * kWeightUnscale;
-                                float x1 = (__uint_as_float(ra[8 * v + 2 * e + 1]) + __uint_as_float(rb[8 * v + 2 * e + 1])) * kWeightUnscale;
+                                float x0 = __uint_as_float(ra[8 * v + 2 * e]) + __uint_as_float(rb[8 * v + 2 * e]);
+                                float x1 = __uint_as_float(ra[8 * v + 2 * e + 1]) + __uint_as_float(rb[8 * v + 2 * e + 1]);
+                                unscale(x0, x1);
                                 if (p.per_column) {
                                     const int pos = scale_single_pos(col + 8 * v + 2 * e);
                                     x0 *= __half2float(p.S[pos]);
@@ -342,8 +343,9 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             uint32_t o[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]) * kWeightUnscale;
-                                float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]) * kWeightUnscale;
+                                float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]);
+                                float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]);
+                                unscale(x0, x1);
                                 if (p.per_column) {
                                     const int pos = scale_single_pos(col + 8 * v + 2 * e);
                                     x0 *= __half2float(p.S[pos]);
