@@ -790,8 +790,9 @@ int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact
         return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
-    // tensor maps of one GEMM: packed words, scales (unused with per-column scales), activations, result (unused when K is split)
-    auto encode_maps = [&](const GemmArgs &q, CUtensorMap *w, CUtensorMap *s, CUtensorMap *x, CUtensorMap *c) {
+    // Tensor maps of one GEMM: packed words, scales (unused with per-column scales), activations (unless x has those of the same ones already),
+    // result (unused when K is split).  A map takes 0.1 us of the host, as much as a tenth of a launch.
+    auto encode_maps = [&](const GemmArgs &q, CUtensorMap *w, CUtensorMap *s, CUtensorMap *x, CUtensorMap *c, bool same_x) {
         {  // packed words: [k/16][2n] int32, boxes of one tile x eight rows (128 K)
             const cuuint64_t dims[2] = {2ull * q.n, static_cast<cuuint64_t>(q.k / 16)}, strides[1] = {8ull * q.n};
             const cuuint32_t box[2] = {2 * kTileCols, kStageK / 16}, estr[2] = {1, 1};
@@ -807,7 +808,7 @@ int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return false;
         }
-        {  // activations [m, k] seen as [k/64][m][64], so that one copy brings both 64-deep tiles of a stage
+        if (!same_x) {  // activations [m, k] seen as [k/64][m][64], so that one copy brings both 64-deep tiles of a stage
             const cuuint64_t dims[3] = {kAtomK, static_cast<cuuint64_t>(q.m), static_cast<cuuint64_t>(q.k / kAtomK)};
             const cuuint64_t strides[2] = {static_cast<cuuint64_t>(q.k) * 2, kAtomK * 2};
             // (test hook: boxes of eight rows less than the kernel announces, so that its waits for them run out)
@@ -820,7 +821,7 @@ int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact
         return splits != 1 || encode(c, q.C, q.swiglu ? q.n / 2 : q.n);
     };
     CUtensorMap tmap_w, tmap_s, tmap_x, tmap_t, tmap_c;
-    if (!encode_maps(a, &tmap_w, &tmap_s, &tmap_x, &tmap_c)) return KILN_W4A16_ERR_CUDA;
+    if (!encode_maps(a, &tmap_w, &tmap_s, &tmap_x, &tmap_c, false)) return KILN_W4A16_ERR_CUDA;
     tmap_t = tmap_x;  // (unused without a LoRA delta)
     const bool lora = a.lora_r > 0 && a.lora_t && a.lora_b;
     if (lora) {
@@ -903,7 +904,11 @@ int launch_smallm_group(const GemmArgs *items, int count, int splits, bool exact
         g.count = count;
         for (int i = 0; i < count; ++i) {
             const GemmArgs &q = items[i];
-            if (!encode_maps(q, &g.w[i], &g.s[i], &g.x[i], &g.c[i])) return KILN_W4A16_ERR_CUDA;
+            g.x[i] = tmap_x;
+            if (i == 0)
+                g.w[0] = tmap_w, g.s[0] = tmap_s, g.c[0] = tmap_c;
+            else if (!encode_maps(q, &g.w[i], &g.s[i], &g.x[i], &g.c[i], q.A == a.A))
+                return KILN_W4A16_ERR_CUDA;
             g.S[i] = static_cast<const __half *>(q.S);
             g.C[i] = static_cast<__nv_bfloat16 *>(q.C);
             g.n[i] = q.n;
