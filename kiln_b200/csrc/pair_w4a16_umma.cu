@@ -277,11 +277,11 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                             float ga = __uint_as_float(ra[2 * e]), gb = __uint_as_float(ra[2 * e + 1]);
                             float ua = __uint_as_float(rb[2 * e]), ub = __uint_as_float(rb[2 * e + 1]);
                             if (p.per_column) {
-                                const int pg = scale_single_pos(nt * TN + pp * 64 + 2 * e), pu = scale_single_pos(nt * TN + pp * 64 + 32 + 2 * e);
-                                ga *= __half2float(p.S[pg]);
-                                gb *= __half2float(p.S[pg + 1]);
-                                ua *= __half2float(p.S[pu]);
-                                ub *= __half2float(p.S[pu + 1]);
+                                const float2 sg = scale_pair(p.S, nt * TN + pp * 64 + 2 * e), su = scale_pair(p.S, nt * TN + pp * 64 + 32 + 2 * e);
+                                ga *= sg.x;
+                                gb *= sg.y;
+                                ua *= su.x;
+                                ub *= su.y;
                             }
                             o[e2] = pack_bf16x2(swiglu_scaled(ga, ua), swiglu_scaled(gb, ub));
                         }
@@ -310,11 +310,12 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                         for (int e = 0; e < 4; ++e) {
                             float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]);
                             float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]);
-                            unscale(x0, x1);
                             if (p.per_column) {
-                                const int pos = scale_single_pos(col + 8 * v + 2 * e);
-                                x0 *= __half2float(p.S[pos]);
-                                x1 *= __half2float(p.S[pos + 1]);
+                                const float2 s = scale_pair(p.S, col + 8 * v + 2 * e);
+                                x0 *= s.x * kWeightUnscale;
+                                x1 *= s.y * kWeightUnscale;
+                            } else {
+                                unscale(x0, x1);
                             }
                             o[e] = pack_bf16x2(x0, x1);
                         }

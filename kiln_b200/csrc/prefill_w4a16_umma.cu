@@ -272,11 +272,12 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             for (int e = 0; e < 4; ++e) {
                                 float x0 = __uint_as_float(ra[8 * v + 2 * e]) + __uint_as_float(rb[8 * v + 2 * e]);
                                 float x1 = __uint_as_float(ra[8 * v + 2 * e + 1]) + __uint_as_float(rb[8 * v + 2 * e + 1]);
-                                unscale(x0, x1);
                                 if (p.per_column) {
-                                    const int pos = scale_single_pos(col + 8 * v + 2 * e);
-                                    x0 *= __half2float(p.S[pos]);
-                                    x1 *= __half2float(p.S[pos + 1]);
+                                    const float2 s = scale_pair(p.S, col + 8 * v + 2 * e);
+                                    x0 *= s.x * kWeightUnscale;
+                                    x1 *= s.y * kWeightUnscale;
+                                } else {
+                                    unscale(x0, x1);
                                 }
                                 o[e] = pack_bf16x2(x0, x1);
                             }
@@ -345,11 +346,12 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             for (int e = 0; e < 4; ++e) {
                                 float x0 = __uint_as_float(half ? rb[8 * v + 2 * e] : ra[8 * v + 2 * e]);
                                 float x1 = __uint_as_float(half ? rb[8 * v + 2 * e + 1] : ra[8 * v + 2 * e + 1]);
-                                unscale(x0, x1);
                                 if (p.per_column) {
-                                    const int pos = scale_single_pos(col + 8 * v + 2 * e);
-                                    x0 *= __half2float(p.S[pos]);
-                                    x1 *= __half2float(p.S[pos + 1]);
+                                    const float2 s = scale_pair(p.S, col + 8 * v + 2 * e);
+                                    x0 *= s.x * kWeightUnscale;
+                                    x1 *= s.y * kWeightUnscale;
+                                } else {
+                                    unscale(x0, x1);
                                 }
                                 o[e] = pack_bf16x2(x0, x1);
                             }
@@ -566,11 +568,8 @@ w4a16_prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 __device__ __forceinline__ uint2 finish4(float4 v, const __half *S, int col, int per_column) {
     v.x *= kWeightUnscale, v.y *= kWeightUnscale, v.z *= kWeightUnscale, v.w *= kWeightUnscale;
     if (per_column) {
-        const int p0 = scale_single_pos(col), p1 = scale_single_pos(col + 2);
-        v.x *= __half2float(S[p0]);
-        v.y *= __half2float(S[p0 + 1]);
-        v.z *= __half2float(S[p1]);
-        v.w *= __half2float(S[p1 + 1]);
+        const float2 s0 = scale_pair(S, col), s1 = scale_pair(S, col + 2);
+        v.x *= s0.x, v.y *= s0.y, v.z *= s1.x, v.w *= s1.y;
     }
     __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
     return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));

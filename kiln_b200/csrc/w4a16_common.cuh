@@ -157,6 +157,11 @@ __device__ __host__ __forceinline__ int scale_single_pos(int col) {
     return (col & ~31) + 8 * ((c32 & 7) >> 1) + 2 * (c32 >> 3) + (c32 & 1);
 }
 
+// per-column scales of an even column and the next one: neighbours in that order, one load of four bytes (S is 16-byte aligned)
+__device__ __forceinline__ float2 scale_pair(const __half *S, int col) {
+    return __half22float2(*reinterpret_cast<const __half2 *>(S + scale_single_pos(col)));
+}
+
 // ---- host side --------------------------------------------------------------------------
 struct GemmArgs {
     const void *A;   // bf16 [m,k]
