@@ -1,6 +1,35 @@
 """How the tcgen05 kernels turn packed nibbles into bf16 weights, restated with numpy (no GPU): a nibble, read as a bf16 where it sits, times
 s * 2^133 or s * 2^129, less 8 s, in one fused multiply-add, everything at 2^-22 of its value (kiln_b200/csrc/w4a16_common.cuh)."""
+import re
+from pathlib import Path
+
 import numpy as np
+
+_SRC = (Path(__file__).parent.parent / "kiln_b200" / "csrc" / "w4a16_common.cuh").read_text()
+
+
+def _constant(name):
+    """A number as the source has it: 0x77007700u, 4194304.f, 1.f / 4194304.f."""
+    text = re.search(r"\b" + name + r" = ([^,;]+)[,;]", _SRC).group(1)
+    value = 1.0
+    for i, part in enumerate(text.split("/")):
+        number = float(int(part.strip().rstrip("u"), 16)) if "0x" in part else float(part.strip().rstrip("f"))
+        value = number if i == 0 else value / number
+    return value
+
+
+def _bf16_pair(name):
+    """The value of a bf16x2 constant, whose halves must be alike."""
+    bits = int(_constant(name))
+    assert bits >> 16 == bits & 0xFFFF
+    return float(np.array([bits & 0xFFFF0000], dtype=np.uint32).view(np.float32)[0])
+
+
+def test_the_constants_of_the_source():
+    assert int(_constant("kNibMask")) == 0x000F000F and int(_constant("kHiNibMask")) == 0x00F000F0
+    factor = _constant("kWeightFactor")
+    assert factor == 2.0 ** -22 and _constant("kWeightUnscale") == 2.0 ** 22
+    assert _bf16_pair("lo") * 2.0 ** -133 == factor and _bf16_pair("hi") * 2.0 ** -129 == factor and _bf16_pair("off") == -8.0 * factor
 
 
 def _bf16_bits(x):
@@ -21,7 +50,7 @@ def test_a_nibble_where_it_sits_is_a_linear_scale_of_bf16():
 def test_fused_multiply_add_rounds_as_subtract_and_multiply_do_for_every_fp16_scale():
     h = np.arange(0, 0x7C00, dtype=np.uint16).view(np.float16)    # zero, subnormals, normals; signs are symmetric
     s = _bf16_bits(h.astype(np.float64))
-    lo, hi, off = s * 2.0 ** 111, s * 2.0 ** 107, -8.0 * s * 2.0 ** -22
+    lo, hi, off = s * _bf16_pair("lo"), s * _bf16_pair("hi"), s * _bf16_pair("off")
     largest = (2.0 - 2.0 ** -7) * 2.0 ** 127
     assert lo.max() <= largest and hi.max() <= largest
     smallest = 2.0 ** -126
