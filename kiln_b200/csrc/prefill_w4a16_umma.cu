@@ -715,7 +715,8 @@ int g_test_drop_a_load = -1;
 int g_smallm_enabled = 1;
 
 // K splits of the small-batch kernel.  Its time in microseconds, fitted to 570 timed launches (CUDA graph over rotating weights;
-// K = 1024..9216 x N = 512..18432 x 9..128 rows x every split; the splits it picks are within 2% of the best).  While its clusters
+// K = 1024..9216 x N = 512..18432 x 9..128 rows x every split; the splits it picked were within 2% of the best.  Dequantisation and
+// exchange have become cheaper since, which it does not know).  While its clusters
 // take at most half the GPU, consecutive launches run side by side and only the chain from the grid-dependency wait to the exit
 // counts; above that a launch starts on the SMs the one before leaves.  A further wave of CTAs repeats that start; how many clusters
 // fit decides when there is one (4096 x 6144 has 48 tiles, and 3 splits need 48 clusters of 3 where 45 fit: 12.2 us, 2 splits 7.9).

@@ -33,7 +33,7 @@
 // Every wait is bounded (w4a16_async.cuh).  Per-column scales (group size -1): the weights are dequantised unscaled and the
 // scale multiplies the finished sums.
 //
-// What bounds it: about 0.3 us per 128 K and CTA up to 64 rows.  The dequant needs some 200 issue slots of every
+// What bounds it: about 0.25 us per 128 K and CTA up to 64 rows.  The dequant needs some 200 issue slots of every
 // sub-partition (nine instructions per packed word), an MMA 32 cycles at 64 rows and 9 at 16, a barrier 160 cycles to answer beside
 // them, and a launch has 2.5 to 3.4 us that no stage hides (the first words' latency after a CTA of the previous kernel has left the SM, the exchange, the
 // exit).  CUDA graph over rotating weights, before (register-streamed words, quad transposes, split-K through global slabs and
